@@ -10,9 +10,10 @@
 // instance whose box is the instance's world box (vertices lo, hi and (lo.x, hi.y, lo.z)); its leaf
 // children are then rewritten to name the instance, as the reference does. Instance records (128 B) and
 // a table of the meshes' node and triangle arrays sit in HBM; a 1024-instance TLAS is ~45 KB and stays
-// in L1/L2. The traversal is one thread per ray: the TLAS with the reference's 128-byte nodes and a
-// 32-entry stack, and per instance the quantised single-ray BLAS traversal of traverse.cu, so an
-// instance's object-space hits equal vt_trace_closest's on the same object-space ray.
+// in L1/L2. The traversal is one flat loop over both levels by persistent warps (k_tlas_trace): the
+// TLAS with the reference's 128-byte nodes, and per instance the quantised BLAS traversal in
+// traverse.cu's order, so an instance's object-space hits equal vt_trace_closest's on the same
+// object-space ray.
 //
 // The ray transform is written with explicitly rounded operations in one fixed order (the oracle
 // repeats it): o'_r = ((l_r.x o.x + l_r.y o.y) + l_r.z o.z) + l_r.w with the products and sums fused as
@@ -30,7 +31,6 @@
 namespace {
 using namespace vtd;
 
-constexpr int kTlasStack = 32;  // mesh_closest's TLAS stack (main.swift:1887)
 constexpr int kTlasBlock = 128;
 
 struct TlasInst {  // vt_instance_record on the device
@@ -58,85 +58,158 @@ __device__ __forceinline__ float xform_dir(float4 l, float x, float y, float z) 
   return __fmaf_rn(l.z, z, __fmaf_rn(l.y, y, __fmul_rn(l.x, x)));
 }
 
-// mesh_closest (kAny = false) / mesh_occluded (kAny = true), one thread per ray.
+// Stack entries of one ray's two levels, one shared-memory column per thread: a BLAS node is its index
+// (< 2^29), a BLAS leaf child ~(node << 2 | slot) (negative), a TLAS node kTlasNode | index and an
+// instance kTlasInstance | index (indices below 2^29 and 2^24).
+constexpr int kTlasNode = 0x40000000, kTlasInstance = 0x60000000, kTlasIndex = 0x1fffffff;
+constexpr int kTlasRefill = 8;  // idle lanes that make a warp take new rays (traverse.cu's k_closest)
+__device__ __forceinline__ int *tlas_slot(int *sstack, int d) { return sstack + d * kTlasBlock + threadIdx.x; }
+
+// mesh_closest (kAny = false) / mesh_occluded (kAny = true): persistent warps over the two levels.
+//
+// Bound: issue and divergence (the TLAS, the records and the meshes sit in L1/L2; a ray moves 52 bytes
+// of HBM). A thread per ray with nested loops and local-memory stacks left most lanes idle while one
+// lane was inside an instance: one flat loop handles one stack entry per lane and iteration instead,
+// the warp running the kind most of its lanes need (BLAS node, BLAS leaf, or world level: a TLAS node
+// or entering an instance), and refills idle lanes. A TLAS visit pushes its inner children below its
+// instances, each far to near, so a ray meets instances and nodes in mesh_closest's order; what an
+// entry pushed before a closer hit holds is culled by the box tests when it is popped.
+// Block b takes the rays of tiles b, b + grid, ... of 32 (through a block counter in shared memory),
+// so a launch needs no device-wide counter and expensive image regions spread over the blocks.
+// Measured on one B200: 1M random rays over 1,024 instances of 20,480-triangle meshes (closest hit)
+// 2.66 -> 1.28 ms.
 template <bool kAny>
-__global__ void __launch_bounds__(kTlasBlock) k_tlas_trace(const float4 *__restrict__ nodes, const TlasInst *__restrict__ inst,
-                                                          const TlasMesh *__restrict__ meshes, float grow, float reach,
-                                                          const float4 *__restrict__ rays, uint32_t n, int4 *__restrict__ hits,
-                                                          uint32_t *__restrict__ instOut, uint8_t *__restrict__ occ) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float4 r0 = __ldcs(rays + 2 * (size_t)i), r1 = __ldcs(rays + 2 * (size_t)i + 1);
-  const float e = __fmul_rn(grow, __fadd_rn(max_abs_origin(r0.x, r0.y, r0.z), reach));
-  const SlabRay sr = make_slab_e(r0.x, r0.y, r0.z, r1.x, r1.y, r1.z, e);
-  const float tMin = r0.w;
-  float closest = r1.w, hb1 = 0.0f, hb2 = 0.0f;
+__global__ void __launch_bounds__(kTlasBlock, 6) k_tlas_trace(const float4 *__restrict__ nodes, const TlasInst *__restrict__ inst,
+                                                             const TlasMesh *__restrict__ meshes, float grow, float reach,
+                                                             const float4 *__restrict__ rays, uint32_t n, int4 *__restrict__ hits,
+                                                             uint32_t *__restrict__ instOut, uint8_t *__restrict__ occ,
+                                                             int stackSize, uint32_t *status) {
+  extern __shared__ int sstack[];
+  __shared__ uint32_t taken;  // rays of this block's tiles handed out
+  if (threadIdx.x == 0) taken = 0;
+  __syncthreads();
+  const unsigned kAll = 0xffffffffu, lane = threadIdx.x & 31u;
+  // This block's tiles and rays (the last tile may be short).
+  const uint32_t tiles = (n + 31u) / 32u;
+  const uint32_t mine = blockIdx.x < tiles ? (tiles - blockIdx.x + gridDim.x - 1u) / gridDim.x * 32u : 0u;
+  int top = 0;  // 0: the lane holds no ray
+  uint32_t rid = 0, hitInst = 0xffffffffu, curInst = 0;
+  WRay wr{};
+  QRay qr{};
+  const float4 *qnodes = nullptr, *tris = nullptr;
+  float tMin = 0.0f, closest = 0.0f, hb1 = 0.0f, hb2 = 0.0f;
   int prim = -1;
-  uint32_t hitInst = 0xffffffffu;
-  uint32_t nv = 0, nt = 0;
-  int stack[kTlasStack];
-  int top = 0;
-  stack[top++] = 0;
-  while (top > 0) {
-    Node4 nd;
-    load_node(nodes, stack[--top], nd);
-    float nearT[4];
-    const int mask = node_hits(nd, sr, tMin, closest, nearT);
-    if (kAny) {
-      // mesh_occluded: children in slot order, inner nodes pushed as met, instances traced as met.
-      for (int k = 0; k < 4; ++k) {
-        if (!(mask >> k & 1)) continue;
-        const int c = i4(nd.child, k);
-        if (c > 0) {
-          if (top < kTlasStack) stack[top++] = c;
-          continue;
-        }
-        const TlasInst I = inst[-c - 1];
-        const TlasMesh M = meshes[I.range.x];
-        const float4 o = make_float4(xform_point(I.local[0], r0.x, r0.y, r0.z), xform_point(I.local[1], r0.x, r0.y, r0.z),
-                                     xform_point(I.local[2], r0.x, r0.y, r0.z), tMin);
-        const float4 d = make_float4(xform_dir(I.local[0], r1.x, r1.y, r1.z), xform_dir(I.local[1], r1.x, r1.y, r1.z),
-                                     xform_dir(I.local[2], r1.x, r1.y, r1.z), r1.w);
-        if (trace_any<false>(M.qnodes, M.tris, I.bound.z, o, d, nv, nt)) {
-          occ[i] = 1;
-          return;
-        }
-      }
-      continue;
-    }
-    // mesh_closest: instances near to far, then inner children pushed far to near.
-    const Sorted4 s = sort_children(nd, mask, nearT);
-#pragma unroll 1
-    for (int j = 0; j < 4; ++j) {
-      if (j >= s.m || s.child[j] > 0 || beyond(s.key[j], closest)) continue;
-      const uint32_t k = (uint32_t)(-s.child[j] - 1);
-      const TlasInst I = inst[k];
-      const TlasMesh M = meshes[I.range.x];
-      const float4 o = make_float4(xform_point(I.local[0], r0.x, r0.y, r0.z), xform_point(I.local[1], r0.x, r0.y, r0.z),
-                                   xform_point(I.local[2], r0.x, r0.y, r0.z), tMin);
-      const float4 d = make_float4(xform_dir(I.local[0], r1.x, r1.y, r1.z), xform_dir(I.local[1], r1.x, r1.y, r1.z),
-                                   xform_dir(I.local[2], r1.x, r1.y, r1.z), closest);
-      float t, b1, b2;
-      int p = -1;
-      if (trace_closest<false>(M.qnodes, M.tris, I.bound.z, o, d, t, b1, b2, p, nv, nt)) {
-        closest = t;
-        hb1 = b1;
-        hb2 = b2;
-        prim = p;
-        hitInst = k;
+  bool exhausted = false;  // warp-uniform
+  while (true) {
+    const unsigned idle = __ballot_sync(kAll, top == 0);
+    if (!exhausted && __popc(idle) >= kTlasRefill) {
+      uint32_t base = 0;
+      if (lane == 0) base = atomicAdd(&taken, (uint32_t)__popc(idle));
+      base = __shfl_sync(kAll, base, 0);
+      if (base + (uint32_t)__popc(idle) >= mine) exhausted = true;
+      const uint32_t q = base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
+      const uint32_t r = ((q >> 5) * gridDim.x + blockIdx.x) * 32u + (q & 31u);
+      if ((idle >> lane & 1u) && q < mine && r < n) {
+        rid = r;
+        tMin = __ldg(&rays[2 * (size_t)r].w);
+        closest = __ldg(&rays[2 * (size_t)r + 1].w);
+        prim = -1;
+        *tlas_slot(sstack, 0) = kTlasNode;
+        top = 1;
       }
     }
+    if (exhausted && !__any_sync(kAll, top > 0)) break;
+    const int entry = top > 0 ? *tlas_slot(sstack, top - 1) : 0;
+    const bool leaf = top > 0 && entry < 0, world = top > 0 && entry >= kTlasNode;
+    const int nLeaf = __popc(__ballot_sync(kAll, leaf)), nWorld = __popc(__ballot_sync(kAll, world)),
+              nInner = __popc(__ballot_sync(kAll, top > 0 && !leaf && !world));
+    const bool leafPhase = nLeaf >= nInner && nLeaf >= nWorld, worldPhase = !leafPhase && nWorld > nInner;
+    if (top == 0 || leaf != leafPhase || world != worldPhase) continue;
+    --top;
+    bool hit = false;
+    if (leaf) {
+      int first, cnt;
+      leaf_range(qnodes, entry, first, cnt);
+      for (int q = 0; q < cnt; ++q) {
+        const float4 *tp = tris + 3 * (size_t)(first + q);
+        const float4 a = __ldg(tp), b = __ldg(tp + 1), cc = __ldg(tp + 2);
+        float t, b1, b2;
+        if (!intersect_tri(wr, a, b, cc, tMin, closest, t, b1, b2)) continue;
+        if (kAny) {
+          hit = true;
+          break;
+        }
+        closest = t; hb1 = b1; hb2 = b2; prim = __float_as_int(a.w); hitInst = curInst;
+      }
+    } else if (!world) {
+      QNode nd;
+      load_qnode(qnodes, entry, nd);
+      float nearT[4];
+      const int mask = qnode_hits(nd, qr, tMin, closest, nearT);
+      if (top + 4 > stackSize) {
+        atomicOr(status, (uint32_t)VT_DEV_STACK);
+        top = stackSize - 4;
+      }
+      if (kAny) {  // slot order
 #pragma unroll
-    for (int j = 3; j >= 0; --j)
-      if (j < s.m && s.child[j] > 0 && !beyond(s.key[j], closest) && top < kTlasStack) stack[top++] = s.child[j];
+        for (int k = 3; k >= 0; --k) {
+          if (!(mask >> k & 1)) continue;
+          const int c = i4(nd.child, k);
+          *tlas_slot(sstack, top++) = c > 0 ? c : leaf_entry_of(entry, k);
+        }
+      } else {
+        const Sorted4 o = sort_qchildren(nd, mask, nearT);
+#pragma unroll
+        for (int j = 3; j >= 0; --j) {
+          if (j >= o.m || beyond(o.key[j], closest)) continue;
+          *tlas_slot(sstack, top++) = o.child[j] > 0 ? o.child[j] : leaf_entry_of(entry, (int)(o.key[j] & 3u));
+        }
+      }
+    } else {
+      const float4 r0 = __ldg(rays + 2 * (size_t)rid), r1 = __ldg(rays + 2 * (size_t)rid + 1);
+      if (entry < kTlasInstance) {
+        const float e = __fmul_rn(grow, __fadd_rn(max_abs_origin(r0.x, r0.y, r0.z), reach));
+        const SlabRay sr = make_slab_e(r0.x, r0.y, r0.z, r1.x, r1.y, r1.z, e);
+        Node4 nd;
+        load_node(nodes, entry & kTlasIndex, nd);
+        float nearT[4];
+        const int mask = node_hits(nd, sr, tMin, closest, nearT);
+        const Sorted4 s = sort_children(nd, mask, nearT);
+#pragma unroll
+        for (int pass = 0; pass < 2; ++pass) {  // inner children, then the instances above them
+#pragma unroll
+          for (int j = 3; j >= 0; --j) {
+            if (j >= s.m || (s.child[j] > 0) != (pass == 0) || beyond(s.key[j], closest)) continue;
+            const int e2 = s.child[j] > 0 ? (kTlasNode | s.child[j]) : (kTlasInstance | (-s.child[j] - 1));
+            if (top < stackSize) *tlas_slot(sstack, top++) = e2;
+            else atomicOr(status, (uint32_t)VT_DEV_STACK);
+          }
+        }
+      } else {
+        curInst = (uint32_t)(entry & kTlasIndex);
+        const TlasInst *I = inst + curInst;
+        const float4 l0 = __ldg(&I->local[0]), l1 = __ldg(&I->local[1]), l2 = __ldg(&I->local[2]);
+        const TlasMesh *M = meshes + __ldg(&I->range.x);
+        qnodes = M->qnodes;
+        tris = M->tris;
+        const float ox = xform_point(l0, r0.x, r0.y, r0.z), oy = xform_point(l1, r0.x, r0.y, r0.z),
+                    oz = xform_point(l2, r0.x, r0.y, r0.z);
+        const float dx = xform_dir(l0, r1.x, r1.y, r1.z), dy = xform_dir(l1, r1.x, r1.y, r1.z),
+                    dz = xform_dir(l2, r1.x, r1.y, r1.z);
+        wr = make_wray(ox, oy, oz, dx, dy, dz);
+        qr = make_qray(ox, oy, oz, dx, dy, dz, __ldg(&I->bound.z));
+        *tlas_slot(sstack, top++) = 0;  // the BLAS root (the popped entry's place)
+      }
+    }
+    if (kAny) {
+      if (hit) top = 0;
+      if (top == 0) occ[rid] = hit ? 1 : 0;
+    } else if (top == 0) {
+      hits[rid] = prim >= 0 ? make_int4(__float_as_int(closest), __float_as_int(hb1), __float_as_int(hb2), prim)
+                            : make_int4(0, 0, 0, -1);
+      if (instOut) instOut[rid] = prim >= 0 ? hitInst : 0xffffffffu;
+    }
   }
-  if (kAny) {
-    occ[i] = 0;
-    return;
-  }
-  hits[i] = prim >= 0 ? make_int4(__float_as_int(closest), __float_as_int(hb1), __float_as_int(hb2), prim)
-                      : make_int4(0, 0, 0, -1);
-  if (instOut) instOut[i] = prim >= 0 ? hitInst : 0xffffffffu;
 }
 
 // The TLAS leaves name instances: child -(first + 1) at BVH position `first` becomes -(order[first] + 1)
@@ -207,6 +280,7 @@ struct vt_tlas {
   TlasInst *d_inst = nullptr;
   TlasMesh *d_meshes = nullptr;
   uint64_t rendered = 0;
+  uint32_t blas_depth = 0;  // the deepest mesh's 4-wide depth (traversal stacks)
   float grow = 0.0f, reach = 0.0f;
   float lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
   float build_ms = 0.0f;
@@ -349,6 +423,7 @@ vt_status vt_tlas_build(vt_ctx *ctx, const vt_mesh *const *meshes, uint32_t nmes
   std::vector<TlasMesh> hm(nmeshes);
   for (uint32_t k = 0; k < nmeshes; ++k) {
     const vt_mesh *mk = meshes[k];
+    t->blas_depth = std::max(t->blas_depth, mk->depth);
     hm[k] = TlasMesh{reinterpret_cast<const float4 *>(mk->d_qnodes), mk->d_tris, mk->d_nrm, mk->d_order, mk->nfaces, mk->root_max, {0, 0}};
   }
   cudaError_t e = cudaMalloc(&t->d_inst, ninstances * sizeof(TlasInst));
@@ -417,17 +492,26 @@ static vt_status tlas_trace(vt_ctx *ctx, const vt_tlas *tlas, const vt_ray *rays
     return vt_fail(ctx, VT_ERR_INVALID, "rays and hits must be 16-byte aligned");
   if (n == 0) return VT_OK;
   VT_CUDA(ctx, cudaSetDevice(ctx->device));
-  const uint32_t grid = (n + kTlasBlock - 1) / kTlasBlock;
+  // Stack entries: the TLAS's root and at most 3 net pushes per level, then the same for a BLAS.
+  const int S = 3 * (int)tlas->boxes->depth + 1 + 3 * (int)tlas->blas_depth + 1;
+  const size_t smem = (size_t)S * kTlasBlock * sizeof(int);
   const float4 *nodes = reinterpret_cast<const float4 *>(tlas->boxes->d_nodes);
-  if (closest)
-    k_tlas_trace<false><<<grid, kTlasBlock, 0, s>>>(nodes, tlas->d_inst, tlas->d_meshes, tlas->grow, tlas->reach,
-                                                   reinterpret_cast<const float4 *>(rays), n, static_cast<int4 *>(out), instOut,
-                                                   nullptr);
-  else
-    k_tlas_trace<true><<<grid, kTlasBlock, 0, s>>>(nodes, tlas->d_inst, tlas->d_meshes, tlas->grow, tlas->reach,
-                                                  reinterpret_cast<const float4 *>(rays), n, nullptr, nullptr,
-                                                  static_cast<uint8_t *>(out));
-  VT_CUDA(ctx, cudaGetLastError());
+  auto launch = [&](auto kernel) -> cudaError_t {
+    if (smem > 48 * 1024) {
+      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+    }
+    int resident = 0;
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, kTlasBlock, smem);
+    if (e != cudaSuccess) return e;
+    const uint32_t grid = std::min<uint32_t>((n + kTlasBlock - 1) / kTlasBlock, (uint32_t)(std::max(1, resident) * ctx->sm_count));
+    kernel<<<grid, kTlasBlock, smem, s>>>(nodes, tlas->d_inst, tlas->d_meshes, tlas->grow, tlas->reach,
+                                         reinterpret_cast<const float4 *>(rays), n, closest ? static_cast<int4 *>(out) : nullptr,
+                                         instOut, closest ? nullptr : static_cast<uint8_t *>(out), S, ctx->d_status + 1);
+    return cudaGetLastError();
+  };
+  if (closest) VT_CUDA(ctx, launch(k_tlas_trace<false>));
+  else VT_CUDA(ctx, launch(k_tlas_trace<true>));
   return VT_OK;
 }
 

@@ -83,6 +83,25 @@ def test_tlas_traversal_matches_oracle(ctx, oracle):
     assert np.array_equal(occ, oocc)
 
 
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 129, 4097])
+@pytest.mark.parametrize("grid", [1, 5])
+def test_tlas_ray_counts_match_oracle(ctx, oracle, n, grid):
+    """Ray counts around the kernel's tiles of 32 and blocks of 128, one instance and many, both signs of
+    tmin: hits, instances and occlusion equal the oracle's bit for bit."""
+    *_, tlas, rec, grow, reach, bf, bv, obvh = _build(ctx, oracle, grid=grid, assets=2, sub=2, seed=5 + grid)
+    p = bv["p"]
+    rays = FI.probe_rays(p.min(0), p.max(0), n, seed=n)[:n]
+    rays[::3, 3] = -0.25
+    rays[1::3, 3] = -0.0
+    hits, inst = tlas.closest(rays)
+    oh, oi = oracle.tlas_trace(tlas.nodes(), tlas.records(), obvh, grow, reach, rays, precision=32)
+    assert np.array_equal(hits.view(np.uint32), oh.view(np.uint32)) and np.array_equal(inst, oi)
+    short = rays.copy()
+    short[:, 7] = np.where(hits["prim"] >= 0, hits["t"] * 1.001, 5.0).astype(np.float32)
+    oocc = oracle.tlas_trace(tlas.nodes(), tlas.records(), obvh, grow, reach, short, closest=False, precision=32)
+    assert np.array_equal(tlas.occluded(short), oocc)
+
+
 def test_tlas_flatten_matches_two_level(ctx, oracle):
     meshes, T, mesh_of, slots, _, gm, tlas, rec, grow, reach, bf, bv, obvh = _build(ctx, oracle)
     flat = tlas.flatten()
