@@ -687,6 +687,9 @@ __global__ void k_collapse_emit(TreeView t, uint32_t L, int leafSize, const int4
         if (c < 0) {
           if (prim >= (uint32_t)t.n) { atomicOr(status, (uint32_t)VT_DEV_TREELET); return; }
           uint32_t f = sorted[-c - 1];
+          // The traversal's leaf loop ends at the triangle marked as its leaf's last (the meshes that
+          // are traversed carry normals here).
+          const float last = nrm && top == 0 ? 1.0f : 0.0f;
           order[prim] = (int32_t)f;
           vt_face fc = faces[f];
           if (fc.a >= nverts || fc.b >= nverts || fc.c >= nverts) {
@@ -696,7 +699,7 @@ __global__ void k_collapse_emit(TreeView t, uint32_t L, int leafSize, const int4
             const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             tris[3 * prim] = make_float4(0.0f, 0.0f, 0.0f, __int_as_float((int)f));
             tris[3 * prim + 1] = z;
-            tris[3 * prim + 2] = z;
+            tris[3 * prim + 2] = make_float4(0.0f, 0.0f, 0.0f, last);
             if (nrm) nrm[3 * prim] = nrm[3 * prim + 1] = nrm[3 * prim + 2] = z;
             ++prim;
             continue;
@@ -704,7 +707,7 @@ __global__ void k_collapse_emit(TreeView t, uint32_t L, int leafSize, const int4
           const vt_vertex &va = verts[fc.a], &vb = verts[fc.b], &vc = verts[fc.c];
           tris[3 * prim] = make_float4(va.px, va.py, va.pz, __int_as_float((int)f));
           tris[3 * prim + 1] = make_float4(vb.px, vb.py, vb.pz, __uint_as_float(fc.tag));
-          tris[3 * prim + 2] = make_float4(vc.px, vc.py, vc.pz, 0.0f);
+          tris[3 * prim + 2] = make_float4(vc.px, vc.py, vc.pz, last);
           if (nrm) {  // vertex normals for smooth shading (mesh_hit_attributes)
             nrm[3 * prim] = make_float4(va.nx, va.ny, va.nz, 0.0f);
             nrm[3 * prim + 1] = make_float4(vb.nx, vb.ny, vb.nz, 0.0f);

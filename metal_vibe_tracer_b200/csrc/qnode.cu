@@ -6,10 +6,12 @@
 // children's union lower corner), a power-of-two step 2^e per axis, and per child and axis the
 // bytes qlo = floor((lo - p) / 2^e) and qhi = ceil((hi - p) / 2^e), so that p + qlo 2^e <= lo and
 // p + qhi 2^e >= hi exactly: each decoded box contains the child's box. Child links and leaf counts
-// are copied. A node is two 32-byte loads instead of four.
+// become traversal stack entries. A node is two 32-byte loads instead of four.
 //
-// Layout (16 words): p.x p.y p.z | biased exponents (e + 127) in bytes 0-2 | qlo.x qlo.y qlo.z |
-// qhi.x qhi.y qhi.z (byte k = child k) | child[4] | leaf counts (4 bits per child) | 0.
+// Layout (16 words): p.x p.y p.z | steps 2^(e + 15) of x and y as bfloat16 halves (so one shift or mask
+// makes a float of each) | qlo.x qlo.y qlo.z | qhi.x qhi.y qhi.z (byte k = child k) | child[4]: the
+// inner node's index, ~(first triangle) of a leaf, 0x80000000 for an empty slot | step of z as the
+// high bfloat16 half | 0. An empty slot's box is inverted (lo 255, hi 0).
 #include <cfloat>
 #include <cmath>
 
@@ -53,9 +55,15 @@ __global__ void k_quantize(const vt_wide_node *__restrict__ in, uint32_t n, vt_q
       const float p = lo[a];
       const int e = quant_exponent((double)hi[a] - (double)p);
       q.w[a] = __float_as_uint(p);
-      q.w[3] |= (uint32_t)(e + 127) << (8 * a);
+      const uint32_t step = (uint32_t)(e + 15 + 127) << 7;  // 2^(e + 15) as bfloat16 bits
+      if (a == 0) q.w[3] |= step;
+      else if (a == 1) q.w[3] |= step << 16;
+      else q.w[14] = step << 16;
       for (int k = 0; k < 4; ++k) {
-        if (nd.child[k] == 0) continue;
+        if (nd.child[k] == 0) {
+          q.w[4 + a] |= 255u << (8 * k);
+          continue;
+        }
         const double l = floor(ldexp((double)clo[a][k] - (double)p, -e));
         const double h = ceil(ldexp((double)chi[a][k] - (double)p, -e));
         const uint32_t ql = (uint32_t)fmin(fmax(l, 0.0), 255.0), qh = (uint32_t)fmin(fmax(h, 0.0), 255.0);
@@ -65,8 +73,7 @@ __global__ void k_quantize(const vt_wide_node *__restrict__ in, uint32_t n, vt_q
     }
   }
   for (int k = 0; k < 4; ++k) {
-    q.w[10 + k] = (uint32_t)nd.child[k];
-    q.w[14] |= ((uint32_t)nd.count[k] & 15u) << (4 * k);
+    q.w[10 + k] = nd.child[k] ? (uint32_t)nd.child[k] : 0x80000000u;  // a leaf is -(first + 1) = ~first already
   }
   out[i] = q;
 }

@@ -59,7 +59,7 @@ __device__ __forceinline__ float xform_dir(float4 l, float x, float y, float z) 
 }
 
 // Stack entries of one ray's two levels, one shared-memory column per thread: a BLAS node is its index
-// (< 2^29), a BLAS leaf child ~(node << 2 | slot) (negative), a TLAS node kTlasNode | index and an
+// (< 2^29), a BLAS leaf ~(its first triangle) (negative), a TLAS node kTlasNode | index and an
 // instance kTlasInstance | index (indices below 2^29 and 2^24).
 constexpr int kTlasNode = 0x40000000, kTlasInstance = 0x60000000, kTlasIndex = 0x1fffffff;
 constexpr int kTlasRefill = 8;  // idle lanes that make a warp take new rays (traverse.cu's k_closest)
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(kTlasBlock, 6) k_tlas_trace(const float4 *__re
       const uint32_t r = ((q >> 5) * gridDim.x + blockIdx.x) * 32u + (q & 31u);
       if ((idle >> lane & 1u) && q < mine && r < n) {
         rid = r;
-        tMin = __ldg(&rays[2 * (size_t)r].w);
+        tMin = __fadd_rn(__ldg(&rays[2 * (size_t)r].w), 0.0f);  // -0 to +0 (sort_qchildren)
         closest = __ldg(&rays[2 * (size_t)r + 1].w);
         prim = -1;
         *tlas_slot(sstack, 0) = kTlasNode;
@@ -128,42 +128,41 @@ __global__ void __launch_bounds__(kTlasBlock, 6) k_tlas_trace(const float4 *__re
     --top;
     bool hit = false;
     if (leaf) {
-      int first, cnt;
-      leaf_range(qnodes, entry, first, cnt);
-      for (int q = 0; q < cnt; ++q) {
-        const float4 *tp = tris + 3 * (size_t)(first + q);
-        const float4 a = __ldg(tp), b = __ldg(tp + 1), cc = __ldg(tp + 2);
-        float t, b1, b2;
-        if (!intersect_tri(wr, a, b, cc, tMin, closest, t, b1, b2)) continue;
-        if (kAny) {
-          hit = true;
-          break;
+      if (entry != kEmptyChild) {
+        const float4 *tp = tris + 3 * (size_t)(~entry);
+        for (int q = 0; q < kMaxLeafTris; ++q, tp += 3) {
+          const float4 a = __ldg(tp), b = __ldg(tp + 1), cc = __ldg(tp + 2);
+          float t, b1, b2;
+          if (intersect_tri(wr, a, b, cc, tMin, closest, t, b1, b2)) {
+            if (kAny) {
+              hit = true;
+              break;
+            }
+            closest = t; hb1 = b1; hb2 = b2; prim = __float_as_int(a.w); hitInst = curInst;
+          }
+          if (leaf_ends(cc)) break;
         }
-        closest = t; hb1 = b1; hb2 = b2; prim = __float_as_int(a.w); hitInst = curInst;
       }
     } else if (!world) {
       QNode nd;
       load_qnode(qnodes, entry, nd);
       float nearT[4];
-      const int mask = qnode_hits(nd, qr, tMin, closest, nearT);
+      bool meets[4];
+      qnode_test(nd, qr, tMin, closest, nearT, meets);
       if (top + 4 > stackSize) {
         atomicOr(status, (uint32_t)VT_DEV_STACK);
         top = stackSize - 4;
       }
       if (kAny) {  // slot order
 #pragma unroll
-        for (int k = 3; k >= 0; --k) {
-          if (!(mask >> k & 1)) continue;
-          const int c = i4(nd.child, k);
-          *tlas_slot(sstack, top++) = c > 0 ? c : leaf_entry_of(entry, k);
-        }
+        for (int k = 3; k >= 0; --k)
+          if (meets[k]) *tlas_slot(sstack, top++) = i4(nd.child, k);
       } else {
-        const Sorted4 o = sort_qchildren(nd, mask, nearT);
+        uint32_t key[4];
+        sort_qchildren(meets, nearT, tMin >= 0.0f, key);
 #pragma unroll
-        for (int j = 3; j >= 0; --j) {
-          if (j >= o.m || beyond(o.key[j], closest)) continue;
-          *tlas_slot(sstack, top++) = o.child[j] > 0 ? o.child[j] : leaf_entry_of(entry, (int)(o.key[j] & 3u));
-        }
+        for (int j = 3; j >= 0; --j)
+          if (key[j] != kMissKey) *tlas_slot(sstack, top++) = pick4(nd.child, key[j] & 3u);
       }
     } else {
       const float4 r0 = __ldg(rays + 2 * (size_t)rid), r1 = __ldg(rays + 2 * (size_t)rid + 1);

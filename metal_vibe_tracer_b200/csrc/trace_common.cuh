@@ -276,33 +276,26 @@ __device__ __forceinline__ QRay make_qray(float ox, float oy, float oz, float dx
 
 struct QNode {
   float px, py, pz;
-  uint32_t e;
+  uint32_t sxy, sz;  // steps 2^(e+15) as bfloat16 bits: x low and y high half; z high half
   uint32_t qlo[3], qhi[3];
-  int4 child;
-  uint32_t counts;
+  int4 child;        // stack entries: inner node index (> 0), leaf ~first triangle, empty kEmptyChild
 };
+
+// An empty child slot: its box is inverted (bytes 255 over 0), so the slab test misses it; where a
+// node's whole box is degenerate the conservative rounding may still report it, and the popped entry
+// is then skipped.
+constexpr int kEmptyChild = (int)0x80000000;
 
 __device__ __forceinline__ void load_qnode(const float4 *__restrict__ qnodes, int i, QNode &n) {
   const float4 *p = qnodes + 4 * (size_t)i;
   float4 a, b, c, d;
   ld256(p, a, b);
   ld256(p + 2, c, d);
-  n.px = a.x; n.py = a.y; n.pz = a.z; n.e = __float_as_uint(a.w);
+  n.px = a.x; n.py = a.y; n.pz = a.z; n.sxy = __float_as_uint(a.w);
   n.qlo[0] = __float_as_uint(b.x); n.qlo[1] = __float_as_uint(b.y); n.qlo[2] = __float_as_uint(b.z);
   n.qhi[0] = __float_as_uint(b.w); n.qhi[1] = __float_as_uint(c.x); n.qhi[2] = __float_as_uint(c.y);
   n.child = make_int4(__float_as_int(c.z), __float_as_int(c.w), __float_as_int(d.x), __float_as_int(d.y));
-  n.counts = __float_as_uint(d.z);
-}
-
-// A leaf child goes on a traversal stack as the entry ~(node << 2 | slot) (node indices are below
-// 2^29); popping it reads the slot's first triangle and count from the node, in L1 since the node's
-// visit.
-__device__ __forceinline__ int leaf_entry_of(int node, int slot) { return ~((node << 2) | slot); }
-__device__ __forceinline__ void leaf_range(const float4 *__restrict__ qnodes, int entry, int &first, int &cnt) {
-  const int code = ~entry, slot = code & 3;
-  const int *nd = reinterpret_cast<const int *>(qnodes + 4 * (size_t)(code >> 2));
-  first = -__ldg(nd + 10 + slot) - 1;
-  cnt = (__ldg(nd + 14) >> (4 * slot)) & 15;
+  n.sz = __float_as_uint(d.z);
 }
 
 // Byte k of w as the float 1 + byte 2^-15 (the byte in mantissa bits 8-15), exact.
@@ -317,10 +310,10 @@ struct QAxis {
 
 // A plane at p + q 2^e lies at (1 + q 2^-15) d + (p * inv - origin * inv - d) with d = 2^(e+15) inv;
 // the bias removal rounds to the safe side too, so the bound loosens by at most 2^-9 of a step.
-__device__ __forceinline__ QAxis q_axis(float p, uint32_t eb, uint32_t qlo, uint32_t qhi, float inv, float nO, float fO,
+__device__ __forceinline__ QAxis q_axis(float p, float step15, uint32_t qlo, uint32_t qhi, float inv, float nO, float fO,
                                         bool neg) {
   QAxis a;
-  a.d = __uint_as_float((eb + 15u) << 23) * inv;  // 2^(e+15) * inv, exact
+  a.d = step15 * inv;  // 2^(e+15) * inv, exact
   a.cn = __fadd_rd(__fmaf_rd(p, inv, -nO), -a.d);
   a.cf = __fadd_ru(__fmaf_ru(p, inv, -fO), -a.d);
   a.nw = neg ? qhi : qlo;
@@ -328,12 +321,11 @@ __device__ __forceinline__ QAxis q_axis(float p, uint32_t eb, uint32_t qlo, uint
   return a;
 }
 
-// Child hit mask and entry distances of a quantised node.
-__device__ __forceinline__ int qnode_hits(const QNode &n, const QRay &r, float tMin, float tMax, float nearT[4]) {
-  const QAxis x = q_axis(n.px, n.e & 0xffu, n.qlo[0], n.qhi[0], r.invx, r.nx, r.fx, (r.neg & 1u) != 0u);
-  const QAxis y = q_axis(n.py, (n.e >> 8) & 0xffu, n.qlo[1], n.qhi[1], r.invy, r.ny, r.fy, (r.neg & 2u) != 0u);
-  const QAxis z = q_axis(n.pz, (n.e >> 16) & 0xffu, n.qlo[2], n.qhi[2], r.invz, r.nz, r.fz, (r.neg & 4u) != 0u);
-  int mask = 0;
+// Entry distances of a quantised node's children, and whether the ray meets each.
+__device__ __forceinline__ void qnode_test(const QNode &n, const QRay &r, float tMin, float tMax, float nearT[4], bool hit[4]) {
+  const QAxis x = q_axis(n.px, __uint_as_float(n.sxy << 16), n.qlo[0], n.qhi[0], r.invx, r.nx, r.fx, (r.neg & 1u) != 0u);
+  const QAxis y = q_axis(n.py, __uint_as_float(n.sxy & 0xffff0000u), n.qlo[1], n.qhi[1], r.invy, r.ny, r.fy, (r.neg & 2u) != 0u);
+  const QAxis z = q_axis(n.pz, __uint_as_float(n.sz), n.qlo[2], n.qhi[2], r.invz, r.nz, r.fz, (r.neg & 4u) != 0u);
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const float nxk = __fmaf_rd(qbyte(x.nw, k), x.d, x.cn), fxk = __fmaf_ru(qbyte(x.fw, k), x.d, x.cf);
@@ -342,86 +334,80 @@ __device__ __forceinline__ int qnode_hits(const QNode &n, const QRay &r, float t
     const float nt = fmaxf(fmax3(nxk, nyk, nzk), tMin);
     const float ft = fminf(fmin3(fxk, fyk, fzk), tMax);
     nearT[k] = nt;
-    mask |= (nt <= ft && i4(n.child, k) != 0) ? (1 << k) : 0;
+    hit[k] = nt <= ft;
   }
-  return mask;
 }
 
-// Hit children of a quantised node near to far (the packed-key network of sort_children).
-__device__ __forceinline__ Sorted4 sort_qchildren(const QNode &nd, int mask, const float nearT[4]) {
-  uint32_t k[4];
+// Sort keys of a quantised node's children, ascending: a hit child's entry distance as an ordered
+// integer with its two low bits replaced by the slot (sort_children's order), a missed child
+// kMissKey. Entry distances are at least tMin, so for tMin >= +0 (`positive`, the ray's own: the
+// caller normalises -0) they are their own ordered integers.
+constexpr uint32_t kMissKey = 0xffffffffu;
+__device__ __forceinline__ void sort_qchildren(const bool hit[4], const float nearT[4], bool positive, uint32_t k[4]) {
+  uint32_t o[4];
 #pragma unroll
-  for (int c = 0; c < 4; ++c)
-    k[c] = (mask >> c & 1) ? ((ord32(__fadd_rn(nearT[c], 0.0f)) & ~3u) | (uint32_t)c) : 0xffffffffu;
+  for (int c = 0; c < 4; ++c) o[c] = __float_as_uint(nearT[c]);
+  if (!positive) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) o[c] = ord32(__fadd_rn(nearT[c], 0.0f));
+  }
+#pragma unroll
+  for (int c = 0; c < 4; ++c) k[c] = hit[c] ? ((o[c] & ~3u) | (uint32_t)c) : kMissKey;
   ucswap(k[0], k[1]);
   ucswap(k[2], k[3]);
   ucswap(k[0], k[2]);
   ucswap(k[1], k[3]);
   ucswap(k[1], k[2]);
-  Sorted4 o;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    o.key[j] = k[j];
-    o.child[j] = pick4(nd.child, k[j] & 3u);
-    o.count[j] = (int)((nd.counts >> (4u * (k[j] & 3u))) & 15u);
-  }
-  o.m = __popc(mask);
-  return o;
 }
+
+// A triangle of the traversal's array (three float4): the third's .w is nonzero on the last triangle
+// of its leaf. A leaf holds at most kMaxLeafTris (the loop's bound in a corrupted array).
+constexpr int kMaxLeafTris = 8;
+__device__ __forceinline__ bool leaf_ends(const float4 &c) { return __float_as_uint(c.w) != 0u; }
 
 // ---- single-ray traversals ------------------------------------------------------------------------
 // In the persistent kernels' order (leaf children pushed as stack entries, near entries popped first),
-// counting node visits and triangle tests when kCount. `r0` is (origin, tmin), `r1` (direction, tmax);
-// the closest hit reports the input face index (vertex a's .w).
-
-template <bool kCount>
-__device__ __forceinline__ bool trace_closest(const float4 *__restrict__ nodes,
-                                              const float4 *__restrict__ tris, float rootMax,
-                                              float4 r0, float4 r1, float &best, float &hb1,
-                                              float &hb2, int &prim, uint32_t &nv, uint32_t &nt) {
+// counting node visits and triangle tests (vt_trace_count). `r0` is (origin, tmin), `r1` (direction,
+// tmax). Entries are not culled when popped, as in the oracle's count.
+__device__ __forceinline__ void count_closest(const float4 *__restrict__ nodes, const float4 *__restrict__ tris, float rootMax,
+                                              float4 r0, float4 r1, uint32_t &nv, uint32_t &nt) {
   const WRay wr = make_wray(r0.x, r0.y, r0.z, r1.x, r1.y, r1.z);
   const QRay qr = make_qray(r0.x, r0.y, r0.z, r1.x, r1.y, r1.z, rootMax);
-  const float tMin = r0.w;
+  const float tMin = __fadd_rn(r0.w, 0.0f);
   float closest = r1.w;
-  bool found = false;
   int stack[kStack];
   int top = 0;
   stack[top++] = 0;
   while (top > 0) {
     const int entry = stack[--top];
+    if (entry == kEmptyChild) continue;
     if (entry < 0) {
-      int first, cnt;
-      leaf_range(nodes, entry, first, cnt);
-      for (int q = 0; q < cnt; ++q) {
-        const float4 *tp = tris + 3 * (size_t)(first + q);
+      const float4 *tp = tris + 3 * (size_t)(~entry);
+      for (int q = 0; q < kMaxLeafTris; ++q, tp += 3) {
         const float4 a = __ldg(tp), b = __ldg(tp + 1), cc = __ldg(tp + 2);
         float t, b1, b2;
-        if (kCount) ++nt;
-        if (!intersect_tri(wr, a, b, cc, tMin, closest, t, b1, b2)) continue;
-        closest = t; hb1 = b1; hb2 = b2; prim = __float_as_int(a.w); found = true;
+        ++nt;
+        if (intersect_tri(wr, a, b, cc, tMin, closest, t, b1, b2)) closest = t;
+        if (leaf_ends(cc)) break;
       }
       continue;
     }
     QNode nd;
     load_qnode(nodes, entry, nd);
-    if (kCount) ++nv;
+    ++nv;
     float nearT[4];
-    const int mask = qnode_hits(nd, qr, tMin, closest, nearT);
-    const Sorted4 o = sort_qchildren(nd, mask, nearT);
+    bool hit[4];
+    uint32_t key[4];
+    qnode_test(nd, qr, tMin, closest, nearT, hit);
+    sort_qchildren(hit, nearT, tMin >= 0.0f, key);
 #pragma unroll
-    for (int j = 3; j >= 0; --j) {
-      if (j >= o.m || beyond(o.key[j], closest) || top >= kStack) continue;
-      stack[top++] = o.child[j] > 0 ? o.child[j] : leaf_entry_of(entry, (int)(o.key[j] & 3u));
-    }
+    for (int j = 3; j >= 0; --j)
+      if (key[j] != kMissKey && top < kStack) stack[top++] = pick4(nd.child, key[j] & 3u);
   }
-  best = closest;
-  return found;
 }
 
-template <bool kCount>
-__device__ __forceinline__ bool trace_any(const float4 *__restrict__ nodes,
-                                          const float4 *__restrict__ tris, float rootMax, float4 r0,
-                                          float4 r1, uint32_t &nv, uint32_t &nt) {
+__device__ __forceinline__ void count_any(const float4 *__restrict__ nodes, const float4 *__restrict__ tris, float rootMax,
+                                          float4 r0, float4 r1, uint32_t &nv, uint32_t &nt) {
   const WRay wr = make_wray(r0.x, r0.y, r0.z, r1.x, r1.y, r1.z);
   const QRay qr = make_qray(r0.x, r0.y, r0.z, r1.x, r1.y, r1.z, rootMax);
   const float tMin = r0.w, tMax = r1.w;
@@ -430,31 +416,28 @@ __device__ __forceinline__ bool trace_any(const float4 *__restrict__ nodes,
   stack[top++] = 0;
   while (top > 0) {
     const int entry = stack[--top];
+    if (entry == kEmptyChild) continue;
     if (entry < 0) {
-      int first, cnt;
-      leaf_range(nodes, entry, first, cnt);
-      for (int q = 0; q < cnt; ++q) {
-        const float4 *tp = tris + 3 * (size_t)(first + q);
+      const float4 *tp = tris + 3 * (size_t)(~entry);
+      for (int q = 0; q < kMaxLeafTris; ++q, tp += 3) {
         const float4 a = __ldg(tp), b = __ldg(tp + 1), cc = __ldg(tp + 2);
         float t, b1, b2;
-        if (kCount) ++nt;
-        if (intersect_tri(wr, a, b, cc, tMin, tMax, t, b1, b2)) return true;
+        ++nt;
+        if (intersect_tri(wr, a, b, cc, tMin, tMax, t, b1, b2)) return;
+        if (leaf_ends(cc)) break;
       }
       continue;
     }
     QNode nd;
     load_qnode(nodes, entry, nd);
-    if (kCount) ++nv;
+    ++nv;
     float nearT[4];
-    const int mask = qnode_hits(nd, qr, tMin, tMax, nearT);
+    bool hit[4];
+    qnode_test(nd, qr, tMin, tMax, nearT, hit);
 #pragma unroll
-    for (int k = 3; k >= 0; --k) {
-      if (!(mask >> k & 1) || top >= kStack) continue;
-      const int c = i4(nd.child, k);
-      stack[top++] = c > 0 ? c : leaf_entry_of(entry, k);
-    }
+    for (int k = 3; k >= 0; --k)
+      if (hit[k] && top < kStack) stack[top++] = i4(nd.child, k);
   }
-  return false;
 }
 
 }  // namespace vtd

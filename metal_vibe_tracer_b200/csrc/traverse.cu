@@ -5,10 +5,10 @@
 // wide_order (main.swift:1758-1785), watertight_ray / watertight_edge / intersect_mesh_triangle
 // (main.swift:1536-1582).
 //
-// Layout: a node is the reference's 128-byte MeshWideNode, fetched as eight 16-byte vector loads
-// through the read-only path; a triangle is three float4 in BVH order (vertex a carries the input
-// face index in .w), 48 bytes fetched as three 16-byte loads. The whole structure of a 1M-triangle
-// mesh (~40 MB nodes + 48 MB triangles) sits in the 126 MB L2.
+// Layout: a node is the 64-byte quantised copy of the reference's MeshWideNode (qnode.cu), fetched as two
+// 32-byte vector loads; a triangle is three float4 in BVH order (vertex a carries the input face index
+// in .w, vertex c the mark of its leaf's last triangle), 48 bytes fetched as three 16-byte loads. The
+// whole structure of a 1M-triangle mesh (19 MB nodes + 48 MB triangles) sits in the 126 MB L2.
 //
 // The watertight arithmetic is written with explicitly rounded intrinsics in one fixed order
 // (each product and sum rounded on its own; the exact FMA fallback on edge ties), which the CPU
@@ -27,19 +27,27 @@ using namespace vtd;
 // Persistent traversal (k_closest, k_any): each warp stays resident and refills idle lanes from a
 // global ray counter: one warp-aggregated atomicAdd hands out as many rays as there are idle lanes,
 // whenever at least kRefill lanes are idle. Each loop iteration handles one stack entry per active
-// lane (a node visit or a leaf's triangles) with the per-ray order of trace_closest / trace_any, so
+// lane (a node visit or a leaf's triangles) with the per-ray order of the single-ray form, so
 // the hits equal those of the single-ray form bit for bit. Rays are read and hits written with
 // streaming cache hints so that the ray stream does not evict the BVH from L2.
-#ifndef VT_TRACE_REFILL
-#define VT_TRACE_REFILL 8
-#endif
-#ifndef VT_TRACE_MIN_BLOCKS
-#define VT_TRACE_MIN_BLOCKS 6
-#endif
+//
+// Bound: issue (ALU) and the latency of dependent loads, not bandwidth. A node visit goes straight on to
+// its nearest hit child, kept in a register, and a warp in its node phase takes up to kSteps nodes per
+// lane before it votes again (a vote costs about a tenth of a visit, and the lanes that meet a leaf
+// earlier wait): of 1, 2, 3, 4, 8 and 16 steps, 4 (closest) and 2 (any hit) measured best. The node
+// test's keys, links and steps are laid out so that a visit needs no index arithmetic (qnode.cu).
+// 8 and 9 blocks per SM (64 and 56 registers) beat 5 to 7 and 10: the loads' latency needs the warps.
+// Measured on one B200, 1M-triangle soup: closest hit of 4M random rays 5.30 -> 4.17 ms, any hit
+// 3.55 -> 2.92 ms; 1080p camera rays 1.37 -> 1.12 and 0.75 -> 0.66 ms; 4,096 rays on 20,000 triangles
+// 110 -> 93 us. Tried and dropped: entry distances on the stack to drop entries beyond a closer hit
+// unvisited (5.76 against 5.20 ms: the larger stacks cost more L1 than the visits saved), loading the
+// next node before pushing the others (5.11 against 4.26 ms).
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kRefill = VT_TRACE_REFILL;      // refill once this many lanes are idle
+// Refill once this many lanes are idle (measured at 4, 8, 12 and 16).
+constexpr int kRefill = 4, kRefillAny = 8;
+constexpr int kSteps = 4, kStepsAny = 2;  // nodes per lane between votes
 constexpr int kBlock = 128;
-constexpr int kMinBlocks = VT_TRACE_MIN_BLOCKS;  // register budget: 65536 / (kBlock * kMinBlocks)
+constexpr int kMinBlocks = 8, kMinBlocksAny = 9;  // register budget: 65536 / (kBlock * blocks)
 
 struct RayState {
   WRay wr;
@@ -72,12 +80,15 @@ __device__ __forceinline__ uint32_t refill(unsigned idle, uint32_t *counter, uin
 // word d * kBlock + t, so every lane of a warp hits its own bank whatever its stack depth.
 __device__ __forceinline__ int *stack_slot(int *sstack, int d) { return sstack + d * kBlock + threadIdx.x; }
 
-// Stack entries: an inner node is its index (>= 0); a leaf child is ~(node << 2 | slot).
+// Entries: an inner node is its index (>= 0), a leaf ~(its first triangle); kIdle marks a lane
+// without a ray. A lane's current entry stays in a register: a node visit goes straight on to its
+// nearest hit child and pushes only the others.
+constexpr int kIdle = 0x7fffffff;
 
-// Per lane, one iteration handles the top stack entry: a node visit (its hit children, leaves
-// included, pushed far to near, so they pop near first) or one leaf's triangle tests. The warp runs
-// only the kind more of its lanes need this iteration; the others wait one iteration. A ray's own
-// order (LIFO over its stack) does not depend on the warp.
+// Per lane, one iteration handles the current entry: a node visit (its hit children, leaves
+// included, near first) or one leaf's triangle tests. The warp runs only the kind more of its lanes
+// need this iteration; the others wait one iteration. A ray's own order (LIFO over its stack) does
+// not depend on the warp.
 // kPos: a hit reports the triangle's BVH position instead of its input face (the integrator's
 // hit record). count: when not null, the queue length on the device (at most n).
 template <bool kPos>
@@ -89,57 +100,73 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) k_closest(const float4 *__
                                                         uint32_t *status, const uint32_t *__restrict__ count) {
   extern __shared__ int sstack[];
   if (count) n = min(n, *count);
-  int top = 0;  // 0: the lane holds no ray
+  int cur = kIdle, top = 0;
   uint32_t rid = 0;
   RayState s;
   float closest = 0.0f, hb1 = 0.0f, hb2 = 0.0f;
   int prim = -1;
   bool exhausted = false;  // warp-uniform
   while (true) {
-    const unsigned idle = __ballot_sync(kFull, top == 0);
+    const unsigned idle = __ballot_sync(kFull, cur == kIdle);
     if (!exhausted && __popc(idle) >= kRefill) {
       const uint32_t r = refill(idle, counter, n, exhausted);
       if (r < n) {
         rid = perm ? __ldcs(perm + r) : r;
         load_ray(rays, rid, s, rootMax);
+        s.tMin = __fadd_rn(s.tMin, 0.0f);  // -0 to +0 (sort_qchildren)
         closest = s.tMax;
         prim = -1;
-        *stack_slot(sstack, 0) = 0;
-        top = 1;
+        cur = 0;
+        top = 0;
       }
     }
-    if (exhausted && !__any_sync(kFull, top > 0)) break;
-    const int entry = top > 0 ? *stack_slot(sstack, top - 1) : 0;
-    const bool leaf = top > 0 && entry < 0;
-    const unsigned leaves = __ballot_sync(kFull, leaf), inner = __ballot_sync(kFull, top > 0 && !leaf);
-    const bool leafPhase = __popc(leaves) >= __popc(inner);
-    if (top == 0 || leaf != leafPhase) continue;
-    --top;
+    const bool leaf = cur < 0;
+    const unsigned leaves = __ballot_sync(kFull, leaf), active = __ballot_sync(kFull, cur != kIdle);
+    if (exhausted && active == 0u) break;
+    const bool leafPhase = 2 * __popc(leaves) >= __popc(active);
+    if (cur == kIdle || leaf != leafPhase) continue;
+    auto pop = [&] { cur = top > 0 ? *stack_slot(sstack, --top) : kIdle; };
     if (leaf) {
-      int first, cnt;
-      leaf_range(nodes, entry, first, cnt);
-      for (int q = 0; q < cnt; ++q) {
-        const float4 *tp = tris + 3 * (size_t)(first + q);
-        const float4 a = __ldg(tp), b = __ldg(tp + 1), cc = __ldg(tp + 2);
-        float t, b1, b2;
-        if (!intersect_tri(s.wr, a, b, cc, s.tMin, closest, t, b1, b2)) continue;
-        closest = t; hb1 = b1; hb2 = b2; prim = kPos ? first + q : __float_as_int(a.w);
+      if (cur != kEmptyChild) {
+        int at = ~cur;
+        const float4 *tp = tris + 3 * (size_t)at;
+        for (int q = 0; q < kMaxLeafTris; ++q, tp += 3, ++at) {
+          const float4 a = __ldg(tp), b = __ldg(tp + 1), cc = __ldg(tp + 2);
+          float t, b1, b2;
+          if (intersect_tri(s.wr, a, b, cc, s.tMin, closest, t, b1, b2)) {
+            closest = t; hb1 = b1; hb2 = b2; prim = kPos ? at : __float_as_int(a.w);
+          }
+          if (leaf_ends(cc)) break;
+        }
       }
+      pop();
     } else {
       QNode nd;
-      load_qnode(nodes, entry, nd);
-      float nearT[4];
-      const int mask = qnode_hits(nd, s.qr, s.tMin, closest, nearT);
-      const Sorted4 o = sort_qchildren(nd, mask, nearT);
+      load_qnode(nodes, cur, nd);
+#pragma unroll 1
+      for (int step = 1;; ++step) {
+        float nearT[4];
+        bool hit[4];
+        uint32_t key[4];
+        qnode_test(nd, s.qr, s.tMin, closest, nearT, hit);
+        sort_qchildren(hit, nearT, s.tMin >= 0.0f, key);
+        // At most three pushes per level of the tree: a full stack means a corrupted tree.
+        if (top + 3 > stackSize) {
+          atomicOr(status, (uint32_t)VT_DEV_STACK);
+          top = stackSize - 3;
+        }
 #pragma unroll
-      for (int j = 3; j >= 0; --j) {
-        if (j >= o.m || beyond(o.key[j], closest)) continue;
-        const int e = o.child[j] > 0 ? o.child[j] : leaf_entry_of(entry, (int)(o.key[j] & 3u));
-        if (top < stackSize) *stack_slot(sstack, top++) = e;
-        else atomicOr(status, (uint32_t)VT_DEV_STACK);
+        for (int j = 3; j >= 1; --j) {
+          if (key[j] == kMissKey) continue;
+          *stack_slot(sstack, top++) = pick4(nd.child, key[j] & 3u);
+        }
+        if (key[0] != kMissKey) cur = pick4(nd.child, key[0] & 3u);
+        else pop();
+        if (cur < 0 || cur == kIdle || step >= kSteps) break;
+        load_qnode(nodes, cur, nd);
       }
     }
-    if (top == 0) {
+    if (cur == kIdle) {
       const int4 out = prim >= 0 ? make_int4(__float_as_int(closest), __float_as_int(hb1), __float_as_int(hb2), prim)
                                  : make_int4(0, 0, 0, -1);
       __stcs(hits + rid, out);
@@ -150,7 +177,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) k_closest(const float4 *__
 // kSlack: each triangle's own rounding bound comes off tmax (the integrator's shadow rays in
 // imported scenes, scene_occluded main.swift:2066-2069). count: as k_closest's.
 template <bool kSlack>
-__global__ void __launch_bounds__(kBlock, kMinBlocks) k_any(const float4 *__restrict__ nodes,
+__global__ void __launch_bounds__(kBlock, kMinBlocksAny) k_any(const float4 *__restrict__ nodes,
                                                     const float4 *__restrict__ tris, float rootMax,
                                                     const float4 *__restrict__ rays, uint32_t n,
                                                     uint8_t *__restrict__ occ, uint32_t *counter,
@@ -158,55 +185,66 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) k_any(const float4 *__rest
                                                     uint32_t *status, const uint32_t *__restrict__ count) {
   extern __shared__ int sstack[];
   if (count) n = min(n, *count);
-  int top = 0;
+  int cur = kIdle, top = 0;
   uint32_t rid = 0;
   RayState s;
   bool exhausted = false;
   while (true) {
-    const unsigned idle = __ballot_sync(kFull, top == 0);
-    if (!exhausted && __popc(idle) >= kRefill) {
+    const unsigned idle = __ballot_sync(kFull, cur == kIdle);
+    if (!exhausted && __popc(idle) >= kRefillAny) {
       const uint32_t r = refill(idle, counter, n, exhausted);
       if (r < n) {
         rid = perm ? __ldcs(perm + r) : r;
         load_ray(rays, rid, s, rootMax);
-        *stack_slot(sstack, 0) = 0;
-        top = 1;
+        cur = 0;
+        top = 0;
       }
     }
-    if (exhausted && !__any_sync(kFull, top > 0)) break;
-    const int entry = top > 0 ? *stack_slot(sstack, top - 1) : 0;
-    const bool leaf = top > 0 && entry < 0;
-    const unsigned leaves = __ballot_sync(kFull, leaf), inner = __ballot_sync(kFull, top > 0 && !leaf);
-    const bool leafPhase = __popc(leaves) >= __popc(inner);
-    if (top == 0 || leaf != leafPhase) continue;
-    --top;
+    const bool leaf = cur < 0;
+    const unsigned leaves = __ballot_sync(kFull, leaf), active = __ballot_sync(kFull, cur != kIdle);
+    if (exhausted && active == 0u) break;
+    const bool leafPhase = 2 * __popc(leaves) >= __popc(active);
+    if (cur == kIdle || leaf != leafPhase) continue;
     bool hit = false;
+    auto pop = [&] { cur = top > 0 ? *stack_slot(sstack, --top) : kIdle; };
     if (leaf) {
-      int first, cnt;
-      leaf_range(nodes, entry, first, cnt);
-      for (int q = 0; q < cnt; ++q) {
-        const float4 *tp = tris + 3 * (size_t)(first + q);
-        const float4 a = __ldg(tp), b = __ldg(tp + 1), cc = __ldg(tp + 2);
-        float t, b1, b2;
-        const float tMax = kSlack ? s.tMax - tri_error_bound(a, b, cc) : s.tMax;
-        if (intersect_tri(s.wr, a, b, cc, s.tMin, tMax, t, b1, b2)) { hit = true; break; }
+      if (cur != kEmptyChild) {
+        const float4 *tp = tris + 3 * (size_t)(~cur);
+        for (int q = 0; q < kMaxLeafTris; ++q, tp += 3) {
+          const float4 a = __ldg(tp), b = __ldg(tp + 1), cc = __ldg(tp + 2);
+          float t, b1, b2;
+          const float tMax = kSlack ? s.tMax - tri_error_bound(a, b, cc) : s.tMax;
+          if (intersect_tri(s.wr, a, b, cc, s.tMin, tMax, t, b1, b2)) { hit = true; break; }
+          if (leaf_ends(cc)) break;
+        }
       }
+      if (hit) cur = kIdle;
+      else pop();
     } else {
-      QNode nd;
-      load_qnode(nodes, entry, nd);
-      float nearT[4];
-      const int mask = qnode_hits(nd, s.qr, s.tMin, s.tMax, nearT);
+#pragma unroll 1
+      for (int step = 0; step < kStepsAny; ++step) {
+        QNode nd;
+        load_qnode(nodes, cur, nd);
+        float nearT[4];
+        bool meets[4];
+        qnode_test(nd, s.qr, s.tMin, s.tMax, nearT, meets);
+        if (top + 3 > stackSize) {
+          atomicOr(status, (uint32_t)VT_DEV_STACK);
+          top = stackSize - 3;
+        }
+        int next = kIdle;
 #pragma unroll
-      for (int k = 3; k >= 0; --k) {
-        if (!(mask >> k & 1)) continue;
-        const int c = i4(nd.child, k);
-        const int e = c > 0 ? c : leaf_entry_of(entry, k);
-        if (top < stackSize) *stack_slot(sstack, top++) = e;
-        else atomicOr(status, (uint32_t)VT_DEV_STACK);
+        for (int k = 3; k >= 0; --k) {
+          if (!meets[k]) continue;
+          if (next != kIdle) *stack_slot(sstack, top++) = next;
+          next = i4(nd.child, k);
+        }
+        if (next != kIdle) cur = next;
+        else pop();
+        if (cur < 0 || cur == kIdle) break;
       }
     }
-    if (hit) top = 0;
-    if (top == 0) occ[rid] = hit ? 1 : 0;
+    if (cur == kIdle) occ[rid] = hit ? 1 : 0;
   }
 }
 
@@ -219,11 +257,9 @@ __global__ void __launch_bounds__(128) k_count(const float4 *__restrict__ nodes,
   if (i < n) {
     const float4 r0 = __ldg(rays + 2 * (size_t)i), r1 = __ldg(rays + 2 * (size_t)i + 1);
     if (closest) {
-      float t, b1, b2;
-      int prim;
-      trace_closest<true>(nodes, tris, rootMax, r0, r1, t, b1, b2, prim, nv, nt);
+      count_closest(nodes, tris, rootMax, r0, r1, nv, nt);
     } else {
-      trace_any<true>(nodes, tris, rootMax, r0, r1, nv, nt);
+      count_any(nodes, tris, rootMax, r0, r1, nv, nt);
     }
   }
   unsigned long long a = nv, b = nt;
@@ -304,9 +340,9 @@ __global__ void k_ray_keys(const float4 *__restrict__ rays, uint32_t n, float3 l
 }
 
 namespace {
-// Stack entries a traversal of a tree of `depth` levels needs: the root, then at most 3 net pushes
-// per level below it (a visit pops one node and pushes up to four).
-inline int stack_entries(uint32_t depth) { return 3 * (int)depth + 1; }
+// Stack entries a traversal of a tree of `depth` levels needs: a visit goes on to one child and
+// pushes at most three.
+inline int stack_entries(uint32_t depth) { return 3 * (int)depth; }
 
 // Resident blocks per SM for a persistent kernel with `smem` bytes of dynamic shared memory.
 template <typename K> int resident_blocks(K kernel, size_t smem) {

@@ -159,3 +159,23 @@ def test_traversal_counts_match_oracle(ctx, oracle):
     assert mesh.count(rays, closest=True) == ref.count(rays, closest=True)
     shadow = scenes.shadow_tmax_np(rays, False)
     assert mesh.count(shadow, closest=False) == ref.count(shadow, closest=False)
+
+
+@pytest.mark.parametrize("faces_n", [1, 2, 5, 700])
+@pytest.mark.parametrize("leaf", [1, 3, 8])
+def test_small_meshes_and_ray_counts(ctx, oracle, faces_n, leaf):
+    """One-leaf trees, part-filled nodes and leaves of up to 8 triangles, ray counts around warps and
+    blocks, tmin negative, -0 and positive: hits and occlusion equal the oracle's bit for bit."""
+    faces, verts = scenes.triangle_soup(faces_n, seed=faces_n, mu=math.log(0.2))
+    mesh = vt.Mesh(ctx, faces, verts, leaf_size=leaf)
+    ref = oracle.Bvh.lbvh(faces, verts, leaf_size=leaf)
+    for n in (1, 31, 33, 129, 3001):
+        rays = scenes.incoherent_rays_np(n, seed=n + leaf)
+        rays[::3, 3] = -0.5
+        rays[1::3, 3] = -0.0
+        rays[2::5, 3] = 0.3
+        hits = gpu_closest(mesh, rays)
+        assert_bit_exact(hits, ref.closest(rays))
+        short = scenes.shadow_tmax_np(rays, False, seed=n)
+        assert np.array_equal(gpu_any(mesh, short), ref.occluded(short))
+    mesh.close()
