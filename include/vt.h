@@ -700,9 +700,9 @@ vt_status vt_render_nrc(vt_ctx *ctx, vt_scene *scene, vt_nrc *nrc, const vt_fram
  *          in .w, b with the face's tag bits in .w, c; 16-byte aligned).
  *   order: nfaces int32 (BVH position -> input face).
  *   info:  host output (build_ms is host wall time).  stream: NULL = the CUDA default stream.
- *          The call blocks the host: it synchronises that stream once per collapse level (the
- *          level's node count sizes the next launch) and at the end, so it returns when the build
- *          is complete; a call that fails after queueing work also waits for that work first.
+ *          The call blocks the host: it synchronises that stream after the collapse (for the node
+ *          count) and at the end, so it returns when the build is complete; a call that fails after
+ *          queueing work also waits for that work first.
  *   error: optional host buffer of error_capacity bytes for the failure message.
  * Meshes over VT_NOALLOC_MAX_FACES faces are rejected with VT_ERR_LIMIT. The first call on each
  * device looks up the static array's address (with that device current), so make that first call

@@ -6,7 +6,9 @@
 // Every arithmetic step that decides topology is written with explicitly rounded intrinsics
 // (__fadd_rn, __fmul_rn, __fdiv_rn) so the CPU oracle (oracle/vt_oracle.cpp, built with
 // -ffp-contract=off) reproduces Morton codes, sorted order and topology bit for bit.
+#include <algorithm>
 #include <cfloat>
+#include <climits>
 #include <vector>
 
 #include "vt_internal.cuh"
@@ -162,10 +164,18 @@ __device__ __forceinline__ int delta(const uint32_t *codes, int n, int i, int j)
   return 32 + __clz((uint32_t)i ^ (uint32_t)j);
 }
 
-__global__ void k_karras(const uint32_t *codes, int n, int2 *child, int32_t *parent) {
+// One thread per sorted position: its leaf box gathered, and internal node i's hierarchy with its
+// visit counter cleared.
+__global__ void k_hierarchy(const uint32_t *codes, const float4 *boxes, const uint32_t *sorted, int n, float4 *leaf, int2 *child,
+                            int32_t *parent, uint32_t *flags) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const uint32_t f = sorted[i];
+  leaf[2 * (size_t)i] = boxes[2 * (size_t)f];
+  leaf[2 * (size_t)i + 1] = boxes[2 * (size_t)f + 1];
   if (i == 0) parent[0] = -1;
   if (i >= n - 1) return;
+  flags[i] = 0u;
   const int d = delta(codes, n, i, i + 1) - delta(codes, n, i, i - 1) > 0 ? 1 : -1;
   const int dmin = delta(codes, n, i, i - d);
   int lmax = 2;
@@ -179,7 +189,7 @@ __global__ void k_karras(const uint32_t *codes, int n, int2 *child, int32_t *par
   for (int div = 2;; div *= 2) {
     const int step = (l + div - 1) / div;
     if (delta(codes, n, i, i + (s + step) * d) > dnode) s += step;
-    if (step == 1) break;
+    if (step <= 1) break;
   }
   const int gamma = i + s * d + min(d, 0);
   const int lo = min(i, j), hi = max(i, j);
@@ -188,14 +198,6 @@ __global__ void k_karras(const uint32_t *codes, int n, int2 *child, int32_t *par
   child[i] = make_int2(left, right);
   parent[left >= 0 ? left : (n - 1 + gamma)] = i;
   parent[right >= 0 ? right : (n - 1 + gamma + 1)] = i;
-}
-
-__global__ void k_leaf_boxes(const float4 *boxes, const uint32_t *sorted, uint32_t n, float4 *leaf) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  uint32_t f = sorted[i];
-  leaf[2 * i] = boxes[2 * f];
-  leaf[2 * i + 1] = boxes[2 * f + 1];
 }
 
 // ---- bottom-up passes ---------------------------------------------------------------------------
@@ -548,17 +550,21 @@ __device__ void restructure_warp(const TreeView &t, int root, int size, uint32_t
   __stcg(t.parent + (ky >= 0 ? ky : (t.n - 1 + (-ky - 1))), node);
 }
 
+constexpr int kMaxWalk = 1 << 14;
+
 // One thread per leaf walks to the root; the second thread to reach a node owns it (its two
-// subtrees are final) and refits it. flags[] must be zero on entry.
+// subtrees are final) and refits it. A pass visits every node twice, so flags[] starts each pass even
+// and the first visitor sees an even count: it is cleared once, by k_hierarchy.
 __global__ void __launch_bounds__(128) k_bottom_up(TreeView t, uint32_t *flags, uint32_t *status) {
   const int leaf = blockIdx.x * blockDim.x + threadIdx.x;
   if (leaf >= t.n) return;
   int node = __ldcg(t.parent + (t.n - 1 + leaf));
-  // A walk longer than the node count means a corrupted parent chain: stop and report.
+  // A walk longer than any tree of 30-bit codes and 32-bit positions is deep means a corrupted parent
+  // chain: stop and report.
   for (int guard = 0; node >= 0; ++guard) {
-    if (guard >= t.n) { atomicOr(status, (uint32_t)VT_DEV_TREELET); return; }
+    if (guard >= kMaxWalk) { atomicOr(status, (uint32_t)VT_DEV_TREELET); return; }
     __threadfence();
-    if (atomicAdd(&flags[node], 1u) == 0u) return;
+    if ((atomicAdd(&flags[node], 1u) & 1u) == 0u) return;
     __threadfence();
     refit_node(t, node);
     __threadfence();
@@ -581,12 +587,12 @@ __global__ void __launch_bounds__(128) k_restructure(TreeView t, uint32_t *flags
   while (true) {
     bool own = false;
     if (node >= 0) {
-      if (guard++ >= t.n) {
+      if (guard++ >= kMaxWalk) {
         atomicOr(status, (uint32_t)VT_DEV_TREELET);
         node = -1;
       } else {
         __threadfence();
-        if (atomicAdd(&flags[node], 1u) == 0u) node = -1;
+        if ((atomicAdd(&flags[node], 1u) & 1u) == 0u) node = -1;
         else own = true;
         __threadfence();
       }
@@ -615,51 +621,46 @@ __global__ void __launch_bounds__(128) k_restructure(TreeView t, uint32_t *flags
 // A wide node rooted at binary node b starts with children [b] and splits the child of largest
 // area among those with more than leafSize leaves (the reference's rule,
 // Sources/Acceleration.swift:255-263) until four children.
-__global__ void k_collapse_count(TreeView t, const int32_t *level, uint32_t L, int leafSize,
-                                 int4 *chOut, uint32_t *nInner, uint32_t *nPrims) {
-  const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= L) return;
-  int ch[4] = {level[w], 0, 0, 0};
+// The children of the wide node at binary node `root`; returns their number.
+__device__ __forceinline__ int collapse_children(const TreeView &t, int root, int leafSize, int ch[4], uint32_t &inner, uint32_t &prims) {
+  uint32_t cnt[4];
+  ch[0] = root;
+  cnt[0] = child_count(t, root);
   int m = 1;
   while (m < 4) {
     int best = -1;
     float bestA = 0.0f;
     for (int k = 0; k < m; ++k) {
-      if (child_count(t, ch[k]) <= (uint32_t)leafSize) continue;
+      if (cnt[k] <= (uint32_t)leafSize) continue;
       Box b = child_box(t, ch[k]);
       float a = box_area(b.lo, b.hi);
       if (best < 0 || a > bestA) { best = k; bestA = a; }
     }
     if (best < 0) break;
     const int c = ch[best];
-    for (int k = m; k > best + 1; --k) ch[k] = ch[k - 1];
+    for (int k = m; k > best + 1; --k) { ch[k] = ch[k - 1]; cnt[k] = cnt[k - 1]; }
     int2 cc = load_child(t, c);
     ch[best] = cc.x;
     ch[best + 1] = cc.y;
+    cnt[best] = child_count(t, cc.x);
+    cnt[best + 1] = child_count(t, cc.y);
     ++m;
   }
-  uint32_t inner = 0, prims = 0;
+  inner = prims = 0;
   for (int k = 0; k < m; ++k) {
-    uint32_t cnt = child_count(t, ch[k]);
-    if (cnt <= (uint32_t)leafSize) prims += cnt;
+    if (cnt[k] <= (uint32_t)leafSize) prims += cnt[k];
     else ++inner;
   }
-  // Unused slots marked INT_MIN (a valid leaf encoding never reaches it).
-  int4 out = make_int4(ch[0], m > 1 ? ch[1] : INT_MIN, m > 2 ? ch[2] : INT_MIN, m > 3 ? ch[3] : INT_MIN);
-  chOut[w] = out;
-  nInner[w] = inner;
-  nPrims[w] = prims;
+  return m;
 }
 
-__global__ void k_collapse_emit(TreeView t, uint32_t L, int leafSize, const int4 *chIn,
-                                const uint32_t *offInner, const uint32_t *offPrims, uint32_t base,
-                                uint32_t nextBase, uint32_t primBase, vt_wide_node *nodes,
-                                int32_t *nextLevel, const uint32_t *sorted, const vt_face *faces,
-                                const vt_vertex *verts, uint32_t nverts, int32_t *order, float4 *tris,
-                                uint32_t *status, float4 *nrm = nullptr) {
-  const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= L) return;
-  int4 c4 = chIn[w];
+// Wide node `at` with children ch (unused slots INT_MIN, which no leaf encoding reaches): its inner
+// children get nodes from nextBase + inner on and entries from nextLevel[inner] on, its leaves'
+// triangles BVH positions from prim on.
+__device__ __forceinline__ void collapse_emit(const TreeView &t, int leafSize, const int4 c4, uint32_t inner, uint32_t prim,
+                                              uint32_t at, uint32_t nextBase, vt_wide_node *nodes, int32_t *nextLevel,
+                                              const uint32_t *sorted, const vt_face *faces, const vt_vertex *verts, uint32_t nverts,
+                                              int32_t *order, float4 *tris, float4 *nrm, bool markLeaves, uint32_t *status) {
   int ch[4] = {c4.x, c4.y, c4.z, c4.w};
   vt_wide_node nd;
 #pragma unroll
@@ -668,7 +669,7 @@ __global__ void k_collapse_emit(TreeView t, uint32_t L, int leafSize, const int4
     nd.child[k] = 0;
     nd.count[k] = 0;
   }
-  uint32_t inner = offInner[w], prim = primBase + offPrims[w];
+#pragma unroll
   for (int k = 0; k < 4; ++k) {
     if (ch[k] == INT_MIN) break;
     Box b = child_box(t, ch[k]);
@@ -687,9 +688,9 @@ __global__ void k_collapse_emit(TreeView t, uint32_t L, int leafSize, const int4
         if (c < 0) {
           if (prim >= (uint32_t)t.n) { atomicOr(status, (uint32_t)VT_DEV_TREELET); return; }
           uint32_t f = sorted[-c - 1];
-          // The traversal's leaf loop ends at the triangle marked as its leaf's last (the meshes that
-          // are traversed carry normals here).
-          const float last = nrm && top == 0 ? 1.0f : 0.0f;
+          // The traversal's leaf loop ends at the triangle marked as its leaf's last.
+          const float last = markLeaves && top == 0 ? 1.0f : 0.0f;
+          const size_t p3 = 3 * (size_t)prim;
           order[prim] = (int32_t)f;
           vt_face fc = faces[f];
           if (fc.a >= nverts || fc.b >= nverts || fc.c >= nverts) {
@@ -697,24 +698,24 @@ __global__ void k_collapse_emit(TreeView t, uint32_t L, int leafSize, const int4
             // returns VT_ERR_INVALID), the slot gets a degenerate triangle at the origin.
             atomicOr(status, (uint32_t)VT_DEV_BAD_INDEX);
             const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            tris[3 * prim] = make_float4(0.0f, 0.0f, 0.0f, __int_as_float((int)f));
-            tris[3 * prim + 1] = z;
-            tris[3 * prim + 2] = make_float4(0.0f, 0.0f, 0.0f, last);
-            if (nrm) nrm[3 * prim] = nrm[3 * prim + 1] = nrm[3 * prim + 2] = z;
+            tris[p3] = make_float4(0.0f, 0.0f, 0.0f, __int_as_float((int)f));
+            tris[p3 + 1] = z;
+            tris[p3 + 2] = make_float4(0.0f, 0.0f, 0.0f, last);
+            if (nrm) nrm[p3] = nrm[p3 + 1] = nrm[p3 + 2] = z;
             ++prim;
             continue;
           }
           const vt_vertex &va = verts[fc.a], &vb = verts[fc.b], &vc = verts[fc.c];
-          tris[3 * prim] = make_float4(va.px, va.py, va.pz, __int_as_float((int)f));
-          tris[3 * prim + 1] = make_float4(vb.px, vb.py, vb.pz, __uint_as_float(fc.tag));
-          tris[3 * prim + 2] = make_float4(vc.px, vc.py, vc.pz, last);
+          tris[p3] = make_float4(va.px, va.py, va.pz, __int_as_float((int)f));
+          tris[p3 + 1] = make_float4(vb.px, vb.py, vb.pz, __uint_as_float(fc.tag));
+          tris[p3 + 2] = make_float4(vc.px, vc.py, vc.pz, last);
           if (nrm) {  // vertex normals for smooth shading (mesh_hit_attributes)
-            nrm[3 * prim] = make_float4(va.nx, va.ny, va.nz, 0.0f);
-            nrm[3 * prim + 1] = make_float4(vb.nx, vb.ny, vb.nz, 0.0f);
-            nrm[3 * prim + 2] = make_float4(vc.nx, vc.ny, vc.nz, 0.0f);
+            nrm[p3] = make_float4(va.nx, va.ny, va.nz, 0.0f);
+            nrm[p3 + 1] = make_float4(vb.nx, vb.ny, vb.nz, 0.0f);
+            nrm[p3 + 2] = make_float4(vc.nx, vc.ny, vc.nz, 0.0f);
             const bool some = va.nx != 0.0f || va.ny != 0.0f || va.nz != 0.0f || vb.nx != 0.0f || vb.ny != 0.0f ||
                               vb.nz != 0.0f || vc.nx != 0.0f || vc.ny != 0.0f || vc.nz != 0.0f;
-            if (some) atomicOr(status, (uint32_t)VT_DEV_NORMALS);
+            if (some && !(__ldcg(status) & (uint32_t)VT_DEV_NORMALS)) atomicOr(status, (uint32_t)VT_DEV_NORMALS);
           }
           ++prim;
           continue;
@@ -726,11 +727,149 @@ __global__ void k_collapse_emit(TreeView t, uint32_t L, int leafSize, const int4
       }
     } else {
       nd.child[k] = (int32_t)(nextBase + inner);
-      nextLevel[inner] = ch[k];
+      __stcg(nextLevel + inner, ch[k]);
       ++inner;
     }
   }
-  nodes[base + w] = nd;
+  nodes[at] = nd;
+}
+
+// What a build reports back, in one copy.
+struct BuildReport {
+  uint32_t bounds[12];                 // k_face_boxes'
+  uint32_t nodes, depth, prims, code;  // the collapse's (code: kCollapse*)
+  uint32_t status, done, pad[2];       // done: 1 once the collapse has run to its end
+};
+enum : uint32_t { kCollapseOk = 0, kCollapseDepth = 1, kCollapseNodes = 2 };
+
+constexpr int kCollapseBlock = 128;
+constexpr uint32_t kBarrierSpins = 1u << 21;  // polls before a grid barrier gives up (VT_DEV_BARRIER)
+
+// Barrier over the grid of a cooperative launch: bar[0] counts arrivals over the kernel's whole life,
+// bar[1] is set when a block gave up. False (block-uniform) once any block did.
+__device__ bool grid_barrier(uint32_t *bar, uint32_t &round, uint32_t *status) {
+  __shared__ bool alive;
+  ++round;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(bar, 1u);
+    const uint32_t target = round * gridDim.x;
+    uint32_t spins = 0;
+    while (vt_poll(bar) < target && vt_poll(bar + 1) == 0u && ++spins < kBarrierSpins) {}
+    if (spins >= kBarrierSpins) {
+      atomicOr(status, (uint32_t)VT_DEV_BARRIER);
+      atomicExch(bar + 1, 1u);
+    }
+    __threadfence();
+    alive = vt_poll(bar + 1) == 0u;
+  }
+  __syncthreads();
+  return alive;
+}
+
+// Sum over the block (every thread gets it).
+__device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t *ws) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = v;
+  __syncthreads();
+  return ws[0] + ws[1] + ws[2] + ws[3];
+}
+
+// The whole collapse in one cooperative launch. Bound: latency (per level a few dependent loads and two
+// grid barriers); a launch per step with the level's size read back by the host spent 60-100 us a
+// level instead (rebuilding and tracing 20,480 triangles: 4.1 -> 1.6 ms with the sort and the pool). Per level each block takes a contiguous part: it counts its wide nodes' inner
+// children and triangles, and after a barrier prefixes the blocks' sums to place its own nodes,
+// children and triangles in the level order of a serial pass.
+__global__ void __launch_bounds__(kCollapseBlock) k_collapse(TreeView t, int leafSize, int maxDepth, uint32_t maxNodes, int32_t *levelA,
+                                                             int32_t *levelB, int4 *children, uint32_t *packed, uint2 *blockSums,
+                                                             uint32_t *bar, vt_wide_node *nodes, const uint32_t *sorted,
+                                                             const vt_face *faces, const vt_vertex *verts, uint32_t nverts,
+                                                             int32_t *order, float4 *tris, float4 *nrm, int markLeaves,
+                                                             const uint32_t *bounds, BuildReport *report, uint32_t *status) {
+  __shared__ uint32_t ws[kCollapseBlock / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t L = 1, base = 0, primBase = 0, depth = 0, code = kCollapseOk, round = 0;
+  int32_t *level = levelA, *nextLevel = levelB;
+  while (L > 0) {
+    if ((int)depth >= maxDepth) { code = kCollapseDepth; break; }
+    ++depth;
+    const uint32_t per = ((L + gridDim.x - 1) / gridDim.x + kCollapseBlock - 1) / kCollapseBlock * kCollapseBlock;
+    const uint32_t w0 = min((uint64_t)L, (uint64_t)blockIdx.x * per), w1 = min(L, w0 + per);
+    uint32_t sumI = 0, sumP = 0;
+    for (uint32_t w = w0 + threadIdx.x; w < w1; w += kCollapseBlock) {
+      const int root = depth == 1 ? (t.n >= 2 ? 0 : -1) : (int)vt_poll(reinterpret_cast<const uint32_t *>(level + w));
+      int ch[4];
+      uint32_t inner, prims;
+      const int m = collapse_children(t, root, leafSize, ch, inner, prims);
+      children[w] = make_int4(ch[0], m > 1 ? ch[1] : INT_MIN, m > 2 ? ch[2] : INT_MIN, m > 3 ? ch[3] : INT_MIN);
+      packed[w] = inner | prims << 16;
+      sumI += inner;
+      sumP += prims;
+    }
+    sumI = block_sum(sumI, ws);
+    sumP = block_sum(sumP, ws);
+    if (threadIdx.x == 0) __stcg(blockSums + blockIdx.x, make_uint2(sumI, sumP));
+    if (!grid_barrier(bar, round, status)) return;
+    uint32_t allI = 0, allP = 0, runI = 0, runP = 0;
+    for (uint32_t q = threadIdx.x; q < gridDim.x; q += kCollapseBlock) {
+      const uint2 v = make_uint2(vt_poll(&blockSums[q].x), vt_poll(&blockSums[q].y));
+      allI += v.x;
+      allP += v.y;
+      if (q < blockIdx.x) { runI += v.x; runP += v.y; }
+    }
+    allI = block_sum(allI, ws);
+    allP = block_sum(allP, ws);
+    runI = block_sum(runI, ws);
+    runP = block_sum(runP, ws);
+    const uint32_t nextBase = base + L;
+    for (uint32_t tile = w0; tile < w1; tile += kCollapseBlock) {  // w0, w1 are block-uniform
+      const uint32_t w = tile + threadIdx.x;
+      // Exclusive prefix of (inner, triangles) over the tile: 16 bits hold either sum.
+      const uint32_t v = w < w1 ? packed[w] : 0u;
+      uint32_t inc = v;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += u;
+      }
+      __syncthreads();
+      if (lane == 31) ws[warp] = inc;
+      __syncthreads();
+      uint32_t before = 0, all = 0;
+#pragma unroll
+      for (int k = 0; k < kCollapseBlock / 32; ++k) {
+        before += k < warp ? ws[k] : 0u;
+        all += ws[k];
+      }
+      before += inc - v;
+      if (w < w1)
+        collapse_emit(t, leafSize, children[w], runI + (before & 0xffffu), primBase + runP + (before >> 16), base + w, nextBase,
+                      nodes, nextLevel, sorted, faces, verts, nverts, order, tris, nrm, markLeaves != 0, status);
+      runI += all & 0xffffu;
+      runP += all >> 16;
+    }
+    if (!grid_barrier(bar, round, status)) return;
+    // No block writes status before the next barrier, so all of them read the same.
+    const uint32_t st = vt_poll(status);
+    primBase += allP;
+    base = nextBase;
+    L = allI;
+    int32_t *x = level; level = nextLevel; nextLevel = x;
+    if (st & (uint32_t)(VT_DEV_TREELET | VT_DEV_BAD_INDEX | VT_DEV_NONFINITE | VT_DEV_SORT)) break;
+    if (base + L > maxNodes) { code = kCollapseNodes; break; }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    for (int k = 0; k < 12; ++k) report->bounds[k] = bounds[k];
+    report->nodes = base;
+    report->depth = depth;
+    report->prims = primBase;
+    report->code = code;
+    report->status = vt_poll(status);
+    report->done = 1u;
+  }
 }
 
 // SAH cost of the wide tree (node cost 1, triangle cost 1, areas over the root box's area).
@@ -763,23 +902,106 @@ __global__ void k_sah(const vt_wide_node *nodes, uint32_t nn, double *acc) {
   if ((threadIdx.x & 31) == 0) atomicAdd(acc, v);
 }
 
-struct DeviceArena {
-  std::vector<void *> ptrs;
-  ~DeviceArena() {
-    for (void *p : ptrs) cudaFree(p);
-  }
-  template <typename T> cudaError_t alloc(T **p, size_t count) {
-    void *q = nullptr;
-    cudaError_t e = cudaMalloc(&q, count * sizeof(T) + 16);
-    if (e == cudaSuccess) {
-      ptrs.push_back(q);
-      *p = static_cast<T *>(q);
-    }
-    return e;
+inline uint32_t blocks(uint32_t n, uint32_t t) { return (n + t - 1) / t; }
+
+// Bump allocator over one device buffer (256-byte aligned regions). With base == nullptr it only
+// measures.
+struct ScratchCarve {
+  unsigned char *base;
+  size_t off = 0;
+  template <typename T> T *take(size_t count) {
+    size_t bytes = (count * sizeof(T) + 16 + 255) & ~size_t(255);
+    T *p = base ? reinterpret_cast<T *>(base + off) : nullptr;
+    off += bytes;
+    return p;
   }
 };
 
-inline uint32_t blocks(uint32_t n, uint32_t t) { return (n + t - 1) / t; }
+// Temporaries of a build of n faces.
+struct BuildScratch {
+  float4 *boxes, *leafBox;
+  uint32_t *bounds, *codesAlt, *valsAlt, *sortTemp, *flags, *count, *packed, *bar;
+  int32_t *parent, *levelA, *levelB;
+  float *cost;
+  int4 *children;
+  uint2 *blockSums;
+  BuildReport *report;
+  double *sah;
+};
+
+constexpr uint32_t kCollapseBlocksMax = 1184;  // 8 per SM
+
+void carve_build(ScratchCarve &c, uint32_t n, BuildScratch &b) {
+  const uint32_t ni = n > 1 ? n - 1 : 1;
+  b.boxes = c.take<float4>(2 * (size_t)n);
+  b.leafBox = c.take<float4>(2 * (size_t)n);
+  b.bounds = c.take<uint32_t>(16);
+  b.codesAlt = c.take<uint32_t>(n);
+  b.valsAlt = c.take<uint32_t>(n);
+  b.sortTemp = c.take<uint32_t>(vt_radix_temp_words(n));
+  b.flags = c.take<uint32_t>(ni);
+  b.count = c.take<uint32_t>(ni);
+  b.parent = c.take<int32_t>(2 * (size_t)n);
+  b.cost = c.take<float>(ni);
+  b.levelA = c.take<int32_t>(n);
+  b.levelB = c.take<int32_t>(n);
+  b.children = c.take<int4>(n);
+  b.packed = c.take<uint32_t>(n);
+  b.blockSums = c.take<uint2>(kCollapseBlocksMax);
+  b.bar = c.take<uint32_t>(2);
+  b.report = c.take<BuildReport>(1);
+  b.sah = c.take<double>(1);
+}
+
+// The build's outputs and the binary hierarchy they come from (either the mesh's own buffers or the
+// caller's).
+struct BuildBuffers {
+  uint32_t *codes, *sorted;  // Morton codes and face indices, sorted
+  int2 *child;               // binary hierarchy: children and boxes per internal node
+  float4 *nodeBox;
+  vt_wide_node *nodes;
+  uint32_t maxNodes;
+  int32_t *order;
+  float4 *tris, *nrm;        // nrm may be null
+  bool markLeaves;           // set the traversal's leaf marks (leaf_ends)
+};
+
+// Queues the build up to the collapse on stream s; the report then holds its outcome.
+cudaError_t queue_build(const vt_face *faces, uint32_t n, const vt_vertex *verts, uint32_t nverts, int leafSize, int treelet,
+                        int rounds, int maxDepth, const BuildBuffers &o, const BuildScratch &b, uint32_t *status, cudaStream_t s) {
+  cudaError_t e = cudaMemsetAsync(status, 0, sizeof(uint32_t), s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(b.bar, 0, 2 * sizeof(uint32_t), s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(b.report, 0, sizeof(BuildReport), s);
+  if (e != cudaSuccess) return e;
+  k_init_bounds<<<1, 32, 0, s>>>(b.bounds);
+  k_face_boxes<<<blocks(n, 256), 256, 0, s>>>(faces, n, verts, nverts, b.boxes, b.bounds, status);
+  k_morton<<<blocks(n, 256), 256, 0, s>>>(b.boxes, n, b.bounds, o.codes, o.sorted);
+  vt_radix_sort_pairs(o.codes, o.sorted, b.codesAlt, b.valsAlt, n, 30, b.sortTemp, status, s);
+  k_hierarchy<<<blocks(n, 256), 256, 0, s>>>(o.codes, b.boxes, o.sorted, (int)n, b.leafBox, o.child, b.parent, b.flags);
+  TreeView t{(int)n, o.child, b.parent, b.leafBox, o.nodeBox, b.count, b.cost};
+  if (n >= 2) {
+    k_bottom_up<<<blocks(n, 128), 128, 0, s>>>(t, b.flags, status);
+    if (treelet > 0 && n >= 3)
+      for (int r = 0; r < rounds; ++r) k_restructure<<<blocks(n, 128), 128, 0, s>>>(t, b.flags, treelet, status);
+  }
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  // Cooperative (its blocks wait on one another): as many blocks as the widest levels can use, at most
+  // what the device holds at once.
+  int dev = 0, sms = 0, per = 0;
+  if ((e = cudaGetDevice(&dev)) != cudaSuccess || (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess ||
+      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_collapse, kCollapseBlock, 0)) != cudaSuccess)
+    return e;
+  const uint32_t most = std::min<uint32_t>(kCollapseBlocksMax, (uint32_t)(sms * std::max(1, per)));
+  const uint32_t grid = std::max(1u, std::min(most, blocks(n, 4 * kCollapseBlock)));
+  uint32_t maxNodes = o.maxNodes, *bounds = b.bounds, nv = nverts;
+  int leaf = leafSize, depth = maxDepth, mark = o.markLeaves ? 1 : 0;
+  BuildBuffers ob = o;
+  BuildScratch sb = b;
+  void *args[] = {&t, &leaf, &depth, &maxNodes, &sb.levelA, &sb.levelB, &sb.children, &sb.packed, &sb.blockSums, &sb.bar,
+                  &ob.nodes, &ob.sorted, &faces, &verts, &nv, &ob.order, &ob.tris, &ob.nrm, &mark, &bounds, &sb.report, &status};
+  return cudaLaunchCooperativeKernel(k_collapse, dim3(grid), dim3(kCollapseBlock), args, 0, s);
+}
 
 }  // namespace
 
@@ -797,150 +1019,80 @@ vt_status vt_lbvh_build(vt_ctx *ctx, const vt_face *faces, uint32_t nfaces, cons
   if (treelet > kMaxTreelet) treelet = kMaxTreelet;
   if (treelet > 0 && treelet < 3) treelet = 3;
 
-  DeviceArena tmp;
-  float4 *boxes, *leafBox, *nodeBox;
-  uint32_t *bounds, *codes, *vals, *codesAlt, *valsAlt, *sortTemp, *flags, *count;
-  int2 *child;
-  int32_t *parent;
-  float *cost;
-  const uint32_t ni = n > 1 ? n - 1 : 1;
-  VT_CUDA(ctx, tmp.alloc(&boxes, 2 * (size_t)n));
-  VT_CUDA(ctx, tmp.alloc(&leafBox, 2 * (size_t)n));
-  VT_CUDA(ctx, tmp.alloc(&nodeBox, 2 * (size_t)ni));
-  VT_CUDA(ctx, tmp.alloc(&bounds, 16));
-  VT_CUDA(ctx, tmp.alloc(&codesAlt, n));
-  VT_CUDA(ctx, tmp.alloc(&valsAlt, n));
-  VT_CUDA(ctx, tmp.alloc(&sortTemp, vt_radix_temp_words(n)));
-  VT_CUDA(ctx, tmp.alloc(&flags, ni));
-  VT_CUDA(ctx, tmp.alloc(&count, ni));
-  VT_CUDA(ctx, tmp.alloc(&child, ni));
-  VT_CUDA(ctx, tmp.alloc(&parent, 2 * (size_t)n));
-  VT_CUDA(ctx, tmp.alloc(&cost, ni));
-  // Outputs kept by the mesh.
-  VT_CUDA(ctx, cudaMalloc(&mesh->d_codes, n * sizeof(uint32_t)));
-  VT_CUDA(ctx, cudaMalloc(&mesh->d_sorted, n * sizeof(int32_t)));
-  VT_CUDA(ctx, cudaMalloc(&mesh->d_order, n * sizeof(int32_t)));
-  VT_CUDA(ctx, cudaMalloc(&mesh->d_tris, 3 * (size_t)n * sizeof(float4)));
-  VT_CUDA(ctx, cudaMalloc(&mesh->d_nrm, 3 * (size_t)n * sizeof(float4)));
-  codes = mesh->d_codes;
-  vals = reinterpret_cast<uint32_t *>(mesh->d_sorted);
-
+  // Temporaries in one buffer of the context's pool, returned to it on every way out.
+  struct Temp {
+    cudaStream_t s;
+    void *p = nullptr;
+    ~Temp() {
+      if (p) cudaFreeAsync(p, s);
+    }
+  } temp{s};
+  ScratchCarve probe{nullptr};
+  BuildScratch b;
+  carve_build(probe, n, b);
+  VT_CUDA(ctx, vt_pool_alloc(ctx, &temp.p, probe.off));
+  ScratchCarve carve{static_cast<unsigned char *>(temp.p)};
+  carve_build(carve, n, b);
+  // Outputs kept by the mesh (the binary hierarchy for parity checks). The wide node count is bounded by
+  // the binary internal count (each wide inner node consumes at least one) plus the root.
+  const uint32_t ni = n > 1 ? n - 1 : 1, maxNodes = ni + 1;
+  auto keep = [&](auto **p, size_t count) { return vt_pool_alloc(ctx, reinterpret_cast<void **>(p), count * sizeof(**p)); };
+  VT_CUDA(ctx, keep(&mesh->d_codes, n));
+  VT_CUDA(ctx, keep(&mesh->d_sorted, n));
+  VT_CUDA(ctx, keep(&mesh->d_order, n));
+  VT_CUDA(ctx, keep(&mesh->d_tris, 3 * (size_t)n));
+  VT_CUDA(ctx, keep(&mesh->d_nrm, 3 * (size_t)n));
+  VT_CUDA(ctx, keep(&mesh->d_nodes, maxNodes));
+  VT_CUDA(ctx, keep(&mesh->d_bin_child, 2 * (size_t)ni));
+  VT_CUDA(ctx, keep(&mesh->d_bin_box, 8 * (size_t)ni));
+  const BuildBuffers o{mesh->d_codes, reinterpret_cast<uint32_t *>(mesh->d_sorted), reinterpret_cast<int2 *>(mesh->d_bin_child),
+                       reinterpret_cast<float4 *>(mesh->d_bin_box), mesh->d_nodes, maxNodes, mesh->d_order, mesh->d_tris,
+                       mesh->d_nrm, true};
   VT_CUDA(ctx, cudaEventRecord(ctx->ev0, s));
-  VT_CUDA(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(uint32_t), s));
-  k_init_bounds<<<1, 32, 0, s>>>(bounds);
-  k_face_boxes<<<blocks(n, 256), 256, 0, s>>>(faces, n, verts, nverts, boxes, bounds, ctx->d_status);
-  k_morton<<<blocks(n, 256), 256, 0, s>>>(boxes, n, bounds, codes, vals);
-  vt_radix_sort_pairs(codes, vals, codesAlt, valsAlt, n, 30, sortTemp, s);
-  k_leaf_boxes<<<blocks(n, 256), 256, 0, s>>>(boxes, vals, n, leafBox);
-  TreeView t{(int)n, child, parent, leafBox, nodeBox, count, cost};
-  if (n >= 2) {
-    k_karras<<<blocks(n - 1, 256), 256, 0, s>>>(codes, (int)n, child, parent);
-    VT_CUDA(ctx, cudaMemsetAsync(flags, 0, ni * sizeof(uint32_t), s));
-    k_bottom_up<<<blocks(n, 128), 128, 0, s>>>(t, flags, ctx->d_status);
-    if (treelet > 0 && n >= 3) {
-      for (int r = 0; r < rounds; ++r) {
-        VT_CUDA(ctx, cudaMemsetAsync(flags, 0, ni * sizeof(uint32_t), s));
-        k_restructure<<<blocks(n, 128), 128, 0, s>>>(t, flags, treelet, ctx->d_status);
-      }
-    }
+  VT_CUDA(ctx, queue_build(faces, n, verts, nverts, leafSize, treelet, rounds, maxDepth, o, b, ctx->d_status, s));
+  BuildReport r;
+  VT_CUDA(ctx, cudaMemcpyAsync(&r, b.report, sizeof r, cudaMemcpyDeviceToHost, s));
+  VT_CUDA(ctx, cudaStreamSynchronize(s));
+  if (!r.done) return vt_fail(ctx, VT_ERR_DEVICE, "the collapse's grid barrier timed out");
+  if (r.status & VT_DEV_SORT) return vt_fail(ctx, VT_ERR_DEVICE, "the Morton sort's look-back timed out");
+  if (r.status & VT_DEV_TREELET) return vt_fail(ctx, VT_ERR_DEVICE, "hierarchy inconsistency during the collapse");
+  if (r.status & VT_DEV_BAD_INDEX) return vt_fail(ctx, VT_ERR_INVALID, "a face indexes past the vertex array");
+  if (r.status & VT_DEV_NONFINITE) return vt_fail(ctx, VT_ERR_INVALID, "a vertex position is not finite");
+  if (r.code == kCollapseDepth)
+    return vt_fail(ctx, VT_ERR_LIMIT, "BVH depth exceeds max_depth (" + std::to_string(maxDepth) + ")");
+  if (r.code == kCollapseNodes) return vt_fail(ctx, VT_ERR_LIMIT, "wide node count exceeds its bound");
+  if (r.prims != n) return vt_fail(ctx, VT_ERR_DEVICE, "collapse emitted " + std::to_string(r.prims) + " of " + std::to_string(n) + " triangles");
+  mesh->nnodes = r.nodes;
+  mesh->depth = r.depth;
+  // A mesh without vertex normals shades with geometric normals: no normal buffer to read.
+  if (!(r.status & VT_DEV_NORMALS)) {
+    VT_CUDA(ctx, cudaFreeAsync(mesh->d_nrm, s));
+    mesh->d_nrm = nullptr;
   }
-  VT_CUDA(ctx, cudaGetLastError());
-
-  // Collapse, level by level. Per-level arrays are sized by the level (at most n wide nodes per
-  // level, fewer in practice); totals come back to the host to size the next level.
-  int32_t *levelA, *levelB;
-  int4 *chBuf;
-  uint32_t *nInner, *nPrims, *scanTemp, *totals;
-  VT_CUDA(ctx, tmp.alloc(&levelA, n));
-  VT_CUDA(ctx, tmp.alloc(&levelB, n));
-  VT_CUDA(ctx, tmp.alloc(&chBuf, n));
-  VT_CUDA(ctx, tmp.alloc(&nInner, n));
-  VT_CUDA(ctx, tmp.alloc(&nPrims, n));
-  VT_CUDA(ctx, tmp.alloc(&scanTemp, vt_scan_temp_words(n)));
-  VT_CUDA(ctx, tmp.alloc(&totals, 4));
-  // Wide node count is bounded by the binary internal count (each wide inner node consumes at
-  // least one binary internal node) plus the root.
-  const uint32_t maxNodes = ni + 1;
-  vt_wide_node *nodes;
-  VT_CUDA(ctx, cudaMalloc(&nodes, maxNodes * sizeof(vt_wide_node)));
-  mesh->d_nodes = nodes;
-  const int32_t rootRef = n >= 2 ? 0 : -1;
-  VT_CUDA(ctx, cudaMemcpyAsync(levelA, &rootRef, sizeof(int32_t), cudaMemcpyHostToDevice, s));
-  uint32_t L = 1, base = 0, primBase = 0, depth = 0;
-  uint32_t host_tot[2];
-  while (L > 0) {
-    ++depth;
-    if ((int)depth > maxDepth) {
-      return vt_fail(ctx, VT_ERR_LIMIT, "BVH depth exceeds max_depth (" + std::to_string(maxDepth) + ")");
-    }
-    k_collapse_count<<<blocks(L, 128), 128, 0, s>>>(t, levelA, L, leafSize, chBuf, nInner, nPrims);
-    vt_scan_exclusive(nInner, nInner, L, scanTemp, totals, s);
-    vt_scan_exclusive(nPrims, nPrims, L, scanTemp, totals + 1, s);
-    const uint32_t nextBase = base + L;
-    k_collapse_emit<<<blocks(L, 128), 128, 0, s>>>(t, L, leafSize, chBuf, nInner, nPrims, base,
-                                                   nextBase, primBase, nodes, levelB, vals, faces,
-                                                   verts, nverts, mesh->d_order, mesh->d_tris, ctx->d_status,
-                                                   mesh->d_nrm);
-    uint32_t st_level = 0;
-    VT_CUDA(ctx, cudaMemcpyAsync(host_tot, totals, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    VT_CUDA(ctx, cudaMemcpyAsync(&st_level, ctx->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    VT_CUDA(ctx, cudaStreamSynchronize(s));
-    if (st_level & VT_DEV_TREELET) return vt_fail(ctx, VT_ERR_DEVICE, "hierarchy inconsistency during the collapse");
-    if (st_level & (VT_DEV_BAD_INDEX | VT_DEV_NONFINITE)) break;
-    primBase += host_tot[1];
-    base = nextBase;
-    L = host_tot[0];
-    if (base + L > maxNodes) return vt_fail(ctx, VT_ERR_LIMIT, "wide node count exceeds its bound");
-    int32_t *x = levelA; levelA = levelB; levelB = x;
+  if (n < 2) {  // no binary hierarchy
+    VT_CUDA(ctx, cudaFreeAsync(mesh->d_bin_child, s));
+    VT_CUDA(ctx, cudaFreeAsync(mesh->d_bin_box, s));
+    mesh->d_bin_child = nullptr;
+    mesh->d_bin_box = nullptr;
   }
-  mesh->nnodes = base;
-  mesh->depth = depth;
-  {
-    uint32_t st0 = 0;
-    VT_CUDA(ctx, cudaMemcpy(&st0, ctx->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost));
-    if (st0 & VT_DEV_BAD_INDEX) return vt_fail(ctx, VT_ERR_INVALID, "a face indexes past the vertex array");
-    if (st0 & VT_DEV_NONFINITE) return vt_fail(ctx, VT_ERR_INVALID, "a vertex position is not finite");
-    // A mesh without vertex normals shades with geometric normals: no normal buffer to read.
-    if (!(st0 & VT_DEV_NORMALS)) {
-      VT_CUDA(ctx, cudaFree(mesh->d_nrm));
-      mesh->d_nrm = nullptr;
-    }
-  }
-  if (primBase != n) return vt_fail(ctx, VT_ERR_DEVICE, "collapse emitted " + std::to_string(primBase) + " of " + std::to_string(n) + " triangles");
-
   {
     const vt_status qs = vt_quantize_nodes(ctx, mesh, s);
     if (qs != VT_OK) return qs;
   }
-  // Keep the refined binary tree for parity checks.
-  if (n >= 2) {
-    VT_CUDA(ctx, cudaMalloc(&mesh->d_bin_child, 2 * (size_t)(n - 1) * sizeof(int32_t)));
-    VT_CUDA(ctx, cudaMalloc(&mesh->d_bin_box, 8 * (size_t)(n - 1) * sizeof(float)));
-    VT_CUDA(ctx, cudaMemcpyAsync(mesh->d_bin_child, child, 2 * (size_t)(n - 1) * sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
-    VT_CUDA(ctx, cudaMemcpyAsync(mesh->d_bin_box, nodeBox, 8 * (size_t)(n - 1) * sizeof(float), cudaMemcpyDeviceToDevice, s));
-  }
-  double *sah;
-  VT_CUDA(ctx, tmp.alloc(&sah, 1));
-  VT_CUDA(ctx, cudaMemsetAsync(sah, 0, sizeof(double), s));
-  k_sah<<<blocks(mesh->nnodes, 256), 256, 0, s>>>(nodes, mesh->nnodes, sah);
+  VT_CUDA(ctx, cudaMemsetAsync(b.sah, 0, sizeof(double), s));
+  k_sah<<<blocks(mesh->nnodes, 256), 256, 0, s>>>(mesh->d_nodes, mesh->nnodes, b.sah);
   VT_CUDA(ctx, cudaEventRecord(ctx->ev1, s));
-  uint32_t hb[12], status = 0;
   double hsah = 0.0;
-  VT_CUDA(ctx, cudaMemcpyAsync(hb, bounds + 0, 12 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  VT_CUDA(ctx, cudaMemcpyAsync(&status, ctx->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  VT_CUDA(ctx, cudaMemcpyAsync(&hsah, sah, sizeof(double), cudaMemcpyDeviceToHost, s));
+  VT_CUDA(ctx, cudaMemcpyAsync(&hsah, b.sah, sizeof(double), cudaMemcpyDeviceToHost, s));
   VT_CUDA(ctx, cudaStreamSynchronize(s));
-  if (status & VT_DEV_BAD_INDEX) return vt_fail(ctx, VT_ERR_INVALID, "a face indexes past the vertex array");
-  if (status & VT_DEV_NONFINITE) return vt_fail(ctx, VT_ERR_INVALID, "a vertex position is not finite");
-  if (status & VT_DEV_TREELET) return vt_fail(ctx, VT_ERR_DEVICE, "treelet restructuring inconsistency");
   float ms = 0.0f;
   cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
   mesh->build_ms = ms;
   mesh->sah = (float)hsah;
   float m = 0.0f;
   for (int k = 0; k < 3; ++k) {
-    mesh->lo[k] = ord2f(hb[6 + k]);
-    mesh->hi[k] = ord2f(hb[9 + k]);
+    mesh->lo[k] = ord2f(r.bounds[6 + k]);
+    mesh->hi[k] = ord2f(r.bounds[9 + k]);
     m = fmaxf(m, fmaxf(fabsf(mesh->lo[k]), fabsf(mesh->hi[k])));
   }
   mesh->root_max = m;
@@ -958,9 +1110,9 @@ vt_status vt_lbvh_build(vt_ctx *ctx, const vt_face *faces, uint32_t nfaces, cons
 // library holds until the process exits. It fits VT_NOALLOC_MAX_FACES faces; larger meshes are
 // rejected. The first call on a device looks the array's address up (cudaGetSymbolAddress, with
 // that device current) and caches it, so that first call should come before any stream capture.
-// Every call blocks the host until its build has finished: it synchronises its stream once per
-// collapse level (the level's node count sizes the next launch) and at the end, and on an error
-// after its first launch it still waits for the work it queued before returning.
+// Every call blocks the host until its build has finished: it synchronises its stream after the
+// collapse (for the node count) and at the end, and on an error after its first launch it still
+// waits for the work it queued before returning.
 // All calls share the one array and find the previous call's contents in it: every region the
 // build needs zeroed is cleared on the call's stream, and two calls overlapping on the GPU (other
 // streams or other host threads) race on it.
@@ -977,56 +1129,22 @@ constexpr int kNoAllocMaxDevices = 64;
 std::mutex g_scratch_mutex;
 unsigned char *g_scratch_addr[kNoAllocMaxDevices] = {};
 
-// Bump allocator over the scratch array (256-byte aligned regions). With base == nullptr it only
-// measures.
-struct ScratchCarve {
-  unsigned char *base;
-  size_t off = 0;
-  template <typename T> T *take(size_t count) {
-    size_t bytes = (count * sizeof(T) + 16 + 255) & ~size_t(255);
-    T *p = base ? reinterpret_cast<T *>(base + off) : nullptr;
-    off += bytes;
-    return p;
-  }
-};
-
 struct NoAllocBuffers {
-  float4 *boxes, *leafBox, *nodeBox;
-  uint32_t *bounds, *codes, *vals, *codesAlt, *valsAlt, *sortTemp, *flags, *count, *status;
+  BuildScratch scratch;
+  float4 *nodeBox;
   int2 *child;
-  int32_t *parent, *levelA, *levelB;
-  float *cost;
-  int4 *chBuf;
-  uint32_t *nInner, *nPrims, *scanTemp, *totals;
-  double *sah;
+  uint32_t *codes, *vals, *status;
 };
 
 size_t carve_noalloc(unsigned char *base, uint32_t n, NoAllocBuffers &b) {
   ScratchCarve c{base};
   const uint32_t ni = n > 1 ? n - 1 : 1;
-  b.boxes = c.take<float4>(2 * (size_t)n);
-  b.leafBox = c.take<float4>(2 * (size_t)n);
+  carve_build(c, n, b.scratch);
   b.nodeBox = c.take<float4>(2 * (size_t)ni);
-  b.bounds = c.take<uint32_t>(16);
+  b.child = c.take<int2>(ni);
   b.codes = c.take<uint32_t>(n);
   b.vals = c.take<uint32_t>(n);
-  b.codesAlt = c.take<uint32_t>(n);
-  b.valsAlt = c.take<uint32_t>(n);
-  b.sortTemp = c.take<uint32_t>(vt_radix_temp_words(n));
-  b.flags = c.take<uint32_t>(ni);
-  b.count = c.take<uint32_t>(ni);
-  b.child = c.take<int2>(ni);
-  b.parent = c.take<int32_t>(2 * (size_t)n);
-  b.cost = c.take<float>(ni);
-  b.levelA = c.take<int32_t>(n);
-  b.levelB = c.take<int32_t>(n);
-  b.chBuf = c.take<int4>(n);
-  b.nInner = c.take<uint32_t>(n);
-  b.nPrims = c.take<uint32_t>(n);
-  b.scanTemp = c.take<uint32_t>(vt_scan_temp_words(n));
-  b.totals = c.take<uint32_t>(4);
   b.status = c.take<uint32_t>(4);
-  b.sah = c.take<double>(1);
   return c.off;
 }
 
@@ -1100,77 +1218,41 @@ extern "C" vt_status vt_mesh_build_noalloc(const vt_face *faces, uint32_t nfaces
   NoAllocBuffers b;
   carve_noalloc(scratch, nfaces, b);
 
-  const uint32_t n = nfaces, ni = n > 1 ? n - 1 : 1;
+  const uint32_t n = nfaces;
 #define VT_NA(call)                                                                  \
   do {                                                                               \
     cudaError_t _e = (call);                                                         \
     if (_e != cudaSuccess) return fail(VT_ERR_CUDA, std::string(#call ": ") + cudaGetErrorString(_e)); \
   } while (0)
   queued = true;
-  VT_NA(cudaMemsetAsync(b.status, 0, 4 * sizeof(uint32_t), s));
-  k_init_bounds<<<1, 32, 0, s>>>(b.bounds);
-  k_face_boxes<<<blocks(n, 256), 256, 0, s>>>(faces, n, verts, nverts, b.boxes, b.bounds, b.status);
-  k_morton<<<blocks(n, 256), 256, 0, s>>>(b.boxes, n, b.bounds, b.codes, b.vals);
-  vt_radix_sort_pairs(b.codes, b.vals, b.codesAlt, b.valsAlt, n, 30, b.sortTemp, s);
-  k_leaf_boxes<<<blocks(n, 256), 256, 0, s>>>(b.boxes, b.vals, n, b.leafBox);
-  TreeView t{(int)n, b.child, b.parent, b.leafBox, b.nodeBox, b.count, b.cost};
-  if (n >= 2) {
-    k_karras<<<blocks(n - 1, 256), 256, 0, s>>>(b.codes, (int)n, b.child, b.parent);
-    VT_NA(cudaMemsetAsync(b.flags, 0, ni * sizeof(uint32_t), s));
-    k_bottom_up<<<blocks(n, 128), 128, 0, s>>>(t, b.flags, b.status);
-    if (treelet > 0 && n >= 3) {
-      for (int r = 0; r < rounds; ++r) {
-        VT_NA(cudaMemsetAsync(b.flags, 0, ni * sizeof(uint32_t), s));
-        k_restructure<<<blocks(n, 128), 128, 0, s>>>(t, b.flags, treelet, b.status);
-      }
-    }
-  }
+  const BuildBuffers out{b.codes, b.vals, b.child, b.nodeBox, nodes, nodes_capacity, order, reinterpret_cast<float4 *>(tris), nullptr, false};
+  VT_NA(queue_build(faces, n, verts, nverts, leafSize, treelet, rounds, maxDepth, out, b.scratch, b.status, s));
+  BuildReport r;
+  VT_NA(cudaMemcpyAsync(&r, b.scratch.report, sizeof r, cudaMemcpyDeviceToHost, s));
+  VT_NA(cudaStreamSynchronize(s));
+  if (!r.done) return fail(VT_ERR_DEVICE, "vt_mesh_build_noalloc: the collapse's grid barrier timed out");
+  if (r.status & VT_DEV_SORT) return fail(VT_ERR_DEVICE, "vt_mesh_build_noalloc: the Morton sort's look-back timed out");
+  if (r.status & VT_DEV_BAD_INDEX) return fail(VT_ERR_INVALID, "vt_mesh_build_noalloc: a face indexes past the vertex array");
+  if (r.status & VT_DEV_NONFINITE) return fail(VT_ERR_INVALID, "vt_mesh_build_noalloc: a vertex position is not finite");
+  if (r.status & VT_DEV_TREELET) return fail(VT_ERR_DEVICE, "vt_mesh_build_noalloc: hierarchy inconsistency");
+  if (r.code == kCollapseDepth) return fail(VT_ERR_LIMIT, "vt_mesh_build_noalloc: BVH depth exceeds max_depth");
+  if (r.code == kCollapseNodes) return fail(VT_ERR_LIMIT, "vt_mesh_build_noalloc: wide nodes exceed nodes_capacity");
+  if (r.prims != n) return fail(VT_ERR_DEVICE, "vt_mesh_build_noalloc: collapse emitted too few triangles");
+  VT_NA(cudaMemsetAsync(b.scratch.sah, 0, sizeof(double), s));
+  k_sah<<<blocks(r.nodes, 256), 256, 0, s>>>(nodes, r.nodes, b.scratch.sah);
   VT_NA(cudaGetLastError());
-  // Root reference of the first level: binary node 0, or leaf 0 (-1, all bits set) for one face.
-  VT_NA(cudaMemsetAsync(b.levelA, n >= 2 ? 0 : 0xff, sizeof(int32_t), s));
-  uint32_t L = 1, base = 0, primBase = 0, depth = 0;
-  int32_t *levelA = b.levelA, *levelB = b.levelB;
-  while (L > 0) {
-    ++depth;
-    if ((int)depth > maxDepth) return fail(VT_ERR_LIMIT, "vt_mesh_build_noalloc: BVH depth exceeds max_depth");
-    k_collapse_count<<<blocks(L, 128), 128, 0, s>>>(t, levelA, L, leafSize, b.chBuf, b.nInner, b.nPrims);
-    vt_scan_exclusive(b.nInner, b.nInner, L, b.scanTemp, b.totals, s);
-    vt_scan_exclusive(b.nPrims, b.nPrims, L, b.scanTemp, b.totals + 1, s);
-    const uint32_t nextBase = base + L;
-    k_collapse_emit<<<blocks(L, 128), 128, 0, s>>>(t, L, leafSize, b.chBuf, b.nInner, b.nPrims, base, nextBase,
-                                                   primBase, nodes, levelB, b.vals, faces, verts, nverts, order,
-                                                   reinterpret_cast<float4 *>(tris), b.status);
-    uint32_t tot[2] = {0, 0}, st = 0;
-    VT_NA(cudaMemcpyAsync(tot, b.totals, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    VT_NA(cudaMemcpyAsync(&st, b.status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    VT_NA(cudaStreamSynchronize(s));
-    if (st & VT_DEV_BAD_INDEX) return fail(VT_ERR_INVALID, "vt_mesh_build_noalloc: a face indexes past the vertex array");
-    if (st & VT_DEV_NONFINITE) return fail(VT_ERR_INVALID, "vt_mesh_build_noalloc: a vertex position is not finite");
-    if (st & VT_DEV_TREELET) return fail(VT_ERR_DEVICE, "vt_mesh_build_noalloc: hierarchy inconsistency");
-    primBase += tot[1];
-    base = nextBase;
-    L = tot[0];
-    if (base + L > nodes_capacity) return fail(VT_ERR_LIMIT, "vt_mesh_build_noalloc: wide nodes exceed nodes_capacity");
-    int32_t *x = levelA; levelA = levelB; levelB = x;
-  }
-  if (primBase != n) return fail(VT_ERR_DEVICE, "vt_mesh_build_noalloc: collapse emitted too few triangles");
-  VT_NA(cudaMemsetAsync(b.sah, 0, sizeof(double), s));
-  k_sah<<<blocks(base, 256), 256, 0, s>>>(nodes, base, b.sah);
-  VT_NA(cudaGetLastError());
-  uint32_t hb[12];
   double hsah = 0.0;
-  VT_NA(cudaMemcpyAsync(hb, b.bounds, 12 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  VT_NA(cudaMemcpyAsync(&hsah, b.sah, sizeof(double), cudaMemcpyDeviceToHost, s));
+  VT_NA(cudaMemcpyAsync(&hsah, b.scratch.sah, sizeof(double), cudaMemcpyDeviceToHost, s));
   VT_NA(cudaStreamSynchronize(s));
 #undef VT_NA
   info->faces = n;
-  info->wide_nodes = base;
+  info->wide_nodes = r.nodes;
   info->binary_nodes = n - 1;
-  info->depth = depth;
+  info->depth = r.depth;
   info->sah_cost = (float)hsah;
   for (int k = 0; k < 3; ++k) {
-    info->lo[k] = ord2f(hb[6 + k]);
-    info->hi[k] = ord2f(hb[9 + k]);
+    info->lo[k] = ord2f(r.bounds[6 + k]);
+    info->hi[k] = ord2f(r.bounds[9 + k]);
   }
   info->build_ms = std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t_start).count();
   return VT_OK;

@@ -5,7 +5,7 @@
 // Through Compressed Wide BVHs", HPG 2017, restated for 4 children): the node's box origin p (its
 // children's union lower corner), a power-of-two step 2^e per axis, and per child and axis the
 // bytes qlo = floor((lo - p) / 2^e) and qhi = ceil((hi - p) / 2^e), so that p + qlo 2^e <= lo and
-// p + qhi 2^e >= hi exactly: each decoded box contains the child's box. Child links and leaf counts
+// p + qhi 2^e >= hi exactly: each decoded box contains the child's box. Child links
 // become traversal stack entries. A node is two 32-byte loads instead of four.
 //
 // Layout (16 words): p.x p.y p.z | steps 2^(e + 15) of x and y as bfloat16 halves (so one shift or mask
@@ -81,10 +81,8 @@ __global__ void k_quantize(const vt_wide_node *__restrict__ in, uint32_t n, vt_q
 }  // namespace
 
 vt_status vt_quantize_nodes(vt_ctx *ctx, vt_mesh *mesh, cudaStream_t s) {
-  cudaFree(mesh->d_qnodes);
-  mesh->d_qnodes = nullptr;
   if (mesh->nnodes == 0) return VT_OK;
-  VT_CUDA(ctx, cudaMalloc(&mesh->d_qnodes, mesh->nnodes * sizeof(vt_qnode)));
+  VT_CUDA(ctx, vt_pool_alloc(ctx, reinterpret_cast<void **>(&mesh->d_qnodes), mesh->nnodes * sizeof(vt_qnode)));
   k_quantize<<<(mesh->nnodes + 255) / 256, 256, 0, s>>>(mesh->d_nodes, mesh->nnodes, mesh->d_qnodes);
   VT_CUDA(ctx, cudaGetLastError());
   return VT_OK;

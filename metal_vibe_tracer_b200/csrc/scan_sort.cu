@@ -1,211 +1,173 @@
-// scan_sort.cu — device prefix sums and the stable LSD radix sort of the LBVH build.
+// scan_sort.cu — the stable LSD radix sort of the LBVH build.
 //
-// Both are HBM-bound integer passes: the scan reads and writes each word once per level; the
-// sort makes one histogram pass and one scatter pass per 4-bit digit over (key, value) pairs,
-// each thread owning 16 consecutive pairs (four 16-byte loads) so a tile is one contiguous 16 KB
-// read. Stability comes from the blocked arrangement: a tile's pairs are ranked by (digit,
-// thread, item), the order they appear in memory.
+// Bound: HBM, or launches for small inputs. One pass over the keys counts the digits of every pass; then
+// each 8-bit digit takes one launch that reads and writes the pairs once (four passes for 30-bit Morton
+// codes): the tiles' running digit offsets come from a decoupled look-back over the tiles before it
+// instead of a histogram launch, a scan and a scatter per digit. Within a tile the pairs are ranked
+// by (digit, warp, item, lane), the order they appear in memory, so the sort is stable, and are
+// reordered in shared memory so that each digit's run is stored contiguously. Eight 4-bit passes of
+// histogram, scan and scatter launches took 391 us for 1M pairs (44 launches) before.
 #include "vt_internal.cuh"
 
 namespace {
 
-constexpr int kScanThreads = 256;
-constexpr int kScanItems = 4;
-constexpr int kScanTile = kScanThreads * kScanItems;  // 1024 words per block
+constexpr int kSortThreads = 256;
+constexpr int kSortWarps = kSortThreads / 32;
+constexpr int kSortItems = 12;
+constexpr int kSortTile = kSortThreads * kSortItems;  // 3072 pairs per tile
+constexpr int kDigits = 256;
+constexpr int kMaxPasses = 4;
+// Tile states of the look-back, in the two top bits of a word whose low bits hold a count (pairs
+// number fewer than 2^30).
+constexpr uint32_t kPartial = 1u << 30, kPrefix = 2u << 30, kCountMask = kPartial - 1u;
+// Look-back polls before a tile gives up (a tile's predecessors have all started, so this is never
+// reached unless a launch is broken); the sort then reports VT_DEV_SORT.
+constexpr uint32_t kSpinLimit = 1u << 21;
 
-__device__ __forceinline__ uint32_t warp_inclusive_scan(uint32_t v) {
-  const int lane = threadIdx.x & 31;
+// Temporary words: digit counts of each pass, tile tickets, then the tile states of each pass.
+constexpr uint32_t kTicketAt = kMaxPasses * kDigits, kStateAt = kTicketAt + 64;
+
+__device__ __forceinline__ uint32_t digit_of(uint32_t key, int shift) { return (key >> shift) & (kDigits - 1); }
+
+__global__ void __launch_bounds__(kSortThreads) k_radix_count(const uint32_t *__restrict__ keys, uint32_t n, int passes,
+                                                                uint32_t *temp) {
+  __shared__ uint32_t cnt[kMaxPasses][kDigits];
+  for (int p = 0; p < passes; ++p) cnt[p][threadIdx.x] = 0;
+  __syncthreads();
+  for (uint32_t i = blockIdx.x * kSortThreads + threadIdx.x; i < n; i += gridDim.x * kSortThreads) {
+    const uint32_t k = keys[i];
+    for (int p = 0; p < passes; ++p) atomicAdd(&cnt[p][digit_of(k, 8 * p)], 1u);
+  }
+  __syncthreads();
+  for (int p = 0; p < passes; ++p)
+    if (cnt[p][threadIdx.x]) atomicAdd(temp + p * kDigits + threadIdx.x, cnt[p][threadIdx.x]);
+}
+
+// Exclusive prefix over the block of one value per thread.
+__device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t *warpSums) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t inc = v;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    uint32_t u = __shfl_up_sync(0xffffffffu, v, o);
-    if (lane >= o) v += u;
+    const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += u;
   }
-  return v;
-}
-
-// Block-wide exclusive scan of one value per thread (blockDim.x == 256). Returns the exclusive
-// prefix; *total receives the block sum.
-__device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *total) {
-  __shared__ uint32_t warp_sums[kScanThreads / 32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t inc = warp_inclusive_scan(v);
-  if (lane == 31) warp_sums[warp] = inc;
+  if (lane == 31) warpSums[warp] = inc;
   __syncthreads();
-  if (warp == 0) {
-    uint32_t w = lane < kScanThreads / 32 ? warp_sums[lane] : 0u;
-    uint32_t wi = warp_inclusive_scan(w);
-    if (lane < kScanThreads / 32) warp_sums[lane] = wi - w;
+  uint32_t before = 0;
+#pragma unroll
+  for (int w = 0; w < kSortWarps; ++w) before += w < warp ? warpSums[w] : 0u;
+  __syncthreads();
+  return before + inc - v;
+}
+
+__global__ void __launch_bounds__(kSortThreads) k_radix_pass(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ vals,
+                                                               uint32_t n, int pass, uint32_t *temp, uint32_t tiles,
+                                                               uint32_t *__restrict__ keysOut, uint32_t *__restrict__ valsOut,
+                                                               uint32_t *status) {
+  __shared__ uint32_t cnt[kSortWarps][kDigits];  // per warp: running digit counts, then offsets in the tile
+  __shared__ uint32_t sKeys[kSortTile], sVals[kSortTile];
+  __shared__ uint32_t out[kDigits];              // destination of a digit's run minus its place in the tile
+  __shared__ uint32_t warpSums[kSortWarps];
+  __shared__ uint32_t sTile;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, shift = 8 * pass;
+  if (t == 0) sTile = atomicAdd(temp + kTicketAt + pass, 1u);  // tiles in the order they start
+#pragma unroll
+  for (int w = 0; w < kSortWarps; ++w) cnt[w][t] = 0;
+  __syncthreads();
+  const uint32_t tile = sTile, base = tile * kSortTile, valid = min((uint32_t)kSortTile, n - base);
+  // Item j of lane l of warp w is pair (w * items + j) * 32 + l of the tile.
+  uint32_t key[kSortItems], val[kSortItems];
+#pragma unroll
+  for (int j = 0; j < kSortItems; ++j) {
+    const uint32_t at = (uint32_t)(warp * kSortItems + j) * 32u + lane;
+    key[j] = at < valid ? keys[base + at] : 0xffffffffu;
+    val[j] = at < valid ? vals[base + at] : 0u;
+  }
+  uint32_t rank[kSortItems];
+#pragma unroll
+  for (int j = 0; j < kSortItems; ++j) {
+    const bool in = (uint32_t)(warp * kSortItems + j) * 32u + lane < valid;
+    const uint32_t d = digit_of(key[j], shift);
+    const unsigned peers = __match_any_sync(0xffffffffu, in ? d : kDigits);  // past-the-end lanes among themselves
+    const uint32_t before = __popc(peers & ((1u << lane) - 1u));
+    rank[j] = in ? cnt[warp][d] + before : 0u;
+    __syncwarp();
+    if (in && before == 0) cnt[warp][d] += __popc(peers);
+    __syncwarp();
   }
   __syncthreads();
-  uint32_t out = warp_sums[warp] + inc - v;
-  if (total) {
-    __shared__ uint32_t tot;
-    if (threadIdx.x == kScanThreads - 1) tot = out + v;
-    __syncthreads();
-    *total = tot;
-  }
-  return out;
-}
-
-__global__ void __launch_bounds__(kScanThreads) k_scan_block(const uint32_t *in, uint32_t *out,
-                                                               uint32_t n, uint32_t *block_sums) {
-  const uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-  uint32_t v[kScanItems];
-  uint32_t sum = 0;
+  // Thread d owns digit d: the warps' counts become offsets, their sum the tile's count.
+  uint32_t total = 0;
 #pragma unroll
-  for (int k = 0; k < kScanItems; ++k) {
-    v[k] = base + k < n ? in[base + k] : 0u;
-    sum += v[k];
+  for (int w = 0; w < kSortWarps; ++w) {
+    const uint32_t c = cnt[w][t];
+    cnt[w][t] = total;
+    total += c;
   }
-  uint32_t total;
-  uint32_t prefix = block_exclusive_scan(sum, &total);
-#pragma unroll
-  for (int k = 0; k < kScanItems; ++k) {
-    if (base + k < n) out[base + k] = prefix;
-    prefix += v[k];
-  }
-  if (threadIdx.x == 0) block_sums[blockIdx.x] = total;
-}
-
-__global__ void k_scan_add(uint32_t *out, uint32_t n, const uint32_t *block_prefix) {
-  const uint32_t add = block_prefix[blockIdx.x];
-  const uint32_t base = blockIdx.x * kScanTile;
-  for (uint32_t k = threadIdx.x; k < kScanTile; k += blockDim.x)
-    if (base + k < n) out[base + k] += add;
-}
-
-__global__ void k_copy_word(const uint32_t *src, uint32_t *dst) { *dst = *src; }
-
-// ---- radix sort ------------------------------------------------------------------------------
-constexpr int kSortThreads = 256;
-constexpr int kSortItems = 16;
-constexpr int kSortTile = kSortThreads * kSortItems;  // 4096 pairs per block
-constexpr int kDigits = 16;
-
-__device__ __forceinline__ void load_tile(const uint32_t *src, uint32_t base, uint32_t n,
-                                          uint32_t (&v)[kSortItems]) {
-  if (base + kSortItems <= n) {
-    const uint4 *p = reinterpret_cast<const uint4 *>(src + base);
-#pragma unroll
-    for (int q = 0; q < kSortItems / 4; ++q) {
-      uint4 x = p[q];
-      v[4 * q] = x.x; v[4 * q + 1] = x.y; v[4 * q + 2] = x.z; v[4 * q + 3] = x.w;
+  uint32_t *state = temp + kStateAt + ((size_t)pass * tiles + tile) * kDigits + t;
+  atomicExch(state, (tile == 0 ? kPrefix : kPartial) | total);
+  const uint32_t start = block_exclusive(total, warpSums);                           // the digit's place in the tile
+  const uint32_t first = block_exclusive(__ldcg(temp + pass * kDigits + t), warpSums);  // and in the output
+  // Pairs of this digit in the tiles before this one.
+  uint32_t before = 0;
+  for (uint32_t p = tile; p > 0;) {
+    uint32_t s = 0, spins = 0;
+    do {
+      s = vt_poll(temp + kStateAt + ((size_t)pass * tiles + (p - 1)) * kDigits + t);
+    } while ((s & ~kCountMask) == 0u && ++spins < kSpinLimit);
+    if ((s & ~kCountMask) == 0u) {
+      atomicOr(status, (uint32_t)VT_DEV_SORT);
+      break;
     }
-  } else {
-#pragma unroll
-    for (int k = 0; k < kSortItems; ++k) v[k] = base + k < n ? src[base + k] : 0u;
+    before += s & kCountMask;
+    if (s & kPrefix) break;
+    --p;
   }
-}
-
-__global__ void __launch_bounds__(kSortThreads) k_radix_hist(const uint32_t *keys, uint32_t n,
-                                                               int shift, uint32_t *hist,
-                                                               uint32_t nblocks) {
-  __shared__ uint32_t cnt[kDigits];
-  if (threadIdx.x < kDigits) cnt[threadIdx.x] = 0;
-  __syncthreads();
-  const uint32_t base = blockIdx.x * kSortTile + threadIdx.x * kSortItems;
-  uint32_t k[kSortItems];
-  load_tile(keys, base, n, k);
+  if (tile > 0) atomicExch(state, kPrefix | (before + total));
+  out[t] = first + before - start;
 #pragma unroll
-  for (int i = 0; i < kSortItems; ++i)
-    if (base + i < n) atomicAdd(&cnt[(k[i] >> shift) & (kDigits - 1)], 1u);
-  __syncthreads();
-  if (threadIdx.x < kDigits) hist[threadIdx.x * nblocks + blockIdx.x] = cnt[threadIdx.x];
-}
-
-__global__ void __launch_bounds__(kSortThreads) k_radix_scatter(
-    const uint32_t *keys, const uint32_t *vals, uint32_t n, int shift, const uint32_t *offsets,
-    uint32_t nblocks, uint32_t *keys_out, uint32_t *vals_out) {
-  __shared__ uint32_t cnt[kDigits][kSortThreads];
-  __shared__ uint32_t dstart[kDigits], goff[kDigits];
-  const int t = threadIdx.x;
-#pragma unroll
-  for (int d = 0; d < kDigits; ++d) cnt[d][t] = 0;
-  const uint32_t base = blockIdx.x * kSortTile + t * kSortItems;
-  uint32_t k[kSortItems], v[kSortItems];
-  load_tile(keys, base, n, k);
-  load_tile(vals, base, n, v);
-  // Column t of cnt is private to thread t here.
-#pragma unroll
-  for (int i = 0; i < kSortItems; ++i)
-    if (base + i < n) cnt[(k[i] >> shift) & (kDigits - 1)][t] += 1u;
-  __syncthreads();
-  // Exclusive scan of cnt in digit-major order: thread t owns the 16 consecutive entries of row
-  // t / 16, columns (t % 16) * 16 ...
-  const int row = t / 16, col0 = (t % 16) * 16;
-  uint32_t local[16];
-  uint32_t sum = 0;
-#pragma unroll
-  for (int j = 0; j < 16; ++j) { local[j] = cnt[row][col0 + j]; sum += local[j]; }
-  uint32_t prefix = block_exclusive_scan(sum, nullptr);
+  for (int w = 0; w < kSortWarps; ++w) cnt[w][t] += start;
   __syncthreads();
 #pragma unroll
-  for (int j = 0; j < 16; ++j) { cnt[row][col0 + j] = prefix; prefix += local[j]; }
-  __syncthreads();
-  if (t < kDigits) {
-    dstart[t] = cnt[t][0];
-    goff[t] = offsets[t * nblocks + blockIdx.x];
+  for (int j = 0; j < kSortItems; ++j) {
+    if ((uint32_t)(warp * kSortItems + j) * 32u + lane >= valid) continue;
+    const uint32_t at = cnt[warp][digit_of(key[j], shift)] + rank[j];
+    sKeys[at] = key[j];
+    sVals[at] = val[j];
   }
   __syncthreads();
-#pragma unroll
-  for (int i = 0; i < kSortItems; ++i) {
-    if (base + i >= n) break;
-    const int d = (k[i] >> shift) & (kDigits - 1);
-    const uint32_t pos = goff[d] + (cnt[d][t] - dstart[d]);
-    cnt[d][t] += 1u;
-    keys_out[pos] = k[i];
-    vals_out[pos] = v[i];
+  for (uint32_t at = t; at < valid; at += kSortThreads) {
+    const uint32_t k = sKeys[at], to = out[digit_of(k, shift)] + at;
+    if (to < n) {  // holds unless a look-back gave up
+      keysOut[to] = k;
+      valsOut[to] = sVals[at];
+    }
   }
 }
 
 }  // namespace
 
-size_t vt_scan_temp_words(uint32_t n) {
-  size_t words = 4;
-  while (n > 1) {
-    n = (n + kScanTile - 1) / kScanTile;
-    words += n;
-  }
-  return words;
-}
-
-void vt_scan_exclusive(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *temp,
-                       uint32_t *total_dev, cudaStream_t s) {
-  if (n == 0) return;
-  const uint32_t nb = (n + kScanTile - 1) / kScanTile;
-  uint32_t *sums = temp;
-  k_scan_block<<<nb, kScanThreads, 0, s>>>(in, out, n, sums);
-  if (nb > 1) {
-    vt_scan_exclusive(sums, sums, nb, temp + nb, total_dev, s);
-    k_scan_add<<<nb, kScanThreads, 0, s>>>(out, n, sums);
-  } else if (total_dev) {
-    k_copy_word<<<1, 1, 0, s>>>(sums, total_dev);
-  }
-}
-
 size_t vt_radix_temp_words(uint32_t n) {
-  const uint32_t nb = (n + kSortTile - 1) / kSortTile;
-  return (size_t)kDigits * nb + vt_scan_temp_words(kDigits * nb) + 4;
+  const size_t tiles = ((size_t)n + kSortTile - 1) / kSortTile;
+  return kStateAt + (size_t)kMaxPasses * tiles * kDigits;
 }
 
 void vt_radix_sort_pairs(uint32_t *keys, uint32_t *vals, uint32_t *keys_alt, uint32_t *vals_alt,
-                         uint32_t n, int bits, uint32_t *temp, cudaStream_t s) {
+                         uint32_t n, int bits, uint32_t *temp, uint32_t *status, cudaStream_t s) {
   if (n <= 1) return;
-  const uint32_t nb = (n + kSortTile - 1) / kSortTile;
-  uint32_t *hist = temp;
-  uint32_t *scan_temp = temp + (size_t)kDigits * nb;
-  uint32_t *src_k = keys, *src_v = vals, *dst_k = keys_alt, *dst_v = vals_alt;
-  int passes = (bits + 3) / 4;
+  const uint32_t tiles = (n + kSortTile - 1) / kSortTile;
+  const int passes = (bits + 7) / 8;
+  cudaMemsetAsync(temp, 0, (kStateAt + (size_t)passes * tiles * kDigits) * sizeof(uint32_t), s);
+  k_radix_count<<<tiles < 592u ? tiles : 592u, kSortThreads, 0, s>>>(keys, n, passes, temp);
+  uint32_t *srcK = keys, *srcV = vals, *dstK = keys_alt, *dstV = vals_alt;
   for (int p = 0; p < passes; ++p) {
-    const int shift = 4 * p;
-    k_radix_hist<<<nb, kSortThreads, 0, s>>>(src_k, n, shift, hist, nb);
-    vt_scan_exclusive(hist, hist, kDigits * nb, scan_temp, nullptr, s);
-    k_radix_scatter<<<nb, kSortThreads, 0, s>>>(src_k, src_v, n, shift, hist, nb, dst_k, dst_v);
-    uint32_t *tk = src_k, *tv = src_v;
-    src_k = dst_k; src_v = dst_v; dst_k = tk; dst_v = tv;
+    k_radix_pass<<<tiles, kSortThreads, 0, s>>>(srcK, srcV, n, p, temp, tiles, dstK, dstV, status);
+    uint32_t *tk = srcK, *tv = srcV;
+    srcK = dstK; srcV = dstV; dstK = tk; dstV = tv;
   }
-  if (src_k != keys) {
-    cudaMemcpyAsync(keys, src_k, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s);
-    cudaMemcpyAsync(vals, src_v, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s);
+  if (srcK != keys) {
+    cudaMemcpyAsync(keys, srcK, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s);
+    cudaMemcpyAsync(vals, srcV, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s);
   }
 }

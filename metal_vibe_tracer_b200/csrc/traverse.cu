@@ -275,70 +275,6 @@ __global__ void __launch_bounds__(128) k_count(const float4 *__restrict__ nodes,
 
 }  // namespace
 
-// ---- ray ordering ----------------------------------------------------------------------------------
-// Large ray batches are traced in the order of a 30-bit key of origin and direction, so that the
-// rays of a warp follow similar paths (fewer idle lanes at divergent branches, shared cache lines).
-// The key is computed per ray, sorted with the LBVH's radix sort, and the persistent kernels read
-// ray perm[q] at queue position q; results still go to each ray's own slot.
-#ifndef VT_TRACE_SORT
-#define VT_TRACE_SORT 0
-#endif
-constexpr uint32_t kSortMinRays = 1u << 20;
-
-__device__ __forceinline__ uint32_t quant(float x, float lo, float inv, uint32_t bits) {
-  float f = (x - lo) * inv;
-  const float top = (float)((1u << bits) - 1u);
-  f = fminf(fmaxf(f, 0.0f), top);
-  return (uint32_t)f;
-}
-// Octahedral map of a unit direction to [0, 1]^2.
-__device__ __forceinline__ float2 octahedral(float dx, float dy, float dz) {
-  const float sum = fabsf(dx) + fabsf(dy) + fabsf(dz);
-  float u = dx / sum, v = dy / sum;
-  if (dz < 0.0f) {
-    const float uu = (1.0f - fabsf(v)) * (u >= 0.0f ? 1.0f : -1.0f);
-    const float vv = (1.0f - fabsf(u)) * (v >= 0.0f ? 1.0f : -1.0f);
-    u = uu; v = vv;
-  }
-  return make_float2(u * 0.5f + 0.5f, v * 0.5f + 0.5f);
-}
-
-__global__ void k_ray_keys(const float4 *__restrict__ rays, uint32_t n, float3 lo, float3 inv,
-                           uint32_t *__restrict__ keys, uint32_t *__restrict__ vals, int mode) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float4 r0 = __ldcs(rays + 2 * (size_t)i), r1 = __ldcs(rays + 2 * (size_t)i + 1);
-  uint32_t key = 0;
-  if (mode == 1 || mode == 2) {
-    // Origin Morton code (10 bits per axis), or octant + 9 bits per axis.
-    const uint32_t b = mode == 1 ? 10u : 9u;
-    const float sc = (float)(1u << b);
-    uint32_t q[3] = {quant(r0.x, lo.x, inv.x * sc, b), quant(r0.y, lo.y, inv.y * sc, b), quant(r0.z, lo.z, inv.z * sc, b)};
-    for (uint32_t bit = 0; bit < b; ++bit)
-      for (int a = 0; a < 3; ++a) key |= ((q[a] >> bit) & 1u) << (3 * bit + (2 - a));
-    if (mode == 2) key |= ((r1.x < 0.0f ? 4u : 0u) | (r1.y < 0.0f ? 2u : 0u) | (r1.z < 0.0f ? 1u : 0u)) << 27;
-  } else if (mode == 3) {
-    // 5-D Morton code: 6 bits each of origin x, y, z and octahedral direction u, v.
-    const float2 o = octahedral(r1.x, r1.y, r1.z);
-    uint32_t q[5] = {quant(r0.x, lo.x, inv.x * 64.0f, 6), quant(r0.y, lo.y, inv.y * 64.0f, 6),
-                     quant(r0.z, lo.z, inv.z * 64.0f, 6), quant(o.x, 0.0f, 64.0f, 6), quant(o.y, 0.0f, 64.0f, 6)};
-    for (uint32_t bit = 0; bit < 6; ++bit)
-      for (int a = 0; a < 5; ++a) key |= ((q[a] >> bit) & 1u) << (5 * bit + (4 - a));
-  } else {
-    // Direction major (5 + 5 octahedral bits), origin Morton minor (20 bits).
-    const float2 o = octahedral(r1.x, r1.y, r1.z);
-    const uint32_t du = quant(o.x, 0.0f, 32.0f, 5), dv = quant(o.y, 0.0f, 32.0f, 5);
-    uint32_t q[3] = {quant(r0.x, lo.x, inv.x * 128.0f, 7), quant(r0.y, lo.y, inv.y * 128.0f, 7), quant(r0.z, lo.z, inv.z * 64.0f, 6)};
-    uint32_t m = 0, pos = 0;
-    for (uint32_t bit = 0; bit < 7; ++bit)
-      for (int a = 0; a < 3; ++a)
-        if (bit < (a == 2 ? 6u : 7u)) m |= ((q[a] >> bit) & 1u) << pos++;
-    key = (du << 25) | (dv << 20) | m;
-  }
-  keys[i] = key;
-  vals[i] = i;
-}
-
 namespace {
 // Stack entries a traversal of a tree of `depth` levels needs: a visit goes on to one child and
 // pushes at most three.
@@ -393,21 +329,4 @@ void vt_launch_count(const vt_mesh *mesh, const vt_ray *rays, uint32_t n, int cl
   k_count<<<(n + 127) / 128, 128, 0, s>>>(reinterpret_cast<const float4 *>(mesh->d_qnodes), mesh->d_tris,
                                          mesh->root_max, reinterpret_cast<const float4 *>(rays), n,
                                          closest, acc);
-}
-
-size_t vt_ray_order_words(uint32_t n) { return 4 * (((size_t)n + 63) & ~size_t(63)) + vt_radix_temp_words(n) + 64; }
-
-const uint32_t *vt_ray_order(const vt_mesh *mesh, const vt_ray *rays, uint32_t n, uint32_t *scratch,
-                             cudaStream_t s) {
-  if (VT_TRACE_SORT == 0 || n < kSortMinRays) return nullptr;
-  // Each array starts on a 256-byte boundary: the sort reads them with 16-byte vector loads.
-  const size_t stride = ((size_t)n + 63) & ~size_t(63);
-  uint32_t *keys = scratch, *vals = keys + stride, *keysAlt = vals + stride, *valsAlt = keysAlt + stride;
-  uint32_t *temp = valsAlt + stride;
-  float3 lo = make_float3(mesh->lo[0], mesh->lo[1], mesh->lo[2]);
-  float ex = mesh->hi[0] - mesh->lo[0], ey = mesh->hi[1] - mesh->lo[1], ez = mesh->hi[2] - mesh->lo[2];
-  float3 inv = make_float3(ex > 0 ? 1.0f / ex : 0.0f, ey > 0 ? 1.0f / ey : 0.0f, ez > 0 ? 1.0f / ez : 0.0f);
-  k_ray_keys<<<(n + 255) / 256, 256, 0, s>>>(reinterpret_cast<const float4 *>(rays), n, lo, inv, keys, vals, VT_TRACE_SORT);
-  vt_radix_sort_pairs(keys, vals, keysAlt, valsAlt, n, 30, temp, s);
-  return vals;
 }

@@ -20,10 +20,35 @@ vt_status vt_cuda_fail(vt_ctx *ctx, cudaError_t err, const char *what) {
   return vt_fail(ctx, err == cudaErrorMemoryAllocation ? VT_ERR_MEMORY : VT_ERR_CUDA, m);
 }
 
+cudaError_t vt_pool_alloc(vt_ctx *ctx, void **p, size_t bytes) {
+  if (!ctx->pool) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = ctx->device;
+    cudaMemPool_t pool;
+    cudaError_t e = cudaMemPoolCreate(&pool, &props);
+    if (e != cudaSuccess) return e;
+    uint64_t keep = kPoolKeep;
+    e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e != cudaSuccess) {
+      cudaMemPoolDestroy(pool);
+      return e;
+    }
+    ctx->pool = pool;
+  }
+  return cudaMallocFromPoolAsync(p, bytes, ctx->pool, ctx->stream);
+}
+
 namespace {
 
+// Waits for every use of the mesh first (freeing pool memory does not, unlike plain cudaFree).
 void free_mesh(vt_mesh *m) {
   if (!m) return;
+  int dev = 0;
+  const bool other = cudaGetDevice(&dev) == cudaSuccess && dev != m->device;
+  if (other) cudaSetDevice(m->device);
+  cudaDeviceSynchronize();
   cudaFree(m->d_nodes);
   cudaFree(m->d_tris);
   cudaFree(m->d_order);
@@ -33,6 +58,7 @@ void free_mesh(vt_mesh *m) {
   cudaFree(m->d_bin_box);
   cudaFree(m->d_qnodes);
   cudaFree(m->d_nrm);
+  if (other) cudaSetDevice(dev);
   delete m;
 }
 
@@ -64,26 +90,11 @@ vt_status ensure_chunks(vt_ctx *ctx, size_t in_bytes, size_t out_bytes) {
   return VT_OK;
 }
 
-// Ray-ordering scratch of `slot` (0: caller streams, 1-2: the host pipeline's streams).
-vt_status order_scratch(vt_ctx *ctx, int slot, uint32_t n, uint32_t **out) {
-  size_t words = vt_ray_order_words(n);
-  if (words > ctx->order_words[slot]) {
-    cudaFree(ctx->d_order[slot]);
-    ctx->d_order[slot] = nullptr;
-    ctx->order_words[slot] = 0;
-    VT_CUDA(ctx, cudaMalloc(&ctx->d_order[slot], words * sizeof(uint32_t)));
-    ctx->order_words[slot] = words;
-  }
-  *out = ctx->d_order[slot];
-  return VT_OK;
-}
-
 vt_status check_trace_args(vt_ctx *ctx, const vt_mesh *mesh, const void *rays, const void *out, uint32_t n) {
   if (!ctx) return VT_ERR_INVALID;
   if (!mesh) return vt_fail(ctx, VT_ERR_INVALID, "mesh is null");
   if (n > 0 && (!rays || !out)) return vt_fail(ctx, VT_ERR_INVALID, "rays or output is null");
   if (n > 0 && mesh->nfaces > 0 && !mesh->d_nodes) return vt_fail(ctx, VT_ERR_INVALID, "mesh has no nodes");
-  // Leaf stack entries hold (node << 2 | slot) in 31 bits.
   if (mesh->nnodes >= (1u << 29)) return vt_fail(ctx, VT_ERR_LIMIT, "traversal supports up to 2^29 - 1 wide nodes");
   return VT_OK;
 }
@@ -134,7 +145,6 @@ vt_status vt_ctx_destroy(vt_ctx *ctx) {
   if (!ctx) return VT_OK;
   cudaSetDevice(ctx->device);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-  for (int k = 0; k < 3; ++k) cudaFree(ctx->d_order[k]);
   for (int k = 0; k < 2; ++k) {
     if (ctx->pipe[k]) cudaStreamSynchronize(ctx->pipe[k]);
     cudaFree(ctx->d_chunk_in[k]);
@@ -149,6 +159,7 @@ vt_status vt_ctx_destroy(vt_ctx *ctx) {
   cudaFree(ctx->d_fgrid);
   cudaFree(ctx->d_pbr);
   cudaFree(ctx->d_gnodes);
+  if (ctx->pool) cudaMemPoolDestroy(ctx->pool);  // meshes still alive keep their memory until freed
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -174,6 +185,7 @@ vt_status vt_mesh_build_device(vt_ctx *ctx, const vt_face *faces_dev, uint32_t n
   if (nfaces > (1u << 30)) return vt_fail(ctx, VT_ERR_LIMIT, "more than 2^30 faces");
   VT_CUDA(ctx, cudaSetDevice(ctx->device));
   vt_mesh *m = new vt_mesh();
+  m->device = ctx->device;
   vt_build_options o = defaults(opts);
   vt_status st = vt_lbvh_build(ctx, faces_dev, nfaces, verts_dev, nverts, o, m);
   if (st != VT_OK) {
@@ -193,18 +205,22 @@ vt_status vt_mesh_build(vt_ctx *ctx, const vt_face *faces, uint32_t nfaces, cons
   vt_face *df = nullptr;
   vt_vertex *dv = nullptr;
   if (nfaces > 0) {
-    VT_CUDA(ctx, cudaMalloc(&df, (size_t)nfaces * sizeof(vt_face)));
-    cudaError_t e = cudaMalloc(&dv, (size_t)(nverts ? nverts : 1) * sizeof(vt_vertex));
-    if (e != cudaSuccess) { cudaFree(df); return vt_cuda_fail(ctx, e, "cudaMalloc(vertices)"); }
+    VT_CUDA(ctx, vt_pool_alloc(ctx, reinterpret_cast<void **>(&df), (size_t)nfaces * sizeof(vt_face)));
+    cudaError_t e = vt_pool_alloc(ctx, reinterpret_cast<void **>(&dv), (size_t)(nverts ? nverts : 1) * sizeof(vt_vertex));
+    if (e != cudaSuccess) { cudaFreeAsync(df, ctx->stream); return vt_cuda_fail(ctx, e, "allocating the vertices"); }
     e = cudaMemcpyAsync(df, faces, (size_t)nfaces * sizeof(vt_face), cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess && nverts)
       e = cudaMemcpyAsync(dv, verts, (size_t)nverts * sizeof(vt_vertex), cudaMemcpyHostToDevice, ctx->stream);
-    if (e != cudaSuccess) { cudaFree(df); cudaFree(dv); return vt_cuda_fail(ctx, e, "cudaMemcpyAsync(mesh)"); }
+    if (e != cudaSuccess) {
+      cudaFreeAsync(df, ctx->stream);
+      cudaFreeAsync(dv, ctx->stream);
+      return vt_cuda_fail(ctx, e, "cudaMemcpyAsync(mesh)");
+    }
   }
   vt_status st = vt_mesh_build_device(ctx, df, nfaces, dv, nverts, opts, out);
   cudaStreamSynchronize(ctx->stream);
-  cudaFree(df);
-  cudaFree(dv);
+  if (df) cudaFreeAsync(df, ctx->stream);
+  if (dv) cudaFreeAsync(dv, ctx->stream);
   return st;
 }
 
@@ -277,9 +293,9 @@ vt_status vt_mesh_get_binary(vt_ctx *ctx, const vt_mesh *mesh, int32_t *children
   return VT_OK;
 }
 
-// Shared body of the device-buffer entry points; `slot` picks the ray-ordering scratch.
+// Shared body of the device-buffer entry points.
 static vt_status trace_device(vt_ctx *ctx, const vt_mesh *mesh, const vt_ray *rays_dev, uint32_t n, void *out,
-                              bool closest, cudaStream_t s, int slot) {
+                              bool closest, cudaStream_t s) {
   vt_status st = check_trace_args(ctx, mesh, rays_dev, out, n);
   if (st) return st;
   if (n == 0) return VT_OK;
@@ -287,12 +303,8 @@ static vt_status trace_device(vt_ctx *ctx, const vt_mesh *mesh, const vt_ray *ra
     if (closest) k_fill_miss<<<(n + 255) / 256, 256, 0, s>>>(static_cast<int4 *>(out), n);
     else VT_CUDA(ctx, cudaMemsetAsync(out, 0, n, s));
   } else {
-    uint32_t *scratch = nullptr;
-    st = order_scratch(ctx, slot, n, &scratch);
-    if (st) return st;
-    const uint32_t *perm = vt_ray_order(mesh, rays_dev, n, scratch, s);
-    if (closest) vt_launch_closest(mesh, rays_dev, n, static_cast<vt_hit *>(out), ctx->sm_count, vt_queue_slot(ctx), perm, ctx->d_status + 1, s);
-    else vt_launch_any(mesh, rays_dev, n, static_cast<uint8_t *>(out), ctx->sm_count, vt_queue_slot(ctx), perm, ctx->d_status + 1, s);
+    if (closest) vt_launch_closest(mesh, rays_dev, n, static_cast<vt_hit *>(out), ctx->sm_count, vt_queue_slot(ctx), nullptr, ctx->d_status + 1, s);
+    else vt_launch_any(mesh, rays_dev, n, static_cast<uint8_t *>(out), ctx->sm_count, vt_queue_slot(ctx), nullptr, ctx->d_status + 1, s);
   }
   VT_CUDA(ctx, cudaGetLastError());
   return VT_OK;
@@ -301,12 +313,12 @@ static vt_status trace_device(vt_ctx *ctx, const vt_mesh *mesh, const vt_ray *ra
 vt_status vt_trace_closest(vt_ctx *ctx, const vt_mesh *mesh, const vt_ray *rays_dev, uint32_t n,
                            vt_hit *hits_dev, void *stream) {
   // NULL stream = the CUDA default stream.
-  return trace_device(ctx, mesh, rays_dev, n, hits_dev, true, static_cast<cudaStream_t>(stream), 0);
+  return trace_device(ctx, mesh, rays_dev, n, hits_dev, true, static_cast<cudaStream_t>(stream));
 }
 
 vt_status vt_trace_any(vt_ctx *ctx, const vt_mesh *mesh, const vt_ray *rays_dev, uint32_t n,
                        uint8_t *occluded_dev, void *stream) {
-  return trace_device(ctx, mesh, rays_dev, n, occluded_dev, false, static_cast<cudaStream_t>(stream), 0);
+  return trace_device(ctx, mesh, rays_dev, n, occluded_dev, false, static_cast<cudaStream_t>(stream));
 }
 
 // Pinned staging buffers for pageable callers (two slots, grown as needed) and their events.
@@ -399,7 +411,7 @@ static vt_status trace_host(vt_ctx *ctx, const vt_mesh *mesh, const vt_ray *rays
       copy_parallel(ctx->h_stage_in[k], rays + first, (size_t)m * sizeof(vt_ray));
       cudaStream_t s = ctx->pipe[k];
       VT_CUDA(ctx, cudaMemcpyAsync(ctx->d_chunk_in[k], ctx->h_stage_in[k], (size_t)m * sizeof(vt_ray), cudaMemcpyHostToDevice, s));
-      st = trace_device(ctx, mesh, static_cast<const vt_ray *>(ctx->d_chunk_in[k]), m, ctx->d_chunk_out[k], closest, s, 1 + k);
+      st = trace_device(ctx, mesh, static_cast<const vt_ray *>(ctx->d_chunk_in[k]), m, ctx->d_chunk_out[k], closest, s);
       if (st) return st;
       VT_CUDA(ctx, cudaMemcpyAsync(ctx->h_stage_out[k], ctx->d_chunk_out[k], (size_t)m * out_stride, cudaMemcpyDeviceToHost, s));
       VT_CUDA(ctx, cudaEventRecord(ctx->stage_ev[k], s));
@@ -417,7 +429,7 @@ static vt_status trace_host(vt_ctx *ctx, const vt_mesh *mesh, const vt_ray *rays
     VT_CUDA(ctx, cudaMemcpyAsync(ctx->d_chunk_in[k], rays + first, (size_t)m * sizeof(vt_ray),
                                  cudaMemcpyHostToDevice, s));
     const vt_ray *dr = static_cast<const vt_ray *>(ctx->d_chunk_in[k]);
-    st = trace_device(ctx, mesh, dr, m, ctx->d_chunk_out[k], closest, s, 1 + k);
+    st = trace_device(ctx, mesh, dr, m, ctx->d_chunk_out[k], closest, s);
     if (st) return st;
     VT_CUDA(ctx, cudaMemcpyAsync(static_cast<char *>(out) + (size_t)first * out_stride, ctx->d_chunk_out[k],
                                  (size_t)m * out_stride, cudaMemcpyDeviceToHost, s));

@@ -32,10 +32,9 @@ struct vt_ctx {
   void *h_stage_out[2] = {nullptr, nullptr};
   size_t stage_in_bytes = 0, stage_out_bytes = 0;
   cudaEvent_t stage_ev[2] = {nullptr, nullptr};
-  // Ray-ordering scratch (keys, permutation, sort buffers), grown on demand. One per pipeline
-  // stream plus one for caller streams, so concurrent launches do not share it.
-  uint32_t *d_order[3] = {nullptr, nullptr, nullptr};
-  size_t order_words[3] = {0, 0, 0};
+  // Memory of the builds (temporaries and the meshes' arrays), created with the first build: freed
+  // blocks stay in it up to kPoolKeep bytes, so that rebuilding a mesh maps no new memory.
+  cudaMemPool_t pool = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // RGB -> spectrum uplift (spectral.cu), built once per context: the moment grid (86^3 float4
   // nodes, then refined 64-entry blocks) and the 86 node values; the colour model it was solved for.
@@ -57,6 +56,7 @@ struct __align__(64) vt_qnode {
 };
 
 struct vt_mesh {
+  int device = 0;            // where its arrays live
   uint32_t nfaces = 0;
   uint32_t nnodes = 0;       // 4-wide nodes
   uint32_t depth = 0;        // 4-wide depth (root = 1)
@@ -185,23 +185,32 @@ enum : uint32_t {
   VT_DEV_NONFINITE = 2u,       // a vertex position is NaN or infinite
   VT_DEV_STACK = 4u,           // traversal stack overflow
   VT_DEV_TREELET = 8u,         // treelet restructuring hit an internal inconsistency
+  VT_DEV_SORT = 32u,           // the Morton sort's look-back gave up
+  VT_DEV_BARRIER = 64u,        // the collapse's grid barrier gave up
   VT_DEV_NORMALS = 16u         // information, not an error: some vertex normal is nonzero
 };
+
+// A word that other blocks of the same launch write: read from L2 at each call (never a kept value).
+__device__ __forceinline__ uint32_t vt_poll(const uint32_t *p) {
+  uint32_t v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
 
 // ---------------------------------------------------------------------------------------------
 // Build helpers implemented in scan_sort.cu / lbvh.cu.
 
-// Exclusive prefix sum of n uint32 values (in place allowed). `temp` must hold
-// vt_scan_temp_words(n) words. Returns the total through *total_dev if non-null (device word).
-size_t vt_scan_temp_words(uint32_t n);
-void vt_scan_exclusive(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *temp,
-                       uint32_t *total_dev, cudaStream_t s);
+// Stream-ordered device memory from the context's pool, usable on ctx->stream (or anywhere once that
+// stream has been synchronised).
+constexpr size_t kPoolKeep = size_t(1) << 30;
+cudaError_t vt_pool_alloc(vt_ctx *ctx, void **p, size_t bytes);
 
 // Stable LSD radix sort of (key, value) pairs on the low `bits` bits of the keys.
-// keys/vals are sorted in place using the alternate buffers; temp is vt_radix_temp_words(n).
+// keys/vals are sorted in place using the alternate buffers; temp is vt_radix_temp_words(n). n below
+// 2^30, bits at most 32; VT_DEV_SORT goes to *status if a tile's look-back gives up.
 size_t vt_radix_temp_words(uint32_t n);
 void vt_radix_sort_pairs(uint32_t *keys, uint32_t *vals, uint32_t *keys_alt, uint32_t *vals_alt,
-                         uint32_t n, int bits, uint32_t *temp, cudaStream_t s);
+                         uint32_t n, int bits, uint32_t *temp, uint32_t *status, cudaStream_t s);
 
 vt_status vt_quantize_nodes(vt_ctx *ctx, vt_mesh *mesh, cudaStream_t s);
 vt_status vt_lbvh_build(vt_ctx *ctx, const vt_face *faces, uint32_t nfaces, const vt_vertex *verts,
@@ -221,10 +230,5 @@ void vt_launch_closest(const vt_mesh *mesh, const vt_ray *rays, uint32_t n, vt_h
 void vt_launch_any(const vt_mesh *mesh, const vt_ray *rays, uint32_t n, uint8_t *occ,
                    int sm_count, uint32_t *counter, const uint32_t *perm, uint32_t *status,
                    cudaStream_t s, const uint32_t *count = nullptr, bool slack = false);
-// Ray ordering for large batches: returns the device permutation (inside `scratch`, which must
-// hold vt_ray_order_words(n) words) or nullptr when the batch is traced in input order.
-size_t vt_ray_order_words(uint32_t n);
-const uint32_t *vt_ray_order(const vt_mesh *mesh, const vt_ray *rays, uint32_t n, uint32_t *scratch,
-                             cudaStream_t s);
 void vt_launch_count(const vt_mesh *mesh, const vt_ray *rays, uint32_t n, int closest,
                      unsigned long long *acc /* 2 device words */, cudaStream_t s);

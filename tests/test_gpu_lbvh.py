@@ -42,6 +42,22 @@ def test_lbvh_bit_exact(ctx, oracle, n, leaf, treelet):
     compare_builds(gpu, ref)
 
 
+@pytest.mark.parametrize("n", [2, 3, 3071, 3072, 3073, 6145, 40_000])
+def test_sort_tiles_and_collapse_blocks(ctx, oracle, n):
+    """Sizes around the Morton sort's tiles of 3,072 pairs and the collapse's blocks, with many equal codes
+    (every centroid near one of 64 points, so stability decides the order) against the oracle; a second
+    build into the reused pool memory gives the same."""
+    faces, verts = scenes.triangle_soup(n, seed=n, mu=math.log(0.01))
+    p = verts["p"].reshape(-1, 3, 3)
+    p += np.floor(p.mean(1, keepdims=True) * 4) / 4 - p.mean(1, keepdims=True)
+    verts["p"] = p.reshape(-1, 3)
+    ref = oracle.Bvh.lbvh(faces, verts)
+    for _ in range(2):
+        gpu = vt.Mesh(ctx, faces, verts)
+        compare_builds(gpu, ref)
+        gpu.close()
+
+
 def test_lbvh_duplicate_centroids_and_welded_patch(ctx, oracle):
     # Coincident centroids (equal Morton codes everywhere) and a welded patch.
     faces, verts = scenes.triangle_soup(500, seed=1)
