@@ -1276,9 +1276,7 @@ __device__ __forceinline__ float3 primary_emission(const RenderArgs &A, const La
 
 // The path after its primary vertex S (the bounce loop of shading_kernel, main.swift:7709-7833):
 // BSDF continuations, NEE with MIS at later vertices, emitter hits weighed by emission_weight and
-// Russian roulette. With diPrimary (sampling mode 0) the primary vertex's direct light came from its
-// ReSTIR DI reservoir, so a BSDF hit on an emitter from it gets no weight (previousMIS false,
-// main.swift:7717-7718).
+// Russian roulette.
 // The cache's query record of a vertex (nrc.cuh's input layout): OpenPBR slots give their
 // roughness and split the base colour by metalness; Lambert slots are rough and diffuse.
 template <bool kPbr>
@@ -1327,27 +1325,18 @@ __device__ __forceinline__ void nrc_store_none(const RenderArgs &A, size_t slot)
   A.nrcT[slot] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 }
 
-// kNrc (vt_render_nrc): the path ends, after the vertex's emission, at vertex A.nrcVertex, or with
-// A.nrcVertex 0 at the first vertex where its spread exceeds spreadLimit (nrc_spread_limit), with
-// its cache query stored in `slot`; `queried` tells whether it got there.
-template <bool kPbr, bool kNrc = false>
+template <bool kPbr>
 __device__ float3 continue_path(const RenderArgs &A, const Lanes &L, Surface S, vt_material m, float3 dir,
-                                Sampler &seed, int *stack, bool diPrimary, float spreadLimit = 0.0f, size_t slot = 0,
-                                bool *queried = nullptr) {
+                                Sampler &seed, int *stack) {
   const int limit = max(0, (int)A.maxDepth - 1);
   const bool nee = A.mode != 3u, mis = A.mode <= 1u;
   float4 T = A.spectral ? make_float4(1.0f, 1.0f, 1.0f, 1.0f) : make_float4(1.0f, 1.0f, 1.0f, 0.0f);
   float3 R = f3(0.0f, 0.0f, 0.0f);
   int scattering = 0;
   bool emissionOnly = false;
-  float spread = 0.0f;  // sum of the vertices' sqrt(d^2 / (p |cos|)) (kNrc)
-  // ReSTIR GI's reservoir estimates the direct light of the secondary diffuse vertex of a path whose
-  // diffuse primary took ReSTIR DI, so that vertex skips NEE (restirGISecondary, main.swift:7801-7803).
-  const bool giPrimary = diPrimary && !kNrc && m.type == VT_MAT_DIFFUSE;
   // Ideal reflections and refractions spend no scattering event (main.swift:7716-7723); `delta`
-  // follows the path's current vertex. The cache-terminated form (kNrc: vt_render_nrc's ReSTIR DI
-  // frames) is compiled without glass and mirrors, and the host refuses scenes that have them there.
-  bool delta = !kNrc && is_delta<kPbr>(A, m);
+  // follows the path's current vertex.
+  bool delta = is_delta<kPbr>(A, m);
   for (int bounce = 1;; ++bounce) {
     if (!delta && scattering >= limit) {
       // BSDF-only paths take one final continuation that may only reach emission.
@@ -1355,7 +1344,7 @@ __device__ float3 continue_path(const RenderArgs &A, const Lanes &L, Surface S, 
       emissionOnly = true;
     }
     if (!delta) ++scattering;
-    const bool previousMIS = mis && !(diPrimary && bounce == 1);
+    const bool previousMIS = mis;
     sampler_event(seed, (uint32_t)bounce, kZBsdf);
     float3 nd;
     float bpdf;
@@ -1396,25 +1385,19 @@ __device__ float3 continue_path(const RenderArgs &A, const Lanes &L, Surface S, 
     }
     S = surface_at(A, h, o, dir);
     m = material(A, S.slot);
-    if (kNrc && !delta) spread += h.t * rsqrtf(fmaxf(bpdf * fabsf(dot3(S.gn, dir)), 1e-30f));
     if (m.type == VT_MAT_EMISSIVE) {
       // emission_weight (main.swift:3462-3466): 1 after an ideal bounce, without NEE or without a
-      // light pdf, else the power heuristic (MIS) or 0 (light sampling, or a ReSTIR DI vertex).
+      // light pdf, else the power heuristic (MIS) or 0 (light sampling).
       const float lpdf = A.imported ? emitter_pdf(A, prev, S.pos, S.face) : light_pdf(A, prev, S.pos);
       const float w = emission_weight(delta, nee, previousMIS, bpdf, lpdf);
       if (!A.imported || S.front) R = add(R, to_rgb(A, L, scale4(mul4(T, emission(A, L, m.emission)), w)));
       break;
     }
     if (emissionOnly) break;
-    // Glass and mirrors take no NEE, and the cache is queried at rough vertices only.
-    const bool nextDelta = !kNrc && is_delta<kPbr>(A, m);
+    // Glass and mirrors take no NEE.
+    const bool nextDelta = is_delta<kPbr>(A, m);
     delta = nextDelta;
-    if (kNrc && !nextDelta && (A.nrcVertex ? (uint32_t)bounce >= A.nrcVertex : spread * spread > spreadLimit)) {
-      nrc_store(A, slot, nrc_query<kPbr>(A, L, S, m, dir), L, T);
-      *queried = true;
-      break;
-    }
-    if (nee && !nextDelta && !(giPrimary && bounce == 1 && m.type == VT_MAT_DIFFUSE)) {
+    if (nee && !nextDelta) {
       sampler_event(seed, (uint32_t)bounce + 1u, kZNee);
       R = add(R, direct_light<kPbr>(A, L, S.pos, S.n, S.gn, S.tri, S.err, mul(dir, -1.0f), T, m, mis && scattering < limit, scattering < limit,
                               seed, stack, false));
@@ -1431,9 +1414,8 @@ __device__ float3 continue_path(const RenderArgs &A, const Lanes &L, Surface S, 
 }
 
 // One path of sampling modes 1-3: camera ray, primary hit, NEE there, then the continuation.
-template <bool kPbr, bool kNrc>
-__device__ __forceinline__ float3 path_sample_body(const RenderArgs &A, uint32_t x, uint32_t y, uint32_t si, uint32_t frame,
-                                                   float2 jit, int *stack, size_t slot, bool &queried) {
+template <bool kPbr>
+__device__ float3 path_sample(const RenderArgs &A, uint32_t x, uint32_t y, uint32_t si, uint32_t frame, float2 jit, int *stack) {
   Sampler seed = pixel_sampler(x, y, A.W, si, A.zSampler != 0u, A.zModel, frame);
   Lanes L;
   if (A.spectral) L = make_lanes(A, wavelength_numbers(seed).x);
@@ -1447,25 +1429,16 @@ __device__ __forceinline__ float3 path_sample_body(const RenderArgs &A, uint32_t
   const vt_material m = material(A, S.slot);
   if (m.type == VT_MAT_EMISSIVE) return primary_emission(A, L, S, m);
   float3 R = f3(0.0f, 0.0f, 0.0f);
-  if (A.mode != 3u && (kNrc || !is_delta<kPbr>(A, m))) {  // no NEE at glass or a mirror (main.swift:7657)
+  if (A.mode != 3u && !is_delta<kPbr>(A, m)) {  // no NEE at glass or a mirror (main.swift:7657)
     const int limit = max(0, (int)A.maxDepth - 1);
     const float4 T = A.spectral ? make_float4(1.0f, 1.0f, 1.0f, 1.0f) : make_float4(1.0f, 1.0f, 1.0f, 0.0f);
     sampler_event(seed, 1u, kZNee);
     R = direct_light<kPbr>(A, L, S.pos, S.n, S.gn, S.tri, S.err, mul(dir0, -1.0f), T, m, A.mode == 1u && limit > 0, limit > 0, seed,
                      stack, true);
   }
-  const float spreadLimit = kNrc ? nrc_spread_limit(A, h.t, S.gn, dir0) : 0.0f;
-  R = add(R, continue_path<kPbr, kNrc>(A, L, S, m, dir0, seed, stack, false, spreadLimit, slot, &queried));
+  R = add(R, continue_path<kPbr>(A, L, S, m, dir0, seed, stack));
   if (!isfinite(R.x) || !isfinite(R.y) || !isfinite(R.z)) R = f3(0.0f, 0.0f, 0.0f);
   return R;
-}
-template <bool kPbr, bool kNrc = false>
-__device__ float3 path_sample(const RenderArgs &A, uint32_t x, uint32_t y, uint32_t si, uint32_t frame, float2 jit,
-                              int *stack, size_t slot = 0) {
-  bool queried = false;
-  const float3 c = path_sample_body<kPbr, kNrc>(A, x, y, si, frame, jit, stack, slot, queried);
-  if (kNrc && !queried) nrc_store_none(A, slot);
-  return c;
 }
 
 // ---- ReSTIR GI (sampling mode 0): the first indirect diffuse vertex ------------------------------
@@ -1525,17 +1498,21 @@ __device__ __forceinline__ float gi_target(const RenderArgs &A, float3 x1, float
   const float3 v = to_rgb(A, L, scale4(mul4(reflectance(A, L, m), c.rad), f * geometry));
   return sqrtf(dot3(v, v));
 }
-// gi_connection_visible (main.swift:3238-3252): x1 sees x2 (the endpoint tolerance at x2).
-__device__ __forceinline__ bool gi_visible(const RenderArgs &A, float3 x1, float3 n1, float3 x2, float err, int *stack) {
+// gi_connection_visible (main.swift:3238-3252): the ray that tells whether x1 sees x2 (the endpoint
+// tolerance at x2); false when x2 is too close to see.
+__device__ __forceinline__ bool gi_ray(const RenderArgs &A, float3 x1, float3 n1, float3 x2, float err, float3 &o, float3 &dir,
+                                       float &tmax) {
   float3 delta = sub(x2, x1);
   const float dist = sqrtf(dot3(delta, delta));
   if (dist <= 2.0f * ray_eps(A, x1)) return false;
-  const float3 o = ray_origin(A, x1, n1, mul(delta, 1.0f / dist), err);
+  o = ray_origin(A, x1, n1, mul(delta, 1.0f / dist), err);
   const float3 e = sub(x2, o);
   const float d = sqrtf(dot3(e, e));
   const float legacy = 2.0f * ray_eps(A, x2);
   const float tol = A.imported ? fmaxf(legacy, 1.907349e-6f * (max_abs(o) + max_abs(x2) + d)) : legacy;
-  return !rt_any(A, o, mul(e, 1.0f / d), ray_tmin(A, o), d - tol, stack, A.imported != 0u);
+  dir = mul(e, 1.0f / d);
+  tmax = d - tol;
+  return true;
 }
 __device__ __forceinline__ GISample gi_load(const float4 *pos, const float4 *nrm, const float4 *rad, const float4 *w,
                                             uint32_t j) {
@@ -1549,290 +1526,10 @@ __device__ __forceinline__ GISample gi_load(const float4 *pos, const float4 *nrm
   return s;
 }
 
-// restir_gi_initial (main.swift:4718-4770) at the diffuse primary vertex S (material m), seen along
-// view: (reservoir sample, weight sum); M is 1.
-__device__ GISample gi_initial(const RenderArgs &A, const Surface &S, const vt_material &m, float3 view, float u,
-                               Sampler &seed, int *stack, float &wsum) {
-  GISample r;
-  r.pos = r.nrm = f3(0.0f, 0.0f, 0.0f);
-  r.rad = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  r.pdf = 0.0f;
-  r.u = u;
-  wsum = 0.0f;
-  const int limit = max(0, (int)A.maxDepth - 1);
-  sampler_event(seed, 1u, kZGiBsdf);
-  const float3 rr = rand_f3(seed);  // sample_bsdf's Lambert branch: the direction from the last two
-  const float3 gd = cosine_hemisphere(S.n, rr.y, rr.z);
-  const float bpdf = fmaxf(0.0f, dot3(S.n, gd)) * kInvPi;
-  if (!(bpdf > 0.0f) || !(dot3(gd, S.gn) > 0.0f)) return r;
-  const float3 o = ray_origin(A, S.pos, S.gn, gd, S.err);
-  Hit h;
-  if (!rt_closest(A, o, gd, ray_tmin(A, o), __int_as_float(0x7f800000), h, stack)) return r;
-  const Surface S2 = surface_at(A, h, o, gd);
-  const vt_material m2 = material(A, S2.slot);
-  if (m2.type != VT_MAT_DIFFUSE) return r;
-  Lanes L;
-  if (A.spectral) L = make_lanes(A, u);
-  float4 rad = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  sampler_event(seed, 2u, kZGiNee);
-  const LightSample ls = sample_direct(A, S2.pos, S2.n, seed, limit >= 2);
-  if (ls.pdf > 0.0f && light_visible(A, S2.pos, S2.gn, S2.err, ls, stack)) {
-    const float c2 = fmaxf(0.0f, dot3(S2.n, ls.wi));
-    float pdf2;
-    const float f2 = lambert_eval(S2.n, S2.gn, mul(gd, -1.0f), ls.wi, pdf2);
-    // The power heuristic only when a second continuation can sample x2's BSDF
-    // (restir_gi_has_complementary_bsdf, main.swift:3482-3484).
-    const float mis = limit >= 2 ? power_heuristic(ls.pdf, pdf2) : 1.0f;
-    const float le[3] = {ls.emission.x, ls.emission.y, ls.emission.z};
-    rad = scale4(mul4(reflectance(A, L, m2), emission(A, L, le)), f2 * c2 * mis / ls.pdf);
-  }
-  const float3 delta = sub(S2.pos, S.pos);
-  const float d2 = dot3(delta, delta);
-  const float cos2 = fmaxf(0.0f, -dot3(S2.n, gd));
-  const float srcPdf = d2 > 1e-10f ? bpdf * cos2 / d2 : 0.0f;
-  GISample c;
-  c.pos = S2.pos;
-  c.nrm = S2.n;
-  c.rad = rad;
-  c.pdf = srcPdf;
-  c.u = u;
-  const float pHat = gi_target(A, S.pos, S.n, S.gn, view, m, c);
-  if (srcPdf > 0.0f && pHat > 0.0f) {
-    r = c;
-    wsum = pHat / srcPdf;
-  }
-  return r;
-}
-
-// ReSTIR DI pass 1 for frame k (restir_temporal_kernel, main.swift:4842-5005): the primary hit into
-// the primary-surface cache, then at a diffuse (Lambert) hit the initial reservoir (RIS over the
-// frame's candidates, restir_di_initial, main.swift:4638-4668), merged with the previous frame's
-// reservoir of the backprojected pixel when it saw the same surface (restir_di_merge, main.swift:
-// 4686-4699, confidence capped at 20), stored with W = wsum / (M p_hat) (restir_di_encode); then,
-// with a scattering budget, the ReSTIR GI reservoir the same way (restir_gi_initial / _merge /
-// _encode). Other primaries get empty reservoirs and shade with NEE in pass 2 (main.swift:4931-4943).
-template <bool kPbr>
-__global__ void __launch_bounds__(kRenderBlock, kPbr ? 3 : 4) k_di_primary(RenderArgs A, uint32_t k) {
-  int stack[kRenderStack];
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= A.W * A.H) return;
-  const uint32_t x = i % A.W, y = i / A.W;
-  Sampler seed = pixel_sampler(x, y, A.W, A.first + k, A.zSampler != 0u, A.zModel, A.firstFrame + k);
-  const float u = A.spectral ? wavelength_numbers(seed).x : 0.0f;
-  float3 dir0 = camera_dir(A, x, y, A.jitter[k]), o0 = A.cam;
-  lens_ray(A, o0, dir0, seed);
-  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  Hit h;
-  if (!rt_closest(A, o0, dir0, ray_tmin(A, o0), __int_as_float(0x7f800000), h, stack)) {
-    A.gPos[i] = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
-    A.gNrm[i] = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
-    A.rPos[i] = zero; A.rEmit[i] = zero; A.rW[i] = zero;
-    A.giPos[i] = zero; A.giNrm[i] = zero; A.giRad[i] = zero; A.giW[i] = zero;
-    return;
-  }
-  const Surface S = surface_at(A, h, o0, dir0);
-  const vt_material m = material(A, S.slot);
-  const float4 gp = make_float4(S.pos.x, S.pos.y, S.pos.z, h.t), gn = make_float4(S.n.x, S.n.y, S.n.z, float(m.type));
-  A.gPos[i] = gp;
-  A.gNrm[i] = gn;
-  A.gGeo[i] = make_float4(S.gn.x, S.gn.y, S.gn.z, 0.0f);
-  A.gInfo[i] = make_uint4(S.face, S.slot | (S.front ? 0x80000000u : 0u), __float_as_uint(S.err), S.tri);
-  if (m.type != VT_MAT_DIFFUSE) {
-    A.rPos[i] = zero; A.rEmit[i] = zero; A.rW[i] = zero;
-    A.giPos[i] = zero; A.giNrm[i] = zero; A.giRad[i] = zero; A.giW[i] = zero;
-    return;
-  }
-  DIReservoir r;
-  r.s.pos = f3(0.0f, 0.0f, 0.0f); r.s.emission = f3(0.0f, 0.0f, 0.0f);
-  r.s.pdf = 0.0f; r.s.u = u; r.s.id = 0u;
-  r.wsum = 0.0f;
-  r.M = 0.0f;
-  for (uint32_t c = 0; c < A.diCandidates; ++c) {
-    sampler_candidate(seed, 1u, kZDi, c, A.diBits);
-    const LightSample ls = sample_direct(A, S.pos, S.n, seed, (int)A.maxDepth - 1 > 0);
-    r.M += 1.0f;  // zero-weight candidates still count
-    if (!(ls.pdf > 0.0f)) continue;
-    DISample cand;
-    cand.pos = ls.pos; cand.emission = ls.emission; cand.pdf = ls.pdf; cand.u = u;
-    cand.id = ls.face == 0xffffffffu ? 0u : ls.face + 2u;
-    const float pHat = di_target<kPbr>(A, S.pos, S.n, S.gn, S.tri, dir0, m, cand);
-    const float proposal = cand.pdf * light_geometry(A, S.pos, cand);
-    const float w = proposal > 0.0f ? pHat / proposal : 0.0f;
-    r.wsum += w;
-    if (rand_decision(seed) * r.wsum < w) r.s = cand;
-  }
-  int px, py;
-  const bool temporal = backproject(A, S.pos, px, py);
-  const uint32_t j = temporal ? (uint32_t)py * A.W + (uint32_t)px : 0u;
-  if (temporal) {
-    const float4 hw = A.hrW[j];
-    if (same_surface(gp, gn, A.hPos[j], A.hNrm[j]) && hw.y > 0.0f && hw.z > 0.0f) {
-      const DISample hs = load_di(A.hrPos, A.hrEmit, A.hrW, j);
-      const float cM = fminf(hw.y, 20.0f);
-      const float w = di_target<kPbr>(A, S.pos, S.n, S.gn, S.tri, dir0, m, hs) * hw.z * cM;
-      r.M += cM;
-      r.wsum += w;
-      if (rand_decision(seed) * r.wsum < w) r.s = hs;
-    }
-  }
-  const float pHat = di_target<kPbr>(A, S.pos, S.n, S.gn, S.tri, dir0, m, r.s);
-  const float W = r.M > 0.0f && pHat > 0.0f ? r.wsum / (r.M * pHat) : 0.0f;
-  A.rPos[i] = make_float4(r.s.pos.x, r.s.pos.y, r.s.pos.z, __uint_as_float(r.s.id));
-  A.rEmit[i] = make_float4(r.s.emission.x, r.s.emission.y, r.s.emission.z, r.s.pdf);
-  A.rW[i] = make_float4(r.wsum, r.M, W, r.s.u);
-  // ReSTIR GI: depth 1 has no indirect bounce for it (restir_gi_enabled, main.swift:3476-3478).
-  if ((int)A.maxDepth - 1 < 1) {
-    A.giPos[i] = zero; A.giNrm[i] = zero; A.giRad[i] = zero; A.giW[i] = zero;
-    return;
-  }
-  float gwsum, gM = 1.0f;
-  GISample g = gi_initial(A, S, m, dir0, u, seed, stack, gwsum);
-  if (temporal) {
-    const float4 ow = A.hgiW[j], op = A.hgiPos[j], on = A.hgiNrm[j], hp = A.hPos[j];
-    if (same_surface(gp, gn, hp, A.hNrm[j]) && ow.y > 0.0f && ow.z > 0.0f && op.w > 0.0f && on.w > 0.0f) {
-      const GISample hs = gi_load(A.hgiPos, A.hgiNrm, A.hgiRad, A.hgiW, j);
-      if (gi_accepts_shift(S.pos, f3(hp.x, hp.y, hp.z), hs.pos, hs.nrm)) {
-        const float cM = fminf(ow.y, 20.0f);
-        const float w = gi_target(A, S.pos, S.n, S.gn, dir0, m, hs) * ow.z * cM;
-        gM += cM;
-        gwsum += w;
-        if (pcg_rand(seed.state) * gwsum < w) g = hs;
-      }
-    }
-  }
-  const float gHat = gi_target(A, S.pos, S.n, S.gn, dir0, m, g);
-  const float gW = gM > 0.0f && gHat > 0.0f ? gwsum / (gM * gHat) : 0.0f;
-  A.giPos[i] = make_float4(g.pos.x, g.pos.y, g.pos.z, g.pdf);
-  A.giNrm[i] = make_float4(g.nrm.x, g.nrm.y, g.nrm.z, g.pdf > 0.0f ? 1.0f : 0.0f);
-  A.giRad[i] = g.rad;
-  A.giW[i] = make_float4(gwsum, gM, gW, g.u);
-}
-
-// ReSTIR DI pass 2 for frame k (shading_kernel, main.swift:7484-7656): at a diffuse primary, spatial
-// reuse of 4 uniform taps in a 32-pixel box that pass RESTIR2020's compatibility test
-// (uniform_neighbor, main.swift:5025-5027), the selected sample's contribution W * bsdf * Le * cos *
-// G when visible; then the same for the GI reservoirs (the reconnection x1 -> x2 shaded with the
-// secondary radiance, W and the area-measure geometry term); other primaries take NEE with MIS
-// (main.swift:7767-7780). Then the path's continuation (MIS at later vertices). The sample is added
-// to the FP64 accumulation.
-template <bool kPbr, bool kNrc = false>
-__global__ void __launch_bounds__(kRenderBlock, kPbr ? 3 : 4) k_di_shade(RenderArgs A, uint32_t k) {
-  int stack[kRenderStack];
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= A.W * A.H) return;
-  const size_t slot = (size_t)k * A.W * A.H + i;
-  bool queried = false;
-  const uint32_t x = i % A.W, y = i / A.W;
-  Sampler seed = pixel_sampler(x, y, A.W, A.first + k, A.zSampler != 0u, A.zModel, A.firstFrame + k);
-  Lanes L;
-  if (A.spectral) L = make_lanes(A, wavelength_numbers(seed).x);
-  float3 dir0 = camera_dir(A, x, y, A.jitter[k]), o0 = A.cam;
-  lens_ray(A, o0, dir0, seed);  // the same draws as pass 1
-  seed.state = pcg_hash(seed.state ^ 0x27d4eb2fu);  // decorrelate_shading_seed
-  const float4 gp = A.gPos[i];
-  if (gp.w <= 0.0f) {
-    if (kNrc) nrc_store_none(A, slot);
-    return;
-  }
-  const float4 gn = A.gNrm[i];
-  const uint4 gi = A.gInfo[i];
-  Surface S;
-  S.pos = f3(gp.x, gp.y, gp.z);
-  S.n = f3(gn.x, gn.y, gn.z);
-  const float4 gg = A.gGeo[i];
-  S.gn = f3(gg.x, gg.y, gg.z);
-  S.face = gi.x;
-  S.slot = gi.y & 0x7fffffffu;
-  S.front = (gi.y >> 31) != 0u;
-  S.err = __uint_as_float(gi.z);
-  S.tri = gi.w;
-  const vt_material m = material(A, S.slot);
-  float3 R;
-  if (m.type == VT_MAT_EMISSIVE) {
-    R = primary_emission(A, L, S, m);
-  } else if (m.type != VT_MAT_DIFFUSE) {
-    const int limit = max(0, (int)A.maxDepth - 1);
-    const float4 T = A.spectral ? make_float4(1.0f, 1.0f, 1.0f, 1.0f) : make_float4(1.0f, 1.0f, 1.0f, 0.0f);
-    R = f3(0.0f, 0.0f, 0.0f);
-    if (kNrc || !is_delta<kPbr>(A, m)) {  // no NEE at glass or a mirror (main.swift:7657)
-      sampler_event(seed, 1u, kZNee);
-      R = direct_light<kPbr>(A, L, S.pos, S.n, S.gn, S.tri, S.err, mul(dir0, -1.0f), T, m, limit > 0, limit > 0, seed, stack, true);
-    }
-    const float spreadLimit = kNrc ? nrc_spread_limit(A, gp.w, S.gn, dir0) : 0.0f;
-    R = add(R, continue_path<kPbr, kNrc>(A, L, S, m, dir0, seed, stack, false, spreadLimit, slot, &queried));
-  } else {
-    const float4 cw = A.rW[i];
-    DISample sel = load_di(A.rPos, A.rEmit, A.rW, i);
-    float wsum = di_target<kPbr>(A, S.pos, S.n, S.gn, S.tri, dir0, m, sel) * cw.z * cw.y, M = cw.y;
-    for (int t = 0; t < 4; ++t) {
-      const float ox = pcg_rand(seed.state), oy = pcg_rand(seed.state);
-      const int nx = (int)x + (int)((ox * 2.0f - 1.0f) * 16.0f), ny = (int)y + (int)((oy * 2.0f - 1.0f) * 16.0f);
-      if (nx < 0 || nx >= (int)A.W || ny < 0 || ny >= (int)A.H) continue;
-      const uint32_t j = (uint32_t)ny * A.W + (uint32_t)nx;
-      if (!compatible(gp, gn, A.gPos[j], A.gNrm[j])) continue;
-      const float4 nw = A.rW[j];
-      if (!(nw.y > 0.0f && nw.z > 0.0f)) continue;
-      const DISample ns = load_di(A.rPos, A.rEmit, A.rW, j);
-      const float w = di_target<kPbr>(A, S.pos, S.n, S.gn, S.tri, dir0, m, ns) * nw.z * nw.y;
-      wsum += w;
-      M += nw.y;
-      if (rand_decision(seed) * wsum < w) sel = ns;
-    }
-    const float pHat = di_target<kPbr>(A, S.pos, S.n, S.gn, S.tri, dir0, m, sel);
-    const float W = M > 0.0f && pHat > 0.0f ? wsum / (M * pHat) : 0.0f;
-    R = f3(0.0f, 0.0f, 0.0f);
-    if (W > 0.0f && light_visible(A, S.pos, S.gn, S.err, di_light_sample(sel, S.pos), stack))
-      R = mul(di_contribution<kPbr>(A, S.pos, S.n, S.gn, S.tri, dir0, m, sel), W);
-    // ReSTIR GI (a cache-terminated path's cache covers this light, so the cache's kernel leaves it out).
-    if (!kNrc && (int)A.maxDepth - 1 >= 1) {
-      const float4 cgw = A.giW[i];
-      GISample gsel = gi_load(A.giPos, A.giNrm, A.giRad, A.giW, i);
-      bool gvalid = A.giNrm[i].w > 0.0f;
-      float gwsum = gvalid ? gi_target(A, S.pos, S.n, S.gn, dir0, m, gsel) * cgw.z * cgw.y : 0.0f, gM = cgw.y;
-      for (int t = 0; t < 4; ++t) {
-        const float ox = pcg_rand(seed.state), oy = pcg_rand(seed.state);
-        const int nx = (int)x + (int)((ox * 2.0f - 1.0f) * 16.0f), ny = (int)y + (int)((oy * 2.0f - 1.0f) * 16.0f);
-        if (nx < 0 || nx >= (int)A.W || ny < 0 || ny >= (int)A.H) continue;
-        const uint32_t j = (uint32_t)ny * A.W + (uint32_t)nx;
-        const float4 q = A.gPos[j];
-        if (!compatible(gp, gn, q, A.gNrm[j])) continue;
-        const float4 nw = A.giW[j], np = A.giPos[j], nn = A.giNrm[j];
-        if (nw.y <= 0.0f || nw.z <= 0.0f || np.w <= 0.0f || nn.w <= 0.0f) continue;
-        if (!gi_accepts_shift(S.pos, f3(q.x, q.y, q.z), f3(np.x, np.y, np.z), f3(nn.x, nn.y, nn.z))) continue;
-        const GISample ns = gi_load(A.giPos, A.giNrm, A.giRad, A.giW, j);
-        const float w = gi_target(A, S.pos, S.n, S.gn, dir0, m, ns) * nw.z * nw.y;
-        gwsum += w;
-        gM += nw.y;
-        if (rand_decision(seed) * gwsum < w) {
-          gsel = ns;
-          gvalid = true;
-        }
-      }
-      const float gHat = gvalid ? gi_target(A, S.pos, S.n, S.gn, dir0, m, gsel) : 0.0f;
-      const float gW = gM > 0.0f && gHat > 0.0f ? gwsum / (gM * gHat) : 0.0f;
-      if (gW > 0.0f && gi_visible(A, S.pos, S.gn, gsel.pos, S.err, stack)) {
-        const float3 dir = normalize3(sub(gsel.pos, S.pos));
-        Lanes Ls;
-        if (A.spectral) Ls = make_lanes(A, gsel.u);
-        float pdf;
-        const float f = lambert_eval(S.n, S.gn, mul(dir0, -1.0f), dir, pdf);
-        const float geometry = gi_geometry(S.pos, S.n, gsel.pos, gsel.nrm);
-        R = add(R, to_rgb(A, Ls, scale4(mul4(reflectance(A, Ls, m), gsel.rad), f * geometry * gW)));
-      }
-    }
-    const float spreadLimit = kNrc ? nrc_spread_limit(A, gp.w, S.gn, dir0) : 0.0f;
-    R = add(R, continue_path<kPbr, kNrc>(A, L, S, m, dir0, seed, stack, true, spreadLimit, slot, &queried));
-  }
-  if (kNrc && !queried) nrc_store_none(A, slot);
-  if (!isfinite(R.x) || !isfinite(R.y) || !isfinite(R.z)) return;
-  double *acc = A.accum + 3 * (size_t)i;
-  acc[0] += R.x; acc[1] += R.y; acc[2] += R.z;
-}
-
 // Work item i = (sample group g, pixel p), pixel-major within a group so that a warp traces
 // neighbouring pixels; a group covers `per` consecutive samples of the call. Each item adds its
 // FP64 sum to the pixel with one atomic per channel (groups > 1) or a plain add (groups = 1).
-template <bool kPbr, bool kNrc = false>
+template <bool kPbr>
 __global__ void __launch_bounds__(kRenderBlock, kPbr ? 3 : 4) k_render(RenderArgs A, uint32_t groups, uint32_t per) {
   int stack[kRenderStack];
   const uint32_t npix = A.OW * A.OH;  // accumulation pixels: the frame's pixels (s i, s j)
@@ -1843,8 +1540,7 @@ __global__ void __launch_bounds__(kRenderBlock, kPbr ? 3 : 4) k_render(RenderArg
     const uint32_t k0 = g * per, k1 = min(A.spp, k0 + per);
     double sr = 0.0, sg = 0.0, sb = 0.0;
     for (uint32_t k = k0; k < k1; ++k) {
-      const float3 c = path_sample<kPbr, kNrc>(A, x, y, A.first + k, A.firstFrame + k, A.jitter[k], stack,
-                                               (size_t)k * npix + p);
+      const float3 c = path_sample<kPbr>(A, x, y, A.first + k, A.firstFrame + k, A.jitter[k], stack);
       sr += c.x;
       sg += c.y;
       sb += c.z;
@@ -1891,7 +1587,7 @@ __device__ __forceinline__ float2 frame_jitter(uint32_t sampleIndex) {
 // summed in k_render's order) to its pixel's FP64 accumulation.
 constexpr int kWfBlock = 256;
 constexpr uint32_t kWfShadow = 1u, kWfShadowPrimary = 2u, kWfEmissionOnly = 4u, kWfPrevMIS = 8u, kWfQueried = 16u,
-                   kWfDead = 32u, kWfPrevDelta = 64u;
+                   kWfDead = 32u, kWfPrevDelta = 64u, kWfGiPrimary = 128u;
 
 struct WfArgs {
   float4 *T;      // throughput per lane
@@ -1913,12 +1609,18 @@ struct WfArgs {
   uint32_t *shQ, *shCount;        // shadow rays of this bounce
   uint32_t *grpQ;                 // the live queue regrouped by material (k_wf_group)
   uint32_t npix, paths, k0;       // accumulation pixels; paths of the pass; its first sample (of the call)
+  uint32_t p0;                    // the pass's first pixel (sampling mode 0: a band of one frame; else 0)
+  // Sampling mode 0: the GI reservoir's connection from the primary vertex.
+  float4 *gray;                   // its shadow ray (vt_ray)
+  float4 *gcon;                   // its contribution (rgb)
+  const uint8_t *gocc;            // its occlusion
+  uint32_t *giQ, *giCount;        // paths with a connection
   uint32_t compact;               // 1: this bounce compacts the live queue; 0: it keeps every entry in
                                   // place (ended paths flagged kWfDead, their next ray empty)
   uint32_t deadFlags;             // 1: some bounce of the pass keeps ended paths queued
 };
-// The cache's query slot of path i: sample k0 + i / npix of pixel i % npix (k_render's slots).
-__device__ __forceinline__ size_t wf_slot(const WfArgs &W, uint32_t i) { return (size_t)W.k0 * W.npix + i; }
+// The cache's query slot of path i: sample k0 + i / npix of pixel p0 + i % npix (k_render's slots).
+__device__ __forceinline__ size_t wf_slot(const WfArgs &W, uint32_t i) { return (size_t)W.k0 * W.npix + W.p0 + i; }
 
 __device__ __forceinline__ void wf_store_seed(const WfArgs &W, uint32_t i, const Sampler &s) {
   W.seedA[i] = make_uint4(s.state, s.key, s.dimension, s.sub);
@@ -2013,9 +1715,57 @@ __device__ __forceinline__ bool wf_nee(const RenderArgs &A, const WfArgs &W, uin
   return true;
 }
 
+// continue_path's loop head at bounce nb: the BSDF continuation from vertex S (material m, met along
+// `dir`). Stores the next ray, the vertex and the throughput and returns whether the path goes on;
+// `mis`: an emitter the continuation meets is weighed against NEE (previousMIS).
+template <bool kPbr>
+__device__ __forceinline__ bool wf_continue(const RenderArgs &A, const WfArgs &W, uint32_t i, uint32_t nb, const Lanes &L,
+                                            const Surface &S, const vt_material &m, float3 dir, float4 T, Sampler &seed,
+                                            int &scattering, bool &emissionOnly, bool mis, float u, uint32_t &flags) {
+  const int limit = max(0, (int)A.maxDepth - 1);
+  const bool delta = is_delta<kPbr>(A, m);
+  if (!delta && scattering >= limit) {
+    const bool stop = A.mode != 3u || emissionOnly;
+    emissionOnly = true;
+    if (stop) return false;
+  }
+  if (!delta) ++scattering;
+  sampler_event(seed, nb, kZBsdf);
+  float3 nd;
+  float bpdf;
+  if (delta) {
+    float4 w;
+    bpdf = 0.0f;
+    if (!sample_delta(A, L, m, S.n, S.gn, dir, S.front, seed, nd, w)) return false;
+    T = mul4(T, w);
+  } else {
+    const float3 r = rand_f3(seed);
+    if (is_pbr<kPbr>(A, m)) {
+      float4 w;
+      if (!pbr_sample_lanes(A, L, m, S.n, S.gn, S.tri, mul(dir, -1.0f), r, nd, w, bpdf)) return false;
+      T = mul4(T, w);
+    } else {
+      nd = cosine_hemisphere(S.n, r.y, r.z);
+      bpdf = fmaxf(0.0f, dot3(S.n, nd)) * kInvPi;
+      if (!(bpdf > 0.0f) || !(dot3(nd, S.gn) > 0.0f)) return false;
+      T = mul4(T, reflectance(A, L, m));
+    }
+  }
+  if (!isfinite(T.x) || !isfinite(T.y) || !isfinite(T.z) || !isfinite(T.w) || max4(A, T) <= 0.0f) return false;
+  const float3 no = ray_origin(A, S.pos, S.gn, nd, S.err);
+  wf_set_ray(W.ray, i, no, ray_tmin(A, no), nd, __int_as_float(0x7f800000));
+  W.prev[i] = make_float4(S.pos.x, S.pos.y, S.pos.z, bpdf);
+  W.prevN[i] = make_float4(S.n.x, S.n.y, S.n.z, u);
+  W.T[i] = T;
+  flags = mis ? (flags | kWfPrevMIS) : (flags & ~kWfPrevMIS);
+  flags = delta ? (flags | kWfPrevDelta) : (flags & ~kWfPrevDelta);
+  return true;
+}
+
 // One vertex of path i at bounce b (0: the primary hit). Sets `next` when the path continues and
-// `shadow` when it queued a shadow ray. kNrc: the path ends with a cache query where continue_path's
-// query rule stops it (vt_render_nrc).
+// `shadow` when it queued a shadow ray. kNrc (vt_render_nrc): the path ends, after the vertex's
+// emission, at vertex A.nrcVertex, or with A.nrcVertex 0 at the first vertex where its spread exceeds
+// its limit (nrc_spread_limit), with its cache query stored in its slot.
 template <bool kPbr, bool kNrc>
 __device__ __forceinline__ void wf_vertex(const RenderArgs &A, const WfArgs &W, uint32_t i, uint32_t b, bool &next,
                                           bool &shadow) {
@@ -2113,7 +1863,9 @@ __device__ __forceinline__ void wf_vertex(const RenderArgs &A, const WfArgs &W, 
         flags |= kWfQueried;
         alive = false;
       } else {
-        if (nee && !delta) {
+        // The secondary diffuse vertex of a path with a GI reservoir takes no NEE (the reservoir
+        // estimates its direct light).
+        if (nee && !delta && !(b == 1u && (flags & kWfGiPrimary) && m.type == VT_MAT_DIFFUSE)) {
           sampler_event(seed, b + 1u, kZNee);
           if (wf_nee<kPbr>(A, W, i, L, S, mul(dir, -1.0f), T, m, mis && scattering < limit, scattering < limit, seed, false)) {
             shadow = true;
@@ -2129,50 +1881,8 @@ __device__ __forceinline__ void wf_vertex(const RenderArgs &A, const WfArgs &W, 
       }
     }
   }
-  if (alive) {  // continue_path's loop head at bounce b + 1: the BSDF continuation
-    const uint32_t nb = b + 1u;
-    const bool delta = is_delta<kPbr>(A, m);
-    if (!delta && scattering >= limit) {
-      if (nee || emissionOnly) alive = false;
-      emissionOnly = true;
-    }
-    if (alive) {
-      if (!delta) ++scattering;
-      sampler_event(seed, nb, kZBsdf);
-      float3 nd;
-      float bpdf;
-      if (delta) {
-        float4 w;
-        bpdf = 0.0f;
-        if (!sample_delta(A, L, m, S.n, S.gn, dir, S.front, seed, nd, w)) alive = false;
-        else T = mul4(T, w);
-      } else {
-        const float3 r = rand_f3(seed);
-        if (is_pbr<kPbr>(A, m)) {
-          float4 w;
-          if (!pbr_sample_lanes(A, L, m, S.n, S.gn, S.tri, mul(dir, -1.0f), r, nd, w, bpdf)) alive = false;
-          else T = mul4(T, w);
-        } else {
-          nd = cosine_hemisphere(S.n, r.y, r.z);
-          bpdf = fmaxf(0.0f, dot3(S.n, nd)) * kInvPi;
-          if (!(bpdf > 0.0f) || !(dot3(nd, S.gn) > 0.0f)) alive = false;
-          else T = mul4(T, reflectance(A, L, m));
-        }
-      }
-      if (alive && (!isfinite(T.x) || !isfinite(T.y) || !isfinite(T.z) || !isfinite(T.w) || max4(A, T) <= 0.0f))
-        alive = false;
-      if (alive) {
-        const float3 no = ray_origin(A, S.pos, S.gn, nd, S.err);
-        wf_set_ray(W.ray, i, no, ray_tmin(A, no), nd, __int_as_float(0x7f800000));
-        W.prev[i] = make_float4(S.pos.x, S.pos.y, S.pos.z, bpdf);
-        W.prevN[i] = make_float4(S.n.x, S.n.y, S.n.z, pn.w);
-        W.T[i] = T;
-        flags = mis ? (flags | kWfPrevMIS) : (flags & ~kWfPrevMIS);
-        flags = delta ? (flags | kWfPrevDelta) : (flags & ~kWfPrevDelta);
-        next = true;
-      }
-    }
-  }
+  if (alive)
+    next = wf_continue<kPbr>(A, W, i, b + 1u, L, S, m, dir, T, seed, scattering, emissionOnly, mis, pn.w, flags);
   flags = emissionOnly ? (flags | kWfEmissionOnly) : (flags & ~kWfEmissionOnly);
   W.meta[i] = make_uint4(meta.x, next ? b + 1u : b, (uint32_t)scattering, flags);
   W.Rc[i] = Rc;
@@ -2185,7 +1895,7 @@ __device__ __forceinline__ void wf_vertex(const RenderArgs &A, const WfArgs &W, 
 // of accumulation pixel i % npix.
 __global__ void __launch_bounds__(kWfBlock) k_wf_generate(RenderArgs A, WfArgs W) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < W.paths; i += gridDim.x * blockDim.x) {
-    const uint32_t p = i % W.npix, k = W.k0 + i / W.npix;
+    const uint32_t p = W.p0 + i % W.npix, k = W.k0 + i / W.npix;
     const uint32_t x = (p % A.OW) * A.stride, y = (p / A.OW) * A.stride;
     Sampler seed = pixel_sampler(x, y, A.W, A.first + k, A.zSampler != 0u, A.zModel, A.firstFrame + k);
     const float u = A.spectral ? wavelength_numbers(seed).x : 0.0f;
@@ -2255,6 +1965,395 @@ __global__ void __launch_bounds__(kWfBlock) k_wf_finish(RenderArgs A, WfArgs W) 
     atomicAdd(acc, (double)R.x);
     atomicAdd(acc + 1, (double)R.y);
     atomicAdd(acc + 2, (double)R.z);
+  }
+}
+
+// ---- ReSTIR frames through the wavefront stages (sampling mode 0) ---------------------------------
+// A frame k, per band of at most 4M pixels (path i of a band is pixel p0 + i):
+//   k_wf_generate, extend      camera rays and their hits;
+//   k_di_primary               the primary-surface cache, the DI reservoir, the GI candidate's ray;
+//   extend, k_gi_secondary     the candidate's vertex x2, its NEE sample's shadow ray; shadow;
+//   k_gi_merge                 the GI reservoir;
+// then, once every band has its reservoirs (spatial reuse reads neighbours), per band:
+//   k_di_shade                 spatial reuse; the primary's radiance, its shadow rays, the path's
+//                              first continuation; shadow (NEE or DI sample, GI connection);
+//   k_gi_connect               adds the visible GI connections;
+//   extend, k_wf_shade, shadow per bounce from 1, then k_wf_finish, as for the other modes.
+// Bound: latency and divergence of the stages, as the other modes'. One kernel per pass with
+// inline traversals (a thread per pixel, local-memory stacks) idled most lanes in its longest path.
+// Measured on one B200: four 1001 x 563 frames of a 300,000-triangle scene at depth 6 with 16
+// candidates 43 -> 26 ms.
+
+// restir_temporal_kernel (main.swift:4842-5005) up to the GI candidate: the primary hit into the
+// primary-surface cache, then at a diffuse (Lambert) hit the initial reservoir (RIS over the frame's
+// candidates, restir_di_initial, main.swift:4638-4668), merged with the previous frame's reservoir
+// of the backprojected pixel when it saw the same surface (restir_di_merge, main.swift:4686-4699,
+// confidence capped at 20), stored with W = wsum / (M p_hat) (restir_di_encode); then, with a
+// scattering budget, the direction of the GI candidate (restir_gi_initial, main.swift:4718-4770: one
+// BSDF sample). Other primaries get empty reservoirs and shade with NEE (main.swift:4931-4943).
+// Leaves the camera ray's direction and wavelength number in W.T, the BSDF pdf in W.prev.w, the
+// sampler in W.seedA/B.
+template <bool kPbr>
+__global__ void __launch_bounds__(kRenderBlock) k_di_primary(RenderArgs A, WfArgs W) {
+  __shared__ uint32_t sTotal, sBase;
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  bool push = false;
+  [&] {  // one pixel; every thread of the block joins the queue push below
+    if (i >= W.paths) return;
+    const uint32_t p = W.p0 + i, k = W.k0, x = p % A.W, y = p / A.W;
+    Sampler seed = pixel_sampler(x, y, A.W, A.first + k, A.zSampler != 0u, A.zModel, A.firstFrame + k);
+    const float u = A.spectral ? wavelength_numbers(seed).x : 0.0f;
+    float3 dir0 = camera_dir(A, x, y, A.jitter[k]), o0 = A.cam;
+    lens_ray(A, o0, dir0, seed);
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const int4 h4 = W.hit[i];
+    Hit h;
+    h.t = __int_as_float(h4.x); h.b1 = __int_as_float(h4.y); h.b2 = __int_as_float(h4.z); h.pos = h4.w;
+    if (h.pos < 0) {
+      A.gPos[p] = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
+      A.gNrm[p] = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
+      A.rPos[p] = zero; A.rEmit[p] = zero; A.rW[p] = zero;
+      A.giPos[p] = zero; A.giNrm[p] = zero; A.giRad[p] = zero; A.giW[p] = zero;
+      return;
+    }
+    const Surface S = surface_at(A, h, o0, dir0);
+    const vt_material m = material(A, S.slot);
+    const float4 gp = make_float4(S.pos.x, S.pos.y, S.pos.z, h.t), gn = make_float4(S.n.x, S.n.y, S.n.z, float(m.type));
+    A.gPos[p] = gp;
+    A.gNrm[p] = gn;
+    A.gGeo[p] = make_float4(S.gn.x, S.gn.y, S.gn.z, 0.0f);
+    A.gInfo[p] = make_uint4(S.face, S.slot | (S.front ? 0x80000000u : 0u), __float_as_uint(S.err), S.tri);
+    // The GI reservoir is empty until k_gi_secondary and k_gi_merge fill it (depth 1 has no indirect
+    // bounce for it, restir_gi_enabled, main.swift:3476-3478).
+    A.giPos[p] = zero; A.giNrm[p] = zero; A.giRad[p] = zero; A.giW[p] = zero;
+    if (m.type != VT_MAT_DIFFUSE) {
+      A.rPos[p] = zero; A.rEmit[p] = zero; A.rW[p] = zero;
+      return;
+    }
+    DIReservoir r;
+    r.s.pos = f3(0.0f, 0.0f, 0.0f); r.s.emission = f3(0.0f, 0.0f, 0.0f);
+    r.s.pdf = 0.0f; r.s.u = u; r.s.id = 0u;
+    r.wsum = 0.0f;
+    r.M = 0.0f;
+    for (uint32_t c = 0; c < A.diCandidates; ++c) {
+      sampler_candidate(seed, 1u, kZDi, c, A.diBits);
+      const LightSample ls = sample_direct(A, S.pos, S.n, seed, (int)A.maxDepth - 1 > 0);
+      r.M += 1.0f;  // zero-weight candidates still count
+      if (!(ls.pdf > 0.0f)) continue;
+      DISample cand;
+      cand.pos = ls.pos; cand.emission = ls.emission; cand.pdf = ls.pdf; cand.u = u;
+      cand.id = ls.face == 0xffffffffu ? 0u : ls.face + 2u;
+      const float pHat = di_target<kPbr>(A, S.pos, S.n, S.gn, S.tri, dir0, m, cand);
+      const float proposal = cand.pdf * light_geometry(A, S.pos, cand);
+      const float w = proposal > 0.0f ? pHat / proposal : 0.0f;
+      r.wsum += w;
+      if (rand_decision(seed) * r.wsum < w) r.s = cand;
+    }
+    int px, py;
+    if (backproject(A, S.pos, px, py)) {
+      const uint32_t j = (uint32_t)py * A.W + (uint32_t)px;
+      const float4 hw = A.hrW[j];
+      if (same_surface(gp, gn, A.hPos[j], A.hNrm[j]) && hw.y > 0.0f && hw.z > 0.0f) {
+        const DISample hs = load_di(A.hrPos, A.hrEmit, A.hrW, j);
+        const float cM = fminf(hw.y, 20.0f);
+        const float w = di_target<kPbr>(A, S.pos, S.n, S.gn, S.tri, dir0, m, hs) * hw.z * cM;
+        r.M += cM;
+        r.wsum += w;
+        if (rand_decision(seed) * r.wsum < w) r.s = hs;
+      }
+    }
+    const float pHat = di_target<kPbr>(A, S.pos, S.n, S.gn, S.tri, dir0, m, r.s);
+    const float Wr = r.M > 0.0f && pHat > 0.0f ? r.wsum / (r.M * pHat) : 0.0f;
+    A.rPos[p] = make_float4(r.s.pos.x, r.s.pos.y, r.s.pos.z, __uint_as_float(r.s.id));
+    A.rEmit[p] = make_float4(r.s.emission.x, r.s.emission.y, r.s.emission.z, r.s.pdf);
+    A.rW[p] = make_float4(r.wsum, r.M, Wr, r.s.u);
+    if ((int)A.maxDepth - 1 < 1) return;
+    sampler_event(seed, 1u, kZGiBsdf);
+    const float3 rr = rand_f3(seed);  // sample_bsdf's Lambert branch: the direction from the last two
+    const float3 gd = cosine_hemisphere(S.n, rr.y, rr.z);
+    const float bpdf = fmaxf(0.0f, dot3(S.n, gd)) * kInvPi;
+    push = bpdf > 0.0f && dot3(gd, S.gn) > 0.0f;
+    if (push) {
+      const float3 o = ray_origin(A, S.pos, S.gn, gd, S.err);
+      wf_set_ray(W.ray, i, o, ray_tmin(A, o), gd, __int_as_float(0x7f800000));
+    }
+    W.T[i] = make_float4(dir0.x, dir0.y, dir0.z, u);
+    W.prev[i] = make_float4(0.0f, 0.0f, 0.0f, bpdf);
+    W.meta[i] = make_uint4(p, 0u, 0u, 0u);
+    wf_store_seed(W, i, seed);
+  }();
+  wf_push(push, i, W.outQ, W.outCount, sTotal, sBase);
+}
+
+// restir_gi_initial (main.swift:4718-4770) at the candidate's hit x2 (diffuse, or there is no
+// candidate): position, normal, source pdf and the radiance of one NEE sample, its visibility
+// pending (kWfShadow).
+__global__ void __launch_bounds__(kWfBlock) k_gi_secondary(RenderArgs A, WfArgs W) {
+  __shared__ uint32_t sTotal, sBase;
+  const uint32_t n = min(*W.inCount, W.paths);
+  for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
+    const uint32_t q = base + threadIdx.x;
+    uint32_t i = 0;
+    bool shadow = false;
+    if (q < n) {
+      i = W.inQ[q];
+      const uint32_t p = W.p0 + i;
+      const int4 h4 = W.hit[i];
+      Hit h;
+      h.t = __int_as_float(h4.x); h.b1 = __int_as_float(h4.y); h.b2 = __int_as_float(h4.z); h.pos = h4.w;
+      if (h.pos >= 0) {
+        const float4 r0 = W.ray[2 * (size_t)i], r1 = W.ray[2 * (size_t)i + 1];
+        const float3 gd = f3(r1.x, r1.y, r1.z);
+        const Surface S2 = surface_at(A, h, f3(r0.x, r0.y, r0.z), gd);
+        const vt_material m2 = material(A, S2.slot);
+        if (m2.type == VT_MAT_DIFFUSE) {
+          const int limit = max(0, (int)A.maxDepth - 1);
+          const float u = W.T[i].w, bpdf = W.prev[i].w;
+          Lanes L;
+          if (A.spectral) L = make_lanes(A, u);
+          Sampler seed = wf_load_seed(W, i);
+          float4 rad = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          sampler_event(seed, 2u, kZGiNee);
+          const LightSample ls = sample_direct(A, S2.pos, S2.n, seed, limit >= 2);
+          float3 so, sd;
+          float tmax;
+          if (ls.pdf > 0.0f && shadow_ray(A, S2.pos, S2.gn, S2.err, ls, so, sd, tmax)) {
+            const float c2 = fmaxf(0.0f, dot3(S2.n, ls.wi));
+            float pdf2;
+            const float f2 = lambert_eval(S2.n, S2.gn, mul(gd, -1.0f), ls.wi, pdf2);
+            // The power heuristic only when a second continuation can sample x2's BSDF
+            // (restir_gi_has_complementary_bsdf, main.swift:3482-3484).
+            const float mis = limit >= 2 ? power_heuristic(ls.pdf, pdf2) : 1.0f;
+            const float le[3] = {ls.emission.x, ls.emission.y, ls.emission.z};
+            rad = scale4(mul4(reflectance(A, L, m2), emission(A, L, le)), f2 * c2 * mis / ls.pdf);
+            wf_set_ray(W.sray, i, so, ray_tmin(A, so), sd, tmax);
+            shadow = true;
+          }
+          const float4 gp = A.gPos[p];
+          const float3 delta = sub(S2.pos, f3(gp.x, gp.y, gp.z));
+          const float d2 = dot3(delta, delta);
+          const float cos2 = fmaxf(0.0f, -dot3(S2.n, gd));
+          A.giPos[p] = make_float4(S2.pos.x, S2.pos.y, S2.pos.z, d2 > 1e-10f ? bpdf * cos2 / d2 : 0.0f);
+          A.giNrm[p] = make_float4(S2.n.x, S2.n.y, S2.n.z, 1.0f);
+          A.giRad[p] = rad;
+          wf_store_seed(W, i, seed);
+          if (shadow) W.meta[i].w = kWfShadow;
+        }
+      }
+    }
+    wf_push(shadow, i, W.shQ, W.shCount, sTotal, sBase);
+  }
+}
+
+// The GI reservoir: the candidate's weight, the merge with the previous frame's reservoir of the
+// backprojected pixel (restir_gi_merge, main.swift:4775-4795) and its encoding (:4797-4806).
+__global__ void __launch_bounds__(kWfBlock) k_gi_merge(RenderArgs A, WfArgs W) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= W.paths) return;
+  const uint32_t p = W.p0 + i;
+  const float4 gp = A.gPos[p], gn = A.gNrm[p];
+  if (!(gp.w > 0.0f) || gn.w != float(VT_MAT_DIFFUSE)) return;
+  const uint4 info = A.gInfo[p];
+  const float4 gg = A.gGeo[p], view4 = W.T[i];
+  const float3 pos = f3(gp.x, gp.y, gp.z), nrm = f3(gn.x, gn.y, gn.z), geo = f3(gg.x, gg.y, gg.z),
+               view = f3(view4.x, view4.y, view4.z);
+  const vt_material m = material(A, info.y & 0x7fffffffu);
+  Sampler seed = wf_load_seed(W, i);
+  GISample g;
+  g.pos = g.nrm = f3(0.0f, 0.0f, 0.0f);
+  g.rad = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  g.pdf = 0.0f;
+  g.u = view4.w;
+  float gwsum = 0.0f, gM = 1.0f;
+  const float4 cn = A.giNrm[p];
+  if (cn.w > 0.0f) {
+    const float4 cp = A.giPos[p];
+    GISample c;
+    c.pos = f3(cp.x, cp.y, cp.z);
+    c.nrm = f3(cn.x, cn.y, cn.z);
+    c.rad = A.giRad[p];
+    c.pdf = cp.w;
+    c.u = view4.w;
+    if ((W.meta[i].w & kWfShadow) && W.occ[i]) c.rad = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const float pHat = gi_target(A, pos, nrm, geo, view, m, c);
+    if (c.pdf > 0.0f && pHat > 0.0f) {
+      g = c;
+      gwsum = pHat / c.pdf;
+    }
+  }
+  int px, py;
+  if (backproject(A, pos, px, py)) {
+    const uint32_t j = (uint32_t)py * A.W + (uint32_t)px;
+    const float4 ow = A.hgiW[j], op = A.hgiPos[j], on = A.hgiNrm[j], hp = A.hPos[j];
+    if (same_surface(gp, gn, hp, A.hNrm[j]) && ow.y > 0.0f && ow.z > 0.0f && op.w > 0.0f && on.w > 0.0f) {
+      const GISample hs = gi_load(A.hgiPos, A.hgiNrm, A.hgiRad, A.hgiW, j);
+      if (gi_accepts_shift(pos, f3(hp.x, hp.y, hp.z), hs.pos, hs.nrm)) {
+        const float cM = fminf(ow.y, 20.0f);
+        const float w = gi_target(A, pos, nrm, geo, view, m, hs) * ow.z * cM;
+        gM += cM;
+        gwsum += w;
+        if (pcg_rand(seed.state) * gwsum < w) g = hs;
+      }
+    }
+  }
+  const float gHat = gi_target(A, pos, nrm, geo, view, m, g);
+  const float gW = gM > 0.0f && gHat > 0.0f ? gwsum / (gM * gHat) : 0.0f;
+  A.giPos[p] = make_float4(g.pos.x, g.pos.y, g.pos.z, g.pdf);
+  A.giNrm[p] = make_float4(g.nrm.x, g.nrm.y, g.nrm.z, g.pdf > 0.0f ? 1.0f : 0.0f);
+  A.giRad[p] = g.rad;
+  A.giW[p] = make_float4(gwsum, gM, gW, g.u);
+}
+
+// ReSTIR pass 2 (shading_kernel, main.swift:7484-7656) at the primary vertex: at a diffuse one, spatial
+// reuse of 4 uniform taps in a 32-pixel box that pass RESTIR2020's compatibility test
+// (uniform_neighbor, main.swift:5025-5027), the selected sample's contribution W * bsdf * Le * cos *
+// G when visible; then the same for the GI reservoirs (the reconnection x1 -> x2 shaded with the
+// secondary radiance, W and the area-measure geometry term); other primaries take NEE with MIS
+// (main.swift:7767-7780). Then the path's first continuation. Visibility is pending: the DI or NEE
+// sample's shadow ray goes to the shadow queue, the GI connection's to its own.
+// kNrc: the path goes on toward a cache query, whose prediction covers the GI light.
+template <bool kPbr, bool kNrc>
+__global__ void __launch_bounds__(kRenderBlock) k_di_shade(RenderArgs A, WfArgs W) {
+  __shared__ uint32_t sTotal, sBase;
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  bool next = false, shadow = false, connect = false;
+  [&] {
+    if (i >= W.paths) return;
+    const uint32_t p = W.p0 + i, k = W.k0, x = p % A.W, y = p / A.W;
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    W.Rc[i] = zero;
+    W.Rp[i] = zero;
+    W.meta[i] = make_uint4(p, 0u, 0u, 0u);
+    Sampler seed = pixel_sampler(x, y, A.W, A.first + k, A.zSampler != 0u, A.zModel, A.firstFrame + k);
+    Lanes L;
+    const float u = A.spectral ? wavelength_numbers(seed).x : 0.0f;
+    if (A.spectral) L = make_lanes(A, u);
+    float3 dir0 = camera_dir(A, x, y, A.jitter[k]), o0 = A.cam;
+    lens_ray(A, o0, dir0, seed);  // the same draws as pass 1
+    seed.state = pcg_hash(seed.state ^ 0x27d4eb2fu);  // decorrelate_shading_seed
+    const float4 gp = A.gPos[p];
+    if (gp.w <= 0.0f) return;
+    const float4 gn = A.gNrm[p];
+    const uint4 gi = A.gInfo[p];
+    Surface S;
+    S.pos = f3(gp.x, gp.y, gp.z);
+    S.n = f3(gn.x, gn.y, gn.z);
+    const float4 gg = A.gGeo[p];
+    S.gn = f3(gg.x, gg.y, gg.z);
+    S.face = gi.x;
+    S.slot = gi.y & 0x7fffffffu;
+    S.front = (gi.y >> 31) != 0u;
+    S.err = __uint_as_float(gi.z);
+    S.tri = gi.w;
+    const vt_material m = material(A, S.slot);
+    if (m.type == VT_MAT_EMISSIVE) {
+      const float3 e = primary_emission(A, L, S, m);
+      W.Rp[i] = make_float4(e.x, e.y, e.z, 0.0f);
+      return;
+    }
+    const int limit = max(0, (int)A.maxDepth - 1);
+    const float4 T = A.spectral ? make_float4(1.0f, 1.0f, 1.0f, 1.0f) : make_float4(1.0f, 1.0f, 1.0f, 0.0f);
+    uint32_t flags = 0u;
+    const bool diffuse = m.type == VT_MAT_DIFFUSE;
+    if (!diffuse) {
+      if (!is_delta<kPbr>(A, m)) {  // no NEE at glass or a mirror (main.swift:7657)
+        sampler_event(seed, 1u, kZNee);
+        shadow = wf_nee<kPbr>(A, W, i, L, S, mul(dir0, -1.0f), T, m, limit > 0, limit > 0, seed, true);
+      }
+    } else {
+      const float4 cw = A.rW[p];
+      DISample sel = load_di(A.rPos, A.rEmit, A.rW, p);
+      float wsum = di_target<kPbr>(A, S.pos, S.n, S.gn, S.tri, dir0, m, sel) * cw.z * cw.y, M = cw.y;
+      for (int t = 0; t < 4; ++t) {
+        const float ox = pcg_rand(seed.state), oy = pcg_rand(seed.state);
+        const int nx = (int)x + (int)((ox * 2.0f - 1.0f) * 16.0f), ny = (int)y + (int)((oy * 2.0f - 1.0f) * 16.0f);
+        if (nx < 0 || nx >= (int)A.W || ny < 0 || ny >= (int)A.H) continue;
+        const uint32_t j = (uint32_t)ny * A.W + (uint32_t)nx;
+        if (!compatible(gp, gn, A.gPos[j], A.gNrm[j])) continue;
+        const float4 nw = A.rW[j];
+        if (!(nw.y > 0.0f && nw.z > 0.0f)) continue;
+        const DISample ns = load_di(A.rPos, A.rEmit, A.rW, j);
+        const float w = di_target<kPbr>(A, S.pos, S.n, S.gn, S.tri, dir0, m, ns) * nw.z * nw.y;
+        wsum += w;
+        M += nw.y;
+        if (rand_decision(seed) * wsum < w) sel = ns;
+      }
+      const float pHat = di_target<kPbr>(A, S.pos, S.n, S.gn, S.tri, dir0, m, sel);
+      const float Wr = M > 0.0f && pHat > 0.0f ? wsum / (M * pHat) : 0.0f;
+      float3 so, sd;
+      float tmax;
+      if (Wr > 0.0f && shadow_ray(A, S.pos, S.gn, S.err, di_light_sample(sel, S.pos), so, sd, tmax)) {
+        const float3 c = mul(di_contribution<kPbr>(A, S.pos, S.n, S.gn, S.tri, dir0, m, sel), Wr);
+        W.scon[i] = make_float4(c.x, c.y, c.z, 0.0f);
+        wf_set_ray(W.sray, i, so, ray_tmin(A, so), sd, tmax);
+        shadow = true;
+      }
+      // ReSTIR GI (a cache-terminated path's cache covers this light, so the cache's kernel leaves it out).
+      if (!kNrc && limit >= 1) {
+        const float4 cgw = A.giW[p];
+        GISample gsel = gi_load(A.giPos, A.giNrm, A.giRad, A.giW, p);
+        bool gvalid = A.giNrm[p].w > 0.0f;
+        float gwsum = gvalid ? gi_target(A, S.pos, S.n, S.gn, dir0, m, gsel) * cgw.z * cgw.y : 0.0f, gM = cgw.y;
+        for (int t = 0; t < 4; ++t) {
+          const float ox = pcg_rand(seed.state), oy = pcg_rand(seed.state);
+          const int nx = (int)x + (int)((ox * 2.0f - 1.0f) * 16.0f), ny = (int)y + (int)((oy * 2.0f - 1.0f) * 16.0f);
+          if (nx < 0 || nx >= (int)A.W || ny < 0 || ny >= (int)A.H) continue;
+          const uint32_t j = (uint32_t)ny * A.W + (uint32_t)nx;
+          const float4 q = A.gPos[j];
+          if (!compatible(gp, gn, q, A.gNrm[j])) continue;
+          const float4 nw = A.giW[j], np = A.giPos[j], nn = A.giNrm[j];
+          if (nw.y <= 0.0f || nw.z <= 0.0f || np.w <= 0.0f || nn.w <= 0.0f) continue;
+          if (!gi_accepts_shift(S.pos, f3(q.x, q.y, q.z), f3(np.x, np.y, np.z), f3(nn.x, nn.y, nn.z))) continue;
+          const GISample ns = gi_load(A.giPos, A.giNrm, A.giRad, A.giW, j);
+          const float w = gi_target(A, S.pos, S.n, S.gn, dir0, m, ns) * nw.z * nw.y;
+          gwsum += w;
+          gM += nw.y;
+          if (rand_decision(seed) * gwsum < w) {
+            gsel = ns;
+            gvalid = true;
+          }
+        }
+        const float gHat = gvalid ? gi_target(A, S.pos, S.n, S.gn, dir0, m, gsel) : 0.0f;
+        const float gW = gM > 0.0f && gHat > 0.0f ? gwsum / (gM * gHat) : 0.0f;
+        if (gW > 0.0f && gi_ray(A, S.pos, S.gn, gsel.pos, S.err, so, sd, tmax)) {
+          const float3 dir = normalize3(sub(gsel.pos, S.pos));
+          Lanes Ls;
+          if (A.spectral) Ls = make_lanes(A, gsel.u);
+          float pdf;
+          const float f = lambert_eval(S.n, S.gn, mul(dir0, -1.0f), dir, pdf);
+          const float geometry = gi_geometry(S.pos, S.n, gsel.pos, gsel.nrm);
+          const float3 c = to_rgb(A, Ls, scale4(mul4(reflectance(A, Ls, m), gsel.rad), f * geometry * gW));
+          W.gcon[i] = make_float4(c.x, c.y, c.z, 0.0f);
+          wf_set_ray(W.gray, i, so, ray_tmin(A, so), sd, tmax);
+          connect = true;
+        }
+      }
+      if (!kNrc) flags |= kWfGiPrimary;
+    }
+    if (shadow) flags |= kWfShadow | kWfShadowPrimary;
+    if (kNrc) W.spread[i] = make_float2(0.0f, nrc_spread_limit(A, gp.w, S.gn, dir0));
+    // A BSDF hit on an emitter from a vertex whose direct light came from its reservoir gets no weight
+    // (previousMIS false, main.swift:7717-7718).
+    int scattering = 0;
+    bool emissionOnly = false;
+    next = wf_continue<kPbr>(A, W, i, 1u, L, S, m, dir0, T, seed, scattering, emissionOnly, !diffuse, u, flags);
+    if (emissionOnly) flags |= kWfEmissionOnly;
+    W.meta[i] = make_uint4(p, next ? 1u : 0u, (uint32_t)scattering, flags);
+    if (next) wf_store_seed(W, i, seed);
+  }();
+  wf_push(next, i, W.outQ, W.outCount, sTotal, sBase);
+  wf_push(shadow, i, W.shQ, W.shCount, sTotal, sBase);
+  wf_push(connect, i, W.giQ, W.giCount, sTotal, sBase);
+}
+
+// Adds the visible GI connections to their paths' primary radiance.
+__global__ void __launch_bounds__(kWfBlock) k_gi_connect(WfArgs W) {
+  const uint32_t n = min(*W.giCount, W.paths);
+  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+    const uint32_t i = W.giQ[q];
+    if (W.gocc[i]) continue;
+    const float4 R = W.Rp[i], c = W.gcon[i];
+    W.Rp[i] = make_float4(R.x + c.x, R.y + c.y, R.z + c.z, 0.0f);
   }
 }
 
@@ -2475,7 +2574,7 @@ __global__ void __launch_bounds__(256) k_render_batch(const RenderArgs *__restri
       const uint32_t x = p % A.W, y = p / A.W, f0 = firstSample[lo], fr0 = firstFrame[lo];
       double sr = 0.0, sg = 0.0, sb = 0.0;
       for (uint32_t k = 0; k < A.spp; ++k) {
-        const float3 c = path_sample<kPbr, false>(A, x, y, f0 + k, fr0 + k, frame_jitter(f0 + k), stack);
+        const float3 c = path_sample<kPbr>(A, x, y, f0 + k, fr0 + k, frame_jitter(f0 + k), stack);
         sr += c.x; sg += c.y; sb += c.z;
       }
       double *acc = A.accum + 3 * (size_t)p;
@@ -2719,6 +2818,7 @@ void scene_free(vt_scene *scene) {
   cudaFree(scene->d_face_pos);
   cudaFree(scene->d_di);
   cudaFree(scene->d_wf);
+  cudaFree(scene->d_wf_gi);
   cudaFree(scene->d_env_img);
   cudaFree(scene->d_env_rows);
   cudaFree(scene->d_env_cols);
@@ -3083,6 +3183,210 @@ vt_status nrc_finish(vt_ctx *ctx, vt_nrc *nrc, const RenderArgs &A, uint32_t spp
   return VT_OK;
 }
 
+// ---- wavefront integrator: host side ------------------------------------------------------------
+// Paths per pass: as many whole samples of the frame as fit 4M paths (about 1 GB of state).
+constexpr uint32_t kWfMaxPaths = 1u << 22;
+
+// The wavefront state's buffers that the host hands to the stages: the two live queues, their counts
+// (words 0, 1), the shadow (2), grouping (3, 4) and GI connection (5) counts, hits and occlusion.
+struct WfBuffers {
+  uint32_t *q[2], *counts;
+  uint8_t *occ;
+  int4 *hit;
+};
+
+// Bytes of wavefront state for `cap` paths (each array 256-byte aligned), and its arrays at `base`.
+size_t wf_carve(unsigned char *base, uint32_t cap, WfArgs &W, WfBuffers &B) {
+  size_t off = 0;
+  auto take = [&](size_t bytes) {
+    unsigned char *p = base ? base + off : nullptr;
+    off += (bytes + 255) & ~size_t(255);
+    return p;
+  };
+  const size_t n = cap;
+  W.T = reinterpret_cast<float4 *>(take(16 * n));
+  W.Rc = reinterpret_cast<float4 *>(take(16 * n));
+  W.Rp = reinterpret_cast<float4 *>(take(16 * n));
+  W.prev = reinterpret_cast<float4 *>(take(16 * n));
+  W.prevN = reinterpret_cast<float4 *>(take(16 * n));
+  W.seedA = reinterpret_cast<uint4 *>(take(16 * n));
+  W.seedB = reinterpret_cast<uint2 *>(take(8 * n));
+  W.meta = reinterpret_cast<uint4 *>(take(16 * n));
+  W.spread = reinterpret_cast<float2 *>(take(8 * n));
+  W.ray = reinterpret_cast<float4 *>(take(32 * n));
+  B.hit = reinterpret_cast<int4 *>(take(16 * n));
+  W.sray = reinterpret_cast<float4 *>(take(32 * n));
+  W.scon = reinterpret_cast<float4 *>(take(16 * n));
+  B.occ = reinterpret_cast<uint8_t *>(take(n));
+  B.q[0] = reinterpret_cast<uint32_t *>(take(4 * n));
+  B.q[1] = reinterpret_cast<uint32_t *>(take(4 * n));
+  W.shQ = reinterpret_cast<uint32_t *>(take(4 * n));
+  W.grpQ = reinterpret_cast<uint32_t *>(take(4 * n));
+  B.counts = reinterpret_cast<uint32_t *>(take(64));
+  W.hit = B.hit;
+  W.occ = B.occ;
+  W.p0 = 0u;
+  return off;
+}
+
+// The connection arrays of sampling mode 0.
+size_t wf_carve_gi(unsigned char *base, uint32_t cap, WfArgs &W, uint8_t **occ) {
+  size_t off = 0;
+  auto take = [&](size_t bytes) {
+    unsigned char *p = base ? base + off : nullptr;
+    off += (bytes + 255) & ~size_t(255);
+    return p;
+  };
+  const size_t n = cap;
+  W.gray = reinterpret_cast<float4 *>(take(32 * n));
+  W.gcon = reinterpret_cast<float4 *>(take(16 * n));
+  *occ = reinterpret_cast<uint8_t *>(take(n));
+  W.gocc = *occ;
+  W.giQ = reinterpret_cast<uint32_t *>(take(4 * n));
+  return off;
+}
+
+// What the stages of one render share.
+struct WfStages {
+  vt_ctx *ctx;
+  const vt_mesh *mesh;
+  WfBuffers B;
+  uint32_t *slot;          // the traversals' ray-queue word
+  int block;               // stage kernels' block size
+  uint32_t gridMax, every; // their most blocks; the live queue is compacted on every n-th bounce
+  bool pbr, unbounded, group, nrc;
+  cudaStream_t s;
+  uint32_t grid(uint32_t paths) const { return std::min<uint32_t>((paths + (uint32_t)block - 1) / (uint32_t)block, gridMax); }
+};
+
+WfStages wf_stages(vt_ctx *ctx, const vt_scene *scene, const RenderArgs &A, const WfBuffers &B, int block, uint32_t every, bool nrc,
+                   cudaStream_t s) {
+  WfStages S;
+  S.ctx = ctx;
+  S.mesh = scene->mesh;
+  S.B = B;
+  S.slot = vt_queue_slot(ctx);
+  S.block = block;
+  S.gridMax = (uint32_t)ctx->sm_count * (8u * kWfBlock / (uint32_t)block);
+  S.every = every;
+  S.pbr = A.layered != 0u;
+  S.unbounded = scene_has_delta(scene);
+  S.group = S.pbr && A.spectral && scene->has_film;
+  S.nrc = nrc;
+  S.s = s;
+  return S;
+}
+
+// The bounces of the paths of W from bounce `first` on (0: every path, its ray just generated; else the
+// live queue q[first & 1]), then their radiance into the accumulation.
+vt_status wf_bounces(const WfStages &S, const RenderArgs &A, WfArgs W, uint32_t first) {
+  vt_ctx *ctx = S.ctx;
+  cudaStream_t s = S.s;
+  uint32_t *counts = S.B.counts;
+  const uint32_t P = W.paths, grid = S.grid(P);
+  for (uint32_t b = first;; ++b) {
+    if (b > A.maxDepth) {
+      // Ideal reflections and refractions spend no scattering event, so paths through glass and
+      // mirrors can outlive the depth (Russian roulette ends them): bounce on while a path lives,
+      // its count read back every 8 bounces (compacted queues from the depth on).
+      if (!S.unbounded) break;
+      if ((b - A.maxDepth - 1u) % 8u == 0u) {
+        uint32_t live = 0;
+        VT_CUDA(ctx, cudaMemcpyAsync(&live, counts + (b & 1u), sizeof live, cudaMemcpyDeviceToHost, s));
+        VT_CUDA(ctx, cudaStreamSynchronize(s));
+        if (live == 0u) break;
+      }
+    }
+    W.compact = ((b + 1u) % S.every == 0u || b >= A.maxDepth) ? 1u : 0u;
+    // Live queue of bounce b (all paths at b = 0), the next bounce's queue and the shadow queue.
+    W.inQ = b == 0 ? nullptr : S.B.q[b & 1u];
+    W.inCount = b == 0 ? nullptr : counts + (b & 1u);
+    W.outQ = S.B.q[(b + 1) & 1u];
+    W.outCount = counts + ((b + 1) & 1u);
+    W.shCount = counts + 2;
+    VT_CUDA(ctx, cudaMemsetAsync(W.outCount, 0, sizeof(uint32_t), s));
+    VT_CUDA(ctx, cudaMemsetAsync(W.shCount, 0, sizeof(uint32_t), s));
+    vt_launch_closest(S.mesh, reinterpret_cast<const vt_ray *>(W.ray), P, reinterpret_cast<vt_hit *>(S.B.hit), ctx->sm_count,
+                      S.slot, W.inQ, ctx->d_status + 1, s, W.inCount, true);
+    if (S.group) {
+      VT_CUDA(ctx, cudaMemsetAsync(counts + 3, 0, 2 * sizeof(uint32_t), s));
+      k_wf_group<<<grid, S.block, 0, s>>>(A, W, counts + 3);
+      W.inQ = W.grpQ;  // the same entries, regrouped (the count stays)
+    }
+    if (S.nrc) {
+      if (S.pbr) k_wf_shade<true, true><<<grid, S.block, 0, s>>>(A, W, b);
+      else k_wf_shade<false, true><<<grid, S.block, 0, s>>>(A, W, b);
+    } else {
+      if (S.pbr) k_wf_shade<true, false><<<grid, S.block, 0, s>>>(A, W, b);
+      else k_wf_shade<false, false><<<grid, S.block, 0, s>>>(A, W, b);
+    }
+    vt_launch_any(S.mesh, reinterpret_cast<const vt_ray *>(W.sray), P, S.B.occ, ctx->sm_count, S.slot, W.shQ, ctx->d_status + 1, s,
+                  W.shCount, A.imported != 0u);
+    VT_CUDA(ctx, cudaGetLastError());
+  }
+  if (S.nrc) k_wf_finish<true><<<grid, S.block, 0, s>>>(A, W);
+  else k_wf_finish<false><<<grid, S.block, 0, s>>>(A, W);
+  VT_CUDA(ctx, cudaGetLastError());
+  return VT_OK;
+}
+
+// One band of a mode-0 frame up to its reservoirs (A holds the frame's reservoir arrays).
+vt_status di_reservoirs(const WfStages &S, const RenderArgs &A, WfArgs W) {
+  vt_ctx *ctx = S.ctx;
+  cudaStream_t s = S.s;
+  uint32_t *counts = S.B.counts;
+  const uint32_t P = W.paths, grid = S.grid(P), pixels = (P + kRenderBlock - 1) / kRenderBlock;
+  const vt_ray *ray = reinterpret_cast<const vt_ray *>(W.ray), *sray = reinterpret_cast<const vt_ray *>(W.sray);
+  vt_hit *hit = reinterpret_cast<vt_hit *>(S.B.hit);
+  VT_CUDA(ctx, cudaMemsetAsync(counts, 0, 64, s));
+  k_wf_generate<<<grid, S.block, 0, s>>>(A, W);
+  vt_launch_closest(S.mesh, ray, P, hit, ctx->sm_count, S.slot, nullptr, ctx->d_status + 1, s, nullptr, true);
+  W.outQ = S.B.q[1];
+  W.outCount = counts + 1;
+  if (S.pbr) k_di_primary<true><<<pixels, kRenderBlock, 0, s>>>(A, W);
+  else k_di_primary<false><<<pixels, kRenderBlock, 0, s>>>(A, W);
+  if (A.maxDepth > 1u) {
+    vt_launch_closest(S.mesh, ray, P, hit, ctx->sm_count, S.slot, S.B.q[1], ctx->d_status + 1, s, counts + 1, true);
+    W.inQ = S.B.q[1];
+    W.inCount = counts + 1;
+    W.shCount = counts + 2;
+    k_gi_secondary<<<grid, S.block, 0, s>>>(A, W);
+    vt_launch_any(S.mesh, sray, P, S.B.occ, ctx->sm_count, S.slot, W.shQ, ctx->d_status + 1, s, W.shCount, A.imported != 0u);
+    k_gi_merge<<<(P + kWfBlock - 1) / kWfBlock, kWfBlock, 0, s>>>(A, W);
+  }
+  VT_CUDA(ctx, cudaGetLastError());
+  return VT_OK;
+}
+
+// One band of a mode-0 frame from its reservoirs to the accumulation.
+vt_status di_paths(const WfStages &S, const RenderArgs &A, WfArgs W, uint8_t *gocc) {
+  vt_ctx *ctx = S.ctx;
+  cudaStream_t s = S.s;
+  uint32_t *counts = S.B.counts;
+  const uint32_t P = W.paths, pixels = (P + kRenderBlock - 1) / kRenderBlock;
+  VT_CUDA(ctx, cudaMemsetAsync(counts, 0, 64, s));
+  W.outQ = S.B.q[1];
+  W.outCount = counts + 1;
+  W.shCount = counts + 2;
+  W.giCount = counts + 5;
+  if (S.nrc) {
+    if (S.pbr) k_di_shade<true, true><<<pixels, kRenderBlock, 0, s>>>(A, W);
+    else k_di_shade<false, true><<<pixels, kRenderBlock, 0, s>>>(A, W);
+  } else {
+    if (S.pbr) k_di_shade<true, false><<<pixels, kRenderBlock, 0, s>>>(A, W);
+    else k_di_shade<false, false><<<pixels, kRenderBlock, 0, s>>>(A, W);
+  }
+  vt_launch_any(S.mesh, reinterpret_cast<const vt_ray *>(W.sray), P, S.B.occ, ctx->sm_count, S.slot, W.shQ, ctx->d_status + 1, s,
+                W.shCount, A.imported != 0u);
+  if (!S.nrc && A.maxDepth > 1u) {
+    vt_launch_any(S.mesh, reinterpret_cast<const vt_ray *>(W.gray), P, gocc, ctx->sm_count, S.slot, W.giQ, ctx->d_status + 1, s,
+                  W.giCount, A.imported != 0u);
+    k_gi_connect<<<S.grid(P), S.block, 0, s>>>(W);
+  }
+  VT_CUDA(ctx, cudaGetLastError());
+  return wf_bounces(S, A, W, 1u);
+}
+
 // vt_render, and with a cache (nrc not null) vt_render_nrc's rendering: the same frames, paths
 // ending at the cache's query vertex, then the predictions and the resolve.
 vt_status render_impl(vt_ctx *ctx, vt_scene *scene, const vt_frame_params *p, uint32_t spp, void *stream,
@@ -3128,7 +3432,7 @@ vt_status render_impl(vt_ctx *ctx, vt_scene *scene, const vt_frame_params *p, ui
     A.nrcSpread = nrc->cfg.spread;
   }
   if (p->sampling_mode == 0u) {
-    // ReSTIR DI: frames in order, two launches each (the primary pass, then reuse and shading).
+    // ReSTIR: frames in order, each through the wavefront stages (k_di_primary's comment lists them).
     if (!scene->d_di || scene->di_width != p->width || scene->di_height != p->height) {
       cudaFree(scene->d_di);
       scene->d_di = nullptr;
@@ -3149,7 +3453,38 @@ vt_status render_impl(vt_ctx *ctx, vt_scene *scene, const vt_frame_params *p, ui
     A.gGeo = base + 19 * (size_t)npix;
     const float cam[14] = {A.cam.x, A.cam.y, A.cam.z, A.fwd.x, A.fwd.y, A.fwd.z, A.right.x, A.right.y, A.right.z,
                            A.up.x, A.up.y, A.up.z, A.aspect, A.fovScale};
-    const unsigned blocks = (npix + kRenderBlock - 1) / kRenderBlock;
+    // The stages' state for a band of pixels: the whole frame up to 4M pixels, less where memory is short.
+    uint32_t band = std::min(npix, kWfMaxPaths);
+    WfArgs W{};
+    WfBuffers B;
+    uint8_t *gocc = nullptr;
+    while (scene->wf_cap < band || scene->wf_gi_cap < band) {
+      cudaError_t e = cudaSuccess;
+      if (scene->wf_cap < band) {
+        cudaFree(scene->d_wf);
+        scene->d_wf = nullptr;
+        scene->wf_cap = 0;
+        e = cudaMalloc(&scene->d_wf, wf_carve(nullptr, band, W, B));
+        if (e == cudaSuccess) scene->wf_cap = band;
+      }
+      if (e == cudaSuccess && scene->wf_gi_cap < band) {
+        cudaFree(scene->d_wf_gi);
+        scene->d_wf_gi = nullptr;
+        scene->wf_gi_cap = 0;
+        e = cudaMalloc(&scene->d_wf_gi, wf_carve_gi(nullptr, band, W, &gocc));
+        if (e == cudaSuccess) scene->wf_gi_cap = band;
+      }
+      if (e == cudaSuccess) break;
+      cudaGetLastError();
+      if (e != cudaErrorMemoryAllocation || band <= (1u << 16)) return vt_cuda_fail(ctx, e, "allocating the frame's path state");
+      band = (band + 1u) / 2u;
+    }
+    wf_carve(scene->d_wf, scene->wf_cap, W, B);
+    wf_carve_gi(scene->d_wf_gi, scene->wf_gi_cap, W, &gocc);
+    W.npix = npix;
+    W.deadFlags = 0u;
+    A.kernelId = nrc ? 5u : 4u;
+    const WfStages S = wf_stages(ctx, scene, A, B, kWfBlock, 1u, nrc != nullptr, s);
     for (uint32_t k = 0; k < spp; ++k) {
       float4 *cur = base + 9 * (size_t)npix * scene->di_parity, *prev = base + 9 * (size_t)npix * (scene->di_parity ^ 1u);
       A.gPos = cur; A.gNrm = cur + npix; A.rPos = cur + 2 * (size_t)npix; A.rEmit = cur + 3 * (size_t)npix;
@@ -3168,20 +3503,21 @@ vt_status render_impl(vt_ctx *ctx, vt_scene *scene, const vt_frame_params *p, ui
       A.pup = make_float3(pc[9], pc[10], pc[11]);
       A.paspect = pc[12];
       A.pfovScale = pc[13];
-      if (A.layered) {
-        A.kernelId = 3;
-        k_di_primary<true><<<blocks, kRenderBlock, 0, s>>>(A, k);
-        A.kernelId = nrc ? 5 : 4;
-        if (nrc) k_di_shade<true, true><<<blocks, kRenderBlock, 0, s>>>(A, k);
-        else k_di_shade<true><<<blocks, kRenderBlock, 0, s>>>(A, k);
-      } else {
-        A.kernelId = 3;
-        k_di_primary<false><<<blocks, kRenderBlock, 0, s>>>(A, k);
-        A.kernelId = nrc ? 5 : 4;
-        if (nrc) k_di_shade<false, true><<<blocks, kRenderBlock, 0, s>>>(A, k);
-        else k_di_shade<false><<<blocks, kRenderBlock, 0, s>>>(A, k);
+      W.k0 = k;
+      const bool whole = band >= npix;
+      for (uint32_t p0 = 0; p0 < npix; p0 += band) {
+        W.p0 = p0;
+        W.paths = std::min(band, npix - p0);
+        vt_status st = di_reservoirs(S, A, W);
+        if (st == VT_OK && whole) st = di_paths(S, A, W, gocc);
+        if (st != VT_OK) return st;
       }
-      VT_CUDA(ctx, cudaGetLastError());
+      for (uint32_t p0 = 0; p0 < npix && !whole; p0 += band) {
+        W.p0 = p0;
+        W.paths = std::min(band, npix - p0);
+        const vt_status st = di_paths(S, A, W, gocc);
+        if (st != VT_OK) return st;
+      }
       scene->di_parity ^= 1u;
       ++scene->di_frames;
       std::memcpy(scene->di_cam, cam, sizeof cam);
@@ -3200,61 +3536,14 @@ vt_status render_impl(vt_ctx *ctx, vt_scene *scene, const vt_frame_params *p, ui
   groups = (spp + per - 1) / per;
   const uint64_t items = (uint64_t)npix * groups;
   const uint32_t grid = (uint32_t)std::min<uint64_t>((items + kRenderBlock - 1) / kRenderBlock, (uint64_t)ctx->sm_count * 32u);
-  if (nrc) {
-    A.kernelId = 2;
-    if (A.layered) k_render<true, true><<<grid, kRenderBlock, 0, s>>>(A, groups, per);
-    else k_render<false, true><<<grid, kRenderBlock, 0, s>>>(A, groups, per);
-    VT_CUDA(ctx, cudaGetLastError());
-    const vt_status st = nrc_finish(ctx, nrc, A, spp, s);
-    if (st != VT_OK) return st;
-  } else {
-    A.kernelId = 1;
-    if (A.layered) k_render<true><<<grid, kRenderBlock, 0, s>>>(A, groups, per);
-    else k_render<false><<<grid, kRenderBlock, 0, s>>>(A, groups, per);
-    VT_CUDA(ctx, cudaGetLastError());
-  }
+  A.kernelId = 1;
+  if (A.layered) k_render<true><<<grid, kRenderBlock, 0, s>>>(A, groups, per);
+  else k_render<false><<<grid, kRenderBlock, 0, s>>>(A, groups, per);
+  VT_CUDA(ctx, cudaGetLastError());
   scene->samples += spp;
   return VT_OK;
 }
 
-
-// ---- wavefront integrator: host side ------------------------------------------------------------
-// Paths per pass: as many whole samples of the frame as fit 4M paths (about 1 GB of state).
-constexpr uint32_t kWfMaxPaths = 1u << 22;
-
-// Bytes of wavefront state per path (each array 256-byte aligned in wf_carve).
-size_t wf_carve(unsigned char *base, uint32_t cap, WfArgs &W, uint32_t **q0, uint32_t **q1, uint32_t **counts,
-                uint8_t **occ, int4 **hit) {
-  size_t off = 0;
-  auto take = [&](size_t bytes) {
-    unsigned char *p = base ? base + off : nullptr;
-    off += (bytes + 255) & ~size_t(255);
-    return p;
-  };
-  const size_t n = cap;
-  W.T = reinterpret_cast<float4 *>(take(16 * n));
-  W.Rc = reinterpret_cast<float4 *>(take(16 * n));
-  W.Rp = reinterpret_cast<float4 *>(take(16 * n));
-  W.prev = reinterpret_cast<float4 *>(take(16 * n));
-  W.prevN = reinterpret_cast<float4 *>(take(16 * n));
-  W.seedA = reinterpret_cast<uint4 *>(take(16 * n));
-  W.seedB = reinterpret_cast<uint2 *>(take(8 * n));
-  W.meta = reinterpret_cast<uint4 *>(take(16 * n));
-  W.spread = reinterpret_cast<float2 *>(take(8 * n));
-  W.ray = reinterpret_cast<float4 *>(take(32 * n));
-  *hit = reinterpret_cast<int4 *>(take(16 * n));
-  W.sray = reinterpret_cast<float4 *>(take(32 * n));
-  W.scon = reinterpret_cast<float4 *>(take(16 * n));
-  *occ = reinterpret_cast<uint8_t *>(take(n));
-  *q0 = reinterpret_cast<uint32_t *>(take(4 * n));
-  *q1 = reinterpret_cast<uint32_t *>(take(4 * n));
-  W.shQ = reinterpret_cast<uint32_t *>(take(4 * n));
-  W.grpQ = reinterpret_cast<uint32_t *>(take(4 * n));
-  *counts = reinterpret_cast<uint32_t *>(take(64));
-  return off;
-}
-
-vt_status nrc_finish(vt_ctx *ctx, vt_nrc *nrc, const RenderArgs &A, uint32_t spp, cudaStream_t s);
 
 // Launch settings of a wavefront render and where its state lives. The defaults are vt_render_wavefront's:
 // the scene's own state, up to 4M paths per pass, 256-thread stage blocks, compaction every bounce and the
@@ -3329,80 +3618,25 @@ vt_status wavefront_impl(vt_ctx *ctx, vt_scene *scene, const vt_frame_params *p,
     *state = nullptr;
     *stateCap = 0;
     WfArgs probe;
-    uint32_t *a, *b, *c;
-    uint8_t *o;
-    int4 *h;
-    const size_t bytes = wf_carve(nullptr, cap, probe, &a, &b, &c, &o, &h);
+    WfBuffers unused;
+    const size_t bytes = wf_carve(nullptr, cap, probe, unused);
     VT_CUDA(ctx, cudaMalloc(state, bytes));
     *stateCap = cap;
   }
-  WfArgs W;
-  uint32_t *q[2], *counts;
-  uint8_t *occ;
-  int4 *hit;
-  wf_carve(*state, *stateCap, W, &q[0], &q[1], &counts, &occ, &hit);
-  W.hit = hit;
-  W.occ = occ;
+  WfArgs W{};
+  WfBuffers B;
+  wf_carve(*state, *stateCap, W, B);
   W.npix = npix;
   const uint32_t every = std::max(1u, run.compactEvery);
   W.deadFlags = every > 1u ? 1u : 0u;
-  const int block = std::max(32, std::min(run.block, kWfBlock));
-  const bool pbr = A.layered != 0u, unbounded = scene_has_delta(scene);
-  const bool group = pbr && A.spectral && scene->has_film;
-  const uint32_t gridMax = (uint32_t)ctx->sm_count * (8u * kWfBlock / (uint32_t)block);
-  uint32_t *slot = vt_queue_slot(ctx);
+  const WfStages S = wf_stages(ctx, scene, A, B, std::max(32, std::min(run.block, kWfBlock)), every, nrc != nullptr, s);
   for (uint32_t k0 = 0; k0 < spp; k0 += chunk) {
-    const uint32_t P = npix * std::min(chunk, spp - k0);
-    W.paths = P;
+    W.paths = npix * std::min(chunk, spp - k0);
     W.k0 = k0;
-    const uint32_t grid = std::min<uint32_t>((P + block - 1) / block, gridMax);
-    k_wf_generate<<<grid, block, 0, s>>>(A, W);
+    k_wf_generate<<<S.grid(W.paths), S.block, 0, s>>>(A, W);
     VT_CUDA(ctx, cudaGetLastError());
-    for (uint32_t b = 0;; ++b) {
-      if (b > A.maxDepth) {
-        // Ideal reflections and refractions spend no scattering event, so paths through glass and
-        // mirrors can outlive the depth (Russian roulette ends them): bounce on while a path lives,
-        // its count read back every 8 bounces (compacted queues from the depth on).
-        if (!unbounded) break;
-        if ((b - A.maxDepth - 1u) % 8u == 0u) {
-          uint32_t live = 0;
-          VT_CUDA(ctx, cudaMemcpyAsync(&live, counts + (b & 1u), sizeof live, cudaMemcpyDeviceToHost, s));
-          VT_CUDA(ctx, cudaStreamSynchronize(s));
-          if (live == 0u) break;
-        }
-      }
-      W.compact = ((b + 1u) % every == 0u || b >= A.maxDepth) ? 1u : 0u;
-      // Live queue of bounce b (all paths at b = 0), the next bounce's queue and the shadow queue.
-      const uint32_t *inQ = b == 0 ? nullptr : q[b & 1u];
-      const uint32_t *inCount = b == 0 ? nullptr : counts + (b & 1u);
-      W.inQ = inQ;
-      W.inCount = inCount;
-      W.outQ = q[(b + 1) & 1u];
-      W.outCount = counts + ((b + 1) & 1u);
-      W.shCount = counts + 2;
-      VT_CUDA(ctx, cudaMemsetAsync(W.outCount, 0, sizeof(uint32_t), s));
-      VT_CUDA(ctx, cudaMemsetAsync(W.shCount, 0, sizeof(uint32_t), s));
-      vt_launch_closest(mesh, reinterpret_cast<const vt_ray *>(W.ray), P, reinterpret_cast<vt_hit *>(hit), ctx->sm_count,
-                        slot, inQ, ctx->d_status + 1, s, inCount, true);
-      if (group) {
-        VT_CUDA(ctx, cudaMemsetAsync(counts + 3, 0, 2 * sizeof(uint32_t), s));
-        k_wf_group<<<grid, block, 0, s>>>(A, W, counts + 3);
-        W.inQ = W.grpQ;  // the same entries, regrouped (the count stays)
-      }
-      if (nrc) {
-        if (pbr) k_wf_shade<true, true><<<grid, block, 0, s>>>(A, W, b);
-        else k_wf_shade<false, true><<<grid, block, 0, s>>>(A, W, b);
-      } else {
-        if (pbr) k_wf_shade<true, false><<<grid, block, 0, s>>>(A, W, b);
-        else k_wf_shade<false, false><<<grid, block, 0, s>>>(A, W, b);
-      }
-      vt_launch_any(mesh, reinterpret_cast<const vt_ray *>(W.sray), P, occ, ctx->sm_count, slot, W.shQ, ctx->d_status + 1, s,
-                    W.shCount, A.imported != 0u);
-      VT_CUDA(ctx, cudaGetLastError());
-    }
-    if (nrc) k_wf_finish<true><<<grid, block, 0, s>>>(A, W);
-    else k_wf_finish<false><<<grid, block, 0, s>>>(A, W);
-    VT_CUDA(ctx, cudaGetLastError());
+    const vt_status st = wf_bounces(S, A, W, 0u);
+    if (st != VT_OK) return st;
   }
   if (nrc) {
     const vt_status st = nrc_finish(ctx, nrc, A, spp, s);
@@ -3498,8 +3732,7 @@ vt_status vt_render_nrc(vt_ctx *ctx, vt_scene *scene, vt_nrc *nrc, const vt_fram
     }
   }
   if (flags & VT_NRC_RENDER) {
-    // MIS primaries through the wavefront integrator; ReSTIR DI's frames through its two passes
-    // (compiled without glass and mirrors, see continue_path).
+    // Both through the wavefront stages: MIS primaries, or ReSTIR's (without glass and mirrors).
     const vt_status st = p->sampling_mode == 1u ? wavefront_impl(ctx, scene, p, spp, stream, nrc)
                                                 : render_impl(ctx, scene, p, spp, stream, nrc);
     if (both) {
