@@ -60,7 +60,7 @@ static_assert(sizeof(ResultDev) == sizeof(vt_openpbr_result), "vt_openpbr_result
 
 __device__ __forceinline__ PbrParams case_params(const CaseDev &c) {
   PbrParams P;
-  P.base = pf3(psat(c.base[0]), psat(c.base[1]), psat(c.base[2]));
+  P.base = pf4(psat(c.base[0]), psat(c.base[1]), psat(c.base[2]), psat(c.base[2]));
   P.metal = c.metal;
   P.rough = fmaxf(0.03f, c.rough);
   P.ior = fmaxf(1.01f, c.ior);
@@ -70,7 +70,8 @@ __device__ __forceinline__ PbrParams case_params(const CaseDev &c) {
   P.tfThickness = c.tfThickness;
   P.tfIor = c.tfIor;
   // The upstream RGB wavelengths unless the case gives its own (openpbr_bsdf.h: OpenPBR_BaseRgbWavelengths_nm).
-  P.lambda = c.lambda[0] > 0.0f ? pf3(c.lambda[0], c.lambda[1], c.lambda[2]) : pf3(kPbrRgbNm[0], kPbrRgbNm[1], kPbrRgbNm[2]);
+  P.lambda = c.lambda[0] > 0.0f ? pf4(c.lambda[0], c.lambda[1], c.lambda[2], c.lambda[2])
+                                : pf4(kPbrRgbNm[0], kPbrRgbNm[1], kPbrRgbNm[2], kPbrRgbNm[2]);
   P.coat = c.coat;
   P.fuzz = c.fuzz;
   P.aniso = c.aniso;
@@ -81,14 +82,15 @@ __global__ void k_openpbr_cases(PbrTables T, const CaseDev *__restrict__ cases, 
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const CaseDev c = cases[i];
-  const PbrPrepared p = pbr_prepare(case_params(c), T, pf3(c.n[0], c.n[1], c.n[2]), pf3(c.wo[0], c.wo[1], c.wo[2]), true,
+  const PbrPrepared p = pbr_prepare(case_params(c), T, pf3(c.n[0], c.n[1], c.n[2]), pf3(c.wo[0], c.wo[1], c.wo[2]),
                                     pf3(c.tangent[0], c.tangent[1], c.tangent[2]));
   const float3 wi = pf3(c.wi[0], c.wi[1], c.wi[2]);
-  const float3 f = pbr_eval(p, T, wi);
   ResultDev r;
+  float specPdf;
+  const float4 f = pbr_eval_pdf(p, T, wi, nullptr, r.pdf, specPdf);
   r.fcos[0] = f.x; r.fcos[1] = f.y; r.fcos[2] = f.z;
-  r.pdf = pbr_pdf(p, T, wi);
-  float3 d = pf3(0.0f, 0.0f, 0.0f), w = pf3(0.0f, 0.0f, 0.0f);
+  float3 d = pf3(0.0f, 0.0f, 0.0f);
+  float4 w = pf4(0.0f, 0.0f, 0.0f, 0.0f);
   float q = 0.0f;
   const bool ok = pbr_sample(p, T, pf3(c.rand[0], c.rand[1], c.rand[2]), d, w, q);
   r.dir[0] = d.x; r.dir[1] = d.y; r.dir[2] = d.z;

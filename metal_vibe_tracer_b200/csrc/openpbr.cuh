@@ -55,13 +55,18 @@ constexpr int kPbrLtc = 32;              // the fuzz LTC table's size per axis
 // The upstream library's wavelengths for R, G and B (openpbr_constants.h: OpenPBR_BaseRgbWavelengths_nm).
 __device__ constexpr float kPbrRgbNm[3] = {620.0f, 540.0f, 450.0f};
 
+// Colours have four channels: a path's four hero wavelengths, or rgb with the fourth unused. Every value
+// is computed per channel from the same geometry, so one preparation and one evaluation serve all
+// four; lobe weights and pdfs come from the first three, as upstream's (its adapter evaluates lane 3
+// as a second preparation of its own).
+//
 // Per slot: base colour (clamped), metalness, roughness (>= 0.03), IOR (>= 1.01), specular weight,
 // diffuse roughness.
 struct PbrParams {
-  float3 base;
+  float4 base;
   float metal, rough, ior, sw, diffRough;
   float tfWeight, tfThickness, tfIor;  // thin film: weight, thickness (micrometres), IOR
-  float3 lambda;                       // the preparation's three wavelengths (nm)
+  float4 lambda;                       // the channels' wavelengths (nm)
   float coat;                          // coat weight (roughness 0.12, IOR 1.6, white, darkening 1)
   float fuzz;                          // fuzz weight (roughness 0.5, white)
   float aniso;                         // specular_roughness_anisotropy in [0, 1]
@@ -94,7 +99,12 @@ __device__ __forceinline__ float3 pnormalize(float3 a) {
   const float l = sqrtf(pdot(a, a));
   return pf3(a.x / l, a.y / l, a.z / l);
 }
-__device__ __forceinline__ float pmax3(float3 v) { return fmaxf(fmaxf(v.x, v.y), v.z); }
+__device__ __forceinline__ float4 pf4(float x, float y, float z, float w) { return make_float4(x, y, z, w); }
+__device__ __forceinline__ float4 padd(float4 a, float4 b) { return pf4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+__device__ __forceinline__ float4 pmul(float4 a, float4 b) { return pf4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); }
+__device__ __forceinline__ float4 pscale(float4 a, float s) { return pf4(a.x * s, a.y * s, a.z * s, a.w * s); }
+// The largest of the channels that weights and pdfs are taken from.
+__device__ __forceinline__ float pmax3(float4 v) { return fmaxf(fmaxf(v.x, v.y), v.z); }
 __device__ __forceinline__ float psq(float x) { return x * x; }
 __device__ __forceinline__ float pmix(float a, float b, float t) { return a + (b - a) * t; }
 __device__ __forceinline__ float psat(float x) { return x < 0.0f ? 0.0f : (x > 1.0f ? 1.0f : x); }
@@ -166,26 +176,15 @@ __device__ __forceinline__ float pbr_fresnel(float eta, float ci) {
   const float rp = psq((ct - eci) / (ct + eci));
   return 0.5f * (rs + rp);
 }
-// F82-tinted Schlick for the metal (white tint: b = r (1 - cos_max)^5 ... with t = 1 gives b = 0).
-__device__ __forceinline__ float3 pbr_f82_b(float3 f0, float3 tint) {
-  const float cm = 1.0f / 7.0f, omc = 1.0f - cm;
-  const float omc2 = omc * omc;
-  const float p5 = omc2 * omc2 * omc, p6 = omc2 * omc2 * omc2;
-  const float rden = 1.0f / (cm * p6);
-  return pf3((f0.x + (1.0f - f0.x) * p5) * (1.0f - tint.x) * rden, (f0.y + (1.0f - f0.y) * p5) * (1.0f - tint.y) * rden,
-             (f0.z + (1.0f - f0.z) * p5) * (1.0f - tint.z) * rden);
-}
-__device__ __forceinline__ float3 pbr_metal_fresnel(float3 f0, float cosT) {
-  const float3 b = pbr_f82_b(f0, pf3(1.0f, 1.0f, 1.0f));
+// F82-tinted Schlick for the metal with a white tint, whose F82 term vanishes.
+__device__ __forceinline__ float4 pbr_metal_fresnel(float4 f0, float cosT) {
   const float omc = 1.0f - cosT, omc2 = omc * omc, p5 = omc2 * omc2 * omc;
-  return pf3(psat(f0.x + ((1.0f - f0.x) - b.x * cosT * omc) * p5), psat(f0.y + ((1.0f - f0.y) - b.y * cosT * omc) * p5),
-             psat(f0.z + ((1.0f - f0.z) - b.z * cosT * omc) * p5));
+  return pf4(psat(f0.x + (1.0f - f0.x) * p5), psat(f0.y + (1.0f - f0.y) * p5), psat(f0.z + (1.0f - f0.z) * p5),
+             psat(f0.w + (1.0f - f0.w) * p5));
 }
-__device__ __forceinline__ float3 pbr_metal_average_fresnel(float3 f0) {
-  const float3 b = pbr_f82_b(f0, pf3(1.0f, 1.0f, 1.0f));
-  return pf3(psat(f0.x + (1.0f - f0.x) * (1.0f / 21.0f) - b.x * (1.0f / 126.0f)),
-             psat(f0.y + (1.0f - f0.y) * (1.0f / 21.0f) - b.y * (1.0f / 126.0f)),
-             psat(f0.z + (1.0f - f0.z) * (1.0f / 21.0f) - b.z * (1.0f / 126.0f)));
+__device__ __forceinline__ float4 pbr_metal_average_fresnel(float4 f0) {
+  return pf4(psat(f0.x + (1.0f - f0.x) * (1.0f / 21.0f)), psat(f0.y + (1.0f - f0.y) * (1.0f / 21.0f)),
+             psat(f0.z + (1.0f - f0.z) * (1.0f / 21.0f)), psat(f0.w + (1.0f - f0.w) * (1.0f / 21.0f)));
 }
 // specular_weight applied to a relative IOR (openpbr_apply_specular_weight_to_ior).
 __device__ __forceinline__ float pbr_weighted_ior(float eta, float sw) {
@@ -339,37 +338,30 @@ __device__ __forceinline__ float pbr_airy_sp(float2 r12, float2 t12, float2 r21,
 }
 // openpbr_thin_film_and_base_reflectance: the dielectric base's and the metal base's reflectance per
 // channel at cos ci from the exterior (no dispersion; the metal's F82 tint is white).
-static __device__ void pbr_thin_film(float ci, float eExt, float eFilm, float eBase, float3 f0, bool diel, bool metal, float nm,
-                              float3 lambda, float3 &rd, float3 &rm) {
-  rd = pf3(0.0f, 0.0f, 0.0f);
-  rm = pf3(0.0f, 0.0f, 0.0f);
+// Not inlined: a preparation and its evaluations share one copy of the code.
+static __device__ __noinline__ void pbr_thin_film(float ci, float eExt, float eFilm, float eBase, float4 f0, bool diel, bool metal,
+                                                  float nm, float4 lambda, float4 &rd, float4 &rm) {
+  rd = pf4(0.0f, 0.0f, 0.0f, 0.0f);
+  rm = pf4(0.0f, 0.0f, 0.0f, 0.0f);
   if (!(diel || metal)) return;
   float2 r12, t12;
   float ct;
   pbr_fresnel_amp(ci, eExt, eFilm, r12, t12, ct);
   if (ct <= 0.0f) {
-    if (diel) rd = pf3(1.0f, 1.0f, 1.0f);
-    if (metal) rm = pf3(1.0f, 1.0f, 1.0f);
+    if (diel) rd = pf4(1.0f, 1.0f, 1.0f, 1.0f);
+    if (metal) rm = pf4(1.0f, 1.0f, 1.0f, 1.0f);
     return;
   }
   const float2 r21 = make_float2(-r12.x, -r12.y);
   const float scale = (eFilm * ct) / (eExt * fmaxf(ci, kPbrMinDenom));
   const float2 t21 = make_float2(t12.x * scale, t12.y * scale);
   const float opd = 2.0f * eFilm * nm * ct;
-  // A preparation at one wavelength with a grey base (the spectral lane-3 preparation) has three equal
-  // channels: the first is computed and copied.
-  const bool mono = lambda.x == lambda.y && lambda.x == lambda.z && (!metal || (f0.x == f0.y && f0.x == f0.z));
-  const float lam[3] = {lambda.x, lambda.y, lambda.z}, f[3] = {f0.x, f0.y, f0.z};
+  const float lam[4] = {lambda.x, lambda.y, lambda.z, lambda.w}, f[4] = {f0.x, f0.y, f0.z, f0.w};
   PbrCx ds = cx(0.0f, 0.0f), dp = cx(0.0f, 0.0f);
   if (diel) pbr_fresnel_amp_cx(ct, eFilm, cx(eBase, 0.0f), ds, dp);
-  float od[3] = {0.0f, 0.0f, 0.0f}, om[3] = {0.0f, 0.0f, 0.0f};
+  float od[4] = {0.0f, 0.0f, 0.0f, 0.0f}, om[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    if (c > 0 && mono) {
-      od[c] = od[0];
-      om[c] = om[0];
-      continue;
-    }
+  for (int c = 0; c < 4; ++c) {
     const float dphi = 2.0f * kPbrPi * opd / lam[c];
     if (diel) od[c] = pbr_airy_sp(r12, t12, r21, t21, ds, dp, dphi);
     if (metal) {
@@ -378,8 +370,8 @@ static __device__ void pbr_thin_film(float ci, float eExt, float eFilm, float eB
       om[c] = pbr_airy_sp(r12, t12, r21, t21, rs, rp, dphi);
     }
   }
-  if (diel) rd = pf3(od[0], od[1], od[2]);
-  if (metal) rm = pf3(om[0], om[1], om[2]);
+  if (diel) rd = pf4(od[0], od[1], od[2], od[3]);
+  if (metal) rm = pf4(om[0], om[1], om[2], om[3]);
 }
 // openpbr_thin_film_presence_multiplier: smoothstep from 1e-9 to 30 nm.
 __device__ __forceinline__ float pbr_thin_film_presence(float weight, float nm) {
@@ -396,23 +388,24 @@ struct PbrPrepared {
   float etaOpaque;     // relative IOR of the opaque reflection
   float scaleOpaque;   // opaque dielectric share (specular colour 1)
   float metalAmount;   // darkened metal
-  float3 f0;           // weighted base colour: the metal's normal-incidence reflectance
-  float3 metalScale;   // metal multiple-scattering scale
-  float metalEc;       // metal energy complement at the view
-  float3 diffAlbedo;
+  float4 f0;           // weighted base colour: the metal's normal-incidence reflectance
+  float4 metalScale;   // metal multiple-scattering scale
+  float metalEc;       // metal energy complement at the view, and its average
+  float metalAvg;
+  float4 diffAlbedo;
   float diffRough, diffComp;
   float wSpec, wMetal, wDiff, total;
   // Thin film: presence (weight x thickness ramp), thickness (nm), the IORs outside, of and under the
   // film, the wavelengths.
   float tfPresence, tfNm, tfExt, tfIor, tfInt;
-  float3 lambda;
+  float4 lambda;
   // Coat (the coating lobe): presence, hit from inside (then only the base counts), relative IOR,
   // alpha (isotropic and clamped), the share reflected at the view, the base's scale under it
   // (transmission at the view times the darkening), and the probability of sampling the coat.
   float coat;
   bool inside;
   float coatEta, coatAlpha, coatAx, inRefl;
-  float3 inScale;
+  float4 inScale;
   float coatProb;
   // Fuzz (the sheen lobe over the coated base): presence (0 from inside), its basis about the
   // face-forwarded normal, the view in it, the share it reflects at the view, its probability.
@@ -425,19 +418,21 @@ struct PbrPrepared {
 // Reflection coefficient of the specular lobe at cos c to the half vector (openpbr_reflection_coefficient):
 // the opaque dielectric's Fresnel and the metal's F82 Schlick, blended with the thin film's reflectances
 // by its presence (computed only where it is partial or whole).
-__device__ __forceinline__ float3 pbr_spec_coeff(const PbrPrepared &p, float c) {
-  float3 standard = pf3(0.0f, 0.0f, 0.0f);
+__device__ __forceinline__ float4 pbr_spec_coeff(const PbrPrepared &p, float c) {
+  float4 standard = pf4(0.0f, 0.0f, 0.0f, 0.0f);
   if (p.tfPresence < 1.0f) {
-    const float F = pbr_fresnel(p.etaOpaque, c);
-    const float3 fm = pbr_metal_fresnel(p.f0, c);
-    standard = padd(pf3(p.scaleOpaque * F, p.scaleOpaque * F, p.scaleOpaque * F), pscale(fm, p.metalAmount));
+    if (p.scaleOpaque > 0.0f) {
+      const float F = p.scaleOpaque * pbr_fresnel(p.etaOpaque, c);
+      standard = pf4(F, F, F, F);
+    }
+    if (p.metalAmount > 0.0f) standard = padd(standard, pscale(pbr_metal_fresnel(p.f0, c), p.metalAmount));
   }
   if (!(p.tfPresence > 0.0f) || c < 0.0f) return standard;
-  float3 rd, rm;
+  float4 rd, rm;
   pbr_thin_film(c, p.tfExt, p.tfIor, p.tfInt, p.f0, p.scaleOpaque > 0.0f, p.metalAmount > 0.0f, p.tfNm, p.lambda, rd, rm);
-  const float3 film = padd(pscale(rd, p.scaleOpaque), pscale(rm, p.metalAmount));
+  const float4 film = padd(pscale(rd, p.scaleOpaque), pscale(rm, p.metalAmount));
   const float t = p.tfPresence;
-  return pf3(standard.x * (1.0f - t) + film.x * t, standard.y * (1.0f - t) + film.y * t, standard.z * (1.0f - t) + film.z * t);
+  return padd(pscale(standard, 1.0f - t), pscale(film, t));
 }
 
 // openpbr_average_fresnel: the fitted hemispherical average of the dielectric Fresnel reflectance.
@@ -473,15 +468,13 @@ __device__ __forceinline__ float3 pbr_ltc_fetch(const PbrTables &T, float alpha,
   return pf3(pmix(m0.x, m1.x, rf), pmix(m0.y, m1.y, rf), pmix(m0.z, m1.z, rf));
 }
 
-// openpbr_prepare for an opaque material seen from `wo` with shading normal n (both unit). Without
-// `weights` the lobe-selection weights (which only pbr_pdf and pbr_sample read) are left at zero: a
-// preparation that is only evaluated skips the specular coefficient at the view. `tangent` is the
+// openpbr_prepare for an opaque material seen from `wo` with shading normal n (both unit). A purely
+// metallic or dielectric slot skips the other part's lookups, whose lobes are exactly zero. `tangent` is the
 // surface's unit tangent (the adapter's mat.tangent); an anisotropic material takes its basis from it
 // when it is usable (prepare_openpbr, main.swift:2510-2511), an isotropic one from the normal alone:
 // the isotropic lobes are symmetric about the normal, so the frame's rotation changes neither their
 // values nor the distribution of their samples.
-__device__ __forceinline__ PbrPrepared pbr_prepare(const PbrParams &P, const PbrTables &T, float3 n, float3 wo,
-                                                   bool weights = true, float3 tangent = make_float3(0.0f, 0.0f, 0.0f)) {
+__device__ __forceinline__ PbrPrepared pbr_prepare(const PbrParams &P, const PbrTables &T, float3 n, float3 wo, float3 tangent) {
   PbrPrepared p;
   p.wo = wo;
   p.B = P.aniso > 0.0f && pdot(tangent, tangent) > 0.5f && fabsf(pdot(tangent, n)) < 0.99f ? pbr_basis_tangent(n, tangent)
@@ -531,10 +524,14 @@ __device__ __forceinline__ PbrPrepared pbr_prepare(const PbrParams &P, const Pbr
   p.scaleOpaque = 1.0f * 1.0f * dielectric;
   p.metalAmount = P.metal * P.sw;
   p.f0 = pscale(P.base, 1.0f);  // base_weight 1
-  const float3 maf = pbr_metal_average_fresnel(p.f0);
+  const float4 maf = pbr_metal_average_fresnel(p.f0);
   p.metalScale = pscale(pmul(maf, maf), p.metalAmount);
   const float idotn = pdot(wo, p.B.n);
-  p.metalEc = p.alpha < kPbrMinAlphaEnergyLoss ? 0.0f : pbr_metal_energy(T, p.alpha, idotn);
+  p.metalEc = p.metalAvg = 0.0f;
+  if (p.alpha >= kPbrMinAlphaEnergyLoss && p.metalAmount > 0.0f) {
+    p.metalEc = pbr_metal_energy(T, p.alpha, idotn);
+    p.metalAvg = pbr_metal_average(T, p.alpha);
+  }
   p.diffAlbedo = pscale(p.f0, p.scaleOpaque);
   p.diffRough = P.diffRough;
   // Thin film (openpbr_bsdf.h:678-690 with no coat): from outside the film lies between the ambient
@@ -545,7 +542,8 @@ __device__ __forceinline__ PbrPrepared pbr_prepare(const PbrParams &P, const Pbr
   p.tfInt = back ? wcoat : wior;
   p.tfIor = P.tfIor;
   p.lambda = P.lambda;
-  {
+  p.diffComp = 0.0f;
+  if (p.scaleOpaque > 0.0f) {
     const float num = pbr_opaque_energy(T, p.etaOpaque, p.alpha, idotn);
     const float den = pbr_opaque_average(T, p.etaOpaque, p.alpha);
     p.diffComp = num / fmaxf(den, 1e-12f);
@@ -560,7 +558,7 @@ __device__ __forceinline__ PbrPrepared pbr_prepare(const PbrParams &P, const Pbr
   p.coatAlpha = psq(coatRough);
   p.coatAx = fmaxf(p.coatAlpha, 1e-6f);
   p.inRefl = 0.0f;
-  p.inScale = pf3(1.0f, 1.0f, 1.0f);
+  p.inScale = pf4(1.0f, 1.0f, 1.0f, 1.0f);
   p.coatProb = 0.0f;
   if (P.coat > 0.0f) {
     const float Ks = pbr_average_fresnel(relCoat);
@@ -568,11 +566,12 @@ __device__ __forceinline__ PbrPrepared pbr_prepare(const PbrParams &P, const Pbr
     const float specOpaque = pbr_average_fresnel(p.etaOpaque);
     const float specBase = dielectric * specOpaque + P.metal;
     const float K = pmix(Ks, Kr, pmix(1.0f, rough, specBase));
-    const float3 Eb = padd(pscale(maf, p.metalAmount),
-                           pscale(pf3(pmix(p.f0.x, 1.0f, specOpaque), pmix(p.f0.y, 1.0f, specOpaque), pmix(p.f0.z, 1.0f, specOpaque)),
+    const float4 Eb = padd(pscale(maf, p.metalAmount),
+                           pscale(pf4(pmix(p.f0.x, 1.0f, specOpaque), pmix(p.f0.y, 1.0f, specOpaque), pmix(p.f0.z, 1.0f, specOpaque),
+                                      pmix(p.f0.w, 1.0f, specOpaque)),
                                   dielectric));
-    const float3 delta = pf3((1.0f - K) / (1.0f - Eb.x * K), (1.0f - K) / (1.0f - Eb.y * K), (1.0f - K) / (1.0f - Eb.z * K));
-    const float3 darkening = pf3(pmix(1.0f, delta.x, P.coat), pmix(1.0f, delta.y, P.coat), pmix(1.0f, delta.z, P.coat));
+    const float4 darkening = pf4(pmix(1.0f, (1.0f - K) / (1.0f - Eb.x * K), P.coat), pmix(1.0f, (1.0f - K) / (1.0f - Eb.y * K), P.coat),
+                                 pmix(1.0f, (1.0f - K) / (1.0f - Eb.z * K), P.coat), pmix(1.0f, (1.0f - K) / (1.0f - Eb.w * K), P.coat));
     p.inRefl = idotn > 0.0f ? pbr_dielectric_energy_reflected(T, relCoat, p.coatAlpha, idotn) * P.coat : 0.0f;
     p.inScale = pscale(darkening, 1.0f - p.inRefl);
   }
@@ -588,12 +587,8 @@ __device__ __forceinline__ PbrPrepared pbr_prepare(const PbrParams &P, const Pbr
     p.fuzzRefl = p.fwo.z <= 0.0f ? 0.0f : p.fuzz * pbr_ltc_fetch(T, kPbrFuzzRoughness, p.fwo.z).z;
   }
   // Lobe weights (estimated contributions with a white throughput).
-  if (!weights) {
-    p.wSpec = p.wMetal = p.wDiff = p.total = 0.0f;
-    return p;
-  }
   p.wSpec = pmax3(pbr_spec_coeff(p, idotn));
-  p.wMetal = p.alpha < kPbrMinAlphaEnergyLoss ? 0.0f : pmax3(p.metalScale) * p.metalEc;
+  p.wMetal = pmax3(p.metalScale) * p.metalEc;
   p.wDiff = pmax3(pscale(p.diffAlbedo, p.diffComp));
   p.total = ((((p.wSpec + 0.0f) + p.wMetal) + p.wDiff) + 0.0f) + 0.0f;
   if (p.coat > 0.0f && !p.inside)
@@ -610,272 +605,72 @@ __device__ __forceinline__ PbrPrepared pbr_prepare(const PbrParams &P, const Pbr
 
 
 
-__device__ __forceinline__ float3 pbr_spec_value(const PbrPrepared &p, float3 wi) {
-  const float idotn = pdot(p.B.n, p.wo), odotn = pdot(p.B.n, wi);
-  if (!(idotn * odotn > 0.0f)) return pf3(0.0f, 0.0f, 0.0f);
-  const float3 h = pnormalize(padd(p.wo, wi));
-  const float idoth = pdot(p.wo, h);
-  const float D = ggx_d(pbr_to_local(p.B, h), p.ax, p.ay);
-  const float other = 1.0f / (4.0f * idotn);
-  const float3 F = pbr_spec_coeff(p, fabsf(idoth));
-  const float3 DoF = pscale(F, D * other);
-  const float G = smith_g1(pbr_to_local(p.B, p.wo), p.ax, p.ay) * smith_g1(pbr_to_local(p.B, wi), p.ax, p.ay);
-  return pscale(DoF, G);
-}
-// The specular lobe's pdf: transmission has zero probability, reflection probability 1 unless the
-// reflection coefficient is zero.
-__device__ __forceinline__ float pbr_spec_pdf(const PbrPrepared &p, float3 wi) {
-  const float idotn = pdot(p.B.n, p.wo), odotn = pdot(p.B.n, wi);
-  if (!(idotn * odotn > 0.0f)) return 0.0f;
-  const float3 h = pnormalize(padd(p.wo, wi));
-  const float idoth = pdot(p.wo, h), odoth = pdot(wi, h);
-  if (idoth * odoth < 0.0f) return 0.0f;
-  const float D = ggx_d(pbr_to_local(p.B, h), p.ax, p.ay);
-  const float other = idoth / (4.0f * odoth * idotn);
-  const float rmax = pmax3(pbr_spec_coeff(p, fabsf(idoth)));
-  const float Fprob = psafe_div(rmax, rmax + 0.0f, 0.0f);
-  return smith_g1(pbr_to_local(p.B, p.wo), p.ax, p.ay) * (Fprob * D * other);
-}
-__device__ __forceinline__ bool pbr_spec_sample(const PbrPrepared &p, float3 r, float3 &wi, float3 &w, float &pdf) {
-  const float idotn = pdot(p.wo, p.B.n);
-  const float3 hl = ggx_sample_vndf(p.ax, p.ay, pbr_to_local(p.B, p.wo), make_float2(r.x, r.y));
-  const float3 h = pbr_to_world(p.B, hl);
-  const float idoth = pdot(p.wo, h);
-  if (idoth < 0.0f) return false;
-  const float3 Fr = pbr_spec_coeff(p, idoth);
-  const float rmax = pmax3(Fr);
-  const float Prefl = psafe_div(rmax, rmax + 0.0f, 0.0f);
-  if (Prefl + 0.0f == 0.0f) return false;
-  wi = pnormalize(padd(pscale(p.wo, -1.0f), pscale(h, 2.0f * idoth)));
-  const float odotn = pdot(p.B.n, wi);
-  if (idotn * odotn <= 0.0f) return false;
-  const float odoth = pdot(wi, h);
-  const float Gs = smith_g1(pbr_to_local(p.B, wi), p.ax, p.ay);
-  w = pscale(pscale(Fr, 1.0f / Prefl), Gs);
-  const float D = ggx_d(pbr_to_local(p.B, h), p.ax, p.ay);
-  if (D <= 0.0f) return false;
-  const float Gm = smith_g1(pbr_to_local(p.B, p.wo), p.ax, p.ay);
-  pdf = Prefl * D * Gm * idoth / (4.0f * odoth * idotn);
-  return true;
-}
-
-// Metal multiple scattering: a cosine-weighted lobe restoring the energy single scattering loses.
-__device__ __forceinline__ float pbr_metal_factor(const PbrPrepared &p, const PbrTables &T, float odotn) {
-  const float f = p.metalEc * pbr_metal_energy(T, p.alpha, odotn) / fmaxf(pbr_metal_average(T, p.alpha), 1e-12f);
-  return fminf(f, psafe_div(1.0f, odotn, 0.0f));
-}
-__device__ __forceinline__ float3 pbr_metal_value(const PbrPrepared &p, const PbrTables &T, float3 wi) {
-  if (p.alpha < kPbrMinAlphaEnergyLoss) return pf3(0.0f, 0.0f, 0.0f);
-  const float odotn = pdot(wi, p.B.n);
-  if (!(odotn > 0.0f)) return pf3(0.0f, 0.0f, 0.0f);
-  return pscale(p.metalScale, pbr_metal_factor(p, T, odotn) * kPbrRcpPi * odotn);
-}
-__device__ __forceinline__ float pbr_metal_pdf(const PbrPrepared &p, float3 wi) {
-  if (p.alpha < kPbrMinAlphaEnergyLoss) return 0.0f;
-  return pdot(wi, p.B.n) > 0.0f ? kPbrRcpTwoPi : 0.0f;
-}
-__device__ __forceinline__ bool pbr_metal_sample(const PbrPrepared &p, const PbrTables &T, float3 r, float3 &wi, float3 &w,
-                                                 float &pdf) {
-  if (p.alpha < kPbrMinAlphaEnergyLoss) return false;
-  const float z = r.x, horizontal = sqrtf(1.0f - psq(z)), az = kPbrTwoPi * r.y;
-  wi = pbr_to_world(pbr_basis(p.B.n), pf3(cosf(az) * horizontal, sinf(az) * horizontal, z));
-  const float odotn = pdot(wi, p.B.n);
-  w = pscale(p.metalScale, 2.0f * odotn * pbr_metal_factor(p, T, odotn));
-  pdf = kPbrRcpTwoPi;
-  return true;
-}
-
 // EON diffuse (Fujii-Oren-Nayar with the approximate albedo), scaled by the opaque specular's
-// energy complement at the light (openpbr_diffuse_lobe.h).
+// energy complement at the light (openpbr_diffuse_lobe.h); cosines of the view and the light to the
+// normal, and of the two to each other.
 __device__ __forceinline__ float pbr_e_fon(float mu, float r) {
   const float mc = 1.0f - mu;
   const float g = mc * (0.0571085289f + mc * (0.491881867f + mc * (-0.332181442f + mc * 0.0714429953f)));
   return (1.0f + r * g) / (1.0f + (0.5f - 2.0f / (3.0f * kPbrPi)) * r);
 }
-__device__ __forceinline__ float3 pbr_diffuse_local(const PbrPrepared &p, const PbrTables &T, float3 vi, float3 vo) {
+__device__ __forceinline__ float4 pbr_diffuse(const PbrPrepared &p, const PbrTables &T, float mui, float muo, float cosIO) {
   const float A = 0.5f - 2.0f / (3.0f * kPbrPi), Bc = 2.0f / 3.0f - 28.0f / (15.0f * kPbrPi);
-  const float r = p.diffRough, mui = vi.z, muo = vo.z;
-  const float s = pdot(vi, vo) - mui * muo;
+  const float r = p.diffRough;
+  const float s = cosIO - mui * muo;
   const float sot = s > 0.0f ? s / fmaxf(mui, muo) : s;
   const float AF = 1.0f / (1.0f + A * r);
-  const float3 rho = p.diffAlbedo;
-  const float ks = 1.0f + r * sot;
-  const float3 fss = pf3(rho.x * kPbrRcpPi * AF * ks, rho.y * kPbrRcpPi * AF * ks, rho.z * kPbrRcpPi * AF * ks);
+  const float4 rho = p.diffAlbedo;
+  const float4 fss = pscale(rho, kPbrRcpPi * AF * (1.0f + r * sot));
   const float EFo = pbr_e_fon(muo, r), EFi = pbr_e_fon(mui, r);
   const float avg = AF * (1.0f + Bc * r);
   const float mo = fmaxf(1e-7f, 1.0f - EFo), mi = fmaxf(1e-7f, 1.0f - EFi), ma = fmaxf(1e-7f, 1.0f - avg);
-  const float3 rms = pf3(rho.x * rho.x * avg / (1.0f - rho.x * (1.0f - avg)), rho.y * rho.y * avg / (1.0f - rho.y * (1.0f - avg)),
-                         rho.z * rho.z * avg / (1.0f - rho.z * (1.0f - avg)));
-  const float3 fms = pf3(rms.x * kPbrRcpPi * mo * mi / ma, rms.y * kPbrRcpPi * mo * mi / ma, rms.z * kPbrRcpPi * mo * mi / ma);
-  const float comp = p.diffComp * pbr_opaque_energy(T, p.etaOpaque, p.alpha, muo);
-  return pscale(padd(fss, fms), comp);
-}
-__device__ __forceinline__ float3 pbr_diffuse_value(const PbrPrepared &p, const PbrTables &T, float3 wi) {
-  const float co = pdot(wi, p.B.n);
-  if (co <= 0.0f) return pf3(0.0f, 0.0f, 0.0f);
-  const PbrBasis b = pbr_basis(p.B.n);
-  return pscale(pbr_diffuse_local(p, T, pbr_to_local(b, p.wo), pbr_to_local(b, wi)), co);
-}
-__device__ __forceinline__ float pbr_diffuse_pdf(const PbrPrepared &p, float3 wi) { return fmaxf(pdot(wi, p.B.n), 0.0f) * kPbrRcpPi; }
-__device__ __forceinline__ bool pbr_diffuse_sample(const PbrPrepared &p, const PbrTables &T, float3 r, float3 &wi, float3 &w,
-                                                   float &pdf) {
-  const float phi = kPbrTwoPi * r.x, z = sqrtf(r.y), rr = sqrtf(1.0f - r.y);
-  const float3 lo = pf3(cosf(phi) * rr, sinf(phi) * rr, z);
-  if (lo.z == 0.0f) return false;
-  const PbrBasis b = pbr_basis(p.B.n);
-  wi = pbr_to_world(b, lo);
-  w = pscale(pbr_diffuse_local(p, T, pbr_to_local(b, p.wo), lo), kPbrPi);
-  pdf = lo.z * kPbrRcpPi;
-  return true;
+  const float4 rms = pf4(rho.x * rho.x * avg / (1.0f - rho.x * (1.0f - avg)), rho.y * rho.y * avg / (1.0f - rho.y * (1.0f - avg)),
+                         rho.z * rho.z * avg / (1.0f - rho.z * (1.0f - avg)), rho.w * rho.w * avg / (1.0f - rho.w * (1.0f - avg)));
+  const float4 fms = pscale(rms, kPbrRcpPi * mo * mi / ma);
+  return pscale(padd(fss, fms), p.diffComp * pbr_opaque_energy(T, p.etaOpaque, p.alpha, muo));
 }
 
-// The aggregate: f |cos| and the lobe-weighted pdf.
-__device__ __forceinline__ float3 pbr_base_eval(const PbrPrepared &p, const PbrTables &T, float3 wi) {
-  float3 v = pbr_spec_value(p, wi);
-  v = padd(v, pbr_metal_value(p, T, wi));
-  v = padd(v, pbr_diffuse_value(p, T, wi));
+// The base (the aggregate lobe: microfacet specular, metal multiple scattering, diffuse): f |cos| and
+// the lobe-weighted pdf at wi, h the half vector. specPdf: the specular lobe's own pdf (transmission
+// has zero probability, reflection probability 1 unless the reflection coefficient is zero).
+__device__ __forceinline__ float4 pbr_base(const PbrPrepared &p, const PbrTables &T, float3 wi, float3 h, float &pdf, float &specPdf) {
+  const float idotn = pdot(p.B.n, p.wo), odotn = pdot(p.B.n, wi);
+  float4 v = pf4(0.0f, 0.0f, 0.0f, 0.0f);
+  specPdf = 0.0f;
+  if (idotn * odotn > 0.0f) {
+    const float idoth = pdot(p.wo, h), odoth = pdot(wi, h);
+    const float D = ggx_d(pbr_to_local(p.B, h), p.ax, p.ay);
+    const float Gi = smith_g1(pbr_to_local(p.B, p.wo), p.ax, p.ay), Go = smith_g1(pbr_to_local(p.B, wi), p.ax, p.ay);
+    const float4 F = pbr_spec_coeff(p, fabsf(idoth));
+    v = pscale(pscale(F, D * (1.0f / (4.0f * idotn))), Gi * Go);
+    if (!(idoth * odoth < 0.0f) && pmax3(F) != 0.0f) specPdf = Gi * (D * (idoth / (4.0f * odoth * idotn)));
+  }
+  float sum = p.wSpec * specPdf;
+  // Metal multiple scattering: a uniform lobe restoring the energy single scattering loses.
+  if (p.metalEc != 0.0f && odotn > 0.0f) {
+    const float f = fminf(p.metalEc * pbr_metal_energy(T, p.alpha, odotn) / fmaxf(p.metalAvg, 1e-12f), psafe_div(1.0f, odotn, 0.0f));
+    v = padd(v, pscale(p.metalScale, f * kPbrRcpPi * odotn));
+    sum += p.wMetal * kPbrRcpTwoPi;
+  }
+  if (p.scaleOpaque > 0.0f && odotn > 0.0f) {
+    v = padd(v, pscale(pbr_diffuse(p, T, idotn, odotn, pdot(p.wo, wi)), odotn));
+    sum += p.wDiff * (odotn * kPbrRcpPi);
+  }
+  pdf = p.total > 0.0f ? sum / p.total : 0.0f;
   return v;
-}
-__device__ __forceinline__ float pbr_base_pdf(const PbrPrepared &p, float3 wi) {
-  float sum = p.wSpec * pbr_spec_pdf(p, wi);
-  sum += p.wMetal * pbr_metal_pdf(p, wi);
-  sum += p.wDiff * pbr_diffuse_pdf(p, wi);
-  return p.total > 0.0f ? sum / p.total : 0.0f;
-}
-// One sample of the base (the aggregate lobe) from three numbers: direction, weight f |cos| / pdf and
-// pdf; false when none.
-__device__ __forceinline__ bool pbr_base_sample(const PbrPrepared &p, const PbrTables &T, float3 r, float3 &wi, float3 &w,
-                                                float &pdf) {
-  if (p.total <= kPbrFloatMin) return false;
-  float rx = r.x * p.total;
-  int lobe;
-  float sel;
-  if (rx < p.wSpec) {
-    lobe = 0; sel = p.wSpec; rx = rx / sel;
-  } else if (rx < p.wSpec + 0.0f + p.wMetal) {
-    lobe = 2; sel = p.wMetal; rx = (rx - (p.wSpec + 0.0f)) / sel;
-  } else {
-    lobe = 3; sel = p.wDiff; rx = (rx - ((p.wSpec + 0.0f) + p.wMetal)) / sel;
-  }
-  rx = pclamp_rand(rx);
-  const float3 rr = pf3(rx, r.y, r.z);
-  float3 lw;
-  float lp;
-  bool ok;
-  if (lobe == 0) ok = pbr_spec_sample(p, rr, wi, lw, lp);
-  else if (lobe == 2) ok = pbr_metal_sample(p, T, rr, wi, lw, lp);
-  else ok = pbr_diffuse_sample(p, T, rr, wi, lw, lp);
-  if (!ok) return false;
-  float3 fc = pscale(lw, lp);
-  float q = lp * sel;
-  if (lobe != 0) {
-    fc = padd(fc, pbr_spec_value(p, wi));
-    q += p.wSpec * pbr_spec_pdf(p, wi);
-  }
-  if (lobe != 2) {
-    fc = padd(fc, pbr_metal_value(p, T, wi));
-    q += p.wMetal * pbr_metal_pdf(p, wi);
-  }
-  if (lobe != 3) {
-    fc = padd(fc, pbr_diffuse_value(p, T, wi));
-    q += p.wDiff * pbr_diffuse_pdf(p, wi);
-  }
-  q /= p.total;
-  w = pscale(fc, 1.0f / q);
-  pdf = q;
-  return true;
 }
 
 // The coat's reflection (the generic minimal microfacet lobe with the coat's dielectric Fresnel,
 // impl/openpbr_generic_minimal_microfacet_lobe.h): GGX of the coat's alpha about the same normal.
-__device__ __forceinline__ float3 pbr_coat_value(const PbrPrepared &p, float3 wi) {
+__device__ __forceinline__ float pbr_coat(const PbrPrepared &p, float3 wi, float3 h, float &pdf) {
   const float idotn = pdot(p.B.n, p.wo), odotn = pdot(p.B.n, wi);
-  if (!(idotn * odotn > 0.0f)) return pf3(0.0f, 0.0f, 0.0f);
-  const float3 h = pnormalize(padd(p.wo, wi));
-  const float idoth = pdot(p.wo, h);
-  const float D = ggx_d(pbr_to_local(p.B, h), p.coatAx, p.coatAx);
-  const float other = 1.0f / (4.0f * idotn);
-  const float F = pbr_fresnel(p.coatEta, fabsf(idoth));
-  const float DoF = F * (D * other);
-  const float G = smith_g1(pbr_to_local(p.B, p.wo), p.coatAx, p.coatAx) * smith_g1(pbr_to_local(p.B, wi), p.coatAx, p.coatAx);
-  return pf3(DoF * G, DoF * G, DoF * G);
-}
-__device__ __forceinline__ float pbr_coat_pdf(const PbrPrepared &p, float3 wi) {
-  const float idotn = pdot(p.B.n, p.wo), odotn = pdot(p.B.n, wi);
+  pdf = 0.0f;
   if (!(idotn * odotn > 0.0f)) return 0.0f;
-  const float3 h = pnormalize(padd(p.wo, wi));
   const float idoth = pdot(p.wo, h), odoth = pdot(wi, h);
-  if (idoth * odoth < 0.0f) return 0.0f;
   const float D = ggx_d(pbr_to_local(p.B, h), p.coatAx, p.coatAx);
-  const float other = idoth / (4.0f * odoth * idotn);
-  return smith_g1(pbr_to_local(p.B, p.wo), p.coatAx, p.coatAx) * (D * other);
-}
-__device__ __forceinline__ bool pbr_coat_sample(const PbrPrepared &p, float3 r, float3 &wi, float3 &w, float &pdf) {
-  const float idotn = pdot(p.wo, p.B.n);
-  const float3 h = pbr_to_world(p.B, ggx_sample_vndf(p.coatAx, p.coatAx, pbr_to_local(p.B, p.wo), make_float2(r.x, r.y)));
-  const float idoth = pdot(p.wo, h);
-  if (idoth < 0.0f) return false;
-  wi = pnormalize(padd(pscale(p.wo, -1.0f), pscale(h, 2.0f * idoth)));
-  const float odotn = pdot(p.B.n, wi);
-  if (idotn * odotn <= 0.0f) return false;
-  const float odoth = pdot(wi, h);
-  const float F = pbr_fresnel(p.coatEta, idoth);
-  const float Gs = smith_g1(pbr_to_local(p.B, wi), p.coatAx, p.coatAx);
-  w = pf3(F * Gs, F * Gs, F * Gs);
-  const float D = ggx_d(pbr_to_local(p.B, h), p.coatAx, p.coatAx);
-  if (D <= 0.0f) return false;
-  const float Gm = smith_g1(pbr_to_local(p.B, p.wo), p.coatAx, p.coatAx);
-  pdf = D * Gm * idoth / (4.0f * odoth * idotn);
-  return true;
-}
-
-// The coating layer over the base (impl/openpbr_coating_lobe.h) and the fuzz layer over it (weight 0:
-// it passes the coated base through). Outside: f = coat presence x coat reflection + base x the base's
-// scale at the view (no attenuation on the light's side, OPENPBR_RECIPROCAL_COAT_AND_FUZZ 0); the pdf
-// mixes the coat's and the base's by the coat's sampling probability. From inside only the base
-// counts (a white coat tints nothing). Without a coat the coat's terms vanish and are skipped.
-__device__ __forceinline__ float3 pbr_coating_eval(const PbrPrepared &p, const PbrTables &T, float3 wi) {
-  const float3 base = pbr_base_eval(p, T, wi);
-  if (p.inside || !(p.coat > 0.0f)) return base;
-  return padd(pscale(pbr_coat_value(p, wi), p.coat), pmul(base, p.inScale));
-}
-__device__ __forceinline__ float pbr_coating_pdf(const PbrPrepared &p, float3 wi) {
-  const float pb = pbr_base_pdf(p, wi);
-  if (p.inside || !(p.coat > 0.0f)) return pb;
-  return pmix(pb, pbr_coat_pdf(p, wi), p.coatProb);
-}
-// One sample from three numbers: direction, weight f |cos| / pdf and pdf; false when none. Outside,
-// the coat or the base is chosen by r.x against the coat's probability (r.x remapped), and the weight
-// recomputed from both layers' f |cos| and pdfs; the fuzz layer recomputes it once more.
-__device__ __forceinline__ bool pbr_coating_sample(const PbrPrepared &p, const PbrTables &T, float3 r, float3 &wi, float3 &w,
-                                                   float &pdf) {
-  if (p.inside) {
-    if (!pbr_base_sample(p, T, r, wi, w, pdf)) return false;
-  } else {
-    const float cp = p.coatProb;
-    if (r.x < cp) {
-      const float rx = pclamp_rand(r.x * (1.0f / cp));
-      float3 wc;
-      float pc;
-      if (!pbr_coat_sample(p, pf3(rx, r.y, r.z), wi, wc, pc)) return false;
-      const float3 fc = padd(pscale(pscale(wc, pc), p.coat), pmul(pbr_base_eval(p, T, wi), p.inScale));
-      pdf = pmix(pbr_base_pdf(p, wi), pc, cp);
-      w = pscale(fc, 1.0f / pdf);
-    } else {
-      const float rx = pclamp_rand((r.x - cp) * (1.0f / (1.0f - cp)));
-      float3 wb;
-      float pb;
-      if (!pbr_base_sample(p, T, pf3(rx, r.y, r.z), wi, wb, pb)) return false;
-      float3 fc = pscale(wb, pb);
-      pdf = pb;
-      if (p.coat > 0.0f) {
-        fc = padd(pscale(pbr_coat_value(p, wi), p.coat), pmul(fc, p.inScale));
-        pdf = pmix(pb, pbr_coat_pdf(p, wi), cp);
-      }
-      w = pscale(fc, 1.0f / pdf);
-    }
-  }
-  return true;
+  const float Gi = smith_g1(pbr_to_local(p.B, p.wo), p.coatAx, p.coatAx), Go = smith_g1(pbr_to_local(p.B, wi), p.coatAx, p.coatAx);
+  if (!(idoth * odoth < 0.0f)) pdf = Gi * (D * (idoth / (4.0f * odoth * idotn)));
+  return pbr_fresnel(p.coatEta, fabsf(idoth)) * (D * (1.0f / (4.0f * idotn))) * (Gi * Go);
 }
 
 // The fuzz (Disney sheen) lobe as linearly transformed cosines (Zeltner, Burley and Chiang 2022;
@@ -896,12 +691,11 @@ __device__ __forceinline__ float pbr_sheen_ltc(float3 wl, float3 k) {
   const float t = k.x / len2;
   return kPbrRcpPi * (z * t) * t;
 }
-__device__ __forceinline__ float3 pbr_sheen_f(const PbrPrepared &p, const PbrTables &T, float3 wl) {
-  if (p.fwo.z <= 0.0f || wl.z <= 0.0f) return pf3(0.0f, 0.0f, 0.0f);
+__device__ __forceinline__ float pbr_sheen_f(const PbrPrepared &p, const PbrTables &T, float3 wl) {
+  if (p.fwo.z <= 0.0f || wl.z <= 0.0f) return 0.0f;
   const float3 ws = pbr_sheen_rotate(wl, p.fwo.x, -p.fwo.y);
   const float3 k = pbr_ltc_fetch(T, kPbrFuzzRoughness, p.fwo.z);
-  const float v = pbr_sheen_ltc(ws, k) * (p.fuzz * k.z * 1.0f);
-  return pf3(v, v, v);
+  return pbr_sheen_ltc(ws, k) * (p.fuzz * k.z * 1.0f);
 }
 __device__ __forceinline__ float pbr_sheen_pdf(const PbrPrepared &p, const PbrTables &T, float3 wl) {
   if (p.fwo.z <= 0.0f || wl.z <= 0.0f) return 0.0f;
@@ -918,43 +712,106 @@ __device__ __forceinline__ bool pbr_sheen_sample(const PbrPrepared &p, const Pbr
   return p.fwo.z * wl.z > 0.0f;
 }
 
-// The fuzz layer over the coated base: f = coated base x (1 - the fuzz's share at the view) + sheen;
-// the pdf mixes the two by the fuzz's sampling probability. Without fuzz the sheen terms vanish and are
-// skipped; the layer still recomputes a sample's weight from f |cos| and the pdf.
-__device__ __forceinline__ float3 pbr_eval(const PbrPrepared &p, const PbrTables &T, float3 wi) {
-  const float3 coated = pbr_coating_eval(p, T, wi);
-  if (!(p.fuzz > 0.0f)) return coated;
-  return padd(pscale(coated, 1.0f - p.fuzzRefl), pbr_sheen_f(p, T, pbr_to_local(p.FB, wi)));
-}
-__device__ __forceinline__ float pbr_pdf(const PbrPrepared &p, const PbrTables &T, float3 wi) {
-  const float pc = pbr_coating_pdf(p, wi);
-  if (!(p.fuzz > 0.0f)) return pc;
-  return pmix(pc, pbr_sheen_pdf(p, T, pbr_to_local(p.FB, wi)), p.fuzzProb);
-}
-__device__ __forceinline__ bool pbr_sample(const PbrPrepared &p, const PbrTables &T, float3 r, float3 &wi, float3 &w, float &pdf) {
+// f |cos| and the pdf at wi. The coating layer over the base (impl/openpbr_coating_lobe.h): outside,
+// f = coat presence x coat reflection + base x the base's scale at the view (no attenuation on the
+// light's side, OPENPBR_RECIPROCAL_COAT_AND_FUZZ 0); the pdf mixes the coat's and the base's by the
+// coat's sampling probability. From inside only the base counts (a white coat tints nothing). The
+// fuzz layer over it: f = coated base x (1 - the fuzz's share at the view) + sheen, the pdf mixed by
+// the fuzz's sampling probability. Absent layers are skipped.
+// `half`: the half vector when the caller sampled it (it is then not rebuilt from the directions,
+// which a narrow lobe would feel), else null.
+__device__ __forceinline__ float4 pbr_eval_pdf(const PbrPrepared &p, const PbrTables &T, float3 wi, const float3 *half, float &pdf,
+                                               float &specPdf) {
+  float3 h = half ? *half : padd(p.wo, wi);
+  if (!half) h = pnormalize(h);
+  float4 v = pbr_base(p, T, wi, h, pdf, specPdf);
+  if (p.coat > 0.0f && !p.inside) {
+    float pc;
+    const float c = pbr_coat(p, wi, h, pc) * p.coat;
+    v = padd(pf4(c, c, c, c), pmul(v, p.inScale));
+    pdf = pmix(pdf, pc, p.coatProb);
+  }
   if (p.fuzz > 0.0f) {
-    const float sp = p.fuzzProb, bp = 1.0f - sp;
+    const float3 wl = pbr_to_local(p.FB, wi);
+    const float f = pbr_sheen_f(p, T, wl);
+    v = padd(pscale(v, 1.0f - p.fuzzRefl), pf4(f, f, f, f));
+    pdf = pmix(pdf, pbr_sheen_pdf(p, T, wl), p.fuzzProb);
+  }
+  return v;
+}
+
+// A direction from three numbers: the fuzz, the coat or the base is chosen by r.x against their
+// probabilities (r.x remapped), the base's lobe by estimated contribution. `half` is the direction's
+// half vector; `spec` tells that the specular lobe was sampled. False when there is none.
+__device__ __forceinline__ bool pbr_sample_direction(const PbrPrepared &p, const PbrTables &T, float3 r, float3 &wi, float3 &half,
+                                                     bool &spec) {
+  spec = false;
+  if (p.fuzz > 0.0f) {
+    const float sp = p.fuzzProb;
     if (r.x < sp) {
       float3 wl;
       if (!pbr_sheen_sample(p, T, make_float2(r.y, r.z), wl)) return false;
       wi = pnormalize(pbr_to_world(p.FB, wl));
-      pdf = pbr_sheen_pdf(p, T, wl) * sp;
-      pdf += pbr_coating_pdf(p, wi) * bp;
-      w = pscale(pbr_eval(p, T, wi), 1.0f / pdf);
+      half = pnormalize(padd(p.wo, wi));
       return true;
     }
-    const float rx = pclamp_rand((r.x - sp) * (1.0f / bp));
-    if (!pbr_coating_sample(p, T, pf3(rx, r.y, r.z), wi, w, pdf)) return false;
-    const float3 wl = pbr_to_local(p.FB, wi);
-    float3 fc = pscale(pscale(w, pdf), 1.0f - p.fuzzRefl);
-    fc = padd(fc, pbr_sheen_f(p, T, wl));
-    pdf *= bp;
-    pdf += pbr_sheen_pdf(p, T, wl) * sp;
-    w = pscale(fc, 1.0f / pdf);
-    return true;
+    r.x = pclamp_rand((r.x - sp) * (1.0f / (1.0f - sp)));
   }
-  if (!pbr_coating_sample(p, T, r, wi, w, pdf)) return false;
-  w = pscale(pscale(w, pdf), 1.0f / pdf);
+  float ax = p.ax, ay = p.ay;  // the microfacet lobe to sample: the base's or the coat's
+  bool facet = false;
+  if (!p.inside) {
+    const float cp = p.coatProb;
+    if (r.x < cp) {
+      r.x = pclamp_rand(r.x * (1.0f / cp));
+      ax = ay = p.coatAx;
+      facet = true;
+    } else {
+      r.x = pclamp_rand((r.x - cp) * (1.0f / (1.0f - cp)));
+    }
+  }
+  int lobe = 0;
+  if (!facet) {
+    if (p.total <= kPbrFloatMin) return false;
+    float rx = r.x * p.total;
+    if (rx < p.wSpec) {
+      rx = rx / p.wSpec;
+      facet = spec = true;
+    } else if (rx < p.wSpec + p.wMetal) {
+      lobe = 2;
+      rx = (rx - p.wSpec) / p.wMetal;
+    } else {
+      lobe = 3;
+      rx = (rx - (p.wSpec + p.wMetal)) / p.wDiff;
+    }
+    r.x = pclamp_rand(rx);
+  }
+  if (facet) {
+    const float idotn = pdot(p.wo, p.B.n);
+    half = pbr_to_world(p.B, ggx_sample_vndf(ax, ay, pbr_to_local(p.B, p.wo), make_float2(r.x, r.y)));
+    const float idoth = pdot(p.wo, half);
+    if (idoth < 0.0f) return false;
+    wi = pnormalize(padd(pscale(p.wo, -1.0f), pscale(half, 2.0f * idoth)));
+    return !(idotn * pdot(p.B.n, wi) <= 0.0f);
+  }
+  // Uniform (metal) or cosine-weighted (diffuse) about the normal.
+  const float az = kPbrTwoPi * (lobe == 2 ? r.y : r.x);
+  const float z = lobe == 2 ? r.x : sqrtf(r.y), horizontal = sqrtf(1.0f - (lobe == 2 ? psq(z) : r.y));
+  if (lobe == 3 && z == 0.0f) return false;
+  wi = pbr_to_world(pbr_basis(p.B.n), pf3(cosf(az) * horizontal, sinf(az) * horizontal, z));
+  half = pnormalize(padd(p.wo, wi));
+  return true;
+}
+
+// One sample: direction, weight f |cos| / pdf and pdf; false when none.
+__device__ __forceinline__ bool pbr_sample(const PbrPrepared &p, const PbrTables &T, float3 r, float3 &wi, float4 &w, float &pdf) {
+  float3 half;
+  bool spec;
+  pdf = 0.0f;
+  if (!pbr_sample_direction(p, T, r, wi, half, spec)) return false;
+  float specPdf;
+  const float4 f = pbr_eval_pdf(p, T, wi, &half, pdf, specPdf);
+  if (spec && !(specPdf > 0.0f)) return false;
+  w = pscale(f, 1.0f / pdf);
   return true;
 }
 
