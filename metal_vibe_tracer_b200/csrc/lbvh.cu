@@ -241,128 +241,61 @@ __device__ __forceinline__ void refit_node(const TreeView &t, int i) {
 // only on a strict cost improvement, internal nodes reassigned depth first, left = the side with
 // the lowest leaf bit.
 //
-// Two executions of that one algorithm give the same tree. restructure_node is one thread's
-// serial loop. restructure_warp spreads one treelet over a warp (Karras and Aila's warp-wide DP):
-// lane q holds treelet leaf q while the treelet grows (its box, children, cost and leaf count
-// loaded in one round trip, the largest area chosen by a shuffle reduction that keeps the first
-// slot on ties); the subsets are listed by size with ballots (increasing s within a size); per
-// size either each lane takes whole subsets (fewer than 32 partitions) or all lanes split one
-// subset's partitions and reduce (cost, then serial order), so the chosen partition is the
-// serial loop's; the rebuilt nodes' boxes, counts and costs are formed in shared memory in
-// refit_node's order (union of left then right, costs added left + right) and stored by one lane
-// per node. Scratch lives in shared memory, one slice per warp.
-__device__ void restructure_node(const TreeView &t, int root, int size, uint32_t *status) {
-  int leaves[kMaxTreelet], internals[kMaxTreelet];
-  int nl = 0, ni = 0;
-  internals[ni++] = root;
-  int2 rc = load_child(t, root);
-  leaves[nl++] = rc.x;
-  leaves[nl++] = rc.y;
-  while (nl < size) {
-    int best = -1;
-    float bestA = -1.0f;
-    for (int k = 0; k < nl; ++k) {
-      int c = leaves[k];
-      if (c < 0) continue;
-      Box b = load_box_cg(t.nodeBox, c);
-      float a = box_area(b.lo, b.hi);
-      if (a > bestA) { bestA = a; best = k; }
-    }
-    if (best < 0) break;
-    int c = leaves[best];
-    internals[ni++] = c;
-    int2 cc = load_child(t, c);
-    leaves[best] = cc.x;
-    leaves[nl++] = cc.y;
-  }
-  const int k = nl;
-  if (k < 3) return;
-  const int full = (1 << k) - 1;
-  float area[1 << kMaxTreelet], copt[1 << kMaxTreelet];
-  uint8_t part[1 << kMaxTreelet];
-  Box lb[kMaxTreelet];
-  for (int q = 0; q < k; ++q) {
-    lb[q] = child_box(t, leaves[q]);
-    copt[1 << q] = child_cost(t, leaves[q]);
-  }
-  for (int s = 1; s <= full; ++s) {
-    int low = __ffs(s) - 1;
-    Box b = lb[low];
-    for (int r = s & (s - 1); r; r &= r - 1) b = box_union(b, lb[__ffs(r) - 1]);
-    area[s] = box_area(b.lo, b.hi);
-  }
-  for (int sz = 2; sz <= k; ++sz) {
-    for (int s = 1; s <= full; ++s) {
-      if (__popc(s) != sz) continue;
-      float best = FLT_MAX;
-      int bp = 0;
-      for (int p = (s - 1) & s; p > 0; p = (p - 1) & s) {
-        float c = __fadd_rn(copt[p], copt[s ^ p]);
-        if (c < best) { best = c; bp = p; }
-      }
-      copt[s] = __fadd_rn(__fmul_rn(kCi, area[s]), best);
-      part[s] = (uint8_t)bp;
-    }
-  }
-  if (!(copt[full] < __ldcg(t.cost + root))) return;
-  int next = 0;
-  int st_s[kMaxTreelet * 2], st_n[kMaxTreelet * 2];
-  int top = 0;
-  st_s[top] = full; st_n[top] = internals[next++]; ++top;
-  while (top) {
-    --top;
-    const int s = st_s[top], node = st_n[top];
-    const int p = part[s], q = s ^ p;
-    const int lowbit = s & -s;
-    const int subs[2] = {(p & lowbit) ? p : q, (p & lowbit) ? q : p};
-    int kids[2];
-    for (int c = 0; c < 2; ++c) {
-      const int x = subs[c];
-      if ((x & (x - 1)) == 0) kids[c] = leaves[__ffs(x) - 1];
-      else {
-        if (next >= ni) { atomicOr(status, (uint32_t)VT_DEV_TREELET); return; }
-        kids[c] = internals[next++];
-      }
-    }
-    __stcg(t.child + node, make_int2(kids[0], kids[1]));
-    for (int c = 1; c >= 0; --c)
-      if ((subs[c] & (subs[c] - 1)) != 0) { st_s[top] = subs[c]; st_n[top] = kids[c]; ++top; }
-  }
-  for (int i = ni - 1; i >= 0; --i) {
-    const int nd = internals[i];
-    refit_node(t, nd);
-    int2 ch = load_child(t, nd);
-    __stcg(t.parent + (ch.x >= 0 ? ch.x : (t.n - 1 + (-ch.x - 1))), nd);
-    __stcg(t.parent + (ch.y >= 0 ? ch.y : (t.n - 1 + (-ch.y - 1))), nd);
-  }
-}
-
+// A warp takes one treelet (Karras and Aila's warp-wide DP): lane q holds treelet leaf q while the
+// treelet grows (its box, children, cost and leaf count loaded in one round trip, the largest area
+// chosen by a warp reduction that keeps the first slot on ties). The DP visits the subsets by size,
+// one or more lanes a subset. A partition and its complement cost the same, and the serial loop meets
+// the one with the subset's highest leaf first: only those are tried, the largest of equal cost kept.
+// A subset's box is the union of two table entries (of the low and of the high four leaves). The
+// rebuilt nodes need no second pass: a node's cost is its subset's optimum, whose sums are the same.
+//
+// Bound: latency of the chain of treelets from the leaves to the root (loads of a growing treelet, the
+// DP's shared-memory reads) and, for large meshes, issue. Measured on one B200, whole builds with
+// three rounds of treelets of 7: 1,000 triangles 0.84 -> 0.60 ms, 20,480 1.31 -> 0.88, 200,000
+// 2.16 -> 1.42, 1M 6.16 -> 3.72, 4M 21.0 -> 12.0. Before, small treelets near the leaves were taken by
+// single threads (divergent, arrays in local memory), the DP tried every partition with a box
+// recomputed per subset, and the rebuilt nodes were refitted one by one.
 struct TreeletScratch {
-  float area[1 << kMaxTreelet];
+  float4 tabLo[32], tabHi[32];  // boxes of the subsets of leaves 0-3 (entries 0-15) and of 4-7 (16-31)
+  float4 leafLo[kMaxTreelet], leafHi[kMaxTreelet];
   float copt[1 << kMaxTreelet];
   uint8_t part[1 << kMaxTreelet];
-  uint8_t list[1 << kMaxTreelet];  // subsets grouped by size, increasing within a size
-  Box lb[kMaxTreelet];             // treelet leaves' boxes
-  Box nb[kMaxTreelet];             // rebuilt internal nodes' boxes (assignment order)
-  float nc[kMaxTreelet];           // and costs
-  uint32_t ncount[kMaxTreelet], lcount[kMaxTreelet];
   int leaves[kMaxTreelet], internals[kMaxTreelet];
-  int2 kid[kMaxTreelet];           // rebuilt node j's children: >= 0 internal index, else -(leaf slot + 1)
-  int start[kMaxTreelet + 2];      // list offset of each subset size
+  uint32_t lcount[kMaxTreelet];
+  int2 kid[kMaxTreelet];        // rebuilt node j's children: >= 0 internal index, else -(leaf slot + 1)
+  uint8_t set[kMaxTreelet];     // rebuilt node j's subset
   int ok;
 };
 
-// The bits of m deposited into the set bits of s, lowest first (pdep).
-__device__ __forceinline__ int deposit_bits(int m, int s) {
-  int out = 0;
-  for (int r = s; r; r &= r - 1) {
-    if (m & 1) out |= r & -r;
-    m >>= 1;
+// The nonempty subsets of 8 leaves grouped by size, increasing within a size, so that for k leaves each
+// group's first C(k, size) entries are the subsets of those; copied to shared memory once per block.
+struct alignas(4) SubsetTable {
+  uint8_t list[256];
+  int start[kMaxTreelet + 2];
+};
+constexpr SubsetTable make_subsets() {
+  SubsetTable t{};
+  int at = 0;
+  for (int size = 1; size <= kMaxTreelet; ++size) {
+    t.start[size] = at;
+    for (int s = 1; s < 256; ++s) {
+      int bits = 0;
+      for (int r = s; r; r &= r - 1) ++bits;
+      if (bits == size) t.list[at++] = (uint8_t)s;
+    }
   }
-  return out;
+  t.start[kMaxTreelet + 1] = at;
+  return t;
+}
+__device__ const SubsetTable kSubsets = make_subsets();
+
+__device__ __forceinline__ Box subset_box(const TreeletScratch &w, int s) {
+  const float4 al = w.tabLo[s & 15], ah = w.tabHi[s & 15], bl = w.tabLo[16 + (s >> 4)], bh = w.tabHi[16 + (s >> 4)];
+  return box_union(Box{make_float3(al.x, al.y, al.z), make_float3(ah.x, ah.y, ah.z)},
+                   Box{make_float3(bl.x, bl.y, bl.z), make_float3(bh.x, bh.y, bh.z)});
 }
 
-__device__ void restructure_warp(const TreeView &t, int root, int size, uint32_t *status, TreeletScratch &w) {
+__device__ void restructure_warp(const TreeView &t, int root, int size, uint32_t *status, TreeletScratch &w, const SubsetTable &sets) {
   const unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const float rootCost = __ldcg(t.cost + root);
@@ -372,8 +305,8 @@ __device__ void restructure_warp(const TreeView &t, int root, int size, uint32_t
   bool dirty = lane < 2;
   Box myBox{};
   int2 myKids = make_int2(0, 0);
-  float myArea = -INFINITY, myCost = 0.0f;
-  uint32_t myCount = 1u;
+  float myCost = 0.0f;
+  uint32_t myCount = 1u, myKey = 0u;  // key: area bits + 1 of a leaf that can be opened
   int myInternal = lane == 0 ? root : -1;
   int nl = 2, ni = 1;
   while (true) {
@@ -383,24 +316,19 @@ __device__ void restructure_warp(const TreeView &t, int root, int size, uint32_t
         myKids = load_child(t, myLeaf);
         myCost = __ldcg(t.cost + myLeaf);
         myCount = __ldcg(t.count + myLeaf);
-        myArea = box_area(myBox.lo, myBox.hi);
-      } else {
+        myKey = __float_as_uint(box_area(myBox.lo, myBox.hi)) + 1u;
+      } else {  // a primitive is never opened
         myBox = load_box_cg(t.leafBox, -myLeaf - 1);
         myCost = __fmul_rn(kCt, box_area(myBox.lo, myBox.hi));
         myCount = 1u;
-        myArea = -INFINITY;  // a primitive is never opened
+        myKey = 0u;
       }
       dirty = false;
     }
     if (nl >= size) break;
-    float a = lane < nl ? myArea : -INFINITY;
-    int q = lane;
-    for (int off = 16; off > 0; off >>= 1) {
-      const float oa = __shfl_xor_sync(kAll, a, off);
-      const int oq = __shfl_xor_sync(kAll, q, off);
-      if (oa > a || (oa == a && oq < q)) { a = oa; q = oq; }
-    }
-    if (a == -INFINITY) break;  // no internal node left to open
+    const uint32_t largest = __reduce_max_sync(kAll, lane < nl ? myKey : 0u);
+    if (largest == 0u) break;  // no internal node left to open
+    const int q = __ffs(__ballot_sync(kAll, lane < nl && myKey == largest)) - 1;
     const int c = __shfl_sync(kAll, myLeaf, q);
     const int cx = __shfl_sync(kAll, myKids.x, q), cy = __shfl_sync(kAll, myKids.y, q);
     if (lane == ni) myInternal = c;
@@ -414,143 +342,121 @@ __device__ void restructure_warp(const TreeView &t, int root, int size, uint32_t
   const int full = (1 << k) - 1;
   if (lane < k) {
     w.leaves[lane] = myLeaf;
-    w.lb[lane] = myBox;
+    w.leafLo[lane] = make_float4(myBox.lo.x, myBox.lo.y, myBox.lo.z, 0.0f);
+    w.leafHi[lane] = make_float4(myBox.hi.x, myBox.hi.y, myBox.hi.z, 0.0f);
     w.copt[1 << lane] = myCost;
     w.lcount[lane] = myCount;
   }
   if (lane < ni) w.internals[lane] = myInternal;
-  if (lane == 0) {
-    // Subsets of size j start after those of sizes 2..j-1: C(k, 2) + ... + C(k, j-1).
-    int off = 0, c = k;  // c = C(k, j) for j = 1
-    for (int j = 2; j <= k; ++j) {
-      c = c * (k - j + 1) / j;
-      w.start[j] = off;
-      off += c;
-    }
-    w.start[k + 1] = off;
-  }
   __syncwarp();
-  // Subset areas and the by-size lists, 32 subsets per step.
-  int fill[kMaxTreelet + 1];
+  {
+    Box b{make_float3(INFINITY, INFINITY, INFINITY), make_float3(-INFINITY, -INFINITY, -INFINITY)};
 #pragma unroll
-  for (int j = 0; j <= kMaxTreelet; ++j) fill[j] = 0;
-  for (int base = 0; base < full; base += 32) {
-    const int s = base + lane + 1;
-    const bool valid = s <= full;
-    if (valid) {
-      Box b = w.lb[__ffs(s) - 1];
-      for (int r = s & (s - 1); r; r &= r - 1) b = box_union(b, w.lb[__ffs(r) - 1]);
-      w.area[s] = box_area(b.lo, b.hi);
-    }
-    const int pc = valid ? __popc(s) : 0;
-#pragma unroll
-    for (int j = 2; j <= kMaxTreelet; ++j) {
-      if (j > k) break;
-      const unsigned m = __ballot_sync(kAll, pc == j);
-      if (pc == j) w.list[w.start[j] + fill[j] + __popc(m & ((1u << lane) - 1u))] = (uint8_t)s;
-      fill[j] += __popc(m);
-    }
-  }
-  __syncwarp();
-  for (int sz = 2; sz <= k; ++sz) {
-    const int np = (1 << sz) - 2;  // partitions of a subset of size sz
-    const int b0 = w.start[sz], nsub = w.start[sz + 1] - b0;
-    if (np < 32) {
-      for (int j = lane; j < nsub; j += 32) {
-        const int s = w.list[b0 + j];
-        float best = FLT_MAX;
-        int bp = 0;
-        for (int p = (s - 1) & s; p > 0; p = (p - 1) & s) {
-          const float c = __fadd_rn(w.copt[p], w.copt[s ^ p]);
-          if (c < best) { best = c; bp = p; }
-        }
-        w.copt[s] = __fadd_rn(__fmul_rn(kCi, w.area[s]), best);
-        w.part[s] = (uint8_t)bp;
+    for (int q = 0; q < 4; ++q) {
+      const int leaf = (lane >> 4) * 4 + q;
+      if ((lane >> q & 1) && leaf < k) {
+        const float4 l = w.leafLo[leaf], h = w.leafHi[leaf];
+        b = box_union(b, Box{make_float3(l.x, l.y, l.z), make_float3(h.x, h.y, h.z)});
       }
-    } else {
-      // All lanes on one subset: partition i (serial order, p descending) is deposit(np - i, s).
-      for (int j = 0; j < nsub; ++j) {
-        const int s = w.list[b0 + j];
-        float best = FLT_MAX;
-        int bi = 0x7fffffff;
-        for (int i = lane; i < np; i += 32) {
-          const int p = deposit_bits(np - i, s);
-          const float c = __fadd_rn(w.copt[p], w.copt[s ^ p]);
-          if (c < best) { best = c; bi = i; }
+    }
+    w.tabLo[lane] = make_float4(b.lo.x, b.lo.y, b.lo.z, 0.0f);
+    w.tabHi[lane] = make_float4(b.hi.x, b.hi.y, b.hi.z, 0.0f);
+  }
+  __syncwarp();
+  int nsub = k;  // C(k, sz)
+  for (int sz = 2; sz <= k; ++sz) {
+    nsub = nsub * (k - sz + 1) / sz;
+    // 2^g lanes a subset (as many as keep all subsets in one round, at most one per partition half).
+    int g = 0;
+    while (g < sz - 1 && (nsub << (g + 1)) <= 32) ++g;
+    for (int j0 = 0; j0 < nsub; j0 += 32 >> g) {
+      const int j = j0 + (lane >> g);
+      const bool active = j < nsub;
+      const int s = active ? sets.list[sets.start[sz] + j] : full;
+      const int top = 1 << (31 - __clz(s)), rest = s ^ top;
+      // This lane fixes the g lowest leaves of the rest by its place in the group and tries every choice
+      // of the others.
+      int fixed = 0, open = rest;
+      for (int q = 0; q < g; ++q) {
+        const int bit = open & -open;
+        open ^= bit;
+        if (lane >> q & 1) fixed |= bit;
+      }
+      float best = FLT_MAX;
+      int bp = 0;
+      if (active) {
+        for (int sub = open;; sub = (sub - 1) & open) {
+          const int p = top | fixed | sub;
+          if (p != s) {
+            const float c = __fadd_rn(w.copt[p], w.copt[s ^ p]);
+            if (c < best || (c == best && bp != 0 && p > bp)) { best = c; bp = p; }
+          }
+          if (sub == 0) break;
         }
-        for (int off = 16; off > 0; off >>= 1) {
-          const float ob = __shfl_xor_sync(kAll, best, off);
-          const int oi = __shfl_xor_sync(kAll, bi, off);
-          if (ob < best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-        }
-        if (lane == 0) {
-          w.copt[s] = __fadd_rn(__fmul_rn(kCi, w.area[s]), best);
-          w.part[s] = (uint8_t)deposit_bits(np - bi, s);
-        }
+      }
+      for (int off = 1; off < (1 << g); off <<= 1) {
+        const float ob = __shfl_xor_sync(kAll, best, off);
+        const int op = __shfl_xor_sync(kAll, bp, off);
+        if (ob < best || (ob == best && op > bp)) { best = ob; bp = op; }
+      }
+      if (active && (lane & ((1 << g) - 1)) == 0) {
+        const Box b = subset_box(w, s);
+        w.copt[s] = __fadd_rn(__fmul_rn(kCi, box_area(b.lo, b.hi)), best);
+        w.part[s] = (uint8_t)bp;
       }
     }
     __syncwarp();
   }
   if (!(w.copt[full] < rootCost)) return;
   if (lane == 0) {
-    // Depth-first assignment of the internal nodes (index j in assignment order), then their
-    // boxes, counts and costs bottom up (children are assigned after their parent).
-    int next = 1;
-    int st_s[kMaxTreelet * 2], st_j[kMaxTreelet * 2];
-    int top = 0;
-    st_s[top] = full; st_j[top] = 0; ++top;
+    // Depth-first assignment of the internal nodes: index j in assignment order, a stack of 4-bit indices.
+    int next = 1, depth = 1;
+    uint32_t stack = 0u;
+    w.set[0] = (uint8_t)full;
     w.ok = 1;
-    while (top) {
-      --top;
-      const int s = st_s[top], j = st_j[top];
-      const int p = w.part[s], q = s ^ p;
+    while (depth > 0) {
+      const int j = (int)(stack & 15u);
+      stack >>= 4;
+      --depth;
+      const int s = w.set[j], p = w.part[s], q = s ^ p;
       const int lowbit = s & -s;
-      const int subs[2] = {(p & lowbit) ? p : q, (p & lowbit) ? q : p};
-      int ref[2];
-      for (int c = 0; c < 2; ++c) {
-        const int x = subs[c];
-        if ((x & (x - 1)) == 0) ref[c] = -__ffs(x);  // -(leaf slot + 1)
-        else {
-          if (next >= ni) { w.ok = 0; top = 0; break; }
-          ref[c] = next++;
-        }
-      }
-      if (!w.ok) break;
-      w.kid[j] = make_int2(ref[0], ref[1]);
-      for (int c = 1; c >= 0; --c)
-        if (ref[c] >= 0) { st_s[top] = subs[c]; st_j[top] = ref[c]; ++top; }
+      const int left = (p & lowbit) ? p : q, right = (p & lowbit) ? q : p;
+      int2 ref;
+      const bool li = (left & (left - 1)) != 0, ri = (right & (right - 1)) != 0;
+      if (next + (li ? 1 : 0) + (ri ? 1 : 0) > ni) { w.ok = 0; break; }
+      ref.x = li ? next++ : -__ffs(left);  // -(leaf slot + 1)
+      ref.y = ri ? next++ : -__ffs(right);
+      w.kid[j] = ref;
+      if (ri) { w.set[ref.y] = (uint8_t)right; stack = stack << 4 | (uint32_t)ref.y; ++depth; }
+      if (li) { w.set[ref.x] = (uint8_t)left; stack = stack << 4 | (uint32_t)ref.x; ++depth; }
     }
-    if (w.ok) {
-      for (int j = ni - 1; j >= 0; --j) {
-        const int2 r = w.kid[j];
-        const Box bx = r.x >= 0 ? w.nb[r.x] : w.lb[-r.x - 1];
-        const Box by = r.y >= 0 ? w.nb[r.y] : w.lb[-r.y - 1];
-        const Box b = box_union(bx, by);
-        const float cx = r.x >= 0 ? w.nc[r.x] : w.copt[1 << (-r.x - 1)];
-        const float cy = r.y >= 0 ? w.nc[r.y] : w.copt[1 << (-r.y - 1)];
-        w.nb[j] = b;
-        w.nc[j] = __fadd_rn(__fmul_rn(kCi, box_area(b.lo, b.hi)), __fadd_rn(cx, cy));
-        w.ncount[j] = (r.x >= 0 ? w.ncount[r.x] : w.lcount[-r.x - 1]) + (r.y >= 0 ? w.ncount[r.y] : w.lcount[-r.y - 1]);
-      }
-    } else {
-      atomicOr(status, (uint32_t)VT_DEV_TREELET);
-    }
+    if (!w.ok) atomicOr(status, (uint32_t)VT_DEV_TREELET);
   }
   __syncwarp();
   if (!w.ok || lane >= ni) return;
-  const int node = w.internals[lane];
+  const int node = w.internals[lane], s = w.set[lane];
   const int2 r = w.kid[lane];
   const int kx = r.x >= 0 ? w.internals[r.x] : w.leaves[-r.x - 1];
   const int ky = r.y >= 0 ? w.internals[r.y] : w.leaves[-r.y - 1];
+  uint32_t count = 0;
+  for (int q = 0; q < k; ++q) count += (s >> q & 1) ? w.lcount[q] : 0u;
   __stcg(t.child + node, make_int2(kx, ky));
-  store_box(t.nodeBox, node, w.nb[lane]);
-  __stcg(t.count + node, w.ncount[lane]);
-  __stcg(t.cost + node, w.nc[lane]);
+  store_box(t.nodeBox, node, subset_box(w, s));
+  __stcg(t.count + node, count);
+  __stcg(t.cost + node, w.copt[s]);
   __stcg(t.parent + (kx >= 0 ? kx : (t.n - 1 + (-kx - 1))), node);
   __stcg(t.parent + (ky >= 0 ? ky : (t.n - 1 + (-ky - 1))), node);
 }
 
 constexpr int kMaxWalk = 1 << 14;
+
+// A visit of a node's counter: everything this thread (and, after a __syncwarp, its warp) wrote below
+// the node is visible to the visitor that comes second, which sees an odd count.
+__device__ __forceinline__ bool second_visit(uint32_t *flag) {
+  uint32_t before;
+  asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(flag) : "memory");
+  return (before & 1u) != 0u;
+}
 
 // One thread per leaf walks to the root; the second thread to reach a node owns it (its two
 // subtrees are final) and refits it. A pass visits every node twice, so flags[] starts each pass even
@@ -563,55 +469,59 @@ __global__ void __launch_bounds__(128) k_bottom_up(TreeView t, uint32_t *flags, 
   // chain: stop and report.
   for (int guard = 0; node >= 0; ++guard) {
     if (guard >= kMaxWalk) { atomicOr(status, (uint32_t)VT_DEV_TREELET); return; }
-    __threadfence();
-    if ((atomicAdd(&flags[node], 1u) & 1u) == 0u) return;
-    __threadfence();
+    if (!second_visit(&flags[node])) return;
     refit_node(t, node);
-    __threadfence();
     node = __ldcg(t.parent + node);
   }
 }
 
-// The same walk for restructuring. Nodes owned by lanes of one warp in the same step are disjoint
-// subtrees (an owner's subtrees are final), so they may be restructured in any order: when more
-// than kWarpTreelets lanes own a node with >= size leaves, each runs restructure_node on its own;
-// otherwise the whole warp takes them one after another (restructure_warp).
-constexpr int kWarpTreelets = 4;
-__global__ void __launch_bounds__(128) k_restructure(TreeView t, uint32_t *flags, int size, uint32_t *status) {
+// The cost of the tree as the first pass found it, kept beside t.cost: a node's restructuring decision
+// compares against its cost before any restructuring below it.
+__device__ __forceinline__ void refit_first(const TreeView &t, float *firstCost, int i) {
+  const int2 ch = load_child(t, i);
+  const Box b = box_union(child_box(t, ch.x), child_box(t, ch.y));
+  auto first = [&](int c) { return c >= 0 ? __ldcg(firstCost + c) : child_cost(t, c); };
+  const float cost = __fadd_rn(__fmul_rn(kCi, box_area(b.lo, b.hi)), __fadd_rn(first(ch.x), first(ch.y)));
+  store_box(t.nodeBox, i, b);
+  __stcg(t.count + i, child_count(t, ch.x) + child_count(t, ch.y));
+  __stcg(t.cost + i, cost);
+  __stcg(firstCost + i, cost);
+}
+
+// The same walk for restructuring; the first round (firstCost not null) refits each node as it comes
+// to own it, which saves a pass of its own. Nodes owned by lanes of one warp in the same step are
+// disjoint subtrees (an owner's subtrees are final), so the warp takes those with >= size leaves one
+// after another in any order.
+__global__ void __launch_bounds__(128) k_restructure(TreeView t, uint32_t *flags, int size, float *firstCost, uint32_t *status) {
   __shared__ TreeletScratch scratch[4];
+  __shared__ SubsetTable sets;
+  for (uint32_t q = threadIdx.x; q < sizeof(SubsetTable) / 4; q += blockDim.x)
+    reinterpret_cast<uint32_t *>(&sets)[q] = reinterpret_cast<const uint32_t *>(&kSubsets)[q];
+  __syncthreads();
   TreeletScratch &w = scratch[threadIdx.x >> 5];
   const unsigned kAll = 0xffffffffu;
   const int leaf = blockIdx.x * blockDim.x + threadIdx.x;
   int node = leaf < t.n ? __ldcg(t.parent + (t.n - 1 + leaf)) : -1;
-  int guard = 0;
-  while (true) {
+  for (int guard = 0;; ++guard) {
     bool own = false;
     if (node >= 0) {
-      if (guard++ >= kMaxWalk) {
+      if (guard >= kMaxWalk) {
         atomicOr(status, (uint32_t)VT_DEV_TREELET);
         node = -1;
       } else {
-        __threadfence();
-        if ((atomicAdd(&flags[node], 1u) & 1u) == 0u) node = -1;
-        else own = true;
-        __threadfence();
+        own = second_visit(&flags[node]);
+        if (!own) node = -1;
       }
     }
-    const bool mine = own && __ldcg(t.count + node) >= (uint32_t)size;
-    unsigned work = __ballot_sync(kAll, mine);
-    if (__popc(work) > kWarpTreelets) {
-      if (mine) restructure_node(t, node, size, status);
-    } else {
-      while (work) {
-        const int src = __ffs(work) - 1;
-        work &= work - 1;
-        const int root = __shfl_sync(kAll, node, src);
-        restructure_warp(t, root, size, status, w);
-        __syncwarp();
-      }
-    }
+    if (own && firstCost) refit_first(t, firstCost, node);
     __syncwarp();
-    __threadfence();
+    unsigned work = __ballot_sync(kAll, own && __ldcg(t.count + node) >= (uint32_t)size);
+    while (work) {
+      const int src = __ffs(work) - 1;
+      work &= work - 1;
+      restructure_warp(t, __shfl_sync(kAll, node, src), size, status, w, sets);
+      __syncwarp();
+    }
     if (own) node = __ldcg(t.parent + node);
     if (!__any_sync(kAll, node >= 0)) break;
   }
@@ -780,9 +690,10 @@ __device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t *ws) {
 
 // The whole collapse in one cooperative launch. Bound: latency (per level a few dependent loads and two
 // grid barriers); a launch per step with the level's size read back by the host spent 60-100 us a
-// level instead (rebuilding and tracing 20,480 triangles: 4.1 -> 1.6 ms with the sort and the pool). Per level each block takes a contiguous part: it counts its wide nodes' inner
-// children and triangles, and after a barrier prefixes the blocks' sums to place its own nodes,
-// children and triangles in the level order of a serial pass.
+// level instead (rebuilding and tracing 20,480 triangles: 4.1 -> 1.6 ms with the sort and the pool). Per
+// level each block takes a contiguous part: it counts its wide nodes' inner children and triangles, and
+// after a barrier prefixes the blocks' sums to place its own nodes, children and triangles in the level
+// order of a serial pass.
 __global__ void __launch_bounds__(kCollapseBlock) k_collapse(TreeView t, int leafSize, int maxDepth, uint32_t maxNodes, int32_t *levelA,
                                                              int32_t *levelB, int4 *children, uint32_t *packed, uint2 *blockSums,
                                                              uint32_t *bar, vt_wide_node *nodes, const uint32_t *sorted,
@@ -922,7 +833,7 @@ struct BuildScratch {
   float4 *boxes, *leafBox;
   uint32_t *bounds, *codesAlt, *valsAlt, *sortTemp, *flags, *count, *packed, *bar;
   int32_t *parent, *levelA, *levelB;
-  float *cost;
+  float *cost, *firstCost;
   int4 *children;
   uint2 *blockSums;
   BuildReport *report;
@@ -943,6 +854,7 @@ void carve_build(ScratchCarve &c, uint32_t n, BuildScratch &b) {
   b.count = c.take<uint32_t>(ni);
   b.parent = c.take<int32_t>(2 * (size_t)n);
   b.cost = c.take<float>(ni);
+  b.firstCost = c.take<float>(ni);
   b.levelA = c.take<int32_t>(n);
   b.levelB = c.take<int32_t>(n);
   b.children = c.take<int4>(n);
@@ -979,10 +891,11 @@ cudaError_t queue_build(const vt_face *faces, uint32_t n, const vt_vertex *verts
   vt_radix_sort_pairs(o.codes, o.sorted, b.codesAlt, b.valsAlt, n, 30, b.sortTemp, status, s);
   k_hierarchy<<<blocks(n, 256), 256, 0, s>>>(o.codes, b.boxes, o.sorted, (int)n, b.leafBox, o.child, b.parent, b.flags);
   TreeView t{(int)n, o.child, b.parent, b.leafBox, o.nodeBox, b.count, b.cost};
-  if (n >= 2) {
+  if (n >= 3 && treelet > 0) {
+    for (int r = 0; r < rounds; ++r)
+      k_restructure<<<blocks(n, 128), 128, 0, s>>>(t, b.flags, treelet, r == 0 ? b.firstCost : nullptr, status);
+  } else if (n >= 2) {
     k_bottom_up<<<blocks(n, 128), 128, 0, s>>>(t, b.flags, status);
-    if (treelet > 0 && n >= 3)
-      for (int r = 0; r < rounds; ++r) k_restructure<<<blocks(n, 128), 128, 0, s>>>(t, b.flags, treelet, status);
   }
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;

@@ -58,6 +58,16 @@ def test_sort_tiles_and_collapse_blocks(ctx, oracle, n):
         gpu.close()
 
 
+@pytest.mark.parametrize("treelet", [3, 4, 6, 8])
+@pytest.mark.parametrize("n", [7, 33, 129, 4097])
+def test_treelet_sizes(ctx, oracle, n, treelet):
+    """Every split of the warp's lanes among a treelet's subsets, on meshes of small integer coordinates (many
+    boxes of equal area, so ties decide) against the oracle's serial restructuring."""
+    faces, verts = scenes.triangle_soup(n, seed=n, mu=math.log(0.05))
+    verts["p"] = np.round(verts["p"] * 8)
+    compare_builds(vt.Mesh(ctx, faces, verts, treelet_size=treelet), oracle.Bvh.lbvh(faces, verts, treelet_size=treelet))
+
+
 def test_lbvh_duplicate_centroids_and_welded_patch(ctx, oracle):
     # Coincident centroids (equal Morton codes everywhere) and a welded patch.
     faces, verts = scenes.triangle_soup(500, seed=1)
