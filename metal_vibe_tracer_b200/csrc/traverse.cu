@@ -294,7 +294,7 @@ template <typename K> void prepare(K kernel, size_t smem) {
 
 void vt_launch_closest(const vt_mesh *mesh, const vt_ray *rays, uint32_t n, vt_hit *hits, int sm_count,
                        uint32_t *counter, const uint32_t *perm, uint32_t *status, cudaStream_t s,
-                       const uint32_t *count, bool bvhPos) {
+                       const uint32_t *count, bool bvhPos, bool cleared) {
   if (n == 0) return;
   const int S = stack_entries(mesh->depth);
   const size_t smem = (size_t)S * kBlock * sizeof(int);
@@ -302,7 +302,7 @@ void vt_launch_closest(const vt_mesh *mesh, const vt_ray *rays, uint32_t n, vt_h
   prepare(kernel, smem);
   const uint32_t want = (n + kBlock - 1) / kBlock;
   const uint32_t grid = std::min<uint32_t>(want, (uint32_t)(resident_blocks(kernel, smem) * sm_count));
-  cudaMemsetAsync(counter, 0, sizeof(uint32_t), s);
+  if (!cleared) cudaMemsetAsync(counter, 0, sizeof(uint32_t), s);
   kernel<<<grid, kBlock, smem, s>>>(reinterpret_cast<const float4 *>(mesh->d_qnodes), mesh->d_tris, mesh->root_max,
                                     reinterpret_cast<const float4 *>(rays), n, reinterpret_cast<int4 *>(hits), counter,
                                     perm, S, status, count);
@@ -310,7 +310,7 @@ void vt_launch_closest(const vt_mesh *mesh, const vt_ray *rays, uint32_t n, vt_h
 
 void vt_launch_any(const vt_mesh *mesh, const vt_ray *rays, uint32_t n, uint8_t *occ, int sm_count,
                    uint32_t *counter, const uint32_t *perm, uint32_t *status, cudaStream_t s,
-                   const uint32_t *count, bool slack) {
+                   const uint32_t *count, bool slack, bool cleared) {
   if (n == 0) return;
   const int S = stack_entries(mesh->depth);
   const size_t smem = (size_t)S * kBlock * sizeof(int);
@@ -318,7 +318,7 @@ void vt_launch_any(const vt_mesh *mesh, const vt_ray *rays, uint32_t n, uint8_t 
   prepare(kernel, smem);
   const uint32_t want = (n + kBlock - 1) / kBlock;
   const uint32_t grid = std::min<uint32_t>(want, (uint32_t)(resident_blocks(kernel, smem) * sm_count));
-  cudaMemsetAsync(counter, 0, sizeof(uint32_t), s);
+  if (!cleared) cudaMemsetAsync(counter, 0, sizeof(uint32_t), s);
   kernel<<<grid, kBlock, smem, s>>>(reinterpret_cast<const float4 *>(mesh->d_qnodes), mesh->d_tris, mesh->root_max,
                                     reinterpret_cast<const float4 *>(rays), n, occ, counter, perm, S, status, count);
 }

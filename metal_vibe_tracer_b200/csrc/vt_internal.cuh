@@ -220,7 +220,7 @@ vt_status vt_lbvh_build(vt_ctx *ctx, const vt_face *faces, uint32_t nfaces, cons
 
 // Traversal launches (traverse.cu).
 // Persistent kernels; `counter` is one device word of scratch (the ray queue head), reset by the
-// launch on stream s.
+// launch on stream s unless the caller has cleared it (`cleared`).
 // `status` receives VT_DEV_STACK if a traversal stack would overflow (it cannot for a tree within
 // the mesh's recorded depth; the check keeps a corrupted tree from writing out of bounds).
 // `count` (optional): the queue length on the device, at most n (the wavefront integrator's queues);
@@ -228,9 +228,9 @@ vt_status vt_lbvh_build(vt_ctx *ctx, const vt_face *faces, uint32_t nfaces, cons
 // triangle's rounding bound early (imported scenes).
 void vt_launch_closest(const vt_mesh *mesh, const vt_ray *rays, uint32_t n, vt_hit *hits,
                        int sm_count, uint32_t *counter, const uint32_t *perm, uint32_t *status,
-                       cudaStream_t s, const uint32_t *count = nullptr, bool bvhPos = false);
+                       cudaStream_t s, const uint32_t *count = nullptr, bool bvhPos = false, bool cleared = false);
 void vt_launch_any(const vt_mesh *mesh, const vt_ray *rays, uint32_t n, uint8_t *occ,
                    int sm_count, uint32_t *counter, const uint32_t *perm, uint32_t *status,
-                   cudaStream_t s, const uint32_t *count = nullptr, bool slack = false);
+                   cudaStream_t s, const uint32_t *count = nullptr, bool slack = false, bool cleared = false);
 void vt_launch_count(const vt_mesh *mesh, const vt_ray *rays, uint32_t n, int closest,
                      unsigned long long *acc /* 2 device words */, cudaStream_t s);

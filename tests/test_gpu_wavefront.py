@@ -90,6 +90,20 @@ def test_layered_openpbr_equals_megakernel(ctx, spectral):
     assert np.all(np.abs(wave.mean((0, 1)) / mega.mean((0, 1)) - 1) < 2e-3)
 
 
+def test_long_paths_equal_megakernel(ctx):
+    """Paths far longer than the stages' 64 slots of counters: a closed box of albedo 0.98 walls."""
+    faces, verts, mats, cam = scenes.cornell_emitters()
+    pts = verts["p"][np.stack([faces["a"], faces["b"], faces["c"]], 1)]
+    front = [((-1, -1, -1), (1, -1, -1), (1, 1, -1)), ((-1, -1, -1), (1, 1, -1), (-1, 1, -1))]
+    faces, verts = scenes._mesh_from_triangles(list(pts) + front, list(faces["tag"]) + [0, 0])
+    mats = [dict(m, albedo=(0.98,) * 3) if m["type"] == 0 else m for m in mats]
+    cam = dict(cam, pos=(0.3, 0.2, -0.9), target=(0.0, -0.1, 0.3))
+    mesh = vt.Mesh(ctx, faces, verts)
+    mega, wave = both(ctx, mesh, mats, None, vt.make_params(cam, 40, 24, 150, 1, False, 1), 4, False)
+    mesh.close()
+    assert_same(mega, wave)
+
+
 def test_passes_and_stride(ctx, cornell):
     mats, light, cam, mesh = cornell
     # 1024 x 1024 x 8 spp = 8M paths: two passes of 4M.
