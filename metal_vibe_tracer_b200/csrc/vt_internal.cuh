@@ -102,6 +102,7 @@ struct vt_scene {
   float env_rot = 0.0f;
   bool env_map = false;
   uint32_t *d_emitters = nullptr;
+  float4 *d_lt_pairs = nullptr;  // the light tree's inner nodes with their children decoded
   std::vector<uint32_t> emitter_words;
   float4 *d_emissions = nullptr;
   int32_t *d_face_pos = nullptr;

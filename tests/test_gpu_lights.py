@@ -101,6 +101,21 @@ def test_lamp_uses_power_sampling_and_eight_lights_a_tree(ctx):
     assert all(r["zero"] == 0 and r["error"] < 1e-3 for r in res)
 
 
+@pytest.mark.parametrize("count", [9, 33, 300])
+def test_tree_of_any_size_samples_by_its_pdf(ctx, count):
+    """Trees of uneven shape, leaves beside inner nodes: the sampling walk and the pdf walk agree (1e-3,
+    as above), and the estimate is the quadrature's."""
+    faces, verts, mats = scenes.ceiling_lights()
+    faces = faces[:count]
+    res, words = estimates(ctx, faces, verts, mats, True)
+    assert words[2 * count + 2] > 1
+    n = PER_POINT * SAMPLES
+    for k, p in enumerate(POINTS):
+        r, exact = res[k], quadrature(faces, verts, mats, p)
+        assert r["zero"] == 0 and r["error"] < 1e-3, (k, r)
+        assert abs(r["mean"] - exact) <= 5 * np.sqrt(r["var"] / n) + 1e-3 * exact, (k, r["mean"], exact)
+
+
 def relmse(a, b):
     return float(np.mean((a - b) ** 2 / (b ** 2 + 1e-2)))
 
