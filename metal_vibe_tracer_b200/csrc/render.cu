@@ -1638,7 +1638,9 @@ struct WfArgs {
   const uint32_t *inQ, *inCount;  // live paths of this bounce (null: paths 0 .. paths - 1)
   uint32_t *outQ, *outCount;      // live paths of the next bounce
   uint32_t *shQ, *shCount;        // shadow rays of this bounce
-  uint32_t *grpQ;                 // the live queue regrouped by material (k_wf_group)
+  uint32_t *grpQ;                 // the live queue regrouped by kind of vertex (k_wf_group): kWfClasses
+  uint32_t grpStride;             // queues of grpStride entries
+  const uint32_t *groups;         // their counts; null: the bounce is not regrouped
   uint32_t npix, paths, k0;       // accumulation pixels; paths of the pass; its first sample (of the call)
   uint32_t p0;                    // the pass's first pixel (sampling mode 0: a band of one frame; else 0)
   // Sampling mode 0: the GI reservoir's connection from the primary vertex.
@@ -1686,45 +1688,55 @@ __device__ __forceinline__ void wf_push(bool push, uint32_t v, uint32_t *q, uint
   __syncthreads();  // sTotal and sBase are reused by the next push
 }
 
-// wf_push from the back: the block's entries go to n - 1 - (reserved rank) of queue q.
-__device__ __forceinline__ void wf_push_back(bool push, uint32_t v, uint32_t *q, uint32_t *count, uint32_t n, uint32_t &sTotal,
-                                             uint32_t &sBase) {
-  const unsigned lane = threadIdx.x & 31u;
-  const unsigned m = __ballot_sync(0xffffffffu, push);
-  if (threadIdx.x == 0) sTotal = 0;
-  __syncthreads();
-  uint32_t w = 0;
-  if (lane == 0 && m) w = atomicAdd(&sTotal, (uint32_t)__popc(m));
-  w = __shfl_sync(0xffffffffu, w, 0);
-  __syncthreads();
-  if (threadIdx.x == 0) sBase = sTotal ? atomicAdd(count, sTotal) : 0u;
-  __syncthreads();
-  if (push) q[n - 1u - (sBase + w + (uint32_t)__popc(m & ((1u << lane) - 1u)))] = v;
-  __syncthreads();
-}
-
-// Shading grouped by material: the live queue of a bounce regrouped so that paths whose hit has a
-// thin film (the costly iridescence evaluations of spectral transport) come after all others. With
-// a tenth of the slots filmed nearly every 32-path warp holds a film vertex; grouped, the shade
-// kernel's warps run one kind of vertex. Others fill W.grpQ from the front, film paths from the
-// back; counts[0] and counts[1] must be zero on entry.
+// Shading grouped by kind of vertex: the live queue of a bounce split into one queue per class of the hit,
+// which k_wf_shade takes one after another in whole warps. In open scenes most rays of the first
+// bounces escape, and slots mix films (the costly iridescence evaluations of spectral transport), pure
+// metals, dielectrics and emitters: ungrouped, 9 of 32 lanes ran on average at bounce 1 of the
+// production scene. Measured on one B200 (the pass itself 7-31 us a bounce of 4M paths): a 1080p
+// production frame of 4 samples 26.9 -> 18.9 ms of device time, 960 x 540 in RGB 6.74 -> 5.13, a 1000 x 600
+// Lambert frame 5.48 -> 4.66. A path that escapes a scene without an environment ends here: its pending shadow
+// result, if any, is added by k_wf_finish. counts[0 .. kWfClasses) must be zero on entry.
+constexpr uint32_t kWfClasses = 5;  // Lambert and ideal; OpenPBR with a dielectric part; pure metal; film;
+                                    // emitters and escapes into the environment
+template <bool kPbr>
 __global__ void __launch_bounds__(kWfBlock) k_wf_group(RenderArgs A, WfArgs W, uint32_t *counts) {
-  __shared__ uint32_t sTotal, sBase;
+  __shared__ uint32_t sCount[kWfClasses], sBase[kWfClasses];
+  const unsigned lane = threadIdx.x & 31u;
   const uint32_t n = W.inCount ? min(*W.inCount, W.paths) : W.paths;
   for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
     const uint32_t q = base + threadIdx.x;
-    uint32_t i = 0;
-    bool film = false;
+    uint32_t i = 0, cls = kWfClasses, rank = 0;
     if (q < n) {
       i = W.inQ ? W.inQ[q] : q;
       const int pos = W.hit[i].w;
-      if (pos >= 0 && (uint32_t)pos < A.faceCount && !(W.deadFlags && (W.meta[i].w & kWfDead))) {
-        const uint32_t slot = __float_as_uint(__ldg(A.tris + 3 * (size_t)pos + 1).w);
-        film = slot < A.nmat && pbr_thin_film_slot(A, material(A, slot));
+      if (W.deadFlags && (W.meta[i].w & kWfDead)) {
+        // Ended on an uncompacted bounce.
+      } else if (pos < 0) {
+        if (A.env) cls = kWfClasses - 1u;
+      } else {
+        cls = 0u;
+        if ((uint32_t)pos < A.faceCount) {
+          const vt_material m = material(A, __float_as_uint(__ldg(A.tris + 3 * (size_t)pos + 1).w));
+          if (m.type == VT_MAT_EMISSIVE) cls = kWfClasses - 1u;
+          else if (is_pbr<kPbr>(A, m)) cls = pbr_thin_film_slot(A, m) ? 3u : (m.type == VT_MAT_GLOSSY || slot_lobe(A, m).y >= 1.0f ? 2u : 1u);
+        }
       }
     }
-    wf_push(q < n && !film, i, W.grpQ, counts, sTotal, sBase);
-    wf_push_back(q < n && film, i, W.grpQ, counts + 1, n, sTotal, sBase);
+    if (threadIdx.x < kWfClasses) sCount[threadIdx.x] = 0;
+    __syncthreads();
+#pragma unroll
+    for (uint32_t c = 0; c < kWfClasses; ++c) {
+      const unsigned m = __ballot_sync(0xffffffffu, cls == c);
+      uint32_t w = 0;
+      if (lane == 0 && m) w = atomicAdd(&sCount[c], (uint32_t)__popc(m));
+      w = __shfl_sync(0xffffffffu, w, 0);
+      if (cls == c) rank = w + (uint32_t)__popc(m & ((1u << lane) - 1u));
+    }
+    __syncthreads();
+    if (threadIdx.x < kWfClasses) sBase[threadIdx.x] = sCount[threadIdx.x] ? atomicAdd(counts + threadIdx.x, sCount[threadIdx.x]) : 0u;
+    __syncthreads();
+    if (cls < kWfClasses) W.grpQ[cls * W.grpStride + sBase[cls] + rank] = i;
+    __syncthreads();
   }
 }
 
@@ -1955,21 +1967,45 @@ __global__ void __launch_bounds__(kWfBlock) k_wf_generate(RenderArgs A, WfArgs W
 template <bool kPbr, bool kNrc>
 __global__ void __launch_bounds__(kWfBlock, 2) k_wf_shade(RenderArgs A, WfArgs W, uint32_t bounce) {
   __shared__ uint32_t sTotal, sBase;
-  const uint32_t n = W.inCount ? min(*W.inCount, W.paths) : W.paths;
+  // Entries of a regrouped queue: the classes one after another, each from a whole warp on.
+  uint32_t n = 0, classes[kWfClasses];
+  if (W.groups) {
+#pragma unroll
+    for (uint32_t c = 0; c < kWfClasses; ++c) {
+      classes[c] = min(W.groups[c], W.paths);
+      n += (classes[c] + 31u) & ~31u;
+    }
+  } else {
+    n = W.inCount ? min(*W.inCount, W.paths) : W.paths;
+  }
   for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
     const uint32_t q = base + threadIdx.x;
-    bool next = false, shadow = false;
+    bool next = false, shadow = false, entry = q < n;
     uint32_t i = 0;
-    if (q < n) {
-      i = W.inQ ? W.inQ[q] : q;
-      const bool dead = W.deadFlags && (W.meta[i].w & kWfDead);
-      if (!dead) {
-        wf_vertex<kPbr, kNrc>(A, W, i, bounce, next, shadow);
-        // A path that ends on a bounce without compaction stays queued: flagged, with an empty ray.
-        if (!next && !W.compact) {
-          W.meta[i].w |= kWfDead;
-          reinterpret_cast<float *>(W.ray + 2 * (size_t)i + 1)[3] = -1.0f;
+    if (W.groups) {
+      uint32_t r = q;
+      bool found = false;
+      entry = false;
+#pragma unroll
+      for (uint32_t c = 0; c < kWfClasses; ++c) {
+        const uint32_t padded = (classes[c] + 31u) & ~31u;
+        if (!found && r < padded) {
+          found = true;
+          entry = r < classes[c];
+          if (entry) i = W.grpQ[c * W.grpStride + r];
         }
+        if (!found) r -= padded;
+      }
+    } else if (entry) {
+      i = W.inQ ? W.inQ[q] : q;
+      entry = !(W.deadFlags && (W.meta[i].w & kWfDead));
+    }
+    if (entry) {
+      wf_vertex<kPbr, kNrc>(A, W, i, bounce, next, shadow);
+      // A path that ends on a bounce without compaction stays queued: flagged, with an empty ray.
+      if (!next && !W.compact) {
+        W.meta[i].w |= kWfDead;
+        reinterpret_cast<float *>(W.ray + 2 * (size_t)i + 1)[3] = -1.0f;
       }
     }
     if (W.compact) {
@@ -3253,9 +3289,9 @@ constexpr uint32_t kWfMaxPaths = 1u << 22;
 // a pass (and one per kWfSlots - 2 bounces beyond) clears them all instead of four or five a bounce, whose
 // gaps counted where a bounce takes some tens of microseconds. Measured on one B200: the spectral
 // Cornell box at 256 x 256, 16 spp, depth 8: 1.23 -> 1.18 ms; four 1080p production samples 28.51 -> 28.36.
-constexpr uint32_t kWfSlots = 64, kWfWords = 8;
-enum : uint32_t { kWfLive = 0, kWfShadows = 1, kWfGroup = 2 /* two words */, kWfExtendHead = 4, kWfShadowHead = 5,
-                  kWfConnections = 6, kWfConnectHead = 7 };
+constexpr uint32_t kWfSlots = 64, kWfWords = 12;
+enum : uint32_t { kWfLive = 0, kWfShadows = 1, kWfExtendHead = 2, kWfShadowHead = 3, kWfConnections = 4, kWfConnectHead = 5,
+                  kWfGroup = 6 /* kWfClasses words */ };
 
 // The wavefront state's buffers that the host hands to the stages: the two live queues, the counters,
 // hits and occlusion.
@@ -3291,7 +3327,8 @@ size_t wf_carve(unsigned char *base, uint32_t cap, WfArgs &W, WfBuffers &B) {
   B.q[0] = reinterpret_cast<uint32_t *>(take(4 * n));
   B.q[1] = reinterpret_cast<uint32_t *>(take(4 * n));
   W.shQ = reinterpret_cast<uint32_t *>(take(4 * n));
-  W.grpQ = reinterpret_cast<uint32_t *>(take(4 * n));
+  W.grpQ = reinterpret_cast<uint32_t *>(take(4 * kWfClasses * n));
+  W.grpStride = cap;
   B.counts = reinterpret_cast<uint32_t *>(take(kWfSlots * kWfWords * sizeof(uint32_t)));
   W.hit = B.hit;
   W.occ = B.occ;
@@ -3341,7 +3378,10 @@ WfStages wf_stages(vt_ctx *ctx, const vt_scene *scene, const RenderArgs &A, cons
   S.every = every;
   S.pbr = A.layered != 0u;
   S.unbounded = scene_has_delta(scene);
-  S.group = S.pbr && A.spectral && scene->has_film;
+  // Regrouping pays where hits differ in kind: scenes with OpenPBR slots, and open scenes (imported ones
+  // may be), where rays escape. The procedural boxes' Lambert walls shade alike, and a pass over the queue
+  // would only add its time (k_wf_group; ReSTIR frames of a Lambert scene gain least, 17.0 -> 16.7 ms).
+    S.group = S.pbr || A.imported;
   S.nrc = nrc;
   S.s = s;
   return S;
@@ -3367,7 +3407,8 @@ vt_status wf_bounces(const WfStages &S, const RenderArgs &A, WfArgs W, uint32_t 
         if (live == 0u) break;
       }
     }
-    W.compact = ((b + 1u) % S.every == 0u || b >= A.maxDepth) ? 1u : 0u;
+    // A regrouped bounce has dropped the paths that ended, so its own queue is compacted anyway.
+    W.compact = (S.group || (b + 1u) % S.every == 0u || b >= A.maxDepth) ? 1u : 0u;
     // Live queue of bounce b (all paths at b = 0), the next bounce's queue and the shadow queue.
     W.inQ = b == 0 ? nullptr : S.B.q[b & 1u];
     W.inCount = b == 0 ? nullptr : S.word(b, kWfLive);
@@ -3383,8 +3424,9 @@ vt_status wf_bounces(const WfStages &S, const RenderArgs &A, WfArgs W, uint32_t 
     vt_launch_closest(S.mesh, reinterpret_cast<const vt_ray *>(W.ray), P, reinterpret_cast<vt_hit *>(S.B.hit), ctx->sm_count,
                       S.word(b, kWfExtendHead), W.inQ, ctx->d_status + 1, s, W.inCount, true, true);
     if (S.group) {
-      k_wf_group<<<grid, S.block, 0, s>>>(A, W, S.word(b, kWfGroup));
-      W.inQ = W.grpQ;  // the same entries, regrouped (the count stays)
+      if (S.pbr) k_wf_group<true><<<grid, S.block, 0, s>>>(A, W, S.word(b, kWfGroup));
+      else k_wf_group<false><<<grid, S.block, 0, s>>>(A, W, S.word(b, kWfGroup));
+      W.groups = S.word(b, kWfGroup);
     }
     if (S.nrc) {
       if (S.pbr) k_wf_shade<true, true><<<grid, S.block, 0, s>>>(A, W, b);

@@ -104,6 +104,26 @@ def test_long_paths_equal_megakernel(ctx):
     assert_same(mega, wave)
 
 
+@pytest.mark.parametrize("spectral", [False, True])
+def test_open_scene_of_every_class_equals_megakernel(ctx, spectral):
+    """An open scene without an environment (escaped paths are dropped, their last light sample still
+    counts) whose slots cover every class the stages regroup by: Lambert, dielectric, metal, film,
+    emitter. (Tolerance as for the layered slots.)"""
+    faces, verts, mats, cam = scenes.sky_scene(emitter=True, subdivisions=3)
+    pbr = dict(type=4, albedo=(0.7, 0.4, 0.3), emission=(0.0, 0.0, 0.0))
+    first = len(mats)
+    mats = mats + [dict(pbr, roughness=0.3), dict(pbr, roughness=0.4, metalness=1.0),
+                   dict(pbr, roughness=0.35, thin_film_weight=1.0, thin_film_thickness=0.4, thin_film_ior=1.4)]
+    sphere = np.flatnonzero(faces["tag"] == 1)
+    faces["tag"][sphere[sphere % 4 > 0]] = first - 1 + (sphere % 4)[sphere % 4 > 0]
+    mesh = vt.Mesh(ctx, faces, verts)
+    mega, wave = both(ctx, mesh, mats, None, vt.make_params(cam, 96, 64, 6, 1, spectral, 1), 8, spectral)
+    mesh.close()
+    same = np.all(np.abs(wave - mega) <= 1e-4 * np.maximum(np.abs(mega), 1e-3), axis=-1)
+    assert same.mean() >= 0.98, same.mean()
+    assert np.all(np.abs(wave.mean((0, 1)) / mega.mean((0, 1)) - 1) < 2e-3)
+
+
 def test_passes_and_stride(ctx, cornell):
     mats, light, cam, mesh = cornell
     # 1024 x 1024 x 8 spp = 8M paths: two passes of 4M.
