@@ -42,12 +42,39 @@ using namespace vtd;
 // 110 -> 93 us. Tried and dropped: entry distances on the stack to drop entries beyond a closer hit
 // unvisited (5.76 against 5.20 ms: the larger stacks cost more L1 than the visits saved), loading the
 // next node before pushing the others (5.11 against 4.26 ms).
+//
+// Few rays (lanes_used) go one or two to a warp: a ray then waits for no others' node and leaf phases, and the
+// chip has room. Measured on one B200 (the whole call): 4,096 rays on 20,000 triangles, closest hit
+// 90 -> 79 us and any hit 72 -> 58; 1,000 rays on 1M triangles 237 -> 184 and 167 -> 111. Spread further it
+// loses: 20,000 rays on 16 warps an SM 99 -> 112 us, on 8 108, on 4 107.
 constexpr unsigned kFull = 0xffffffffu;
 // Refill once this many lanes are idle (measured at 4, 8, 12 and 16).
 constexpr int kRefill = 4, kRefillAny = 8;
 constexpr int kSteps = 4, kStepsAny = 2;  // nodes per lane between votes
 constexpr int kBlock = 128;
 constexpr int kMinBlocks = 8, kMinBlocksAny = 9;  // register budget: 65536 / (kBlock * blocks)
+
+// The rays of a launch and where the results go: perm (null: all rays in order) lists the rays, count (when
+// not null) holds the list's length on the device (at most n), counter the next to hand out.
+template <typename Out>
+struct RaySet {
+  const float4 *rays;
+  uint32_t n;
+  Out *out;
+  uint32_t *counter;
+  const uint32_t *perm, *count;
+  uint32_t sms;
+};
+
+// Lanes of each warp that take rays (kFew: a launch of possibly few rays): one or two while that gives every
+// ray of the launch a place in kFewWarps warps an SM, else all.
+constexpr uint32_t kFewWarps = 16, kFewLanes = 2;
+template <bool kFew>
+__device__ __forceinline__ unsigned lanes_used(uint32_t n, uint32_t sms) {
+  if (!kFew) return kFull;
+  const uint32_t warps = min(gridDim.x * (kBlock / 32u), sms * kFewWarps), lanes = (n + warps - 1u) / warps;
+  return lanes > kFewLanes ? kFull : (1u << lanes) - 1u;
+}
 
 struct RayState {
   WRay wr;
@@ -90,16 +117,12 @@ constexpr int kIdle = 0x7fffffff;
 // need this iteration; the others wait one iteration. A ray's own order (LIFO over its stack) does
 // not depend on the warp.
 // kPos: a hit reports the triangle's BVH position instead of its input face (the integrator's
-// hit record). count: when not null, the queue length on the device (at most n).
-template <bool kPos>
-__global__ void __launch_bounds__(kBlock, kMinBlocks) k_closest(const float4 *__restrict__ nodes,
-                                                        const float4 *__restrict__ tris, float rootMax,
-                                                        const float4 *__restrict__ rays, uint32_t n,
-                                                        int4 *__restrict__ hits, uint32_t *counter,
-                                                        const uint32_t *__restrict__ perm, int stackSize,
-                                                        uint32_t *status, const uint32_t *__restrict__ count) {
-  extern __shared__ int sstack[];
-  if (count) n = min(n, *count);
+// hit record).
+template <bool kPos, bool kFew>
+__device__ __forceinline__ void closest_rays(const float4 *__restrict__ nodes, const float4 *__restrict__ tris, float rootMax,
+                                             const RaySet<int4> &R, int stackSize, uint32_t *status, int *sstack) {
+  const uint32_t n = R.count ? min(R.n, *R.count) : R.n;
+  const unsigned mine = lanes_used<kFew>(n, R.sms);  // of this warp
   int cur = kIdle, top = 0;
   uint32_t rid = 0;
   RayState s;
@@ -107,12 +130,12 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) k_closest(const float4 *__
   int prim = -1;
   bool exhausted = false;  // warp-uniform
   while (true) {
-    const unsigned idle = __ballot_sync(kFull, cur == kIdle);
-    if (!exhausted && __popc(idle) >= kRefill) {
-      const uint32_t r = refill(idle, counter, n, exhausted);
+    const unsigned idle = __ballot_sync(kFull, cur == kIdle) & mine;
+    if (!exhausted && (__popc(idle) >= kRefill || (kFew && idle == mine))) {
+      const uint32_t r = refill(idle, R.counter, n, exhausted);
       if (r < n) {
-        rid = perm ? __ldcs(perm + r) : r;
-        load_ray(rays, rid, s, rootMax);
+        rid = R.perm ? __ldcs(R.perm + r) : r;
+        load_ray(R.rays, rid, s, rootMax);
         s.tMin = __fadd_rn(s.tMin, 0.0f);  // -0 to +0 (sort_qchildren)
         closest = s.tMax;
         prim = -1;
@@ -169,33 +192,29 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) k_closest(const float4 *__
     if (cur == kIdle) {
       const int4 out = prim >= 0 ? make_int4(__float_as_int(closest), __float_as_int(hb1), __float_as_int(hb2), prim)
                                  : make_int4(0, 0, 0, -1);
-      __stcs(hits + rid, out);
+      __stcs(R.out + rid, out);
     }
   }
 }
 
 // kSlack: each triangle's own rounding bound comes off tmax (the integrator's shadow rays in
-// imported scenes, scene_occluded main.swift:2066-2069). count: as k_closest's.
-template <bool kSlack>
-__global__ void __launch_bounds__(kBlock, kMinBlocksAny) k_any(const float4 *__restrict__ nodes,
-                                                    const float4 *__restrict__ tris, float rootMax,
-                                                    const float4 *__restrict__ rays, uint32_t n,
-                                                    uint8_t *__restrict__ occ, uint32_t *counter,
-                                                    const uint32_t *__restrict__ perm, int stackSize,
-                                                    uint32_t *status, const uint32_t *__restrict__ count) {
-  extern __shared__ int sstack[];
-  if (count) n = min(n, *count);
+// imported scenes, scene_occluded main.swift:2066-2069).
+template <bool kSlack, bool kFew>
+__device__ __forceinline__ void any_rays(const float4 *__restrict__ nodes, const float4 *__restrict__ tris, float rootMax,
+                                         const RaySet<uint8_t> &R, int stackSize, uint32_t *status, int *sstack) {
+  const uint32_t n = R.count ? min(R.n, *R.count) : R.n;
+  const unsigned mine = lanes_used<kFew>(n, R.sms);  // of this warp
   int cur = kIdle, top = 0;
   uint32_t rid = 0;
   RayState s;
   bool exhausted = false;
   while (true) {
-    const unsigned idle = __ballot_sync(kFull, cur == kIdle);
-    if (!exhausted && __popc(idle) >= kRefillAny) {
-      const uint32_t r = refill(idle, counter, n, exhausted);
+    const unsigned idle = __ballot_sync(kFull, cur == kIdle) & mine;
+    if (!exhausted && (__popc(idle) >= kRefillAny || (kFew && idle == mine))) {
+      const uint32_t r = refill(idle, R.counter, n, exhausted);
       if (r < n) {
-        rid = perm ? __ldcs(perm + r) : r;
-        load_ray(rays, rid, s, rootMax);
+        rid = R.perm ? __ldcs(R.perm + r) : r;
+        load_ray(R.rays, rid, s, rootMax);
         cur = 0;
         top = 0;
       }
@@ -244,8 +263,21 @@ __global__ void __launch_bounds__(kBlock, kMinBlocksAny) k_any(const float4 *__r
         if (cur < 0 || cur == kIdle) break;
       }
     }
-    if (cur == kIdle) occ[rid] = hit ? 1 : 0;
+    if (cur == kIdle) R.out[rid] = hit ? 1 : 0;
   }
+}
+
+template <bool kPos, bool kFew>
+__global__ void __launch_bounds__(kBlock, kMinBlocks) k_closest(const float4 *__restrict__ nodes, const float4 *__restrict__ tris,
+                                                                float rootMax, const __grid_constant__ RaySet<int4> R, int stackSize, uint32_t *status) {
+  extern __shared__ int sstack[];
+  closest_rays<kPos, kFew>(nodes, tris, rootMax, R, stackSize, status, sstack);
+}
+template <bool kSlack, bool kFew>
+__global__ void __launch_bounds__(kBlock, kMinBlocksAny) k_any(const float4 *__restrict__ nodes, const float4 *__restrict__ tris,
+                                                               float rootMax, const __grid_constant__ RaySet<uint8_t> R, int stackSize, uint32_t *status) {
+  extern __shared__ int sstack[];
+  any_rays<kSlack, kFew>(nodes, tris, rootMax, R, stackSize, status, sstack);
 }
 
 __global__ void __launch_bounds__(128) k_count(const float4 *__restrict__ nodes,
@@ -280,15 +312,21 @@ namespace {
 // pushes at most three.
 inline int stack_entries(uint32_t depth) { return 3 * (int)depth; }
 
-// Resident blocks per SM for a persistent kernel with `smem` bytes of dynamic shared memory.
-template <typename K> int resident_blocks(K kernel, size_t smem) {
-  int b = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, kBlock, smem) != cudaSuccess || b < 1) b = 1;
-  return b;
-}
-
-template <typename K> void prepare(K kernel, size_t smem) {
+// Launches a persistent traversal of n rays: at most a warp per ray, as many blocks as fit the chip, `smem`
+// bytes of stacks in each.
+template <typename K, typename... Args>
+void launch_persistent(K kernel, const vt_mesh *mesh, uint64_t n, int sm_count, cudaStream_t s, uint32_t *status, Args... rays) {
+  const int S = stack_entries(mesh->depth);
+  const size_t smem = (size_t)S * kBlock * sizeof(int);
   if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  int resident = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, kBlock, smem) != cudaSuccess || resident < 1) resident = 1;
+  const uint32_t grid = (uint32_t)std::min<uint64_t>((n + kBlock / 32 - 1) / (kBlock / 32), (uint64_t)resident * sm_count);
+  kernel<<<grid, kBlock, smem, s>>>(reinterpret_cast<const float4 *>(mesh->d_qnodes), mesh->d_tris, mesh->root_max, rays..., S, status);
+}
+template <typename Out, typename T>
+RaySet<Out> ray_set(const vt_ray *rays, uint32_t n, T *out, uint32_t *counter, const uint32_t *perm, const uint32_t *count, int sm_count) {
+  return {reinterpret_cast<const float4 *>(rays), n, reinterpret_cast<Out *>(out), counter, perm, count, (uint32_t)sm_count};
 }
 }  // namespace
 
@@ -296,31 +334,20 @@ void vt_launch_closest(const vt_mesh *mesh, const vt_ray *rays, uint32_t n, vt_h
                        uint32_t *counter, const uint32_t *perm, uint32_t *status, cudaStream_t s,
                        const uint32_t *count, bool bvhPos, bool cleared) {
   if (n == 0) return;
-  const int S = stack_entries(mesh->depth);
-  const size_t smem = (size_t)S * kBlock * sizeof(int);
-  auto kernel = bvhPos ? k_closest<true> : k_closest<false>;
-  prepare(kernel, smem);
-  const uint32_t want = (n + kBlock - 1) / kBlock;
-  const uint32_t grid = std::min<uint32_t>(want, (uint32_t)(resident_blocks(kernel, smem) * sm_count));
   if (!cleared) cudaMemsetAsync(counter, 0, sizeof(uint32_t), s);
-  kernel<<<grid, kBlock, smem, s>>>(reinterpret_cast<const float4 *>(mesh->d_qnodes), mesh->d_tris, mesh->root_max,
-                                    reinterpret_cast<const float4 *>(rays), n, reinterpret_cast<int4 *>(hits), counter,
-                                    perm, S, status, count);
+  const bool few = count || n <= kFewLanes * kFewWarps * (uint32_t)sm_count;
+  launch_persistent(bvhPos ? (few ? k_closest<true, true> : k_closest<true, false>) : few ? k_closest<false, true> : k_closest<false, false>, mesh, n, sm_count, s, status,
+                    ray_set<int4>(rays, n, hits, counter, perm, count, sm_count));
 }
 
 void vt_launch_any(const vt_mesh *mesh, const vt_ray *rays, uint32_t n, uint8_t *occ, int sm_count,
                    uint32_t *counter, const uint32_t *perm, uint32_t *status, cudaStream_t s,
                    const uint32_t *count, bool slack, bool cleared) {
   if (n == 0) return;
-  const int S = stack_entries(mesh->depth);
-  const size_t smem = (size_t)S * kBlock * sizeof(int);
-  auto kernel = slack ? k_any<true> : k_any<false>;
-  prepare(kernel, smem);
-  const uint32_t want = (n + kBlock - 1) / kBlock;
-  const uint32_t grid = std::min<uint32_t>(want, (uint32_t)(resident_blocks(kernel, smem) * sm_count));
   if (!cleared) cudaMemsetAsync(counter, 0, sizeof(uint32_t), s);
-  kernel<<<grid, kBlock, smem, s>>>(reinterpret_cast<const float4 *>(mesh->d_qnodes), mesh->d_tris, mesh->root_max,
-                                    reinterpret_cast<const float4 *>(rays), n, occ, counter, perm, S, status, count);
+  const bool few = count || n <= kFewLanes * kFewWarps * (uint32_t)sm_count;
+  launch_persistent(slack ? (few ? k_any<true, true> : k_any<true, false>) : few ? k_any<false, true> : k_any<false, false>, mesh, n, sm_count, s, status,
+                    ray_set<uint8_t>(rays, n, occ, counter, perm, count, sm_count));
 }
 
 void vt_launch_count(const vt_mesh *mesh, const vt_ray *rays, uint32_t n, int closest,

@@ -179,3 +179,14 @@ def test_small_meshes_and_ray_counts(ctx, oracle, faces_n, leaf):
         short = scenes.shadow_tmax_np(rays, False, seed=n)
         assert np.array_equal(gpu_any(mesh, short), ref.occluded(short))
     mesh.close()
+
+
+@pytest.mark.parametrize("n", [1, 31, 1183, 1185, 4097, 37_000, 38_000, 150_000, 190_000])
+def test_few_rays_equal_a_large_batch(ctx, n):
+    """Counts around the lines between one, a few and all lanes of a warp: the first n rays of a large batch,
+    bit for bit."""
+    faces, verts = scenes.triangle_soup(5000, seed=1, mu=math.log(0.03))
+    mesh = vt.Mesh(ctx, faces, verts)
+    rays = scenes.incoherent_rays_np(300_000, seed=3)
+    assert_bit_exact(gpu_closest(mesh, rays[:n]), gpu_closest(mesh, rays)[:n])
+    assert np.array_equal(gpu_any(mesh, rays[:n]), gpu_any(mesh, rays)[:n])
