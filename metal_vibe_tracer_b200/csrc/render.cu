@@ -3388,13 +3388,20 @@ WfStages wf_stages(vt_ctx *ctx, const vt_scene *scene, const RenderArgs &A, cons
 }
 
 // The bounces of the paths of W from bounce `first` on (0: every path, its ray just generated; else the
-// live queue q[first & 1]), then their radiance into the accumulation. The pass's counters are clear but
-// for what its earlier stages counted.
+// live queue q[first & 1], and the shadow rays queued as bounce first - 1's), then their radiance into the
+// accumulation. The pass's counters are clear but for what its earlier stages counted.
 vt_status wf_bounces(const WfStages &S, const RenderArgs &A, WfArgs W, uint32_t first) {
   vt_ctx *ctx = S.ctx;
   cudaStream_t s = S.s;
   const uint32_t P = W.paths, grid = S.grid(P);
-  for (uint32_t b = first;; ++b) {
+  vt_hit *hits = reinterpret_cast<vt_hit *>(S.B.hit);
+  // The shadow rays queued at bounce b - 1, traced with bounce b's rays (or alone after the last bounce):
+  // their results are read when bounce b is shaded.
+  const auto shadows = [&](uint32_t b) {
+    return vt_ray_queue{reinterpret_cast<const vt_ray *>(W.sray), W.shQ, S.word(b - 1u, kWfShadows), S.word(b - 1u, kWfShadowHead)};
+  };
+  uint32_t b = first;
+  for (;; ++b) {
     if (b > A.maxDepth) {
       // Ideal reflections and refractions spend no scattering event, so paths through glass and
       // mirrors can outlive the depth (Russian roulette ends them): bounce on while a path lives,
@@ -3416,13 +3423,17 @@ vt_status wf_bounces(const WfStages &S, const RenderArgs &A, WfArgs W, uint32_t 
     W.outCount = S.word(b + 1, kWfLive);
     W.shCount = S.word(b, kWfShadows);
     if (b > first && b % (kWfSlots - 2u) == 0u) {
-      // The slots are about to come round again: clear all but this bounce's, whose live count is in use.
-      const uint32_t at = b % kWfSlots;
-      VT_CUDA(ctx, cudaMemsetAsync(S.B.counts, 0, at * kWfWords * sizeof(uint32_t), s));
-      VT_CUDA(ctx, cudaMemsetAsync(S.B.counts + (at + 1u) * kWfWords, 0, (kWfSlots - 1u - at) * kWfWords * sizeof(uint32_t), s));
+      // The slots are about to come round again: clear all but this bounce's (its live count) and the one
+      // before (its shadow rays' count).
+      const uint32_t at = (b + 1u) % kWfSlots, upper = std::min(kWfSlots - 2u, kWfSlots - at);
+      VT_CUDA(ctx, cudaMemsetAsync(S.B.counts + at * kWfWords, 0, upper * kWfWords * sizeof(uint32_t), s));
+      VT_CUDA(ctx, cudaMemsetAsync(S.B.counts, 0, (kWfSlots - 2u - upper) * kWfWords * sizeof(uint32_t), s));
     }
-    vt_launch_closest(S.mesh, reinterpret_cast<const vt_ray *>(W.ray), P, reinterpret_cast<vt_hit *>(S.B.hit), ctx->sm_count,
-                      S.word(b, kWfExtendHead), W.inQ, ctx->d_status + 1, s, W.inCount, true, true);
+    const vt_ray_queue extend{reinterpret_cast<const vt_ray *>(W.ray), W.inQ, W.inCount, S.word(b, kWfExtendHead)};
+    if (b == 0u)
+      vt_launch_closest(S.mesh, extend.rays, P, hits, ctx->sm_count, extend.head, extend.list, ctx->d_status + 1, s, extend.count, true, true);
+    else
+      vt_launch_closest_any(S.mesh, extend, hits, shadows(b), S.B.occ, P, ctx->sm_count, ctx->d_status + 1, s, A.imported != 0u);
     if (S.group) {
       if (S.pbr) k_wf_group<true><<<grid, S.block, 0, s>>>(A, W, S.word(b, kWfGroup));
       else k_wf_group<false><<<grid, S.block, 0, s>>>(A, W, S.word(b, kWfGroup));
@@ -3435,10 +3446,10 @@ vt_status wf_bounces(const WfStages &S, const RenderArgs &A, WfArgs W, uint32_t 
       if (S.pbr) k_wf_shade<true, false><<<grid, S.block, 0, s>>>(A, W, b);
       else k_wf_shade<false, false><<<grid, S.block, 0, s>>>(A, W, b);
     }
-    vt_launch_any(S.mesh, reinterpret_cast<const vt_ray *>(W.sray), P, S.B.occ, ctx->sm_count, S.word(b, kWfShadowHead), W.shQ,
-                  ctx->d_status + 1, s, W.shCount, A.imported != 0u, true);
     VT_CUDA(ctx, cudaGetLastError());
   }
+  const vt_ray_queue last = shadows(b);
+  vt_launch_any(S.mesh, last.rays, P, S.B.occ, ctx->sm_count, last.head, last.list, ctx->d_status + 1, s, last.count, A.imported != 0u, true);
   if (S.nrc) k_wf_finish<true><<<grid, S.block, 0, s>>>(A, W);
   else k_wf_finish<false><<<grid, S.block, 0, s>>>(A, W);
   VT_CUDA(ctx, cudaGetLastError());
@@ -3489,8 +3500,6 @@ vt_status di_paths(const WfStages &S, const RenderArgs &A, WfArgs W, uint8_t *go
     if (S.pbr) k_di_shade<true, false><<<pixels, kRenderBlock, 0, s>>>(A, W);
     else k_di_shade<false, false><<<pixels, kRenderBlock, 0, s>>>(A, W);
   }
-  vt_launch_any(S.mesh, reinterpret_cast<const vt_ray *>(W.sray), P, S.B.occ, ctx->sm_count, S.word(0, kWfShadowHead), W.shQ,
-                ctx->d_status + 1, s, W.shCount, A.imported != 0u, true);
   if (!S.nrc && A.maxDepth > 1u) {
     vt_launch_any(S.mesh, reinterpret_cast<const vt_ray *>(W.gray), P, gocc, ctx->sm_count, S.word(0, kWfConnectHead), W.giQ,
                   ctx->d_status + 1, s, W.giCount, A.imported != 0u, true);

@@ -233,5 +233,13 @@ void vt_launch_closest(const vt_mesh *mesh, const vt_ray *rays, uint32_t n, vt_h
 void vt_launch_any(const vt_mesh *mesh, const vt_ray *rays, uint32_t n, uint8_t *occ,
                    int sm_count, uint32_t *counter, const uint32_t *perm, uint32_t *status,
                    cudaStream_t s, const uint32_t *count = nullptr, bool slack = false, bool cleared = false);
+// Both in one launch (BVH positions), each over its queue of at most n rays with a cleared head.
+struct vt_ray_queue {
+  const vt_ray *rays;
+  const uint32_t *list, *count;
+  uint32_t *head;
+};
+void vt_launch_closest_any(const vt_mesh *mesh, const vt_ray_queue &closest, vt_hit *hits, const vt_ray_queue &any, uint8_t *occ,
+                           uint32_t n, int sm_count, uint32_t *status, cudaStream_t s, bool slack);
 void vt_launch_count(const vt_mesh *mesh, const vt_ray *rays, uint32_t n, int closest,
                      unsigned long long *acc /* 2 device words */, cudaStream_t s);
