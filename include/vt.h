@@ -321,8 +321,8 @@ vt_status vt_render(vt_ctx *ctx, vt_scene *scene, const vt_frame_params *params,
  * and arithmetic per path; a path's primary and continuation radiance are summed apart, so the image
  * equals vt_render's to float rounding (1e-6 relative per pixel). The
  * reference has no wavefront path; its design note proposes the split (docs/KERNEL_SPLIT_DESIGN.md:
- * 72-74). Paths per pass are capped at 4M (whole samples of the frame); the state takes ~250 bytes
- * per path, allocated with the scene on first use. */
+ * 72-74). A frame has at most 4M pixels; a pass holds as many whole samples as fit 16M paths (4M where
+ * memory is short); the state takes ~260 bytes per path, allocated with the scene on first use. */
 vt_status vt_render_wavefront(vt_ctx *ctx, vt_scene *scene, const vt_frame_params *params, uint32_t spp, void *stream);
 vt_status vt_accum_reset(vt_ctx *ctx, vt_scene *scene);
 /* Mean radiance per pixel (linear sRGB, row-major, 3 doubles per pixel; n = width * height * 3

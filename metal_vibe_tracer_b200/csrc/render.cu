@@ -3282,8 +3282,11 @@ vt_status nrc_finish(vt_ctx *ctx, vt_nrc *nrc, const RenderArgs &A, uint32_t spp
 }
 
 // ---- wavefront integrator: host side ------------------------------------------------------------
-// Paths per pass: as many whole samples of the frame as fit 4M paths (about 1 GB of state).
-constexpr uint32_t kWfMaxPaths = 1u << 22;
+// Pixels of a frame at most, and paths per pass: as many whole samples of the frame as fit 16M paths (4.3 GB
+// of state), fewer (down to 4M paths) where memory is short. The late bounces of a pass hold few paths,
+// each some 100 us of dependent loads, whatever the pass's size: a 1080p production frame of 4 samples
+// (8.3M paths) took 17.5 ms in two passes and takes 15.4 in one on one B200.
+constexpr uint32_t kWfMaxPaths = 1u << 22, kWfPassPaths = 1u << 24;
 
 // Counter words of a pass: kWfSlots slots of kWfWords in rotation, one slot per bounce, so that one memset
 // a pass (and one per kWfSlots - 2 bounces beyond) clears them all instead of four or five a bounce, whose
@@ -3731,19 +3734,26 @@ vt_status wavefront_impl(vt_ctx *ctx, vt_scene *scene, const vt_frame_params *p,
     A.nrcVertex = nrc->cfg.query_vertex;
     A.nrcSpread = nrc->cfg.spread;
   }
-  const uint32_t chunk = std::max(1u, std::min(spp, maxPaths / npix));
-  const uint32_t cap = npix * chunk;
   unsigned char **state = run.state ? run.state : &scene->d_wf;
   uint32_t *stateCap = run.state ? run.stateCap : &scene->wf_cap;
-  if (cap > *stateCap) {
+  uint32_t chunk = 1u;
+  for (;;) {
+    const uint32_t passPaths = run.state || scene->wf_short ? maxPaths : kWfPassPaths;
+    chunk = std::max(1u, std::min(spp, passPaths / npix));
+    if (npix * chunk <= *stateCap) break;
     cudaFree(*state);
     *state = nullptr;
     *stateCap = 0;
     WfArgs probe;
     WfBuffers unused;
-    const size_t bytes = wf_carve(nullptr, cap, probe, unused);
-    VT_CUDA(ctx, cudaMalloc(state, bytes));
-    *stateCap = cap;
+    const cudaError_t e = cudaMalloc(state, wf_carve(nullptr, npix * chunk, probe, unused));
+    if (e == cudaSuccess) {
+      *stateCap = npix * chunk;
+      break;
+    }
+    if (e != cudaErrorMemoryAllocation || passPaths == maxPaths) return vt_cuda_fail(ctx, e, "allocating the path state");
+    cudaGetLastError();
+    scene->wf_short = true;  // this scene's passes stay at maxPaths
   }
   WfArgs W{};
   WfBuffers B;

@@ -141,6 +141,7 @@ struct vt_scene {
   // sized for wf_cap paths.
   unsigned char *d_wf = nullptr;
   uint32_t wf_cap = 0;
+  bool wf_short = false;  // memory was too short for the state of the largest passes
   unsigned char *d_wf_gi = nullptr;  // sampling mode 0's connection arrays, for wf_gi_cap paths
   uint32_t wf_gi_cap = 0;
   float di_cam[14] = {};  // previous frame's camera: position, forward, right, up, aspect, fov scale

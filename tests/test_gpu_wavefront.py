@@ -133,6 +133,13 @@ def test_passes_and_stride(ctx, cornell):
     assert_same(mega, wave)
 
 
+def test_largest_passes(ctx, cornell):
+    """More samples than one pass of 16M paths holds: 4 + 1 samples of 4M pixels."""
+    mats, light, cam, mesh = cornell
+    mega, wave = both(ctx, mesh, mats, light, vt.make_params(cam, 2000, 2000, 2, 1, False, 1), 5, False)
+    assert_same(mega, wave)
+
+
 def test_rejects_restir(ctx, cornell):
     mats, light, cam, mesh = cornell
     scene = vt.Scene(ctx, mesh, mats, light, None)
