@@ -4362,9 +4362,7 @@ vt_status vt_accum_readback(vt_ctx *ctx, vt_scene *scene, double *rgb, uint32_t 
                          ", kernel " + std::to_string(w[10] & 0xffu) + "); those accesses were clamped or skipped");
     }
   }
-  if (want) VT_CUDA(ctx, cudaMemcpy(rgb, scene->d_accum, want * sizeof(double), cudaMemcpyDeviceToHost));
-  const double inv = scene->samples ? 1.0 / scene->samples : 0.0;
-  for (size_t i = 0; i < want; ++i) rgb[i] *= inv;
+  if (vt_status st = vt_read_scaled(ctx, rgb, scene->d_accum, want, scene->samples ? 1.0 / scene->samples : 0.0)) return st;
   if (samples) *samples = scene->samples;
   return VT_OK;
 }

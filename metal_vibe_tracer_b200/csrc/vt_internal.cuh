@@ -12,6 +12,10 @@
 // ---------------------------------------------------------------------------------------------
 // Context and mesh objects behind the opaque C handles.
 
+// Staged host copies: slots in flight, chunks a slot's drain lags its fill, bytes a thread copies at once.
+constexpr uint32_t kStageSlots = 6, kStageLag = 2;
+constexpr size_t kStagePiece = 1u << 20;
+
 struct vt_ctx {
   int device = 0;
   int sm_count = 0;
@@ -26,12 +30,11 @@ struct vt_ctx {
   void *d_chunk_in[2] = {nullptr, nullptr};
   void *d_chunk_out[2] = {nullptr, nullptr};
   size_t chunk_in_bytes = 0, chunk_out_bytes = 0;
-  // Pinned host staging for callers' pageable buffers (allocated on first use, grown as needed), and
-  // per staging slot the event recorded after its chunk's copy back.
-  void *h_stage_in[2] = {nullptr, nullptr};
-  void *h_stage_out[2] = {nullptr, nullptr};
+  // Pinned host staging for callers' pageable buffers (kStageSlots slots, allocated on first use, grown as
+  // needed), and per slot the events recorded after its chunk's copy to the device and back.
+  void *h_stage_in = nullptr, *h_stage_out = nullptr;
   size_t stage_in_bytes = 0, stage_out_bytes = 0;
-  cudaEvent_t stage_ev[2] = {nullptr, nullptr};
+  cudaEvent_t stage_in_ev[kStageSlots] = {}, stage_out_ev[kStageSlots] = {};
   // Memory of the builds (temporaries and the meshes' arrays), created with the first build: freed
   // blocks stay in it up to kPoolKeep bytes, so that rebuilding a mesh maps no new memory.
   cudaMemPool_t pool = nullptr;
@@ -208,6 +211,8 @@ __device__ __forceinline__ uint32_t vt_poll(const uint32_t *p) {
 // stream has been synchronised).
 constexpr size_t kPoolKeep = size_t(1) << 30;
 cudaError_t vt_pool_alloc(vt_ctx *ctx, void **p, size_t bytes);
+// n doubles from the device, times scale, into host memory (the device is idle; returns when done).
+vt_status vt_read_scaled(vt_ctx *ctx, double *dst, const double *src, size_t n, double scale);
 
 // Stable LSD radix sort of (key, value) pairs on the low `bits` bits of the keys.
 // keys/vals are sorted in place using the alternate buffers; temp is vt_radix_temp_words(n). n below

@@ -194,3 +194,23 @@ def test_accumulation_save_and_restore_continue_a_render(ctx, cornell, tmp_path)
     b.close()
     assert n == 16
     np.testing.assert_allclose(img, whole[::2, ::2], rtol=1e-12, atol=1e-15)
+
+
+@pytest.mark.parametrize("width,height", [(419, 417), (420, 417), (701, 997), (1280, 721)])
+def test_readback_into_pageable_and_pinned_memory(ctx, width, height):
+    """Image sizes around the threaded readback's lines: ordinary memory (staged, scaled by the threads that
+    drain it) and pinned memory (copied, then scaled) hold the same doubles."""
+    import ctypes as C
+    import torch
+    from metal_vibe_tracer_b200 import _lib
+    faces, verts, mats, light, cam = scenes.cornell_box()
+    mesh = vt.Mesh(ctx, faces, verts)
+    scene = vt.Scene(ctx, mesh, mats, light, None)
+    scene.render_wavefront(vt.make_params(cam, width, height, 2, 1, False, 1), 3)
+    img, n = scene.readback()
+    pinned = torch.zeros(height * width * 3, dtype=torch.float64, pin_memory=True)
+    samples = C.c_uint32()
+    assert _lib.load().vt_accum_readback(ctx.handle, scene._p, pinned.data_ptr(), pinned.numel(), C.byref(samples)) == 0
+    assert n == samples.value == 3 and np.array_equal(img.reshape(-1), pinned.numpy())
+    scene.close()
+    mesh.close()

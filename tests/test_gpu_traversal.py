@@ -190,3 +190,14 @@ def test_few_rays_equal_a_large_batch(ctx, n):
     rays = scenes.incoherent_rays_np(300_000, seed=3)
     assert_bit_exact(gpu_closest(mesh, rays[:n]), gpu_closest(mesh, rays)[:n])
     assert np.array_equal(gpu_any(mesh, rays[:n]), gpu_any(mesh, rays)[:n])
+
+
+@pytest.mark.parametrize("n", [87_381, 87_382, 131_071, 131_073, 786_433, 1_500_001])
+def test_host_chunks(ctx, n):
+    """Ordinary host arrays around the sizes where threads start and chunks end, against device arrays."""
+    faces, verts = scenes.triangle_soup(3000, seed=2, mu=math.log(0.03))
+    mesh = vt.Mesh(ctx, faces, verts)
+    rays = scenes.incoherent_rays_np(n, seed=4)
+    for _ in range(2):
+        assert_bit_exact(mesh.closest(rays), gpu_closest(mesh, rays))
+        assert np.array_equal(mesh.occluded(rays), gpu_any(mesh, rays))
