@@ -2072,10 +2072,9 @@ __global__ void __launch_bounds__(kWfBlock) k_wf_finish(RenderArgs A, WfArgs W) 
 // 64 16.4.
 template <bool kPbr>
 __global__ void __launch_bounds__(kRenderBlock, 6) k_di_primary(RenderArgs A, WfArgs W) {
-  __shared__ uint32_t sTotal, sBase;
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   bool push = false;
-  [&] {  // one pixel; every thread of the block joins the queue push below
+  [&] {  // one pixel; every lane joins the queue push below
     if (i >= W.paths) return;
     const uint32_t p = W.p0 + i, k = W.k0, x = p % A.W, y = p / A.W;
     Sampler seed = pixel_sampler(x, y, A.W, A.first + k, A.zSampler != 0u, A.zModel, A.firstFrame + k);
@@ -2159,7 +2158,12 @@ __global__ void __launch_bounds__(kRenderBlock, 6) k_di_primary(RenderArgs A, Wf
     W.meta[i] = make_uint4(p, 0u, 0u, 0u);
     wf_store_seed(W, i, seed);
   }();
-  wf_push(push, i, W.outQ, W.outCount, sTotal, sBase);
+  // Pushed per warp: a block's warps end far apart, and waiting for the last cost 2 % of a frame.
+  const unsigned lane = threadIdx.x & 31u, pushes = __ballot_sync(0xffffffffu, push);
+  uint32_t base = 0;
+  if (lane == 0 && pushes) base = atomicAdd(W.outCount, (uint32_t)__popc(pushes));
+  base = __shfl_sync(0xffffffffu, base, 0);
+  if (push) W.outQ[base + (uint32_t)__popc(pushes & ((1u << lane) - 1u))] = i;
 }
 
 // restir_gi_initial (main.swift:4718-4770) at the candidate's hit x2 (diffuse, or there is no
