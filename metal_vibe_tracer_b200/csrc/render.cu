@@ -1561,11 +1561,13 @@ __device__ __forceinline__ GISample gi_load(const float4 *pos, const float4 *nrm
 // neighbouring pixels; a group covers `per` consecutive samples of the call. Each item adds its
 // FP64 sum to the pixel with one atomic per channel (groups > 1) or a plain add (groups = 1).
 template <bool kPbr>
-__global__ void __launch_bounds__(kRenderBlock, kPbr ? 3 : 4) k_render(RenderArgs A, uint32_t groups, uint32_t per) {
+__global__ void __launch_bounds__(kRenderBlock, kPbr ? 3 : 4) k_render(RenderArgs A, uint32_t groups, uint32_t per, uint32_t lanes) {
   int stack[kRenderStack];
   const uint32_t npix = A.OW * A.OH;  // accumulation pixels: the frame's pixels (s i, s j)
   const uint64_t items = (uint64_t)npix * groups;
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < items; i += (uint64_t)gridDim.x * blockDim.x) {
+  const uint32_t lane = threadIdx.x & 31u, warp = blockIdx.x * (kRenderBlock / 32) + (threadIdx.x >> 5);
+  if (lane >= lanes) return;
+  for (uint64_t i = warp * (uint64_t)lanes + lane; i < items; i += (uint64_t)gridDim.x * (kRenderBlock / 32) * lanes) {
     const uint32_t p = (uint32_t)(i % npix), g = (uint32_t)(i / npix);
     const uint32_t x = (p % A.OW) * A.stride, y = (p / A.OW) * A.stride;
     const uint32_t k0 = g * per, k1 = min(A.spp, k0 + per);
@@ -3664,10 +3666,17 @@ vt_status render_impl(vt_ctx *ctx, vt_scene *scene, const vt_frame_params *p, ui
   const uint32_t per = (spp + groups - 1) / groups;
   groups = (spp + per - 1) / per;
   const uint64_t items = (uint64_t)npix * groups;
-  const uint32_t grid = (uint32_t)std::min<uint64_t>((items + kRenderBlock - 1) / kRenderBlock, (uint64_t)ctx->sm_count * 32u);
+  // Few items (a small preview) go to a few lanes of each of 8 warps an SM, where a path waits for fewer
+  // others': up to 8 lanes a warp (9,472 items), beyond that whole warps are the faster. Measured on one
+  // B200, one sample of 64 x 64 at depth 5: 36 triangles 68 -> 64 us, 300,000 581 -> 329, the spectral OPENPBR
+  // grid 851 -> 553; 8 lanes of 16 warps lose at 128 x 128 (70 -> 94 us).
+  const uint64_t warps = (uint64_t)ctx->sm_count * 8u;
+  const uint32_t lanes = items <= 8u * warps ? (uint32_t)((items + warps - 1) / warps) : 32u;
+  const uint64_t block = (kRenderBlock / 32) * lanes;
+  const uint32_t grid = (uint32_t)std::min<uint64_t>((items + block - 1) / block, (uint64_t)ctx->sm_count * 32u);
   A.kernelId = 1;
-  if (A.layered) k_render<true><<<grid, kRenderBlock, 0, s>>>(A, groups, per);
-  else k_render<false><<<grid, kRenderBlock, 0, s>>>(A, groups, per);
+  if (A.layered) k_render<true><<<grid, kRenderBlock, 0, s>>>(A, groups, per, lanes);
+  else k_render<false><<<grid, kRenderBlock, 0, s>>>(A, groups, per, lanes);
   VT_CUDA(ctx, cudaGetLastError());
   scene->samples += spp;
   return VT_OK;

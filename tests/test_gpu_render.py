@@ -214,3 +214,21 @@ def test_readback_into_pageable_and_pinned_memory(ctx, width, height):
     assert n == samples.value == 3 and np.array_equal(img.reshape(-1), pinned.numpy())
     scene.close()
     mesh.close()
+
+
+@pytest.mark.parametrize("width,height,spp", [(1, 1, 1), (37, 32, 1), (74, 64, 1), (74, 64, 2), (75, 127, 1)])
+def test_small_frames(ctx, width, height, spp):
+    """Frames around the sizes that give a path one, several or all lanes of a warp: the whole-path integrator's
+    image equals the stage kernels' (1e-6, as the two always agree)."""
+    faces, verts, mats, light, cam = scenes.cornell_box()
+    mesh = vt.Mesh(ctx, faces, verts)
+    images = []
+    for wavefront in (False, True):
+        scene = vt.Scene(ctx, mesh, mats, light, None)
+        (scene.render_wavefront if wavefront else scene.render)(vt.make_params(cam, width, height, 5, 1, False, 1), spp)
+        images.append(scene.readback()[0])
+        scene.close()
+    mesh.close()
+    mega, wave = images
+    same = np.all(np.abs(wave - mega) <= 1e-6 * np.maximum(np.abs(mega), 1e-3), axis=-1)
+    assert same.mean() >= 0.995, same.mean()
