@@ -1620,7 +1620,7 @@ __device__ __forceinline__ float2 frame_jitter(uint32_t sampleIndex) {
 // summed in k_render's order) to its pixel's FP64 accumulation.
 constexpr int kWfBlock = 256;
 constexpr uint32_t kWfShadow = 1u, kWfShadowPrimary = 2u, kWfEmissionOnly = 4u, kWfPrevMIS = 8u, kWfQueried = 16u,
-                   kWfDead = 32u, kWfPrevDelta = 64u, kWfGiPrimary = 128u;
+                   kWfDead = 32u, kWfPrevDelta = 64u, kWfGiPrimary = 128u, kWfLit = 256u;
 
 struct WfArgs {
   float4 *T;      // throughput per lane
@@ -1643,6 +1643,7 @@ struct WfArgs {
   uint32_t *grpQ;                 // the live queue regrouped by kind of vertex (k_wf_group): kWfClasses
   uint32_t grpStride;             // queues of grpStride entries
   const uint32_t *groups;         // their counts; null: the bounce is not regrouped
+  float4 *light;                  // the vertex's light sample (k_wf_light): direction, pdf; emission
   uint32_t npix, paths, k0;       // accumulation pixels; paths of the pass; its first sample (of the call)
   uint32_t p0;                    // the pass's first pixel (sampling mode 0: a band of one frame; else 0)
   // Sampling mode 0: the GI reservoir's connection from the primary vertex.
@@ -1742,6 +1743,45 @@ __global__ void __launch_bounds__(kWfBlock) k_wf_group(RenderArgs A, WfArgs W, u
   }
 }
 
+// Entries of a stage: the first `use` classes of a regrouped queue one after another, each from a whole warp
+// on, or the live queue.
+struct WfEntries {
+  uint32_t n, classes[kWfClasses];
+};
+__device__ __forceinline__ WfEntries wf_entries(const WfArgs &W, uint32_t use) {
+  WfEntries E;
+  if (W.groups) {
+    E.n = 0;
+#pragma unroll
+    for (uint32_t c = 0; c < kWfClasses; ++c) {
+      E.classes[c] = c < use ? min(W.groups[c], W.paths) : 0u;
+      E.n += (E.classes[c] + 31u) & ~31u;
+    }
+  } else {
+    E.n = W.inCount ? min(*W.inCount, W.paths) : W.paths;
+  }
+  return E;
+}
+// Entry q's path into i; false where there is none.
+__device__ __forceinline__ bool wf_entry(const WfArgs &W, const WfEntries &E, uint32_t q, uint32_t &i) {
+  if (!W.groups) {
+    if (q >= E.n) return false;
+    i = W.inQ ? W.inQ[q] : q;
+    return !(W.deadFlags && (W.meta[i].w & kWfDead));
+  }
+#pragma unroll
+  for (uint32_t c = 0; c < kWfClasses; ++c) {
+    const uint32_t padded = (E.classes[c] + 31u) & ~31u;
+    if (q < padded) {
+      if (q >= E.classes[c]) return false;
+      i = W.grpQ[c * W.grpStride + q];
+      return true;
+    }
+    q -= padded;
+  }
+  return false;
+}
+
 // The light sample of one vertex (the draws of direct_light_lanes) and its shadow ray into sray[i];
 // false when there is nothing to trace.
 __device__ __forceinline__ bool wf_light(const RenderArgs &A, const WfArgs &W, uint32_t i, const Surface &S, bool compensated,
@@ -1808,7 +1848,7 @@ __device__ __forceinline__ bool wf_continue(const RenderArgs &A, const WfArgs &W
 // `shadow` when it queued a shadow ray. kNrc (vt_render_nrc): the path ends, after the vertex's
 // emission, at vertex A.nrcVertex, or with A.nrcVertex 0 at the first vertex where its spread exceeds
 // its limit (nrc_spread_limit), with its cache query stored in its slot.
-template <bool kPbr, bool kNrc>
+template <bool kPbr, bool kNrc, bool kSplit>
 __device__ __forceinline__ void wf_vertex(const RenderArgs &A, const WfArgs &W, uint32_t i, uint32_t b, bool &next,
                                           bool &shadow) {
   uint4 meta = W.meta[i];
@@ -1913,7 +1953,15 @@ __device__ __forceinline__ void wf_vertex(const RenderArgs &A, const WfArgs &W, 
     // (Preparing at each use, and again for lane 3, left 1.9x the instructions and several copies of the
     // lobes' code for the instruction cache: a 1080p production frame of 4 samples 56.9 -> 28.5 ms.)
     LightSample ls;
-    if (takesNee) {
+    if (takesNee && kSplit) {
+      shadow = (flags & kWfLit) != 0u;
+      if (shadow) {
+        const float4 l0 = W.light[2 * (size_t)i], l1 = W.light[2 * (size_t)i + 1];
+        ls.wi = f3(l0.x, l0.y, l0.z);
+        ls.pdf = l0.w;
+        ls.emission = f3(l1.x, l1.y, l1.z);
+      }
+    } else if (takesNee) {
       sampler_event(seed, b + 1u, kZNee);
       shadow = wf_light(A, W, i, S, scattering < limit, seed, b == 0u, ls);
     }
@@ -1934,6 +1982,7 @@ __device__ __forceinline__ void wf_vertex(const RenderArgs &A, const WfArgs &W, 
     if (alive)
       next = wf_continue<kPbr>(A, W, i, b + 1u, L, S, m, dir, T, seed, scattering, emissionOnly, mis, pn.w, flags, pbr, prep);
   }
+  if (kSplit) flags &= ~kWfLit;
   flags = emissionOnly ? (flags | kWfEmissionOnly) : (flags & ~kWfEmissionOnly);
   W.meta[i] = make_uint4(meta.x, next ? b + 1u : b, (uint32_t)scattering, flags);
   W.Rc[i] = Rc;
@@ -1966,44 +2015,18 @@ __global__ void __launch_bounds__(kWfBlock) k_wf_generate(RenderArgs A, WfArgs W
 
 // Two blocks of kWfBlock per SM (at most 128 registers): the OpenPBR variant's register demand
 // (with thin films) would otherwise leave one block, and the stage is latency-bound on its loads.
-template <bool kPbr, bool kNrc>
+template <bool kPbr, bool kNrc, bool kSplit>
 __global__ void __launch_bounds__(kWfBlock, 2) k_wf_shade(RenderArgs A, WfArgs W, uint32_t bounce) {
   __shared__ uint32_t sTotal, sBase;
-  // Entries of a regrouped queue: the classes one after another, each from a whole warp on.
-  uint32_t n = 0, classes[kWfClasses];
-  if (W.groups) {
-#pragma unroll
-    for (uint32_t c = 0; c < kWfClasses; ++c) {
-      classes[c] = min(W.groups[c], W.paths);
-      n += (classes[c] + 31u) & ~31u;
-    }
-  } else {
-    n = W.inCount ? min(*W.inCount, W.paths) : W.paths;
-  }
+  const WfEntries E = wf_entries(W, kWfClasses);
+  const uint32_t n = E.n;
   for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
     const uint32_t q = base + threadIdx.x;
-    bool next = false, shadow = false, entry = q < n;
+    bool next = false, shadow = false;
     uint32_t i = 0;
-    if (W.groups) {
-      uint32_t r = q;
-      bool found = false;
-      entry = false;
-#pragma unroll
-      for (uint32_t c = 0; c < kWfClasses; ++c) {
-        const uint32_t padded = (classes[c] + 31u) & ~31u;
-        if (!found && r < padded) {
-          found = true;
-          entry = r < classes[c];
-          if (entry) i = W.grpQ[c * W.grpStride + r];
-        }
-        if (!found) r -= padded;
-      }
-    } else if (entry) {
-      i = W.inQ ? W.inQ[q] : q;
-      entry = !(W.deadFlags && (W.meta[i].w & kWfDead));
-    }
+    const bool entry = wf_entry(W, E, q, i);
     if (entry) {
-      wf_vertex<kPbr, kNrc>(A, W, i, bounce, next, shadow);
+      wf_vertex<kPbr, kNrc, kSplit>(A, W, i, bounce, next, shadow);
       // A path that ends on a bounce without compaction stays queued: flagged, with an empty ray.
       if (!next && !W.compact) {
         W.meta[i].w |= kWfDead;
@@ -2015,6 +2038,44 @@ __global__ void __launch_bounds__(kWfBlock, 2) k_wf_shade(RenderArgs A, WfArgs W
     } else {
       if (q < n) W.outQ[q] = i;
       if (q == 0) *W.outCount = n;
+    }
+    if (!kSplit) wf_push(shadow, i, W.shQ, W.shCount, sTotal, sBase);
+  }
+}
+
+// The light samples of a regrouped bounce's vertices in a launch of their own: half of a production vertex's
+// instructions are the serial walk of the light tree, which wants warps to hide its loads, and the BSDF's
+// registers allow k_wf_shade two blocks an SM. Draws what wf_vertex would, stores the sample (W.light, kWfLit)
+// and the sampler, and queues the shadow ray. Bound: the walk's dependent loads. Measured on one B200, a 1080p
+// production frame of 4 samples: 15.3 -> 14.5 ms of device time (3 and 5 blocks an SM instead of 4: 14.9).
+__global__ void __launch_bounds__(kWfBlock, 4) k_wf_light(RenderArgs A, WfArgs W, uint32_t b) {
+  __shared__ uint32_t sTotal, sBase;
+  const WfEntries E = wf_entries(W, kWfClasses - 1u);  // no emitters
+  for (uint32_t base = blockIdx.x * blockDim.x; base < E.n; base += gridDim.x * blockDim.x) {
+    bool shadow = false;
+    uint32_t i = 0;
+    if (wf_entry(W, E, base + threadIdx.x, i)) {
+      const uint4 meta = W.meta[i];
+      const int4 h4 = W.hit[i];
+      Hit h;
+      h.t = __int_as_float(h4.x); h.b1 = __int_as_float(h4.y); h.b2 = __int_as_float(h4.z); h.pos = h4.w;
+      const float4 r0 = W.ray[2 * (size_t)i], r1 = W.ray[2 * (size_t)i + 1];
+      const Surface S = surface_at(A, h, f3(r0.x, r0.y, r0.z), f3(r1.x, r1.y, r1.z));
+      const vt_material m = material(A, S.slot);
+      const bool emissionOnly = b > 0u && (meta.w & kWfEmissionOnly);
+      if (!emissionOnly && !is_delta<true>(A, m) && !(b == 1u && (meta.w & kWfGiPrimary) && m.type == VT_MAT_DIFFUSE)) {
+        Sampler seed = wf_load_seed(W, i);
+        sampler_event(seed, b + 1u, kZNee);
+        LightSample ls;
+        const int scattering = b == 0u ? 0 : (int)meta.z;
+        shadow = wf_light(A, W, i, S, scattering < max(0, (int)A.maxDepth - 1), seed, b == 0u, ls);
+        wf_store_seed(W, i, seed);
+        if (shadow) {
+          W.light[2 * (size_t)i] = make_float4(ls.wi.x, ls.wi.y, ls.wi.z, ls.pdf);
+          W.light[2 * (size_t)i + 1] = make_float4(ls.emission.x, ls.emission.y, ls.emission.z, 0.0f);
+          W.meta[i].w = meta.w | kWfLit;
+        }
+      }
     }
     wf_push(shadow, i, W.shQ, W.shCount, sTotal, sBase);
   }
@@ -3288,7 +3349,7 @@ vt_status nrc_finish(vt_ctx *ctx, vt_nrc *nrc, const RenderArgs &A, uint32_t spp
 }
 
 // ---- wavefront integrator: host side ------------------------------------------------------------
-// Pixels of a frame at most, and paths per pass: as many whole samples of the frame as fit 16M paths (4.3 GB
+// Pixels of a frame at most, and paths per pass: as many whole samples of the frame as fit 16M paths (4.8 GB
 // of state), fewer (down to 4M paths) where memory is short. The late bounces of a pass hold few paths,
 // each some 100 us of dependent loads, whatever the pass's size: a 1080p production frame of 4 samples
 // (8.3M paths) took 17.5 ms in two passes and takes 15.4 in one on one B200.
@@ -3332,6 +3393,7 @@ size_t wf_carve(unsigned char *base, uint32_t cap, WfArgs &W, WfBuffers &B) {
   B.hit = reinterpret_cast<int4 *>(take(16 * n));
   W.sray = reinterpret_cast<float4 *>(take(32 * n));
   W.scon = reinterpret_cast<float4 *>(take(16 * n));
+  W.light = reinterpret_cast<float4 *>(take(32 * n));
   B.occ = reinterpret_cast<uint8_t *>(take(n));
   B.q[0] = reinterpret_cast<uint32_t *>(take(4 * n));
   B.q[1] = reinterpret_cast<uint32_t *>(take(4 * n));
@@ -3369,7 +3431,7 @@ struct WfStages {
   WfBuffers B;
   int block;               // stage kernels' block size
   uint32_t gridMax, every; // their most blocks; the live queue is compacted on every n-th bounce
-  bool pbr, unbounded, group, nrc;
+  bool pbr, unbounded, group, split, nrc;
   cudaStream_t s;
   uint32_t *word(uint32_t bounce, uint32_t w) const { return B.counts + (bounce % kWfSlots) * kWfWords + w; }
   cudaError_t clear() const { return cudaMemsetAsync(B.counts, 0, kWfSlots * kWfWords * sizeof(uint32_t), s); }
@@ -3392,6 +3454,11 @@ WfStages wf_stages(vt_ctx *ctx, const vt_scene *scene, const RenderArgs &A, cons
   // would only add its time (k_wf_group; ReSTIR frames of a Lambert scene gain least, 17.0 -> 16.7 ms).
     S.group = S.pbr || A.imported;
   S.nrc = nrc;
+  // Light samples in their own launch (k_wf_light) where the walk and the BSDF are both long: with a light
+  // tree, OpenPBR slots and spectral transport. In RGB it gains nothing (4.55 against 4.58 ms for 960 x 540),
+  // and on Lambert slots the second pass over the path state costs more than it saves (4.30 against 4.48 ms
+  // for 1000 x 600). (A cache-terminated path must not draw at the vertex that ends it.)
+  S.split = S.pbr && A.spectral && A.imported && A.treeNodes && !nrc && A.mode != 3u;
   S.s = s;
   return S;
 }
@@ -3448,12 +3515,15 @@ vt_status wf_bounces(const WfStages &S, const RenderArgs &A, WfArgs W, uint32_t 
       else k_wf_group<false><<<grid, S.block, 0, s>>>(A, W, S.word(b, kWfGroup));
       W.groups = S.word(b, kWfGroup);
     }
-    if (S.nrc) {
-      if (S.pbr) k_wf_shade<true, true><<<grid, S.block, 0, s>>>(A, W, b);
-      else k_wf_shade<false, true><<<grid, S.block, 0, s>>>(A, W, b);
+    if (S.split) {
+      k_wf_light<<<grid, S.block, 0, s>>>(A, W, b);
+      k_wf_shade<true, false, true><<<grid, S.block, 0, s>>>(A, W, b);
+    } else if (S.nrc) {
+      if (S.pbr) k_wf_shade<true, true, false><<<grid, S.block, 0, s>>>(A, W, b);
+      else k_wf_shade<false, true, false><<<grid, S.block, 0, s>>>(A, W, b);
     } else {
-      if (S.pbr) k_wf_shade<true, false><<<grid, S.block, 0, s>>>(A, W, b);
-      else k_wf_shade<false, false><<<grid, S.block, 0, s>>>(A, W, b);
+      if (S.pbr) k_wf_shade<true, false, false><<<grid, S.block, 0, s>>>(A, W, b);
+      else k_wf_shade<false, false, false><<<grid, S.block, 0, s>>>(A, W, b);
     }
     VT_CUDA(ctx, cudaGetLastError());
   }
@@ -3684,7 +3754,7 @@ vt_status render_impl(vt_ctx *ctx, vt_scene *scene, const vt_frame_params *p, ui
 
 
 // Launch settings of a wavefront render and where its state lives. The defaults are vt_render_wavefront's:
-// the scene's own state, up to 4M paths per pass, 256-thread stage blocks, compaction every bounce and the
+// the scene's own state, passes of up to kWfPassPaths paths, 256-thread stage blocks, compaction every bounce and the
 // frame jitter uploaded from the host. Batches give each stream its own state and tune the rest.
 struct WfRun {
   unsigned char **state = nullptr;  // state buffer (null: the scene's own)

@@ -124,6 +124,25 @@ def test_open_scene_of_every_class_equals_megakernel(ctx, spectral):
     assert np.all(np.abs(wave.mean((0, 1)) / mega.mean((0, 1)) - 1) < 2e-3)
 
 
+@pytest.mark.parametrize("mode,sampler", [(1, 0), (2, 0), (1, 1)])
+def test_openpbr_under_a_light_tree_equals_megakernel(ctx, mode, sampler):
+    """Spectral OpenPBR slots (a film among them) under a light tree, where the light samples have a launch of
+    their own, beside Lambert and mirror slots. (Tolerance as for the layered slots.)"""
+    faces, verts, mats, cam = scenes.cornell_emitters()
+    pbr = dict(type=4, emission=(0.0, 0.0, 0.0), roughness=0.35, ior=1.5)
+    mats[2] = dict(pbr, albedo=(0.7, 0.6, 0.5))
+    mats[3] = dict(pbr, albedo=(0.6, 0.1, 0.1), thin_film_weight=1.0, thin_film_thickness=0.4, thin_film_ior=1.4)
+    mats[4] = dict(pbr, albedo=(0.9, 0.7, 0.3), metalness=1.0)
+    mats[5] = scenes.cornell_delta()[2][5]
+    mesh = vt.Mesh(ctx, faces, verts)
+    params = vt.make_params(cam, 96, 64, 6, 1, True, mode, sampler=sampler)
+    mega, wave = both(ctx, mesh, mats, None, params, 8, True)
+    mesh.close()
+    same = np.all(np.abs(wave - mega) <= 1e-4 * np.maximum(np.abs(mega), 1e-3), axis=-1)
+    assert same.mean() >= 0.98, same.mean()
+    assert np.all(np.abs(wave.mean((0, 1)) / mega.mean((0, 1)) - 1) < 2e-3)
+
+
 def test_passes_and_stride(ctx, cornell):
     mats, light, cam, mesh = cornell
     # 1024 x 1024 x 8 spp = 8M paths: two passes of 4M.
