@@ -496,8 +496,11 @@ __device__ __forceinline__ void refit_first(const TreeView &t, float *firstCost,
 // to own it, which saves a pass of its own. Nodes owned by lanes of one warp in the same step are
 // disjoint subtrees (an owner's subtrees are final), so the warp takes those with >= size leaves one
 // after another in any order.
-__global__ void __launch_bounds__(128) k_restructure(TreeView t, uint32_t *flags, int size, float *firstCost, uint32_t *status) {
-  __shared__ TreeletScratch scratch[4];
+// Blocks of two warps: a block's slots stay taken until its longest walk ends (128 threads 0.839 and 3.50 ms
+// for whole builds of 20,480 and 1M triangles, 64 0.813 and 3.46, 32 0.866 and 3.52).
+constexpr int kRestructureBlock = 64;
+__global__ void __launch_bounds__(kRestructureBlock) k_restructure(TreeView t, uint32_t *flags, int size, float *firstCost, uint32_t *status) {
+  __shared__ TreeletScratch scratch[kRestructureBlock / 32];
   __shared__ SubsetTable sets;
   for (uint32_t q = threadIdx.x; q < sizeof(SubsetTable) / 4; q += blockDim.x)
     reinterpret_cast<uint32_t *>(&sets)[q] = reinterpret_cast<const uint32_t *>(&kSubsets)[q];
@@ -719,7 +722,7 @@ __global__ void __launch_bounds__(kCollapseBlock) k_collapse(TreeView t, int lea
     const uint32_t w0 = min((uint64_t)L, (uint64_t)blockIdx.x * per), w1 = min(L, w0 + per);
     uint32_t sumI = 0, sumP = 0;
     for (uint32_t w = w0 + threadIdx.x; w < w1; w += kCollapseBlock) {
-      const int root = depth == 1 ? (t.n >= 2 ? 0 : -1) : (int)vt_poll(reinterpret_cast<const uint32_t *>(level + w));
+      const int root = depth == 1 ? (t.n >= 2 ? 0 : -1) : __ldcg(level + w);
       int ch[4];
       uint32_t inner, prims;
       const int m = collapse_children(t, root, leafSize, ch, inner, prims);
@@ -734,7 +737,7 @@ __global__ void __launch_bounds__(kCollapseBlock) k_collapse(TreeView t, int lea
     if (!grid_barrier(bar, round, status)) return;
     uint32_t allI = 0, allP = 0, runI = 0, runP = 0;
     for (uint32_t q = threadIdx.x; q < gridDim.x; q += kCollapseBlock) {
-      const uint2 v = make_uint2(vt_poll(&blockSums[q].x), vt_poll(&blockSums[q].y));
+      const uint2 v = __ldcg(blockSums + q);  // ordered by the barrier
       allI += v.x;
       allP += v.y;
       if (q < blockIdx.x) { runI += v.x; runP += v.y; }
@@ -848,7 +851,7 @@ struct BuildScratch {
   double *sah;
 };
 
-constexpr uint32_t kCollapseBlocksMax = 1184;  // 8 per SM
+constexpr uint32_t kCollapseBlocksMax = 592;  // 4 per SM: more blocks make the barriers and the prefix dearer
 
 void carve_build(ScratchCarve &c, uint32_t n, BuildScratch &b) {
   const uint32_t ni = n > 1 ? n - 1 : 1;
@@ -901,7 +904,7 @@ cudaError_t queue_build(const vt_face *faces, uint32_t n, const vt_vertex *verts
   TreeView t{(int)n, o.child, b.parent, b.leafBox, o.nodeBox, b.count, b.cost};
   if (n >= 3 && treelet > 0) {
     for (int r = 0; r < rounds; ++r)
-      k_restructure<<<blocks(n, 128), 128, 0, s>>>(t, b.flags, treelet, r == 0 ? b.firstCost : nullptr, status);
+      k_restructure<<<blocks(n, kRestructureBlock), kRestructureBlock, 0, s>>>(t, b.flags, treelet, r == 0 ? b.firstCost : nullptr, status);
   } else if (n >= 2) {
     k_bottom_up<<<blocks(n, 128), 128, 0, s>>>(t, b.flags, status);
   }
