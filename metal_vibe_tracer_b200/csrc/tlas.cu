@@ -62,7 +62,9 @@ __device__ __forceinline__ float xform_dir(float4 l, float x, float y, float z) 
 // (< 2^29), a BLAS leaf ~(its first triangle) (negative), a TLAS node kTlasNode | index and an
 // instance kTlasInstance | index (indices below 2^29 and 2^24).
 constexpr int kTlasNode = 0x40000000, kTlasInstance = 0x60000000, kTlasIndex = 0x1fffffff;
-constexpr int kTlasRefill = 8;  // idle lanes that make a warp take new rays (traverse.cu's k_closest)
+constexpr int kTlasIdle = 0x7fffffff;  // no ray
+constexpr int kTlasSteps = 4;        // BLAS nodes per lane between votes
+constexpr int kTlasRefill = 4;  // idle lanes that make a warp take new rays (traverse.cu's k_closest)
 __device__ __forceinline__ int *tlas_slot(int *sstack, int d) { return sstack + d * kTlasBlock + threadIdx.x; }
 
 // mesh_closest (kAny = false) / mesh_occluded (kAny = true): persistent warps over the two levels.
@@ -76,10 +78,12 @@ __device__ __forceinline__ int *tlas_slot(int *sstack, int d) { return sstack + 
 // entry pushed before a closer hit holds is culled by the box tests when it is popped.
 // Block b takes the rays of tiles b, b + grid, ... of 32 (through a block counter in shared memory),
 // so a launch needs no device-wide counter and expensive image regions spread over the blocks.
-// Measured on one B200: 1M random rays over 1,024 instances of 20,480-triangle meshes (closest hit)
-// 2.66 -> 1.28 ms.
+// A BLAS visit goes straight on to its nearest hit child, kept in a register, for up to kTlasSteps nodes
+// per lane between votes (traverse.cu). Measured on one B200: 1M random rays over 1,024 instances of
+// 20,480-triangle meshes (closest hit) 2.66 -> 1.28 ms, with the straight descent 1.17 -> 1.12 (1, 2 and 8
+// steps 1.21, 1.17, 1.28; 6 and 8 blocks an SM instead of 7, 1.15 and 1.21; refill at 8 lanes 1.14).
 template <bool kAny>
-__global__ void __launch_bounds__(kTlasBlock, 6) k_tlas_trace(const float4 *__restrict__ nodes, const TlasInst *__restrict__ inst,
+__global__ void __launch_bounds__(kTlasBlock, 7) k_tlas_trace(const float4 *__restrict__ nodes, const TlasInst *__restrict__ inst,
                                                              const TlasMesh *__restrict__ meshes, float grow, float reach,
                                                              const float4 *__restrict__ rays, uint32_t n, int4 *__restrict__ hits,
                                                              uint32_t *__restrict__ instOut, uint8_t *__restrict__ occ,
@@ -92,7 +96,7 @@ __global__ void __launch_bounds__(kTlasBlock, 6) k_tlas_trace(const float4 *__re
   // This block's tiles and rays (the last tile may be short).
   const uint32_t tiles = (n + 31u) / 32u;
   const uint32_t mine = blockIdx.x < tiles ? (tiles - blockIdx.x + gridDim.x - 1u) / gridDim.x * 32u : 0u;
-  int top = 0;  // 0: the lane holds no ray
+  int cur = kTlasIdle, top = 0;  // the current entry, in a register; entries on the stack
   uint32_t rid = 0, hitInst = 0xffffffffu, curInst = 0;
   WRay wr{};
   QRay qr{};
@@ -101,7 +105,7 @@ __global__ void __launch_bounds__(kTlasBlock, 6) k_tlas_trace(const float4 *__re
   int prim = -1;
   bool exhausted = false;  // warp-uniform
   while (true) {
-    const unsigned idle = __ballot_sync(kAll, top == 0);
+    const unsigned idle = __ballot_sync(kAll, cur == kTlasIdle);
     if (!exhausted && __popc(idle) >= kTlasRefill) {
       uint32_t base = 0;
       if (lane == 0) base = atomicAdd(&taken, (uint32_t)__popc(idle));
@@ -114,19 +118,19 @@ __global__ void __launch_bounds__(kTlasBlock, 6) k_tlas_trace(const float4 *__re
         tMin = __fadd_rn(__ldg(&rays[2 * (size_t)r].w), 0.0f);  // -0 to +0 (sort_qchildren)
         closest = __ldg(&rays[2 * (size_t)r + 1].w);
         prim = -1;
-        *tlas_slot(sstack, 0) = kTlasNode;
-        top = 1;
+        cur = kTlasNode;
+        top = 0;
       }
     }
-    if (exhausted && !__any_sync(kAll, top > 0)) break;
-    const int entry = top > 0 ? *tlas_slot(sstack, top - 1) : 0;
-    const bool leaf = top > 0 && entry < 0, world = top > 0 && entry >= kTlasNode;
+    if (exhausted && !__any_sync(kAll, cur != kTlasIdle)) break;
+    const bool leaf = cur < 0, world = cur >= kTlasNode && cur != kTlasIdle;
     const int nLeaf = __popc(__ballot_sync(kAll, leaf)), nWorld = __popc(__ballot_sync(kAll, world)),
-              nInner = __popc(__ballot_sync(kAll, top > 0 && !leaf && !world));
+              nInner = __popc(__ballot_sync(kAll, !leaf && cur < kTlasNode));
     const bool leafPhase = nLeaf >= nInner && nLeaf >= nWorld, worldPhase = !leafPhase && nWorld > nInner;
-    if (top == 0 || leaf != leafPhase || world != worldPhase) continue;
-    --top;
+    if (cur == kTlasIdle || leaf != leafPhase || world != worldPhase) continue;
+    const int entry = cur;
     bool hit = false;
+    auto pop = [&] { cur = top > 0 ? *tlas_slot(sstack, --top) : kTlasIdle; };
     if (leaf) {
       if (entry != kEmptyChild) {
         const float4 *tp = tris + 3 * (size_t)(~entry);
@@ -143,26 +147,40 @@ __global__ void __launch_bounds__(kTlasBlock, 6) k_tlas_trace(const float4 *__re
           if (leaf_ends(cc)) break;
         }
       }
+      if (kAny && hit) cur = kTlasIdle;
+      else pop();
     } else if (!world) {
-      QNode nd;
-      load_qnode(qnodes, entry, nd);
-      float nearT[4];
-      bool meets[4];
-      qnode_test(nd, qr, tMin, closest, nearT, meets);
-      if (top + 4 > stackSize) {
-        atomicOr(status, (uint32_t)VT_DEV_STACK);
-        top = stackSize - 4;
-      }
-      if (kAny) {  // slot order
+#pragma unroll 1
+      for (int step = 1;; ++step) {
+        QNode nd;
+        load_qnode(qnodes, cur, nd);
+        float nearT[4];
+        bool meets[4];
+        qnode_test(nd, qr, tMin, closest, nearT, meets);
+        if (top + 3 > stackSize) {
+          atomicOr(status, (uint32_t)VT_DEV_STACK);
+          top = stackSize - 3;
+        }
+        if (kAny) {  // slot order
+          int next = kTlasIdle;
 #pragma unroll
-        for (int k = 3; k >= 0; --k)
-          if (meets[k]) *tlas_slot(sstack, top++) = i4(nd.child, k);
-      } else {
-        uint32_t key[4];
-        sort_qchildren(meets, nearT, tMin >= 0.0f, key);
+          for (int k = 3; k >= 0; --k) {
+            if (!meets[k]) continue;
+            if (next != kTlasIdle) *tlas_slot(sstack, top++) = next;
+            next = i4(nd.child, k);
+          }
+          if (next != kTlasIdle) cur = next;
+          else pop();
+        } else {
+          uint32_t key[4];
+          sort_qchildren(meets, nearT, tMin >= 0.0f, key);
 #pragma unroll
-        for (int j = 3; j >= 0; --j)
-          if (key[j] != kMissKey) *tlas_slot(sstack, top++) = pick4(nd.child, key[j] & 3u);
+          for (int j = 3; j >= 1; --j)
+            if (key[j] != kMissKey) *tlas_slot(sstack, top++) = pick4(nd.child, key[j] & 3u);
+          if (key[0] != kMissKey) cur = pick4(nd.child, key[0] & 3u);
+          else pop();
+        }
+        if (cur < 0 || cur >= kTlasNode || step >= kTlasSteps) break;
       }
     } else {
       const float4 r0 = __ldg(rays + 2 * (size_t)rid), r1 = __ldg(rays + 2 * (size_t)rid + 1);
@@ -184,6 +202,7 @@ __global__ void __launch_bounds__(kTlasBlock, 6) k_tlas_trace(const float4 *__re
             else atomicOr(status, (uint32_t)VT_DEV_STACK);
           }
         }
+        pop();
       } else {
         curInst = (uint32_t)(entry & kTlasIndex);
         const TlasInst *I = inst + curInst;
@@ -197,13 +216,12 @@ __global__ void __launch_bounds__(kTlasBlock, 6) k_tlas_trace(const float4 *__re
                     dz = xform_dir(l2, r1.x, r1.y, r1.z);
         wr = make_wray(ox, oy, oz, dx, dy, dz);
         qr = make_qray(ox, oy, oz, dx, dy, dz, __ldg(&I->bound.z));
-        *tlas_slot(sstack, top++) = 0;  // the BLAS root (the popped entry's place)
+        cur = 0;  // the BLAS root
       }
     }
     if (kAny) {
-      if (hit) top = 0;
-      if (top == 0) occ[rid] = hit ? 1 : 0;
-    } else if (top == 0) {
+      if (cur == kTlasIdle) occ[rid] = hit ? 1 : 0;
+    } else if (cur == kTlasIdle) {
       hits[rid] = prim >= 0 ? make_int4(__float_as_int(closest), __float_as_int(hb1), __float_as_int(hb2), prim)
                             : make_int4(0, 0, 0, -1);
       if (instOut) instOut[rid] = prim >= 0 ? hitInst : 0xffffffffu;
