@@ -135,9 +135,9 @@ vt_status vt_trace_any(vt_ctx *ctx, const vt_mesh *mesh, const vt_ray *rays_dev,
                        uint8_t *occluded_dev, void *stream);
 /* The same from HOST arrays: copies in, traces and copies out in pipelined chunks on the context's two
  * streams, then synchronises. Pinned (or registered) buffers are copied directly, 2^22 rays a chunk;
- * ordinary pageable buffers go in chunks of 2^17 to 2^20 rays through the context's pinned staging
- * slots (allocated on first use), filled and drained by up to 8 host threads while the GPU works on
- * other chunks. */
+ * ordinary pageable buffers go through the context's pinned staging memory (allocated on first use):
+ * below 12 MB whole, else in chunks of 2^17 to 2^20 rays, filled and drained by up to 8 host threads
+ * while the GPU works on other chunks. */
 vt_status vt_trace_closest_host(vt_ctx *ctx, const vt_mesh *mesh, const vt_ray *rays, uint32_t n,
                                 vt_hit *hits);
 vt_status vt_trace_any_host(vt_ctx *ctx, const vt_mesh *mesh, const vt_ray *rays, uint32_t n,

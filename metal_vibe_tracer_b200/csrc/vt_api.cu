@@ -3,7 +3,6 @@
 #include <atomic>
 #include <cstring>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -355,11 +354,12 @@ vt_status ensure_stage(vt_ctx *ctx, size_t in_bytes, size_t out_bytes) {
 // as it is filled and its slot is drained. Every wait is for something earlier in that order.
 //
 // Bound: host memory (one core copies, and faults in a new output's pages, at a fraction of the link's
-// rate) and the link. Under kThreadedBytes starting the threads costs more than they save (50,000 rays:
-// 0.61 ms with them, 0.36 without).
-constexpr size_t kThreadedBytes = 4u << 20;
+// rate) and the link. Below these bytes starting the threads costs more than they save: closest hits of
+// 114,544 rays (5.5 MB) 1.29 ms with them and 0.84 without, 180,000 1.14 and 1.12, 250,000 1.17 and 1.44, any hits
+// of 250,000 (8.3 MB) 1.16 and 0.96, 500,000 1.45 and 1.49; an image of 13.5 MB 0.7 and 1.85, of 1.5 MB the same.
+constexpr size_t kThreadedBytes = 4u << 20, kThreadedRayBytes = 12u << 20;
 template <typename In, typename Issue, typename Out>
-vt_status host_pipeline(vt_ctx *ctx, size_t bytes, uint32_t chunks, uint32_t inPieces, uint32_t outPieces, In copyIn, Issue issue, Out copyOut) {
+vt_status host_pipeline(vt_ctx *ctx, bool threads, uint32_t chunks, uint32_t inPieces, uint32_t outPieces, In copyIn, Issue issue, Out copyOut) {
   constexpr uint32_t kMaxWorkers = 8;
   struct Counts {
     std::atomic<uint32_t> in{0}, out{0};
@@ -397,12 +397,12 @@ vt_status host_pipeline(vt_ctx *ctx, size_t bytes, uint32_t chunks, uint32_t inP
     }
   };
   std::thread workers[kMaxWorkers];
-  const uint32_t want = bytes < kThreadedBytes ? 1u : std::min<uint32_t>({kMaxWorkers, std::max(1u, std::thread::hardware_concurrency()), chunks * std::max(inPieces, outPieces)});
+  const uint32_t want = !threads ? 1u : std::min<uint32_t>({kMaxWorkers, std::max(1u, std::thread::hardware_concurrency()), chunks * std::max(inPieces, outPieces)});
   uint32_t started = 0;
   if (want > 1) {
     try {
       for (; started < want; ++started) workers[started] = std::thread(work);
-    } catch (const std::system_error &) {  // no more threads: the ones there are do the work
+    } catch (...) {  // no more threads: the ones there are do the work
     }
   }
   vt_status st = VT_OK;
@@ -441,9 +441,25 @@ bool pageable(const void *p) {
   return a.type == cudaMemoryTypeUnregistered;
 }
 
-// Rays of one chunk of the pageable pipeline: a sixth of the call, so that copies in, traversal and
-// copies out overlap, but at least 128K (a traversal that fills the GPU; fewer bytes than the link's
-// latency is worth) and at most 1M (the slots' pinned memory).
+// A host copy split over a few threads from 8 MB on (a call of one chunk).
+void copy_parallel(void *dst, const void *src, size_t bytes) {
+  const size_t parts = std::min<size_t>(std::max(1u, std::thread::hardware_concurrency()), std::max<size_t>(1, bytes >> 22));
+  const size_t step = (bytes + parts - 1) / parts;
+  std::vector<std::thread> workers;
+  size_t done = step;  // [0, step) is this thread's
+  try {
+    for (; done < bytes; done += step)
+      workers.emplace_back([=] { std::memcpy(static_cast<char *>(dst) + done, static_cast<const char *>(src) + done, std::min(step, bytes - done)); });
+  } catch (...) {  // no more threads
+    std::memcpy(static_cast<char *>(dst) + done, static_cast<const char *>(src) + done, bytes - done);
+  }
+  std::memcpy(dst, src, std::min(step, bytes));
+  for (auto &w : workers) w.join();
+}
+
+// Rays of one chunk of the pageable pipeline with threads: a sixth of the call, so that copies in,
+// traversal and copies out overlap, but at least 128K (a traversal that fills the GPU; fewer bytes than
+// the link's latency is worth) and at most 1M (the slots' pinned memory). Without: the whole call.
 uint32_t stage_chunk(uint32_t n) {
   return std::min(n, std::min(1u << 20, std::max(1u << 17, ((n + 5) / 6 + 1023) & ~1023u)));
 }
@@ -465,7 +481,7 @@ vt_status vt_read_scaled(vt_ctx *ctx, double *dst, const double *src, size_t n, 
   const auto words = [&](uint32_t c) { return std::min(kPiece, n - c * kPiece); };
   const auto slot_of = [&](uint32_t c) { return static_cast<double *>(ctx->h_stage_out) + (c % kStageSlots) * kPiece; };
   return host_pipeline(
-      ctx, n * sizeof(double), (uint32_t)((n + kPiece - 1) / kPiece), 0, 1, [](uint32_t, uint32_t) {},
+      ctx, true, (uint32_t)((n + kPiece - 1) / kPiece), 0, 1, [](uint32_t, uint32_t) {},
       [&](uint32_t c) -> vt_status {
         VT_CUDA(ctx, cudaMemcpyAsync(slot_of(c), src + c * kPiece, words(c) * sizeof(double), cudaMemcpyDeviceToHost, ctx->pipe[0]));
         VT_CUDA(ctx, cudaEventRecord(ctx->stage_out_ev[c % kStageSlots], ctx->pipe[0]));
@@ -493,7 +509,8 @@ static vt_status trace_host(vt_ctx *ctx, const vt_mesh *mesh, const vt_ray *rays
   VT_CUDA(ctx, cudaSetDevice(ctx->device));
   if (n == 0) return VT_OK;
   const bool staged = pageable(rays) || pageable(out);
-  const uint32_t chunk = staged ? stage_chunk(n) : n < kChunk ? n : kChunk;
+  const bool threads = n * (sizeof(vt_ray) + out_stride) >= kThreadedRayBytes;
+  const uint32_t chunk = staged && threads ? stage_chunk(n) : n < kChunk ? n : kChunk;
   st = ensure_chunks(ctx, (size_t)chunk * sizeof(vt_ray), (size_t)chunk * out_stride);
   if (st) return st;
   // The previous user of these buffers may still be in flight on the other stream.
@@ -501,19 +518,21 @@ static vt_status trace_host(vt_ctx *ctx, const vt_mesh *mesh, const vt_ray *rays
   VT_CUDA(ctx, cudaStreamSynchronize(ctx->pipe[1]));
   if (staged) {
     const size_t in_slot = (size_t)chunk * sizeof(vt_ray), out_slot = (size_t)chunk * out_stride;
-    st = ensure_stage(ctx, kStageSlots * in_slot, kStageSlots * out_slot);
+    const uint32_t slots = threads ? kStageSlots : 1u;
+    st = ensure_stage(ctx, slots * in_slot, slots * out_slot);
     if (st) return st;
-    const uint32_t in_pieces = (uint32_t)((in_slot + kStagePiece - 1) / kStagePiece), out_pieces = (uint32_t)((out_slot + kStagePiece - 1) / kStagePiece);
+    const size_t in_size = threads ? kStagePiece : in_slot, out_size = threads ? kStagePiece : out_slot;
+    const uint32_t in_pieces = (uint32_t)((in_slot + in_size - 1) / in_size), out_pieces = (uint32_t)((out_slot + out_size - 1) / out_size);
     const auto rays_of = [&](uint32_t c) { return std::min(chunk, n - c * chunk); };
-    const auto copy_piece = [](char *dst, const char *src, size_t bytes, uint32_t piece) {
-      const size_t at = std::min(bytes, (size_t)piece * kStagePiece);
-      std::memcpy(dst + at, src + at, std::min(bytes - at, kStagePiece));
+    const auto copy_piece = [](char *dst, const char *src, size_t bytes, uint32_t piece, size_t size) {
+      const size_t at = std::min(bytes, piece * size);
+      copy_parallel(dst + at, src + at, std::min(bytes - at, size));
     };
     return host_pipeline(
-        ctx, n * (sizeof(vt_ray) + out_stride), (n + chunk - 1) / chunk, in_pieces, out_pieces,
+        ctx, threads, (n + chunk - 1) / chunk, in_pieces, out_pieces,
         [&](uint32_t c, uint32_t piece) {
           copy_piece(static_cast<char *>(ctx->h_stage_in) + (c % kStageSlots) * in_slot,
-                     reinterpret_cast<const char *>(rays + (size_t)c * chunk), rays_of(c) * sizeof(vt_ray), piece);
+                     reinterpret_cast<const char *>(rays + (size_t)c * chunk), rays_of(c) * sizeof(vt_ray), piece, in_size);
         },
         [&](uint32_t c) -> vt_status {
           const int k = c & 1;
@@ -531,7 +550,7 @@ static vt_status trace_host(vt_ctx *ctx, const vt_mesh *mesh, const vt_ray *rays
         },
         [&](uint32_t c, uint32_t piece) {
           copy_piece(static_cast<char *>(out) + (size_t)c * chunk * out_stride, static_cast<const char *>(ctx->h_stage_out) + (c % kStageSlots) * out_slot,
-                     rays_of(c) * out_stride, piece);
+                     rays_of(c) * out_stride, piece, out_size);
         });
   }
   for (uint32_t c = 0, first = 0; first < n; ++c, first += chunk) {

@@ -192,7 +192,7 @@ def test_few_rays_equal_a_large_batch(ctx, n):
     assert np.array_equal(gpu_any(mesh, rays[:n]), gpu_any(mesh, rays)[:n])
 
 
-@pytest.mark.parametrize("n", [87_381, 87_382, 131_071, 131_073, 786_433, 1_500_001])
+@pytest.mark.parametrize("n", [131_073, 262_143, 262_145, 381_300, 381_301, 786_433, 1_500_001])
 def test_host_chunks(ctx, n):
     """Ordinary host arrays around the sizes where threads start and chunks end, against device arrays."""
     faces, verts = scenes.triangle_soup(3000, seed=2, mu=math.log(0.03))
