@@ -2133,12 +2133,18 @@ __global__ void __launch_bounds__(kWfBlock) k_wf_finish(RenderArgs A, WfArgs W) 
 // (six blocks an SM): the spills cost less than the walks' latency without the warps. Measured on one
 // B200, four 1001 x 563 frames with 16 candidates: 154 registers 19.4 ms, 121 18.6, 96 17.0, 80 16.3-17.0,
 // 64 16.4.
-template <bool kPbr>
-__global__ void __launch_bounds__(kRenderBlock, 6) k_di_primary(RenderArgs A, WfArgs W) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+//
+// A band of at most one pixel per thread of 4 blocks an SM (kFew) runs unspilled at 128 registers, `lanes`
+// pixels to a warp so that all of them fit at once: nothing waits for a block's slot, and a warp
+// diverges over fewer walks. Measured on one B200, four frames at depth 8: 100 x 64 5.83 -> 5.48 ms, 264 x 171
+// 7.51 -> 7.27.
+template <bool kPbr, bool kFew>
+__global__ void __launch_bounds__(kRenderBlock, kFew ? 4 : 6) k_di_primary(RenderArgs A, WfArgs W, uint32_t lanes) {
+  const unsigned lane = threadIdx.x & 31u;
+  const uint32_t i = kFew ? (blockIdx.x * (kRenderBlock / 32) + (threadIdx.x >> 5)) * lanes + lane : blockIdx.x * kRenderBlock + threadIdx.x;
   bool push = false;
   [&] {  // one pixel; every lane joins the queue push below
-    if (i >= W.paths) return;
+    if (i >= W.paths || (kFew && lane >= lanes)) return;
     const uint32_t p = W.p0 + i, k = W.k0, x = p % A.W, y = p / A.W;
     Sampler seed = pixel_sampler(x, y, A.W, A.first + k, A.zSampler != 0u, A.zModel, A.firstFrame + k);
     const float u = A.spectral ? wavelength_numbers(seed).x : 0.0f;
@@ -2222,7 +2228,7 @@ __global__ void __launch_bounds__(kRenderBlock, 6) k_di_primary(RenderArgs A, Wf
     wf_store_seed(W, i, seed);
   }();
   // Pushed per warp: a block's warps end far apart, and waiting for the last cost 2 % of a frame.
-  const unsigned lane = threadIdx.x & 31u, pushes = __ballot_sync(0xffffffffu, push);
+  const unsigned pushes = __ballot_sync(0xffffffffu, push);
   uint32_t base = 0;
   if (lane == 0 && pushes) base = atomicAdd(W.outCount, (uint32_t)__popc(pushes));
   base = __shfl_sync(0xffffffffu, base, 0);
@@ -3547,8 +3553,15 @@ vt_status di_reservoirs(const WfStages &S, const RenderArgs &A, WfArgs W) {
   vt_launch_closest(S.mesh, ray, P, hit, ctx->sm_count, S.word(0, kWfExtendHead), nullptr, ctx->d_status + 1, s, nullptr, true, true);
   W.outQ = S.B.q[1];
   W.outCount = S.word(1, kWfLive);
-  if (S.pbr) k_di_primary<true><<<pixels, kRenderBlock, 0, s>>>(A, W);
-  else k_di_primary<false><<<pixels, kRenderBlock, 0, s>>>(A, W);
+  const uint32_t warps = (uint32_t)ctx->sm_count * 16u, lanes = (P + warps - 1u) / warps;
+  if (lanes <= 32u) {
+    const uint32_t blocks = (P + lanes * (kRenderBlock / 32) - 1u) / (lanes * (kRenderBlock / 32));
+    if (S.pbr) k_di_primary<true, true><<<blocks, kRenderBlock, 0, s>>>(A, W, lanes);
+    else k_di_primary<false, true><<<blocks, kRenderBlock, 0, s>>>(A, W, lanes);
+  } else {
+    if (S.pbr) k_di_primary<true, false><<<pixels, kRenderBlock, 0, s>>>(A, W, 32u);
+    else k_di_primary<false, false><<<pixels, kRenderBlock, 0, s>>>(A, W, 32u);
+  }
   if (A.maxDepth > 1u) {
     vt_launch_closest(S.mesh, ray, P, hit, ctx->sm_count, S.word(1, kWfExtendHead), S.B.q[1], ctx->d_status + 1, s, W.outCount, true, true);
     W.inQ = S.B.q[1];
@@ -3685,7 +3698,10 @@ vt_status render_impl(vt_ctx *ctx, vt_scene *scene, const vt_frame_params *p, ui
     W.npix = npix;
     W.deadFlags = 0u;
     A.kernelId = nrc ? 5u : 4u;
-    const WfStages S = wf_stages(ctx, scene, A, B, kWfBlock, 1u, nrc != nullptr, s);
+    // Blocks of two warps where the band is small: they spread evenly over the SMs (264 x 171: 7.24 -> 7.16 ms for
+    // four frames; large bands want whole blocks in the same code, k_wf_shade).
+    const int stageBlock = band <= (uint32_t)ctx->sm_count * 512u ? 64 : kWfBlock;
+    const WfStages S = wf_stages(ctx, scene, A, B, stageBlock, 1u, nrc != nullptr, s);
     for (uint32_t k = 0; k < spp; ++k) {
       float4 *cur = base + 9 * (size_t)npix * scene->di_parity, *prev = base + 9 * (size_t)npix * (scene->di_parity ^ 1u);
       A.gPos = cur; A.gNrm = cur + npix; A.rPos = cur + 2 * (size_t)npix; A.rEmit = cur + 3 * (size_t)npix;
