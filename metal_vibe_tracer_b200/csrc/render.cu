@@ -4439,33 +4439,6 @@ vt_status vt_scene_gi_weights(vt_ctx *ctx, const vt_scene *scene, float *out, ui
   return VT_OK;
 }
 
-vt_status vt_accum_readback(vt_ctx *ctx, vt_scene *scene, double *rgb, uint32_t n, uint32_t *samples) {
-  if (!ctx) return VT_ERR_INVALID;
-  if (!scene || !rgb) return vt_fail(ctx, VT_ERR_INVALID, "scene or rgb is null");
-  const size_t want = 3 * (size_t)scene->width * scene->height;
-  if (n != want) return vt_fail(ctx, VT_ERR_INVALID, "n must equal width * height * 3");
-  VT_CUDA(ctx, cudaDeviceSynchronize());
-  {
-    uint32_t w[16];
-    VT_CUDA(ctx, cudaMemcpy(w, ctx->d_status, sizeof w, cudaMemcpyDeviceToHost));
-    if (w[1] & VT_DEV_STACK) {
-      VT_CUDA(ctx, cudaMemset(ctx->d_status + 1, 0, sizeof(uint32_t)));
-      return vt_fail(ctx, VT_ERR_DEVICE, "a traversal stack would have overflowed; the entries were dropped");
-    }
-    if (w[2]) {
-      VT_CUDA(ctx, cudaMemset(ctx->d_status + 2, 0, sizeof(uint32_t)));
-      VT_CUDA(ctx, cudaMemset(ctx->d_status + 8, 0, 3 * sizeof(uint32_t)));
-      return vt_fail(ctx, VT_ERR_DEVICE,
-                     "the integrator met an out-of-range index (status " + std::to_string(w[2]) +
-                         ": 4 hit, 8 cache record, 16 emitter face; first: value " + std::to_string(w[9]) +
-                         ", kernel " + std::to_string(w[10] & 0xffu) + "); those accesses were clamped or skipped");
-    }
-  }
-  if (vt_status st = vt_read_scaled(ctx, rgb, scene->d_accum, want, scene->samples ? 1.0 / scene->samples : 0.0)) return st;
-  if (samples) *samples = scene->samples;
-  return VT_OK;
-}
-
 vt_status vt_accum_restore(vt_ctx *ctx, vt_scene *scene, uint32_t width, uint32_t height, uint32_t pixel_stride,
                            const double *rgb, uint32_t n, uint32_t samples) {
   if (!ctx) return VT_ERR_INVALID;

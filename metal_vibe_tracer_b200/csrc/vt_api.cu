@@ -464,13 +464,11 @@ uint32_t stage_chunk(uint32_t n) {
   return std::min(n, std::min(1u << 20, std::max(1u << 17, ((n + 5) / 6 + 1023) & ~1023u)));
 }
 
-}  // namespace
-
-// dst = src x scale for n doubles on the device, to host memory; the device is idle. Pageable memory
+// dst = src x scale for n doubles on the device, to host memory; the device is idle and current. Pageable memory
 // goes through the staging slots, scaled by the threads that drain them. Measured on one B200: the
 // 50 MB of a 1920 x 1080 image 14.5 -> 3.6 ms, the 13.5 MB of 1001 x 563 1.85 -> 0.7 (one copy into the
 // caller's pages by the driver, then a scaling pass by one core).
-vt_status vt_read_scaled(vt_ctx *ctx, double *dst, const double *src, size_t n, double scale) {
+vt_status read_scaled(vt_ctx *ctx, double *dst, const double *src, size_t n, double scale) {
   constexpr size_t kPiece = kStagePiece / sizeof(double);
   if (n * sizeof(double) < kThreadedBytes || !pageable(dst)) {
     if (n) VT_CUDA(ctx, cudaMemcpy(dst, src, n * sizeof(double), cudaMemcpyDeviceToHost));
@@ -493,6 +491,8 @@ vt_status vt_read_scaled(vt_ctx *ctx, double *dst, const double *src, size_t n, 
         for (size_t i = 0, m = words(c); i < m; ++i) to[i] = from[i] * scale;
       });
 }
+
+}  // namespace
 
 extern "C" {
 
@@ -578,6 +578,36 @@ vt_status vt_trace_closest_host(vt_ctx *ctx, const vt_mesh *mesh, const vt_ray *
 vt_status vt_trace_any_host(vt_ctx *ctx, const vt_mesh *mesh, const vt_ray *rays, uint32_t n,
                             uint8_t *occluded) {
   return trace_host(ctx, mesh, rays, n, occluded, 1, false);
+}
+
+vt_status vt_accum_readback(vt_ctx *ctx, vt_scene *scene, double *rgb, uint32_t n, uint32_t *samples) {
+  if (!ctx) return VT_ERR_INVALID;
+  if (!scene || !rgb) return vt_fail(ctx, VT_ERR_INVALID, "scene or rgb is null");
+  const size_t want = 3 * (size_t)scene->width * scene->height;
+  if (n != want) return vt_fail(ctx, VT_ERR_INVALID, "n must equal width * height * 3");
+  // The synchronisation and the staging events below are the current device's, which another context's
+  // call may have left elsewhere.
+  VT_CUDA(ctx, cudaSetDevice(ctx->device));
+  VT_CUDA(ctx, cudaDeviceSynchronize());
+  {
+    uint32_t w[16];
+    VT_CUDA(ctx, cudaMemcpy(w, ctx->d_status, sizeof w, cudaMemcpyDeviceToHost));
+    if (w[1] & VT_DEV_STACK) {
+      VT_CUDA(ctx, cudaMemset(ctx->d_status + 1, 0, sizeof(uint32_t)));
+      return vt_fail(ctx, VT_ERR_DEVICE, "a traversal stack would have overflowed; the entries were dropped");
+    }
+    if (w[2]) {
+      VT_CUDA(ctx, cudaMemset(ctx->d_status + 2, 0, sizeof(uint32_t)));
+      VT_CUDA(ctx, cudaMemset(ctx->d_status + 8, 0, 3 * sizeof(uint32_t)));
+      return vt_fail(ctx, VT_ERR_DEVICE,
+                     "the integrator met an out-of-range index (status " + std::to_string(w[2]) +
+                         ": 4 hit, 8 cache record, 16 emitter face; first: value " + std::to_string(w[9]) +
+                         ", kernel " + std::to_string(w[10] & 0xffu) + "); those accesses were clamped or skipped");
+    }
+  }
+  if (vt_status st = read_scaled(ctx, rgb, scene->d_accum, want, scene->samples ? 1.0 / scene->samples : 0.0)) return st;
+  if (samples) *samples = scene->samples;
+  return VT_OK;
 }
 
 vt_status vt_trace_count(vt_ctx *ctx, const vt_mesh *mesh, const vt_ray *rays_dev, uint32_t n,

@@ -211,8 +211,6 @@ __device__ __forceinline__ uint32_t vt_poll(const uint32_t *p) {
 // stream has been synchronised).
 constexpr size_t kPoolKeep = size_t(1) << 30;
 cudaError_t vt_pool_alloc(vt_ctx *ctx, void **p, size_t bytes);
-// n doubles from the device, times scale, into host memory (the device is idle; returns when done).
-vt_status vt_read_scaled(vt_ctx *ctx, double *dst, const double *src, size_t n, double scale);
 
 // Stable LSD radix sort of (key, value) pairs on the low `bits` bits of the keys.
 // keys/vals are sorted in place using the alternate buffers; temp is vt_radix_temp_words(n). n below
