@@ -1993,24 +1993,25 @@ __device__ __forceinline__ void wf_vertex(const RenderArgs &A, const WfArgs &W, 
 // The pass's paths: sampler, wavelengths and camera ray (path_sample_body's draws before the trace;
 // the shading seed's rehash needs no hit, so it happens here too); path i is sample k0 + i / npix
 // of accumulation pixel i % npix.
+__device__ __forceinline__ void wf_generate(const RenderArgs &A, const WfArgs &W, uint32_t i) {
+  const uint32_t p = W.p0 + i % W.npix, k = W.k0 + i / W.npix;
+  const uint32_t x = (p % A.OW) * A.stride, y = (p / A.OW) * A.stride;
+  Sampler seed = pixel_sampler(x, y, A.W, A.first + k, A.zSampler != 0u, A.zModel, A.firstFrame + k);
+  const float u = A.spectral ? wavelength_numbers(seed).x : 0.0f;
+  float3 dir0 = camera_dir(A, x, y, A.jitter ? A.jitter[k] : frame_jitter(A.first + k)), o0 = A.cam;
+  lens_ray(A, o0, dir0, seed);
+  seed.state = pcg_hash(seed.state ^ 0x27d4eb2fu);  // decorrelate_shading_seed
+  wf_set_ray(W.ray, i, o0, ray_tmin(A, o0), dir0, __int_as_float(0x7f800000));
+  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  W.T[i] = zero;
+  W.Rc[i] = zero;
+  W.Rp[i] = zero;
+  W.prevN[i] = make_float4(0.0f, 0.0f, 0.0f, u);
+  W.meta[i] = make_uint4(p, 0u, 0u, 0u);
+  wf_store_seed(W, i, seed);
+}
 __global__ void __launch_bounds__(kWfBlock) k_wf_generate(RenderArgs A, WfArgs W) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < W.paths; i += gridDim.x * blockDim.x) {
-    const uint32_t p = W.p0 + i % W.npix, k = W.k0 + i / W.npix;
-    const uint32_t x = (p % A.OW) * A.stride, y = (p / A.OW) * A.stride;
-    Sampler seed = pixel_sampler(x, y, A.W, A.first + k, A.zSampler != 0u, A.zModel, A.firstFrame + k);
-    const float u = A.spectral ? wavelength_numbers(seed).x : 0.0f;
-    float3 dir0 = camera_dir(A, x, y, A.jitter ? A.jitter[k] : frame_jitter(A.first + k)), o0 = A.cam;
-    lens_ray(A, o0, dir0, seed);
-    seed.state = pcg_hash(seed.state ^ 0x27d4eb2fu);  // decorrelate_shading_seed
-    wf_set_ray(W.ray, i, o0, ray_tmin(A, o0), dir0, __int_as_float(0x7f800000));
-    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    W.T[i] = zero;
-    W.Rc[i] = zero;
-    W.Rp[i] = zero;
-    W.prevN[i] = make_float4(0.0f, 0.0f, 0.0f, u);
-    W.meta[i] = make_uint4(p, 0u, 0u, 0u);
-    wf_store_seed(W, i, seed);
-  }
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < W.paths; i += gridDim.x * blockDim.x) wf_generate(A, W, i);
 }
 
 // Two blocks of kWfBlock per SM (at most 128 registers): the OpenPBR variant's register demand
@@ -2085,23 +2086,25 @@ __global__ void __launch_bounds__(kWfBlock, 4) k_wf_light(RenderArgs A, WfArgs W
 // continuation, in k_render's order, non-finite sums dropped. kNrc: a path without a query clears its
 // slot's throughput (the resolve skips it).
 template <bool kNrc>
-__global__ void __launch_bounds__(kWfBlock) k_wf_finish(RenderArgs A, WfArgs W) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < W.paths; i += gridDim.x * blockDim.x) {
-    const uint4 meta = W.meta[i];
-    if (kNrc && !(meta.w & kWfQueried)) nrc_store_none(A, wf_slot(W, i));
-    float4 Rc = W.Rc[i], Rp = W.Rp[i];
-    if ((meta.w & kWfShadow) && !W.occ[i]) {
-      const float4 c = W.scon[i];
-      if (meta.w & kWfShadowPrimary) Rp = make_float4(Rp.x + c.x, Rp.y + c.y, Rp.z + c.z, 0.0f);
-      else Rc = make_float4(Rc.x + c.x, Rc.y + c.y, Rc.z + c.z, 0.0f);
-    }
-    const float3 R = add(f3(Rp.x, Rp.y, Rp.z), f3(Rc.x, Rc.y, Rc.z));
-    if (!isfinite(R.x) || !isfinite(R.y) || !isfinite(R.z)) continue;
-    double *acc = A.accum + 3 * (size_t)meta.x;
-    atomicAdd(acc, (double)R.x);
-    atomicAdd(acc + 1, (double)R.y);
-    atomicAdd(acc + 2, (double)R.z);
+__device__ __forceinline__ void wf_finish(const RenderArgs &A, const WfArgs &W, uint32_t i) {
+  const uint4 meta = W.meta[i];
+  if (kNrc && !(meta.w & kWfQueried)) nrc_store_none(A, wf_slot(W, i));
+  float4 Rc = W.Rc[i], Rp = W.Rp[i];
+  if ((meta.w & kWfShadow) && !W.occ[i]) {
+    const float4 c = W.scon[i];
+    if (meta.w & kWfShadowPrimary) Rp = make_float4(Rp.x + c.x, Rp.y + c.y, Rp.z + c.z, 0.0f);
+    else Rc = make_float4(Rc.x + c.x, Rc.y + c.y, Rc.z + c.z, 0.0f);
   }
+  const float3 R = add(f3(Rp.x, Rp.y, Rp.z), f3(Rc.x, Rc.y, Rc.z));
+  if (!isfinite(R.x) || !isfinite(R.y) || !isfinite(R.z)) return;
+  double *acc = A.accum + 3 * (size_t)meta.x;
+  atomicAdd(acc, (double)R.x);
+  atomicAdd(acc + 1, (double)R.y);
+  atomicAdd(acc + 2, (double)R.z);
+}
+template <bool kNrc>
+__global__ void __launch_bounds__(kWfBlock) k_wf_finish(RenderArgs A, WfArgs W) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < W.paths; i += gridDim.x * blockDim.x) wf_finish<kNrc>(A, W, i);
 }
 
 // ---- ReSTIR frames through the wavefront stages (sampling mode 0) ---------------------------------
@@ -2115,6 +2118,7 @@ __global__ void __launch_bounds__(kWfBlock) k_wf_finish(RenderArgs A, WfArgs W) 
 //                              first continuation; shadow (NEE or DI sample, GI connection);
 //   k_gi_connect               adds the visible GI connections;
 //   extend, k_wf_shade, shadow per bounce from 1, then k_wf_finish, as for the other modes.
+// Small frames take the same parts in two launches (k_di_small_reservoirs).
 // Bound: latency and divergence of the stages, as the other modes'. One kernel per pass with
 // inline traversals (a thread per pixel, local-memory stacks) idled most lanes in its longest path.
 // Measured on one B200: four 1001 x 563 frames of a 300,000-triangle scene at depth 6 with 16
@@ -2129,6 +2133,91 @@ __global__ void __launch_bounds__(kWfBlock) k_wf_finish(RenderArgs A, WfArgs W) 
 // BSDF sample). Other primaries get empty reservoirs and shade with NEE (main.swift:4931-4943).
 // Leaves the camera ray's direction and wavelength number in W.T, the BSDF pdf in W.prev.w, the
 // sampler in W.seedA/B.
+__device__ __forceinline__ bool di_primary(const RenderArgs &A, const WfArgs &W, uint32_t i) {
+  const uint32_t p = W.p0 + i, k = W.k0, x = p % A.W, y = p / A.W;
+  Sampler seed = pixel_sampler(x, y, A.W, A.first + k, A.zSampler != 0u, A.zModel, A.firstFrame + k);
+  const float u = A.spectral ? wavelength_numbers(seed).x : 0.0f;
+  float3 dir0 = camera_dir(A, x, y, A.jitter[k]), o0 = A.cam;
+  lens_ray(A, o0, dir0, seed);
+  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  const int4 h4 = W.hit[i];
+  Hit h;
+  h.t = __int_as_float(h4.x); h.b1 = __int_as_float(h4.y); h.b2 = __int_as_float(h4.z); h.pos = h4.w;
+  if (h.pos < 0) {
+    A.gPos[p] = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
+    A.gNrm[p] = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
+    A.rPos[p] = zero; A.rEmit[p] = zero; A.rW[p] = zero;
+    A.giPos[p] = zero; A.giNrm[p] = zero; A.giRad[p] = zero; A.giW[p] = zero;
+    return false;
+  }
+  const Surface S = surface_at(A, h, o0, dir0);
+  const vt_material m = material(A, S.slot);
+  const float4 gp = make_float4(S.pos.x, S.pos.y, S.pos.z, h.t), gn = make_float4(S.n.x, S.n.y, S.n.z, float(m.type));
+  A.gPos[p] = gp;
+  A.gNrm[p] = gn;
+  A.gGeo[p] = make_float4(S.gn.x, S.gn.y, S.gn.z, 0.0f);
+  A.gInfo[p] = make_uint4(S.face, S.slot | (S.front ? 0x80000000u : 0u), __float_as_uint(S.err), S.tri);
+  // The GI reservoir is empty until k_gi_secondary and k_gi_merge fill it (depth 1 has no indirect
+  // bounce for it, restir_gi_enabled, main.swift:3476-3478).
+  A.giPos[p] = zero; A.giNrm[p] = zero; A.giRad[p] = zero; A.giW[p] = zero;
+  if (m.type != VT_MAT_DIFFUSE) {
+    A.rPos[p] = zero; A.rEmit[p] = zero; A.rW[p] = zero;
+    return false;
+  }
+  DIReservoir r;
+  r.s.pos = f3(0.0f, 0.0f, 0.0f); r.s.emission = f3(0.0f, 0.0f, 0.0f);
+  r.s.pdf = 0.0f; r.s.u = u; r.s.id = 0u;
+  r.wsum = 0.0f;
+  r.M = 0.0f;
+  for (uint32_t c = 0; c < A.diCandidates; ++c) {
+    sampler_candidate(seed, 1u, kZDi, c, A.diBits);
+    const LightSample ls = sample_direct(A, S.pos, S.n, seed, (int)A.maxDepth - 1 > 0);
+    r.M += 1.0f;  // zero-weight candidates still count
+    if (!(ls.pdf > 0.0f)) continue;
+    DISample cand;
+    cand.pos = ls.pos; cand.emission = ls.emission; cand.pdf = ls.pdf; cand.u = u;
+    cand.id = ls.face == 0xffffffffu ? 0u : ls.face + 2u;
+    const float pHat = di_target(A, S.pos, S.n, S.gn, dir0, m, cand);
+    const float proposal = cand.pdf * light_geometry(A, S.pos, cand);
+    const float w = proposal > 0.0f ? pHat / proposal : 0.0f;
+    r.wsum += w;
+    if (rand_decision(seed) * r.wsum < w) r.s = cand;
+  }
+  int px, py;
+  if (backproject(A, S.pos, px, py)) {
+    const uint32_t j = (uint32_t)py * A.W + (uint32_t)px;
+    const float4 hw = A.hrW[j];
+    if (same_surface(gp, gn, A.hPos[j], A.hNrm[j]) && hw.y > 0.0f && hw.z > 0.0f) {
+      const DISample hs = load_di(A.hrPos, A.hrEmit, A.hrW, j);
+      const float cM = fminf(hw.y, 20.0f);
+      const float w = di_target(A, S.pos, S.n, S.gn, dir0, m, hs) * hw.z * cM;
+      r.M += cM;
+      r.wsum += w;
+      if (rand_decision(seed) * r.wsum < w) r.s = hs;
+    }
+  }
+  const float pHat = di_target(A, S.pos, S.n, S.gn, dir0, m, r.s);
+  const float Wr = r.M > 0.0f && pHat > 0.0f ? r.wsum / (r.M * pHat) : 0.0f;
+  A.rPos[p] = make_float4(r.s.pos.x, r.s.pos.y, r.s.pos.z, __uint_as_float(r.s.id));
+  A.rEmit[p] = make_float4(r.s.emission.x, r.s.emission.y, r.s.emission.z, r.s.pdf);
+  A.rW[p] = make_float4(r.wsum, r.M, Wr, r.s.u);
+  if ((int)A.maxDepth - 1 < 1) return false;
+  sampler_event(seed, 1u, kZGiBsdf);
+  const float3 rr = rand_f3(seed);  // sample_bsdf's Lambert branch: the direction from the last two
+  const float3 gd = cosine_hemisphere(S.n, rr.y, rr.z);
+  const float bpdf = fmaxf(0.0f, dot3(S.n, gd)) * kInvPi;
+  const bool push = bpdf > 0.0f && dot3(gd, S.gn) > 0.0f;
+  if (push) {
+    const float3 o = ray_origin(A, S.pos, S.gn, gd, S.err);
+    wf_set_ray(W.ray, i, o, ray_tmin(A, o), gd, __int_as_float(0x7f800000));
+  }
+  W.T[i] = make_float4(dir0.x, dir0.y, dir0.z, u);
+  W.prev[i] = make_float4(0.0f, 0.0f, 0.0f, bpdf);
+  W.meta[i] = make_uint4(p, 0u, 0u, 0u);
+  wf_store_seed(W, i, seed);
+  return push;
+}
+
 // Bound: the dependent loads and the issue of one light-tree walk after another. Held to 80 registers
 // (six blocks an SM): the spills cost less than the walks' latency without the warps. Measured on one
 // B200, four 1001 x 563 frames with 16 candidates: 154 registers 19.4 ms, 121 18.6, 96 17.0, 80 16.3-17.0,
@@ -2136,97 +2225,14 @@ __global__ void __launch_bounds__(kWfBlock) k_wf_finish(RenderArgs A, WfArgs W) 
 //
 // A band of at most one pixel per thread of 4 blocks an SM (kFew) runs unspilled at 128 registers, `lanes`
 // pixels to a warp so that all of them fit at once: nothing waits for a block's slot, and a warp
-// diverges over fewer walks. Measured on one B200, four frames at depth 8: 100 x 64 5.83 -> 5.48 ms, 264 x 171
-// 7.51 -> 7.27.
+// diverges over fewer walks. Measured on one B200, a frame of 300,000 triangles, a third of its slots OPENPBR, at
+// depth 3: 191 x 150 1165 -> 1109 us, 264 x 171 1216 -> 1181.
 template <bool kPbr, bool kFew>
 __global__ void __launch_bounds__(kRenderBlock, kFew ? 4 : 6) k_di_primary(RenderArgs A, WfArgs W, uint32_t lanes) {
   const unsigned lane = threadIdx.x & 31u;
   const uint32_t i = kFew ? (blockIdx.x * (kRenderBlock / 32) + (threadIdx.x >> 5)) * lanes + lane : blockIdx.x * kRenderBlock + threadIdx.x;
   bool push = false;
-  [&] {  // one pixel; every lane joins the queue push below
-    if (i >= W.paths || (kFew && lane >= lanes)) return;
-    const uint32_t p = W.p0 + i, k = W.k0, x = p % A.W, y = p / A.W;
-    Sampler seed = pixel_sampler(x, y, A.W, A.first + k, A.zSampler != 0u, A.zModel, A.firstFrame + k);
-    const float u = A.spectral ? wavelength_numbers(seed).x : 0.0f;
-    float3 dir0 = camera_dir(A, x, y, A.jitter[k]), o0 = A.cam;
-    lens_ray(A, o0, dir0, seed);
-    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    const int4 h4 = W.hit[i];
-    Hit h;
-    h.t = __int_as_float(h4.x); h.b1 = __int_as_float(h4.y); h.b2 = __int_as_float(h4.z); h.pos = h4.w;
-    if (h.pos < 0) {
-      A.gPos[p] = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
-      A.gNrm[p] = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
-      A.rPos[p] = zero; A.rEmit[p] = zero; A.rW[p] = zero;
-      A.giPos[p] = zero; A.giNrm[p] = zero; A.giRad[p] = zero; A.giW[p] = zero;
-      return;
-    }
-    const Surface S = surface_at(A, h, o0, dir0);
-    const vt_material m = material(A, S.slot);
-    const float4 gp = make_float4(S.pos.x, S.pos.y, S.pos.z, h.t), gn = make_float4(S.n.x, S.n.y, S.n.z, float(m.type));
-    A.gPos[p] = gp;
-    A.gNrm[p] = gn;
-    A.gGeo[p] = make_float4(S.gn.x, S.gn.y, S.gn.z, 0.0f);
-    A.gInfo[p] = make_uint4(S.face, S.slot | (S.front ? 0x80000000u : 0u), __float_as_uint(S.err), S.tri);
-    // The GI reservoir is empty until k_gi_secondary and k_gi_merge fill it (depth 1 has no indirect
-    // bounce for it, restir_gi_enabled, main.swift:3476-3478).
-    A.giPos[p] = zero; A.giNrm[p] = zero; A.giRad[p] = zero; A.giW[p] = zero;
-    if (m.type != VT_MAT_DIFFUSE) {
-      A.rPos[p] = zero; A.rEmit[p] = zero; A.rW[p] = zero;
-      return;
-    }
-    DIReservoir r;
-    r.s.pos = f3(0.0f, 0.0f, 0.0f); r.s.emission = f3(0.0f, 0.0f, 0.0f);
-    r.s.pdf = 0.0f; r.s.u = u; r.s.id = 0u;
-    r.wsum = 0.0f;
-    r.M = 0.0f;
-    for (uint32_t c = 0; c < A.diCandidates; ++c) {
-      sampler_candidate(seed, 1u, kZDi, c, A.diBits);
-      const LightSample ls = sample_direct(A, S.pos, S.n, seed, (int)A.maxDepth - 1 > 0);
-      r.M += 1.0f;  // zero-weight candidates still count
-      if (!(ls.pdf > 0.0f)) continue;
-      DISample cand;
-      cand.pos = ls.pos; cand.emission = ls.emission; cand.pdf = ls.pdf; cand.u = u;
-      cand.id = ls.face == 0xffffffffu ? 0u : ls.face + 2u;
-      const float pHat = di_target(A, S.pos, S.n, S.gn, dir0, m, cand);
-      const float proposal = cand.pdf * light_geometry(A, S.pos, cand);
-      const float w = proposal > 0.0f ? pHat / proposal : 0.0f;
-      r.wsum += w;
-      if (rand_decision(seed) * r.wsum < w) r.s = cand;
-    }
-    int px, py;
-    if (backproject(A, S.pos, px, py)) {
-      const uint32_t j = (uint32_t)py * A.W + (uint32_t)px;
-      const float4 hw = A.hrW[j];
-      if (same_surface(gp, gn, A.hPos[j], A.hNrm[j]) && hw.y > 0.0f && hw.z > 0.0f) {
-        const DISample hs = load_di(A.hrPos, A.hrEmit, A.hrW, j);
-        const float cM = fminf(hw.y, 20.0f);
-        const float w = di_target(A, S.pos, S.n, S.gn, dir0, m, hs) * hw.z * cM;
-        r.M += cM;
-        r.wsum += w;
-        if (rand_decision(seed) * r.wsum < w) r.s = hs;
-      }
-    }
-    const float pHat = di_target(A, S.pos, S.n, S.gn, dir0, m, r.s);
-    const float Wr = r.M > 0.0f && pHat > 0.0f ? r.wsum / (r.M * pHat) : 0.0f;
-    A.rPos[p] = make_float4(r.s.pos.x, r.s.pos.y, r.s.pos.z, __uint_as_float(r.s.id));
-    A.rEmit[p] = make_float4(r.s.emission.x, r.s.emission.y, r.s.emission.z, r.s.pdf);
-    A.rW[p] = make_float4(r.wsum, r.M, Wr, r.s.u);
-    if ((int)A.maxDepth - 1 < 1) return;
-    sampler_event(seed, 1u, kZGiBsdf);
-    const float3 rr = rand_f3(seed);  // sample_bsdf's Lambert branch: the direction from the last two
-    const float3 gd = cosine_hemisphere(S.n, rr.y, rr.z);
-    const float bpdf = fmaxf(0.0f, dot3(S.n, gd)) * kInvPi;
-    push = bpdf > 0.0f && dot3(gd, S.gn) > 0.0f;
-    if (push) {
-      const float3 o = ray_origin(A, S.pos, S.gn, gd, S.err);
-      wf_set_ray(W.ray, i, o, ray_tmin(A, o), gd, __int_as_float(0x7f800000));
-    }
-    W.T[i] = make_float4(dir0.x, dir0.y, dir0.z, u);
-    W.prev[i] = make_float4(0.0f, 0.0f, 0.0f, bpdf);
-    W.meta[i] = make_uint4(p, 0u, 0u, 0u);
-    wf_store_seed(W, i, seed);
-  }();
+  if (i < W.paths && (!kFew || lane < lanes)) push = di_primary(A, W, i);
   // Pushed per warp: a block's warps end far apart, and waiting for the last cost 2 % of a frame.
   const unsigned pushes = __ballot_sync(0xffffffffu, push);
   uint32_t base = 0;
@@ -2238,6 +2244,53 @@ __global__ void __launch_bounds__(kRenderBlock, kFew ? 4 : 6) k_di_primary(Rende
 // restir_gi_initial (main.swift:4718-4770) at the candidate's hit x2 (diffuse, or there is no
 // candidate): position, normal, source pdf and the radiance of one NEE sample, its visibility
 // pending (kWfShadow).
+__device__ __forceinline__ bool gi_secondary(const RenderArgs &A, const WfArgs &W, uint32_t i) {
+  bool shadow = false;
+  const uint32_t p = W.p0 + i;
+  const int4 h4 = W.hit[i];
+  Hit h;
+  h.t = __int_as_float(h4.x); h.b1 = __int_as_float(h4.y); h.b2 = __int_as_float(h4.z); h.pos = h4.w;
+  if (h.pos >= 0) {
+    const float4 r0 = W.ray[2 * (size_t)i], r1 = W.ray[2 * (size_t)i + 1];
+    const float3 gd = f3(r1.x, r1.y, r1.z);
+    const Surface S2 = surface_at(A, h, f3(r0.x, r0.y, r0.z), gd);
+    const vt_material m2 = material(A, S2.slot);
+    if (m2.type == VT_MAT_DIFFUSE) {
+      const int limit = max(0, (int)A.maxDepth - 1);
+      const float u = W.T[i].w, bpdf = W.prev[i].w;
+      Lanes L;
+      if (A.spectral) L = make_lanes(A, u);
+      Sampler seed = wf_load_seed(W, i);
+      float4 rad = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      sampler_event(seed, 2u, kZGiNee);
+      const LightSample ls = sample_direct(A, S2.pos, S2.n, seed, limit >= 2);
+      float3 so, sd;
+      float tmax;
+      if (ls.pdf > 0.0f && shadow_ray(A, S2.pos, S2.gn, S2.err, ls, so, sd, tmax)) {
+        const float c2 = fmaxf(0.0f, dot3(S2.n, ls.wi));
+        float pdf2;
+        const float f2 = lambert_eval(S2.n, S2.gn, mul(gd, -1.0f), ls.wi, pdf2);
+        // The power heuristic only when a second continuation can sample x2's BSDF
+        // (restir_gi_has_complementary_bsdf, main.swift:3482-3484).
+        const float mis = limit >= 2 ? power_heuristic(ls.pdf, pdf2) : 1.0f;
+        const float le[3] = {ls.emission.x, ls.emission.y, ls.emission.z};
+        rad = scale4(mul4(reflectance(A, L, m2), emission(A, L, le)), f2 * c2 * mis / ls.pdf);
+        wf_set_ray(W.sray, i, so, ray_tmin(A, so), sd, tmax);
+        shadow = true;
+      }
+      const float4 gp = A.gPos[p];
+      const float3 delta = sub(S2.pos, f3(gp.x, gp.y, gp.z));
+      const float d2 = dot3(delta, delta);
+      const float cos2 = fmaxf(0.0f, -dot3(S2.n, gd));
+      A.giPos[p] = make_float4(S2.pos.x, S2.pos.y, S2.pos.z, d2 > 1e-10f ? bpdf * cos2 / d2 : 0.0f);
+      A.giNrm[p] = make_float4(S2.n.x, S2.n.y, S2.n.z, 1.0f);
+      A.giRad[p] = rad;
+      wf_store_seed(W, i, seed);
+      if (shadow) W.meta[i].w = kWfShadow;
+    }
+  }
+  return shadow;
+}
 __global__ void __launch_bounds__(kWfBlock) k_gi_secondary(RenderArgs A, WfArgs W) {
   __shared__ uint32_t sTotal, sBase;
   const uint32_t n = min(*W.inCount, W.paths);
@@ -2247,49 +2300,7 @@ __global__ void __launch_bounds__(kWfBlock) k_gi_secondary(RenderArgs A, WfArgs 
     bool shadow = false;
     if (q < n) {
       i = W.inQ[q];
-      const uint32_t p = W.p0 + i;
-      const int4 h4 = W.hit[i];
-      Hit h;
-      h.t = __int_as_float(h4.x); h.b1 = __int_as_float(h4.y); h.b2 = __int_as_float(h4.z); h.pos = h4.w;
-      if (h.pos >= 0) {
-        const float4 r0 = W.ray[2 * (size_t)i], r1 = W.ray[2 * (size_t)i + 1];
-        const float3 gd = f3(r1.x, r1.y, r1.z);
-        const Surface S2 = surface_at(A, h, f3(r0.x, r0.y, r0.z), gd);
-        const vt_material m2 = material(A, S2.slot);
-        if (m2.type == VT_MAT_DIFFUSE) {
-          const int limit = max(0, (int)A.maxDepth - 1);
-          const float u = W.T[i].w, bpdf = W.prev[i].w;
-          Lanes L;
-          if (A.spectral) L = make_lanes(A, u);
-          Sampler seed = wf_load_seed(W, i);
-          float4 rad = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          sampler_event(seed, 2u, kZGiNee);
-          const LightSample ls = sample_direct(A, S2.pos, S2.n, seed, limit >= 2);
-          float3 so, sd;
-          float tmax;
-          if (ls.pdf > 0.0f && shadow_ray(A, S2.pos, S2.gn, S2.err, ls, so, sd, tmax)) {
-            const float c2 = fmaxf(0.0f, dot3(S2.n, ls.wi));
-            float pdf2;
-            const float f2 = lambert_eval(S2.n, S2.gn, mul(gd, -1.0f), ls.wi, pdf2);
-            // The power heuristic only when a second continuation can sample x2's BSDF
-            // (restir_gi_has_complementary_bsdf, main.swift:3482-3484).
-            const float mis = limit >= 2 ? power_heuristic(ls.pdf, pdf2) : 1.0f;
-            const float le[3] = {ls.emission.x, ls.emission.y, ls.emission.z};
-            rad = scale4(mul4(reflectance(A, L, m2), emission(A, L, le)), f2 * c2 * mis / ls.pdf);
-            wf_set_ray(W.sray, i, so, ray_tmin(A, so), sd, tmax);
-            shadow = true;
-          }
-          const float4 gp = A.gPos[p];
-          const float3 delta = sub(S2.pos, f3(gp.x, gp.y, gp.z));
-          const float d2 = dot3(delta, delta);
-          const float cos2 = fmaxf(0.0f, -dot3(S2.n, gd));
-          A.giPos[p] = make_float4(S2.pos.x, S2.pos.y, S2.pos.z, d2 > 1e-10f ? bpdf * cos2 / d2 : 0.0f);
-          A.giNrm[p] = make_float4(S2.n.x, S2.n.y, S2.n.z, 1.0f);
-          A.giRad[p] = rad;
-          wf_store_seed(W, i, seed);
-          if (shadow) W.meta[i].w = kWfShadow;
-        }
-      }
+      shadow = gi_secondary(A, W, i);
     }
     wf_push(shadow, i, W.shQ, W.shCount, sTotal, sBase);
   }
@@ -2297,9 +2308,7 @@ __global__ void __launch_bounds__(kWfBlock) k_gi_secondary(RenderArgs A, WfArgs 
 
 // The GI reservoir: the candidate's weight, the merge with the previous frame's reservoir of the
 // backprojected pixel (restir_gi_merge, main.swift:4775-4795) and its encoding (:4797-4806).
-__global__ void __launch_bounds__(kWfBlock) k_gi_merge(RenderArgs A, WfArgs W) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= W.paths) return;
+__device__ __forceinline__ void gi_merge(const RenderArgs &A, const WfArgs &W, uint32_t i) {
   const uint32_t p = W.p0 + i;
   const float4 gp = A.gPos[p], gn = A.gNrm[p];
   if (!(gp.w > 0.0f) || gn.w != float(VT_MAT_DIFFUSE)) return;
@@ -2353,6 +2362,10 @@ __global__ void __launch_bounds__(kWfBlock) k_gi_merge(RenderArgs A, WfArgs W) {
   A.giRad[p] = g.rad;
   A.giW[p] = make_float4(gwsum, gM, gW, g.u);
 }
+__global__ void __launch_bounds__(kWfBlock) k_gi_merge(RenderArgs A, WfArgs W) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < W.paths) gi_merge(A, W, i);
+}
 
 // ReSTIR pass 2 (shading_kernel, main.swift:7484-7656) at the primary vertex: at a diffuse one, spatial
 // reuse of 4 uniform taps in a 32-pixel box that pass RESTIR2020's compatibility test
@@ -2363,157 +2376,226 @@ __global__ void __launch_bounds__(kWfBlock) k_gi_merge(RenderArgs A, WfArgs W) {
 // sample's shadow ray goes to the shadow queue, the GI connection's to its own.
 // kNrc: the path goes on toward a cache query, whose prediction covers the GI light.
 template <bool kPbr, bool kNrc>
-__global__ void __launch_bounds__(kRenderBlock) k_di_shade(RenderArgs A, WfArgs W) {
-  __shared__ uint32_t sTotal, sBase;
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  bool next = false, shadow = false, connect = false;
-  [&] {
-    if (i >= W.paths) return;
-    const uint32_t p = W.p0 + i, k = W.k0, x = p % A.W, y = p / A.W;
-    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    W.Rc[i] = zero;
-    W.Rp[i] = zero;
-    W.meta[i] = make_uint4(p, 0u, 0u, 0u);
-    Sampler seed = pixel_sampler(x, y, A.W, A.first + k, A.zSampler != 0u, A.zModel, A.firstFrame + k);
-    Lanes L;
-    const float u = A.spectral ? wavelength_numbers(seed).x : 0.0f;
-    if (A.spectral) L = make_lanes(A, u);
-    float3 dir0 = camera_dir(A, x, y, A.jitter[k]), o0 = A.cam;
-    lens_ray(A, o0, dir0, seed);  // the same draws as pass 1
-    seed.state = pcg_hash(seed.state ^ 0x27d4eb2fu);  // decorrelate_shading_seed
-    const float4 gp = A.gPos[p];
-    if (gp.w <= 0.0f) return;
-    const float4 gn = A.gNrm[p];
-    const uint4 gi = A.gInfo[p];
-    Surface S;
-    S.pos = f3(gp.x, gp.y, gp.z);
-    S.n = f3(gn.x, gn.y, gn.z);
-    const float4 gg = A.gGeo[p];
-    S.gn = f3(gg.x, gg.y, gg.z);
-    S.face = gi.x;
-    S.slot = gi.y & 0x7fffffffu;
-    S.front = (gi.y >> 31) != 0u;
-    S.err = __uint_as_float(gi.z);
-    S.tri = gi.w;
-    const vt_material m = material(A, S.slot);
-    if (m.type == VT_MAT_EMISSIVE) {
-      const float3 e = primary_emission(A, L, S, m);
-      W.Rp[i] = make_float4(e.x, e.y, e.z, 0.0f);
-      return;
+__device__ __forceinline__ void di_shade(const RenderArgs &A, const WfArgs &W, uint32_t i, bool &next, bool &shadow, bool &connect) {
+  const uint32_t p = W.p0 + i, k = W.k0, x = p % A.W, y = p / A.W;
+  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  W.Rc[i] = zero;
+  W.Rp[i] = zero;
+  W.meta[i] = make_uint4(p, 0u, 0u, 0u);
+  Sampler seed = pixel_sampler(x, y, A.W, A.first + k, A.zSampler != 0u, A.zModel, A.firstFrame + k);
+  Lanes L;
+  const float u = A.spectral ? wavelength_numbers(seed).x : 0.0f;
+  if (A.spectral) L = make_lanes(A, u);
+  float3 dir0 = camera_dir(A, x, y, A.jitter[k]), o0 = A.cam;
+  lens_ray(A, o0, dir0, seed);  // the same draws as pass 1
+  seed.state = pcg_hash(seed.state ^ 0x27d4eb2fu);  // decorrelate_shading_seed
+  const float4 gp = A.gPos[p];
+  if (gp.w <= 0.0f) return;
+  const float4 gn = A.gNrm[p];
+  const uint4 gi = A.gInfo[p];
+  Surface S;
+  S.pos = f3(gp.x, gp.y, gp.z);
+  S.n = f3(gn.x, gn.y, gn.z);
+  const float4 gg = A.gGeo[p];
+  S.gn = f3(gg.x, gg.y, gg.z);
+  S.face = gi.x;
+  S.slot = gi.y & 0x7fffffffu;
+  S.front = (gi.y >> 31) != 0u;
+  S.err = __uint_as_float(gi.z);
+  S.tri = gi.w;
+  const vt_material m = material(A, S.slot);
+  if (m.type == VT_MAT_EMISSIVE) {
+    const float3 e = primary_emission(A, L, S, m);
+    W.Rp[i] = make_float4(e.x, e.y, e.z, 0.0f);
+    return;
+  }
+  const int limit = max(0, (int)A.maxDepth - 1);
+  const float4 T = A.spectral ? make_float4(1.0f, 1.0f, 1.0f, 1.0f) : make_float4(1.0f, 1.0f, 1.0f, 0.0f);
+  uint32_t flags = 0u;
+  const bool diffuse = m.type == VT_MAT_DIFFUSE;
+  PbrPrepared prep;
+  bool pbr = false;
+  if (!diffuse) {
+    LightSample ls;
+    if (!is_delta<kPbr>(A, m)) {  // no NEE at glass or a mirror (main.swift:7657)
+      sampler_event(seed, 1u, kZNee);
+      shadow = wf_light(A, W, i, S, limit > 0, seed, true, ls);
     }
-    const int limit = max(0, (int)A.maxDepth - 1);
-    const float4 T = A.spectral ? make_float4(1.0f, 1.0f, 1.0f, 1.0f) : make_float4(1.0f, 1.0f, 1.0f, 0.0f);
-    uint32_t flags = 0u;
-    const bool diffuse = m.type == VT_MAT_DIFFUSE;
-    PbrPrepared prep;
-    bool pbr = false;
-    if (!diffuse) {
-      LightSample ls;
-      if (!is_delta<kPbr>(A, m)) {  // no NEE at glass or a mirror (main.swift:7657)
-        sampler_event(seed, 1u, kZNee);
-        shadow = wf_light(A, W, i, S, limit > 0, seed, true, ls);
-      }
-      pbr = is_pbr<kPbr>(A, m);
-      if (pbr) prep = pbr_prepare(pbr_params_lanes(A, L, m), A.pbrT, S.n, mul(dir0, -1.0f), surface_tangent(A, m, S.tri, S.n));
-      if (shadow) {
-        const float3 c = to_rgb(A, L, nee_lanes(A, L, S.n, S.gn, S.tri, mul(dir0, -1.0f), T, m, limit > 0, ls, pbr, &prep));
-        W.scon[i] = make_float4(c.x, c.y, c.z, 0.0f);
-      }
-    } else {
-      const float4 cw = A.rW[p];
-      DISample sel = load_di(A.rPos, A.rEmit, A.rW, p);
-      float wsum = di_target(A, S.pos, S.n, S.gn, dir0, m, sel) * cw.z * cw.y, M = cw.y;
+    pbr = is_pbr<kPbr>(A, m);
+    if (pbr) prep = pbr_prepare(pbr_params_lanes(A, L, m), A.pbrT, S.n, mul(dir0, -1.0f), surface_tangent(A, m, S.tri, S.n));
+    if (shadow) {
+      const float3 c = to_rgb(A, L, nee_lanes(A, L, S.n, S.gn, S.tri, mul(dir0, -1.0f), T, m, limit > 0, ls, pbr, &prep));
+      W.scon[i] = make_float4(c.x, c.y, c.z, 0.0f);
+    }
+  } else {
+    const float4 cw = A.rW[p];
+    DISample sel = load_di(A.rPos, A.rEmit, A.rW, p);
+    float wsum = di_target(A, S.pos, S.n, S.gn, dir0, m, sel) * cw.z * cw.y, M = cw.y;
+    for (int t = 0; t < 4; ++t) {
+      const float ox = pcg_rand(seed.state), oy = pcg_rand(seed.state);
+      const int nx = (int)x + (int)((ox * 2.0f - 1.0f) * 16.0f), ny = (int)y + (int)((oy * 2.0f - 1.0f) * 16.0f);
+      if (nx < 0 || nx >= (int)A.W || ny < 0 || ny >= (int)A.H) continue;
+      const uint32_t j = (uint32_t)ny * A.W + (uint32_t)nx;
+      if (!compatible(gp, gn, A.gPos[j], A.gNrm[j])) continue;
+      const float4 nw = A.rW[j];
+      if (!(nw.y > 0.0f && nw.z > 0.0f)) continue;
+      const DISample ns = load_di(A.rPos, A.rEmit, A.rW, j);
+      const float w = di_target(A, S.pos, S.n, S.gn, dir0, m, ns) * nw.z * nw.y;
+      wsum += w;
+      M += nw.y;
+      if (rand_decision(seed) * wsum < w) sel = ns;
+    }
+    const float pHat = di_target(A, S.pos, S.n, S.gn, dir0, m, sel);
+    const float Wr = M > 0.0f && pHat > 0.0f ? wsum / (M * pHat) : 0.0f;
+    float3 so, sd;
+    float tmax;
+    if (Wr > 0.0f && shadow_ray(A, S.pos, S.gn, S.err, di_light_sample(sel, S.pos), so, sd, tmax)) {
+      const float3 c = mul(di_contribution(A, S.pos, S.n, S.gn, dir0, m, sel), Wr);
+      W.scon[i] = make_float4(c.x, c.y, c.z, 0.0f);
+      wf_set_ray(W.sray, i, so, ray_tmin(A, so), sd, tmax);
+      shadow = true;
+    }
+    // ReSTIR GI (a cache-terminated path's cache covers this light, so the cache's kernel leaves it out).
+    if (!kNrc && limit >= 1) {
+      const float4 cgw = A.giW[p];
+      GISample gsel = gi_load(A.giPos, A.giNrm, A.giRad, A.giW, p);
+      bool gvalid = A.giNrm[p].w > 0.0f;
+      float gwsum = gvalid ? gi_target(A, S.pos, S.n, S.gn, dir0, m, gsel) * cgw.z * cgw.y : 0.0f, gM = cgw.y;
       for (int t = 0; t < 4; ++t) {
         const float ox = pcg_rand(seed.state), oy = pcg_rand(seed.state);
         const int nx = (int)x + (int)((ox * 2.0f - 1.0f) * 16.0f), ny = (int)y + (int)((oy * 2.0f - 1.0f) * 16.0f);
         if (nx < 0 || nx >= (int)A.W || ny < 0 || ny >= (int)A.H) continue;
         const uint32_t j = (uint32_t)ny * A.W + (uint32_t)nx;
-        if (!compatible(gp, gn, A.gPos[j], A.gNrm[j])) continue;
-        const float4 nw = A.rW[j];
-        if (!(nw.y > 0.0f && nw.z > 0.0f)) continue;
-        const DISample ns = load_di(A.rPos, A.rEmit, A.rW, j);
-        const float w = di_target(A, S.pos, S.n, S.gn, dir0, m, ns) * nw.z * nw.y;
-        wsum += w;
-        M += nw.y;
-        if (rand_decision(seed) * wsum < w) sel = ns;
-      }
-      const float pHat = di_target(A, S.pos, S.n, S.gn, dir0, m, sel);
-      const float Wr = M > 0.0f && pHat > 0.0f ? wsum / (M * pHat) : 0.0f;
-      float3 so, sd;
-      float tmax;
-      if (Wr > 0.0f && shadow_ray(A, S.pos, S.gn, S.err, di_light_sample(sel, S.pos), so, sd, tmax)) {
-        const float3 c = mul(di_contribution(A, S.pos, S.n, S.gn, dir0, m, sel), Wr);
-        W.scon[i] = make_float4(c.x, c.y, c.z, 0.0f);
-        wf_set_ray(W.sray, i, so, ray_tmin(A, so), sd, tmax);
-        shadow = true;
-      }
-      // ReSTIR GI (a cache-terminated path's cache covers this light, so the cache's kernel leaves it out).
-      if (!kNrc && limit >= 1) {
-        const float4 cgw = A.giW[p];
-        GISample gsel = gi_load(A.giPos, A.giNrm, A.giRad, A.giW, p);
-        bool gvalid = A.giNrm[p].w > 0.0f;
-        float gwsum = gvalid ? gi_target(A, S.pos, S.n, S.gn, dir0, m, gsel) * cgw.z * cgw.y : 0.0f, gM = cgw.y;
-        for (int t = 0; t < 4; ++t) {
-          const float ox = pcg_rand(seed.state), oy = pcg_rand(seed.state);
-          const int nx = (int)x + (int)((ox * 2.0f - 1.0f) * 16.0f), ny = (int)y + (int)((oy * 2.0f - 1.0f) * 16.0f);
-          if (nx < 0 || nx >= (int)A.W || ny < 0 || ny >= (int)A.H) continue;
-          const uint32_t j = (uint32_t)ny * A.W + (uint32_t)nx;
-          const float4 q = A.gPos[j];
-          if (!compatible(gp, gn, q, A.gNrm[j])) continue;
-          const float4 nw = A.giW[j], np = A.giPos[j], nn = A.giNrm[j];
-          if (nw.y <= 0.0f || nw.z <= 0.0f || np.w <= 0.0f || nn.w <= 0.0f) continue;
-          if (!gi_accepts_shift(S.pos, f3(q.x, q.y, q.z), f3(np.x, np.y, np.z), f3(nn.x, nn.y, nn.z))) continue;
-          const GISample ns = gi_load(A.giPos, A.giNrm, A.giRad, A.giW, j);
-          const float w = gi_target(A, S.pos, S.n, S.gn, dir0, m, ns) * nw.z * nw.y;
-          gwsum += w;
-          gM += nw.y;
-          if (rand_decision(seed) * gwsum < w) {
-            gsel = ns;
-            gvalid = true;
-          }
-        }
-        const float gHat = gvalid ? gi_target(A, S.pos, S.n, S.gn, dir0, m, gsel) : 0.0f;
-        const float gW = gM > 0.0f && gHat > 0.0f ? gwsum / (gM * gHat) : 0.0f;
-        if (gW > 0.0f && gi_ray(A, S.pos, S.gn, gsel.pos, S.err, so, sd, tmax)) {
-          const float3 dir = normalize3(sub(gsel.pos, S.pos));
-          Lanes Ls;
-          if (A.spectral) Ls = make_lanes(A, gsel.u);
-          float pdf;
-          const float f = lambert_eval(S.n, S.gn, mul(dir0, -1.0f), dir, pdf);
-          const float geometry = gi_geometry(S.pos, S.n, gsel.pos, gsel.nrm);
-          const float3 c = to_rgb(A, Ls, scale4(mul4(reflectance(A, Ls, m), gsel.rad), f * geometry * gW));
-          W.gcon[i] = make_float4(c.x, c.y, c.z, 0.0f);
-          wf_set_ray(W.gray, i, so, ray_tmin(A, so), sd, tmax);
-          connect = true;
+        const float4 q = A.gPos[j];
+        if (!compatible(gp, gn, q, A.gNrm[j])) continue;
+        const float4 nw = A.giW[j], np = A.giPos[j], nn = A.giNrm[j];
+        if (nw.y <= 0.0f || nw.z <= 0.0f || np.w <= 0.0f || nn.w <= 0.0f) continue;
+        if (!gi_accepts_shift(S.pos, f3(q.x, q.y, q.z), f3(np.x, np.y, np.z), f3(nn.x, nn.y, nn.z))) continue;
+        const GISample ns = gi_load(A.giPos, A.giNrm, A.giRad, A.giW, j);
+        const float w = gi_target(A, S.pos, S.n, S.gn, dir0, m, ns) * nw.z * nw.y;
+        gwsum += w;
+        gM += nw.y;
+        if (rand_decision(seed) * gwsum < w) {
+          gsel = ns;
+          gvalid = true;
         }
       }
-      if (!kNrc) flags |= kWfGiPrimary;
+      const float gHat = gvalid ? gi_target(A, S.pos, S.n, S.gn, dir0, m, gsel) : 0.0f;
+      const float gW = gM > 0.0f && gHat > 0.0f ? gwsum / (gM * gHat) : 0.0f;
+      if (gW > 0.0f && gi_ray(A, S.pos, S.gn, gsel.pos, S.err, so, sd, tmax)) {
+        const float3 dir = normalize3(sub(gsel.pos, S.pos));
+        Lanes Ls;
+        if (A.spectral) Ls = make_lanes(A, gsel.u);
+        float pdf;
+        const float f = lambert_eval(S.n, S.gn, mul(dir0, -1.0f), dir, pdf);
+        const float geometry = gi_geometry(S.pos, S.n, gsel.pos, gsel.nrm);
+        const float3 c = to_rgb(A, Ls, scale4(mul4(reflectance(A, Ls, m), gsel.rad), f * geometry * gW));
+        W.gcon[i] = make_float4(c.x, c.y, c.z, 0.0f);
+        wf_set_ray(W.gray, i, so, ray_tmin(A, so), sd, tmax);
+        connect = true;
+      }
     }
-    if (shadow) flags |= kWfShadow | kWfShadowPrimary;
-    if (kNrc) W.spread[i] = make_float2(0.0f, nrc_spread_limit(A, gp.w, S.gn, dir0));
-    // A BSDF hit on an emitter from a vertex whose direct light came from its reservoir gets no weight
-    // (previousMIS false, main.swift:7717-7718).
-    int scattering = 0;
-    bool emissionOnly = false;
-    next = wf_continue<kPbr>(A, W, i, 1u, L, S, m, dir0, T, seed, scattering, emissionOnly, !diffuse, u, flags, pbr, prep);
-    if (emissionOnly) flags |= kWfEmissionOnly;
-    W.meta[i] = make_uint4(p, next ? 1u : 0u, (uint32_t)scattering, flags);
-    if (next) wf_store_seed(W, i, seed);
-  }();
+    if (!kNrc) flags |= kWfGiPrimary;
+  }
+  if (shadow) flags |= kWfShadow | kWfShadowPrimary;
+  if (kNrc) W.spread[i] = make_float2(0.0f, nrc_spread_limit(A, gp.w, S.gn, dir0));
+  // A BSDF hit on an emitter from a vertex whose direct light came from its reservoir gets no weight
+  // (previousMIS false, main.swift:7717-7718).
+  int scattering = 0;
+  bool emissionOnly = false;
+  next = wf_continue<kPbr>(A, W, i, 1u, L, S, m, dir0, T, seed, scattering, emissionOnly, !diffuse, u, flags, pbr, prep);
+  if (emissionOnly) flags |= kWfEmissionOnly;
+  W.meta[i] = make_uint4(p, next ? 1u : 0u, (uint32_t)scattering, flags);
+  if (next) wf_store_seed(W, i, seed);
+}
+template <bool kPbr, bool kNrc>
+__global__ void __launch_bounds__(kRenderBlock) k_di_shade(RenderArgs A, WfArgs W) {
+  __shared__ uint32_t sTotal, sBase;
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  bool next = false, shadow = false, connect = false;
+  if (i < W.paths) di_shade<kPbr, kNrc>(A, W, i, next, shadow, connect);
   wf_push(next, i, W.outQ, W.outCount, sTotal, sBase);
   wf_push(shadow, i, W.shQ, W.shCount, sTotal, sBase);
   wf_push(connect, i, W.giQ, W.giCount, sTotal, sBase);
 }
 
 // Adds the visible GI connections to their paths' primary radiance.
+__device__ __forceinline__ void gi_connect(const WfArgs &W, uint32_t i) {
+  const float4 R = W.Rp[i], c = W.gcon[i];
+  W.Rp[i] = make_float4(R.x + c.x, R.y + c.y, R.z + c.z, 0.0f);
+}
 __global__ void __launch_bounds__(kWfBlock) k_gi_connect(WfArgs W) {
   const uint32_t n = min(*W.giCount, W.paths);
   for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
     const uint32_t i = W.giQ[q];
-    if (W.gocc[i]) continue;
-    const float4 R = W.Rp[i], c = W.gcon[i];
-    W.Rp[i] = make_float4(R.x + c.x, R.y + c.y, R.z + c.z, 0.0f);
+    if (!W.gocc[i]) gi_connect(W, i);
   }
+}
+
+// ---- a path per thread, of the stages' parts ------------------------------------------------------
+// Where the stages' traversals leave hits and occlusion.
+struct WfHits {
+  int4 *hit;
+  uint8_t *occ;
+};
+// Path i's ray to its hit.
+__device__ __forceinline__ void wf_trace(const RenderArgs &A, const WfArgs &W, const WfHits &H, uint32_t i, int *stack) {
+  const float4 r0 = W.ray[2 * (size_t)i], r1 = W.ray[2 * (size_t)i + 1];
+  Hit h;
+  const bool found = rt_closest(A, f3(r0.x, r0.y, r0.z), f3(r1.x, r1.y, r1.z), r0.w, r1.w, h, stack);
+  H.hit[i] = found ? make_int4(__float_as_int(h.t), __float_as_int(h.b1), __float_as_int(h.b2), h.pos) : make_int4(0, 0, 0, -1);
+}
+__device__ __forceinline__ bool wf_occluded(const RenderArgs &A, const float4 *ray, uint32_t i, int *stack) {
+  const float4 r0 = ray[2 * (size_t)i], r1 = ray[2 * (size_t)i + 1];
+  return rt_any(A, f3(r0.x, r0.y, r0.z), f3(r1.x, r1.y, r1.z), r0.w, r1.w, stack, A.imported != 0u);
+}
+// Path i from bounce b, whose ray is set, to its end.
+template <bool kPbr, bool kNrc>
+__device__ __forceinline__ void wf_path(const RenderArgs &A, const WfArgs &W, const WfHits &H, uint32_t i, uint32_t b, int *stack) {
+  for (bool next = true; next; ++b) {
+    bool shadow = false;
+    next = false;
+    wf_trace(A, W, H, i, stack);
+    wf_vertex<kPbr, kNrc, false>(A, W, i, b, next, shadow);
+    if (shadow) H.occ[i] = wf_occluded(A, W.sray, i, stack) ? 1 : 0;
+  }
+}
+
+// Small ReSTIR frames (small_frame): a thread a pixel takes all reservoir stages in one launch and its path in
+// a second, with its own traversals. Bound: the longest path's chain of dependent loads. The stages cost a
+// small frame some 12 launches and two or three a bounce, each as long as the longest ray it holds; a
+// thread waits for its own only. `lanes` pixels to a warp, so that a warp diverges over few paths. Measured on
+// one B200, a frame in us, by stages -> by threads: 100 x 64 Cornell box at depth 3 393 -> 255, at 12 677 -> 347; 300,000
+// triangles 953 -> 618 and 1680 -> 914; OPENPBR grid in spectral transport 582 -> 422 and 1457 -> 792. (16 warps an
+// SM instead of 8: the Cornell box 316 and 423, 300,000 triangles 588 and 870.)
+constexpr uint32_t kDiSmallWarps = 8;
+__device__ __forceinline__ uint32_t few_index(uint32_t lanes) {
+  const uint32_t lane = threadIdx.x & 31u;
+  return lane < lanes ? (blockIdx.x * (kRenderBlock / 32) + (threadIdx.x >> 5)) * lanes + lane : 0xffffffffu;
+}
+__global__ void __launch_bounds__(kRenderBlock, 4) k_di_small_reservoirs(RenderArgs A, WfArgs W, WfHits H, uint32_t lanes) {
+  int stack[kRenderStack];
+  const uint32_t i = few_index(lanes);
+  if (i >= W.paths) return;
+  wf_generate(A, W, i);
+  wf_trace(A, W, H, i, stack);
+  if (di_primary(A, W, i)) {
+    wf_trace(A, W, H, i, stack);
+    if (gi_secondary(A, W, i)) H.occ[i] = wf_occluded(A, W.sray, i, stack) ? 1 : 0;
+  }
+  if (A.maxDepth > 1u) gi_merge(A, W, i);
+}
+template <bool kPbr, bool kNrc>
+__global__ void __launch_bounds__(kRenderBlock, kPbr ? 3 : 4) k_di_small_paths(RenderArgs A, WfArgs W, WfHits H, uint32_t lanes) {
+  int stack[kRenderStack];
+  const uint32_t i = few_index(lanes);
+  if (i >= W.paths) return;
+  bool next = false, shadow = false, connect = false;
+  di_shade<kPbr, kNrc>(A, W, i, next, shadow, connect);
+  if (shadow) H.occ[i] = wf_occluded(A, W.sray, i, stack) ? 1 : 0;
+  if (connect && !wf_occluded(A, W.gray, i, stack)) gi_connect(W, i);
+  if (next) wf_path<kPbr, kNrc>(A, W, H, i, 1u, stack);
+  wf_finish<kNrc>(A, W, i);
 }
 
 // ---- radiance cache: training paths and the resolve (vt_render_nrc) -----------------------------
@@ -3541,6 +3623,36 @@ vt_status wf_bounces(const WfStages &S, const RenderArgs &A, WfArgs W, uint32_t 
   return VT_OK;
 }
 
+// Whether a mode-0 frame goes to k_di_small_reservoirs and k_di_small_paths. In threads of kDiSmallWarps warps an SM:
+// up to 2 pixels a thread, 3/4 where slots are OpenPBR (their paths differ more), and 2/3 of either up to depth 8
+// (the stages pay launches for every bounce). Larger frames are faster in stages. One B200, a frame in us, threads /
+// stages: Cornell box 264 x 171 354 / 418 at depth 3 and 529 / 755 at 12, 320 x 236 476 / 451 and 759 / 828; 300,000
+// triangles 320 x 236 1335 / 1353 and 1911 / 2314; OPENPBR grid 180 x 100 541 / 585 and 1036 / 1424, 190 x 149 708 / 644 and
+// 1388 / 1610, 264 x 171 839 / 690 and 1565 / 1683.
+bool small_frame(const WfStages &S, const RenderArgs &A, uint32_t npix) {
+  const uint32_t full = (uint32_t)S.ctx->sm_count * kDiSmallWarps * 32u, most = S.pbr ? full / 4u * 3u : 2u * full;
+  return npix <= (A.maxDepth > 8u ? most : most / 3u * 2u);
+}
+
+// Such a frame.
+vt_status di_small(const WfStages &S, const RenderArgs &A, const WfArgs &W) {
+  vt_ctx *ctx = S.ctx;
+  cudaStream_t s = S.s;
+  const uint32_t warps = (uint32_t)ctx->sm_count * kDiSmallWarps, lanes = std::min(32u, (W.paths + warps - 1u) / warps);
+  const uint32_t block = lanes * (kRenderBlock / 32), grid = (W.paths + block - 1u) / block;
+  const WfHits H{S.B.hit, S.B.occ};
+  k_di_small_reservoirs<<<grid, kRenderBlock, 0, s>>>(A, W, H, lanes);
+  if (S.nrc) {
+    if (S.pbr) k_di_small_paths<true, true><<<grid, kRenderBlock, 0, s>>>(A, W, H, lanes);
+    else k_di_small_paths<false, true><<<grid, kRenderBlock, 0, s>>>(A, W, H, lanes);
+  } else {
+    if (S.pbr) k_di_small_paths<true, false><<<grid, kRenderBlock, 0, s>>>(A, W, H, lanes);
+    else k_di_small_paths<false, false><<<grid, kRenderBlock, 0, s>>>(A, W, H, lanes);
+  }
+  VT_CUDA(ctx, cudaGetLastError());
+  return VT_OK;
+}
+
 // One band of a mode-0 frame up to its reservoirs (A holds the frame's reservoir arrays).
 vt_status di_reservoirs(const WfStages &S, const RenderArgs &A, WfArgs W) {
   vt_ctx *ctx = S.ctx;
@@ -3698,10 +3810,7 @@ vt_status render_impl(vt_ctx *ctx, vt_scene *scene, const vt_frame_params *p, ui
     W.npix = npix;
     W.deadFlags = 0u;
     A.kernelId = nrc ? 5u : 4u;
-    // Blocks of two warps where the band is small: they spread evenly over the SMs (264 x 171: 7.24 -> 7.16 ms for
-    // four frames; large bands want whole blocks in the same code, k_wf_shade).
-    const int stageBlock = band <= (uint32_t)ctx->sm_count * 512u ? 64 : kWfBlock;
-    const WfStages S = wf_stages(ctx, scene, A, B, stageBlock, 1u, nrc != nullptr, s);
+    const WfStages S = wf_stages(ctx, scene, A, B, kWfBlock, 1u, nrc != nullptr, s);
     for (uint32_t k = 0; k < spp; ++k) {
       float4 *cur = base + 9 * (size_t)npix * scene->di_parity, *prev = base + 9 * (size_t)npix * (scene->di_parity ^ 1u);
       A.gPos = cur; A.gNrm = cur + npix; A.rPos = cur + 2 * (size_t)npix; A.rEmit = cur + 3 * (size_t)npix;
@@ -3721,8 +3830,13 @@ vt_status render_impl(vt_ctx *ctx, vt_scene *scene, const vt_frame_params *p, ui
       A.paspect = pc[12];
       A.pfovScale = pc[13];
       W.k0 = k;
-      const bool whole = band >= npix;
-      for (uint32_t p0 = 0; p0 < npix; p0 += band) {
+      const bool whole = band >= npix, small = whole && small_frame(S, A, npix);
+      if (small) {
+        W.p0 = 0u;
+        W.paths = npix;
+        if (const vt_status st = di_small(S, A, W)) return st;
+      }
+      for (uint32_t p0 = 0; p0 < npix && !small; p0 += band) {
         W.p0 = p0;
         W.paths = std::min(band, npix - p0);
         vt_status st = di_reservoirs(S, A, W);
