@@ -15,8 +15,11 @@ double can still part at a total-internal-reflection or Fresnel threshold, and a
 the light through the glass carries a caustic firefly worth a few percent of the image mean. So means
 and relMSE are compared over the pixels outside the 0.5 % that differ most.
 """
+import time
+
 import numpy as np
 import pytest
+import torch
 
 import metal_vibe_tracer_b200 as vt
 from metal_vibe_tracer_b200 import scenes, spectral_tables
@@ -92,6 +95,50 @@ def test_delta_restir_matches_oracle(ctx, oracle):
     other = oracle.render(faces, verts, mats, light, cam, 64, 64, 32, max_depth=8, mode=0, first_sample=5001)
     # Reservoirs pass samples between pixels, so a parted path moves its neighbours too.
     assert_agrees(gpu, ref, other, frac=0.9)
+
+
+def test_staged_delta_restir_matches_oracle(ctx, oracle):
+    """As above, of a frame large enough for the stages: paths that outlive the depth end in k_wf_rest."""
+    faces, verts, mats, light, cam = scenes.cornell_delta()
+    mesh = vt.Mesh(ctx, faces, verts)
+    gpu = gpu_render(ctx, mesh, mats, light, vt.make_params(cam, 200, 160, 3, 1, False, 0), 8, False)
+    mesh.close()
+    ref = oracle.render(faces, verts, mats, light, cam, 200, 160, 8, max_depth=3, mode=0)
+    other = oracle.render(faces, verts, mats, light, cam, 200, 160, 8, max_depth=3, mode=0, first_sample=5001)
+    assert_agrees(gpu, ref, other, frac=0.9)
+
+
+@pytest.mark.parametrize("size", [(96, 72), (200, 160)])
+def test_delta_restir_keeps_the_mis_energy(ctx, size):
+    """By threads and by stages, at a depth that most paths through the glass outlive: the reference's 6 %."""
+    faces, verts, mats, light, cam = scenes.cornell_delta()
+    mesh = vt.Mesh(ctx, faces, verts)
+    restir, mis = (gpu_render(ctx, mesh, mats, light, vt.make_params(cam, *size, 3, 1, False, mode), 96, False).mean() for mode in (0, 1))
+    mesh.close()
+    assert abs(restir / mis - 1) < 0.06, (restir, mis)
+
+
+@pytest.mark.parametrize("size", [(64, 48), (200, 160)])
+def test_restir_of_delta_scenes_is_stream_ordered(ctx, size):
+    """vt_render queues a mode-0 frame of glass and mirrors behind half a second of other work on its stream and
+    returns: nothing is read back in between."""
+    faces, verts, mats, light, cam = scenes.cornell_delta()
+    mesh = vt.Mesh(ctx, faces, verts)
+    scene = vt.Scene(ctx, mesh, mats, light)
+    params = vt.make_params(cam, *size, 8, 1, False, 0)
+    scene.render(params, 2)  # allocates
+    torch.cuda.synchronize()
+    begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    begin.record()
+    torch.cuda._sleep(1_000_000_000)
+    end.record()
+    started = time.perf_counter()
+    scene.render(params, 2)
+    took = time.perf_counter() - started
+    torch.cuda.synchronize()
+    assert took < 0.25e-3 * begin.elapsed_time(end), (took, begin.elapsed_time(end))
+    scene.close()
+    mesh.close()
 
 
 def test_cache_takes_delta_scenes_in_mode_1_only(ctx):
