@@ -168,12 +168,21 @@ __device__ __forceinline__ int delta(const uint32_t *codes, int n, int i, int j)
   return 32 + __clz((uint32_t)i ^ (uint32_t)j);
 }
 
+// Whether the sort gave up: its face indices are then any numbers and nothing is built on them. k_hierarchy leaves
+// every leaf without a parent, so that the treelet walks end where they start, the collapse has no level, and the
+// build reports the error.
+__device__ __forceinline__ bool unsorted(const uint32_t *status) { return (__ldcg(status) & (uint32_t)VT_DEV_SORT) != 0u; }
+
 // One thread per sorted position: its leaf box gathered, and internal node i's hierarchy with its
 // visit counter cleared.
 __global__ void k_hierarchy(const uint32_t *codes, const float4 *boxes, const uint32_t *sorted, int n, float4 *leaf, int2 *child,
-                            int32_t *parent, uint32_t *flags) {
+                            int32_t *parent, uint32_t *flags, const uint32_t *status) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
+  if (unsorted(status)) {
+    parent[n - 1 + i] = -1;
+    return;
+  }
   const uint32_t f = sorted[i];
   leaf[2 * (size_t)i] = boxes[2 * (size_t)f];
   leaf[2 * (size_t)i + 1] = boxes[2 * (size_t)f + 1];
@@ -713,7 +722,7 @@ __global__ void __launch_bounds__(kCollapseBlock) k_collapse(TreeView t, int lea
                                                              const uint32_t *bounds, BuildReport *report, uint32_t *status) {
   __shared__ uint32_t ws[kCollapseBlock / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t L = 1, base = 0, primBase = 0, depth = 0, code = kCollapseOk, round = 0;
+  uint32_t L = unsorted(status) ? 0u : 1u, base = 0, primBase = 0, depth = 0, code = kCollapseOk, round = 0;
   int32_t *level = levelA, *nextLevel = levelB;
   while (L > 0) {
     if ((int)depth >= maxDepth) { code = kCollapseDepth; break; }
@@ -780,7 +789,7 @@ __global__ void __launch_bounds__(kCollapseBlock) k_collapse(TreeView t, int lea
     base = nextBase;
     L = allI;
     int32_t *x = level; level = nextLevel; nextLevel = x;
-    if (st & (uint32_t)(VT_DEV_TREELET | VT_DEV_BAD_INDEX | VT_DEV_NONFINITE | VT_DEV_SORT)) break;
+    if (st & (uint32_t)(VT_DEV_TREELET | VT_DEV_BAD_INDEX | VT_DEV_NONFINITE)) break;
     if (base + L > maxNodes) { code = kCollapseNodes; break; }
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -900,7 +909,7 @@ cudaError_t queue_build(const vt_face *faces, uint32_t n, const vt_vertex *verts
   k_face_boxes<<<blocks(n, 256), 256, 0, s>>>(faces, n, verts, nverts, b.boxes, b.bounds, status);
   k_morton<<<blocks(n, 256), 256, 0, s>>>(b.boxes, n, b.bounds, o.codes, o.sorted);
   vt_radix_sort_pairs(o.codes, o.sorted, b.codesAlt, b.valsAlt, n, 30, b.sortTemp, status, s);
-  k_hierarchy<<<blocks(n, 256), 256, 0, s>>>(o.codes, b.boxes, o.sorted, (int)n, b.leafBox, o.child, b.parent, b.flags);
+  k_hierarchy<<<blocks(n, 256), 256, 0, s>>>(o.codes, b.boxes, o.sorted, (int)n, b.leafBox, o.child, b.parent, b.flags, status);
   TreeView t{(int)n, o.child, b.parent, b.leafBox, o.nodeBox, b.count, b.cost};
   if (n >= 3 && treelet > 0) {
     for (int r = 0; r < rounds; ++r)

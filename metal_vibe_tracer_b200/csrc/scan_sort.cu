@@ -21,8 +21,12 @@ constexpr int kMaxPasses = 4;
 // number fewer than 2^30).
 constexpr uint32_t kPartial = 1u << 30, kPrefix = 2u << 30, kCountMask = kPartial - 1u;
 // Look-back polls before a tile gives up (a tile's predecessors have all started, so this is never
-// reached unless a launch is broken); the sort then reports VT_DEV_SORT.
-constexpr uint32_t kSpinLimit = 1u << 21;
+// reached unless a launch is broken); the sort then reports VT_DEV_SORT, and its output holds some pairs twice
+// and others' slots unwritten. (0: every look-back gives up, for the test of that.)
+#ifndef VT_SORT_SPIN_LIMIT
+#define VT_SORT_SPIN_LIMIT (1u << 21)
+#endif
+constexpr uint32_t kSpinLimit = VT_SORT_SPIN_LIMIT;
 
 // Temporary words: digit counts of each pass, tile tickets, then the tile states of each pass.
 constexpr uint32_t kTicketAt = kMaxPasses * kDigits, kStateAt = kTicketAt + 64;
@@ -112,10 +116,9 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_pass(const uint32_t *__r
   // Pairs of this digit in the tiles before this one.
   uint32_t before = 0;
   for (uint32_t p = tile; p > 0;) {
-    uint32_t s = 0, spins = 0;
-    do {
+    uint32_t s = 0;
+    for (uint32_t spins = 0; spins < kSpinLimit && (s & ~kCountMask) == 0u; ++spins)
       s = vt_poll(temp + kStateAt + ((size_t)pass * tiles + (p - 1)) * kDigits + t);
-    } while ((s & ~kCountMask) == 0u && ++spins < kSpinLimit);
     if ((s & ~kCountMask) == 0u) {
       atomicOr(status, (uint32_t)VT_DEV_SORT);
       break;

@@ -107,3 +107,41 @@ def test_build_rejects_bad_input(ctx):
     # The context stays usable after an error.
     m = vt.Mesh(ctx, faces, verts)
     assert m.info().faces == 100
+
+
+def test_a_sort_that_gives_up_ends_in_an_error(tmp_path):
+    """The library with a look-back limit of no polls: a mesh of more than one tile of the Morton sort gets an error
+    from both build entries (nothing is built on the unsorted indices), one of a single tile builds."""
+    import ctypes as C
+    import subprocess
+
+    import torch
+
+    from metal_vibe_tracer_b200 import _lib, build
+
+    if not (build.OBJ / "lbvh.o").exists():
+        build.build()
+    obj, so = tmp_path / "scan_sort.o", tmp_path / "libvt_gives_up.so"
+    subprocess.run([build.nvcc(), *build.ARCH, *build.NVCC_FLAGS, "-DVT_SORT_SPIN_LIMIT=0", "-I", str(build.INCLUDE), "-c",
+                    str(build.CSRC / "scan_sort.cu"), "-o", str(obj)], check=True)
+    others = [str(o) for o in sorted(build.OBJ.glob("*.o")) if o.stem != "scan_sort"]
+    subprocess.run([build.nvcc(), *build.ARCH, "-shared", "--cudart", "static", "-Xlinker", "-Bsymbolic", "-o", str(so), str(obj), *others],
+                   check=True)
+    lib = C.CDLL(str(so))
+    for name, (res, args) in _lib.SIGNATURES.items():
+        getattr(lib, name).restype, getattr(lib, name).argtypes = res, args
+    ctx, mesh, opts = C.c_void_p(), C.c_void_p(), _lib.BuildOptions(2, 7, 2, 31)
+    assert lib.vt_ctx_create(0, C.byref(ctx)) == 0
+    for n, ok in ((20_000, False), (3_072, True), (3_073, False), (1, True)):
+        faces, verts = scenes.triangle_soup(n, seed=3)
+        st = lib.vt_mesh_build(ctx, faces.ctypes.data, n, verts.ctypes.data, len(verts), C.byref(opts), C.byref(mesh))
+        assert (st == 0) == ok and (ok or (_lib.STATUS_NAMES[st] == "VT_ERR_DEVICE" and b"look-back" in lib.vt_last_error(ctx))), (n, st)
+        if ok:
+            assert lib.vt_mesh_destroy(ctx, mesh) == 0
+        f, v = torch.from_numpy(faces.view(np.int32).reshape(n, 4).copy()).cuda(), torch.from_numpy(verts.view(np.float32).reshape(-1, 8).copy()).cuda()
+        nodes, tris = torch.zeros(n, 32, dtype=torch.int32, device="cuda"), torch.zeros(n, 12, device="cuda")
+        order, info, err = torch.zeros(n, dtype=torch.int32, device="cuda"), _lib.MeshInfo(), C.create_string_buffer(256)
+        st = lib.vt_mesh_build_noalloc(f.data_ptr(), n, v.data_ptr(), len(verts), C.byref(opts), nodes.data_ptr(), n, tris.data_ptr(),
+                                       order.data_ptr(), C.byref(info), torch.cuda.current_stream().cuda_stream, err, len(err))
+        assert (st == 0) == ok and (ok or b"look-back" in err.value), (n, st, err.value)
+    assert lib.vt_ctx_destroy(ctx) == 0
