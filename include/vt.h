@@ -323,7 +323,8 @@ vt_status vt_render(vt_ctx *ctx, vt_scene *scene, const vt_frame_params *params,
  * equals vt_render's to float rounding (1e-6 relative per pixel). The
  * reference has no wavefront path; its design note proposes the split (docs/KERNEL_SPLIT_DESIGN.md:
  * 72-74). A frame has at most 4M pixels; a pass holds as many whole samples as fit 16M paths (4M where
- * memory is short); the state takes ~260 bytes per path, allocated with the scene on first use. */
+ * memory is short); the state takes 229 bytes per path, 249 with OPENPBR slots or imported meshes, 281 for spectral
+ * OPENPBR under a light tree, 8 more with a radiance cache, allocated on first use and kept with the scene. */
 vt_status vt_render_wavefront(vt_ctx *ctx, vt_scene *scene, const vt_frame_params *params, uint32_t spp, void *stream);
 vt_status vt_accum_reset(vt_ctx *ctx, vt_scene *scene);
 /* Mean radiance per pixel (linear sRGB, row-major, 3 doubles per pixel; n = width * height * 3

@@ -3470,8 +3470,25 @@ struct WfBuffers {
   int4 *hit;
 };
 
-// Bytes of wavefront state for `cap` paths (each array 256-byte aligned), and its arrays at `base`.
-size_t wf_carve(unsigned char *base, uint32_t cap, WfArgs &W, WfBuffers &B) {
+// Which stages a render takes, and so which arrays its paths need.
+struct WfLayout {
+  bool group, split, nrc;
+};
+WfLayout wf_layout(const RenderArgs &A, bool nrc) {
+  // Regrouping pays where hits differ in kind: scenes with OpenPBR slots, and open scenes (imported ones
+  // may be), where rays escape. The procedural boxes' Lambert walls shade alike, and a pass over the queue
+  // would only add its time (k_wf_group; ReSTIR frames of a Lambert scene gain least, 17.0 -> 16.7 ms).
+  //
+  // Light samples in their own launch (k_wf_light) where the walk and the BSDF are both long: with a light
+  // tree, OpenPBR slots and spectral transport. In RGB it gains nothing (4.55 against 4.58 ms for 960 x 540),
+  // and on Lambert slots the second pass over the path state costs more than it saves (4.30 against 4.48 ms
+  // for 1000 x 600). (A cache-terminated path must not draw at the vertex that ends it.)
+  return {A.layered || A.imported, A.layered && A.spectral && A.imported && A.treeNodes && !nrc && A.mode != 3u, nrc};
+}
+
+// Bytes of wavefront state for `cap` paths (each array 256-byte aligned), and its arrays at `base`: 229 a path, 8 more
+// for a cache's render, 20 for regrouping, 32 for light samples of their own.
+size_t wf_carve(unsigned char *base, uint32_t cap, const WfLayout &need, WfArgs &W, WfBuffers &B) {
   size_t off = 0;
   auto take = [&](size_t bytes) {
     unsigned char *p = base ? base + off : nullptr;
@@ -3487,17 +3504,17 @@ size_t wf_carve(unsigned char *base, uint32_t cap, WfArgs &W, WfBuffers &B) {
   W.seedA = reinterpret_cast<uint4 *>(take(16 * n));
   W.seedB = reinterpret_cast<uint2 *>(take(8 * n));
   W.meta = reinterpret_cast<uint4 *>(take(16 * n));
-  W.spread = reinterpret_cast<float2 *>(take(8 * n));
+  W.spread = need.nrc ? reinterpret_cast<float2 *>(take(8 * n)) : nullptr;
   W.ray = reinterpret_cast<float4 *>(take(32 * n));
   B.hit = reinterpret_cast<int4 *>(take(16 * n));
   W.sray = reinterpret_cast<float4 *>(take(32 * n));
   W.scon = reinterpret_cast<float4 *>(take(16 * n));
-  W.light = reinterpret_cast<float4 *>(take(32 * n));
+  W.light = need.split ? reinterpret_cast<float4 *>(take(32 * n)) : nullptr;
   B.occ = reinterpret_cast<uint8_t *>(take(n));
   B.q[0] = reinterpret_cast<uint32_t *>(take(4 * n));
   B.q[1] = reinterpret_cast<uint32_t *>(take(4 * n));
   W.shQ = reinterpret_cast<uint32_t *>(take(4 * n));
-  W.grpQ = reinterpret_cast<uint32_t *>(take(4 * kWfClasses * n));
+  W.grpQ = need.group ? reinterpret_cast<uint32_t *>(take(4 * kWfClasses * n)) : nullptr;
   W.grpStride = cap;
   B.counts = reinterpret_cast<uint32_t *>(take(kWfSlots * kWfWords * sizeof(uint32_t)));
   W.hit = B.hit;
@@ -3537,8 +3554,8 @@ struct WfStages {
   uint32_t grid(uint32_t paths) const { return std::min<uint32_t>((paths + (uint32_t)block - 1) / (uint32_t)block, gridMax); }
 };
 
-WfStages wf_stages(vt_ctx *ctx, const vt_scene *scene, const RenderArgs &A, const WfBuffers &B, int block, uint32_t every, bool nrc,
-                   cudaStream_t s) {
+WfStages wf_stages(vt_ctx *ctx, const vt_scene *scene, const RenderArgs &A, const WfBuffers &B, int block, uint32_t every,
+                   const WfLayout &layout, cudaStream_t s) {
   WfStages S;
   S.ctx = ctx;
   S.mesh = scene->mesh;
@@ -3548,16 +3565,9 @@ WfStages wf_stages(vt_ctx *ctx, const vt_scene *scene, const RenderArgs &A, cons
   S.every = every;
   S.pbr = A.layered != 0u;
   S.unbounded = scene_has_delta(scene);
-  // Regrouping pays where hits differ in kind: scenes with OpenPBR slots, and open scenes (imported ones
-  // may be), where rays escape. The procedural boxes' Lambert walls shade alike, and a pass over the queue
-  // would only add its time (k_wf_group; ReSTIR frames of a Lambert scene gain least, 17.0 -> 16.7 ms).
-    S.group = S.pbr || A.imported;
-  S.nrc = nrc;
-  // Light samples in their own launch (k_wf_light) where the walk and the BSDF are both long: with a light
-  // tree, OpenPBR slots and spectral transport. In RGB it gains nothing (4.55 against 4.58 ms for 960 x 540),
-  // and on Lambert slots the second pass over the path state costs more than it saves (4.30 against 4.48 ms
-  // for 1000 x 600). (A cache-terminated path must not draw at the vertex that ends it.)
-  S.split = S.pbr && A.spectral && A.imported && A.treeNodes && !nrc && A.mode != 3u;
+  S.group = layout.group;
+  S.split = layout.split;
+  S.nrc = layout.nrc;
   S.s = s;
   return S;
 }
@@ -3799,14 +3809,15 @@ vt_status render_impl(vt_ctx *ctx, vt_scene *scene, const vt_frame_params *p, ui
     WfArgs W{};
     WfBuffers B;
     uint8_t *gocc = nullptr;
-    while (scene->wf_cap < band || scene->wf_gi_cap < band) {
+    const WfLayout layout = wf_layout(A, nrc != nullptr);
+    for (;;) {
       cudaError_t e = cudaSuccess;
-      if (scene->wf_cap < band) {
+      if (const size_t bytes = wf_carve(nullptr, band, layout, W, B); scene->wf_bytes < bytes) {
         cudaFree(scene->d_wf);
         scene->d_wf = nullptr;
-        scene->wf_cap = 0;
-        e = cudaMalloc(&scene->d_wf, wf_carve(nullptr, band, W, B));
-        if (e == cudaSuccess) scene->wf_cap = band;
+        scene->wf_bytes = 0;
+        e = cudaMalloc(&scene->d_wf, bytes);
+        if (e == cudaSuccess) scene->wf_bytes = bytes;
       }
       if (e == cudaSuccess && scene->wf_gi_cap < band) {
         cudaFree(scene->d_wf_gi);
@@ -3820,12 +3831,12 @@ vt_status render_impl(vt_ctx *ctx, vt_scene *scene, const vt_frame_params *p, ui
       if (e != cudaErrorMemoryAllocation || band <= (1u << 16)) return vt_cuda_fail(ctx, e, "allocating the frame's path state");
       band = (band + 1u) / 2u;
     }
-    wf_carve(scene->d_wf, scene->wf_cap, W, B);
+    wf_carve(scene->d_wf, band, layout, W, B);
     wf_carve_gi(scene->d_wf_gi, scene->wf_gi_cap, W, &gocc);
     W.npix = npix;
     W.deadFlags = 0u;
     A.kernelId = nrc ? 5u : 4u;
-    const WfStages S = wf_stages(ctx, scene, A, B, kWfBlock, 1u, nrc != nullptr, s);
+    const WfStages S = wf_stages(ctx, scene, A, B, kWfBlock, 1u, layout, s);
     for (uint32_t k = 0; k < spp; ++k) {
       float4 *cur = base + 9 * (size_t)npix * scene->di_parity, *prev = base + 9 * (size_t)npix * (scene->di_parity ^ 1u);
       A.gPos = cur; A.gNrm = cur + npix; A.rPos = cur + 2 * (size_t)npix; A.rEmit = cur + 3 * (size_t)npix;
@@ -3903,7 +3914,7 @@ vt_status render_impl(vt_ctx *ctx, vt_scene *scene, const vt_frame_params *p, ui
 // frame jitter uploaded from the host. Batches give each stream its own state and tune the rest.
 struct WfRun {
   unsigned char **state = nullptr;  // state buffer (null: the scene's own)
-  uint32_t *stateCap = nullptr;     // its capacity in paths
+  size_t *stateBytes = nullptr;     // its size
   uint32_t maxPaths = kWfMaxPaths;  // queue size: paths per pass
   int block = kWfBlock;             // stage kernels' block size (at most kWfBlock)
   uint32_t compactEvery = 1;        // compact the live queue on every n-th bounce
@@ -3963,33 +3974,33 @@ vt_status wavefront_impl(vt_ctx *ctx, vt_scene *scene, const vt_frame_params *p,
     A.nrcSpread = nrc->cfg.spread;
   }
   unsigned char **state = run.state ? run.state : &scene->d_wf;
-  uint32_t *stateCap = run.state ? run.stateCap : &scene->wf_cap;
+  size_t *stateBytes = run.state ? run.stateBytes : &scene->wf_bytes;
+  const WfLayout layout = wf_layout(A, nrc != nullptr);
+  WfArgs W{};
+  WfBuffers B;
   uint32_t chunk = 1u;
   for (;;) {
     const uint32_t passPaths = run.state || scene->wf_short ? maxPaths : kWfPassPaths;
     chunk = std::max(1u, std::min(spp, passPaths / npix));
-    if (npix * chunk <= *stateCap) break;
+    const size_t bytes = wf_carve(nullptr, npix * chunk, layout, W, B);
+    if (bytes <= *stateBytes) break;
     cudaFree(*state);
     *state = nullptr;
-    *stateCap = 0;
-    WfArgs probe;
-    WfBuffers unused;
-    const cudaError_t e = cudaMalloc(state, wf_carve(nullptr, npix * chunk, probe, unused));
+    *stateBytes = 0;
+    const cudaError_t e = cudaMalloc(state, bytes);
     if (e == cudaSuccess) {
-      *stateCap = npix * chunk;
+      *stateBytes = bytes;
       break;
     }
     if (e != cudaErrorMemoryAllocation || passPaths == maxPaths) return vt_cuda_fail(ctx, e, "allocating the path state");
     cudaGetLastError();
     scene->wf_short = true;  // this scene's passes stay at maxPaths
   }
-  WfArgs W{};
-  WfBuffers B;
-  wf_carve(*state, *stateCap, W, B);
+  wf_carve(*state, npix * chunk, layout, W, B);
   W.npix = npix;
   const uint32_t every = std::max(1u, run.compactEvery);
   W.deadFlags = every > 1u ? 1u : 0u;
-  const WfStages S = wf_stages(ctx, scene, A, B, std::max(32, std::min(run.block, kWfBlock)), every, nrc != nullptr, s);
+  const WfStages S = wf_stages(ctx, scene, A, B, std::max(32, std::min(run.block, kWfBlock)), every, layout, s);
   for (uint32_t k0 = 0; k0 < spp; k0 += chunk) {
     W.paths = npix * std::min(chunk, spp - k0);
     W.k0 = k0;
@@ -4148,7 +4159,7 @@ struct vt_batch {
   cudaStream_t streams[kStreams] = {};
   cudaEvent_t fork = nullptr, join[kStreams] = {};
   unsigned char *state[kStreams] = {};
-  uint32_t stateCap[kStreams] = {};
+  size_t stateBytes[kStreams] = {};
   std::vector<cudaEvent_t> sceneEv;
   std::vector<int> streamOf;     // stream of each scene (longest-processing-time assignment)
   std::vector<uint32_t> orderBy; // scenes by decreasing work
@@ -4409,7 +4420,7 @@ vt_status vt_batch_render_wavefront(vt_ctx *ctx, vt_batch *b, void *stream) {
     const int k = b->streamOf[i];
     WfRun run;
     run.state = &b->state[k];
-    run.stateCap = &b->stateCap[k];
+    run.stateBytes = &b->stateBytes[k];
     run.maxPaths = c.queue;
     run.block = c.block;
     run.compactEvery = c.every;

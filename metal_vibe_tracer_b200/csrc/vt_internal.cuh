@@ -141,9 +141,9 @@ struct vt_scene {
   float4 *d_di = nullptr;
   uint32_t di_width = 0, di_height = 0, di_frames = 0, di_parity = 0;
   // Wavefront integrator (vt_render_wavefront): the paths' state, rays and queues, one allocation
-  // sized for wf_cap paths.
+  // of wf_bytes, carved anew for each render.
   unsigned char *d_wf = nullptr;
-  uint32_t wf_cap = 0;
+  size_t wf_bytes = 0;
   bool wf_short = false;  // memory was too short for the state of the largest passes
   unsigned char *d_wf_gi = nullptr;  // sampling mode 0's connection arrays, for wf_gi_cap paths
   uint32_t wf_gi_cap = 0;

@@ -12,6 +12,7 @@ pixels, and their means to well within the estimator's noise:
 """
 import numpy as np
 import pytest
+import torch
 
 import metal_vibe_tracer_b200 as vt
 from metal_vibe_tracer_b200 import scenes, spectral_tables
@@ -157,6 +158,25 @@ def test_largest_passes(ctx, cornell):
     mats, light, cam, mesh = cornell
     mega, wave = both(ctx, mesh, mats, light, vt.make_params(cam, 2000, 2000, 2, 1, False, 1), 5, False)
     assert_same(mega, wave)
+
+
+def test_state_holds_only_what_the_render_uses(ctx, cornell):
+    """The path state of a first wavefront render: 229 bytes a path, and 20 more for the queues by kind of vertex
+    where slots are OPENPBR (no light samples of their own in RGB, no spread without a cache)."""
+    spp, paths = 4, 4 * 1024 * 1024
+    faces, verts, mats, light, cam = scenes.cornell_openpbr()
+    mesh = vt.Mesh(ctx, faces, verts)
+    for m, materials, per_path in ((cornell[3], cornell[0], 229), (mesh, mats, 249)):
+        scene = vt.Scene(ctx, m, materials, cornell[1], None)
+        params = vt.make_params(cam, 1024, 1024, 2, 1, False, 1)
+        scene.render(params, spp)  # the accumulation and the jitter
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        scene.render_wavefront(params, spp)
+        taken = before - torch.cuda.mem_get_info()[0]
+        assert per_path * paths - (8 << 20) <= taken <= per_path * paths + (8 << 20), taken / paths
+        scene.close()
+    mesh.close()
 
 
 def test_rejects_restir(ctx, cornell):
