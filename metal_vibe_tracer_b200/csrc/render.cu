@@ -2133,7 +2133,7 @@ __global__ void __launch_bounds__(kWfBlock) k_wf_finish(RenderArgs A, WfArgs W) 
 // BSDF sample). Other primaries get empty reservoirs and shade with NEE (main.swift:4931-4943).
 // Leaves the camera ray's direction and wavelength number in W.T, the BSDF pdf in W.prev.w, the
 // sampler in W.seedA/B.
-__device__ __forceinline__ bool di_primary(const RenderArgs &A, const WfArgs &W, uint32_t i) {
+__device__ __forceinline__ void di_primary(const RenderArgs &A, const WfArgs &W, uint32_t i, bool &push) {
   const uint32_t p = W.p0 + i, k = W.k0, x = p % A.W, y = p / A.W;
   Sampler seed = pixel_sampler(x, y, A.W, A.first + k, A.zSampler != 0u, A.zModel, A.firstFrame + k);
   const float u = A.spectral ? wavelength_numbers(seed).x : 0.0f;
@@ -2148,7 +2148,7 @@ __device__ __forceinline__ bool di_primary(const RenderArgs &A, const WfArgs &W,
     A.gNrm[p] = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
     A.rPos[p] = zero; A.rEmit[p] = zero; A.rW[p] = zero;
     A.giPos[p] = zero; A.giNrm[p] = zero; A.giRad[p] = zero; A.giW[p] = zero;
-    return false;
+    return;
   }
   const Surface S = surface_at(A, h, o0, dir0);
   const vt_material m = material(A, S.slot);
@@ -2162,7 +2162,7 @@ __device__ __forceinline__ bool di_primary(const RenderArgs &A, const WfArgs &W,
   A.giPos[p] = zero; A.giNrm[p] = zero; A.giRad[p] = zero; A.giW[p] = zero;
   if (m.type != VT_MAT_DIFFUSE) {
     A.rPos[p] = zero; A.rEmit[p] = zero; A.rW[p] = zero;
-    return false;
+    return;
   }
   DIReservoir r;
   r.s.pos = f3(0.0f, 0.0f, 0.0f); r.s.emission = f3(0.0f, 0.0f, 0.0f);
@@ -2201,12 +2201,12 @@ __device__ __forceinline__ bool di_primary(const RenderArgs &A, const WfArgs &W,
   A.rPos[p] = make_float4(r.s.pos.x, r.s.pos.y, r.s.pos.z, __uint_as_float(r.s.id));
   A.rEmit[p] = make_float4(r.s.emission.x, r.s.emission.y, r.s.emission.z, r.s.pdf);
   A.rW[p] = make_float4(r.wsum, r.M, Wr, r.s.u);
-  if ((int)A.maxDepth - 1 < 1) return false;
+  if ((int)A.maxDepth - 1 < 1) return;
   sampler_event(seed, 1u, kZGiBsdf);
   const float3 rr = rand_f3(seed);  // sample_bsdf's Lambert branch: the direction from the last two
   const float3 gd = cosine_hemisphere(S.n, rr.y, rr.z);
   const float bpdf = fmaxf(0.0f, dot3(S.n, gd)) * kInvPi;
-  const bool push = bpdf > 0.0f && dot3(gd, S.gn) > 0.0f;
+  push = bpdf > 0.0f && dot3(gd, S.gn) > 0.0f;
   if (push) {
     const float3 o = ray_origin(A, S.pos, S.gn, gd, S.err);
     wf_set_ray(W.ray, i, o, ray_tmin(A, o), gd, __int_as_float(0x7f800000));
@@ -2215,7 +2215,6 @@ __device__ __forceinline__ bool di_primary(const RenderArgs &A, const WfArgs &W,
   W.prev[i] = make_float4(0.0f, 0.0f, 0.0f, bpdf);
   W.meta[i] = make_uint4(p, 0u, 0u, 0u);
   wf_store_seed(W, i, seed);
-  return push;
 }
 
 // Bound: the dependent loads and the issue of one light-tree walk after another. Held to 80 registers
@@ -2227,12 +2226,15 @@ __device__ __forceinline__ bool di_primary(const RenderArgs &A, const WfArgs &W,
 // pixels to a warp so that all of them fit at once: nothing waits for a block's slot, and a warp
 // diverges over fewer walks. Measured on one B200, a frame of 300,000 triangles, a third of its slots OPENPBR, at
 // depth 3: 191 x 150 1165 -> 1109 us, 264 x 171 1216 -> 1181.
-template <bool kPbr, bool kFew>
+template <bool kFew>
 __global__ void __launch_bounds__(kRenderBlock, kFew ? 4 : 6) k_di_primary(RenderArgs A, WfArgs W, uint32_t lanes) {
   const unsigned lane = threadIdx.x & 31u;
   const uint32_t i = kFew ? (blockIdx.x * (kRenderBlock / 32) + (threadIdx.x >> 5)) * lanes + lane : blockIdx.x * kRenderBlock + threadIdx.x;
   bool push = false;
-  if (i < W.paths && (!kFew || lane < lanes)) push = di_primary(A, W, i);
+  [&] {  // every lane joins the push below (the early return: `if (...) di_primary(...)` spills 44 bytes more, 0.8 % of a frame)
+    if (i >= W.paths || (kFew && lane >= lanes)) return;
+    di_primary(A, W, i, push);
+  }();
   // Pushed per warp: a block's warps end far apart, and waiting for the last cost 2 % of a frame.
   const unsigned pushes = __ballot_sync(0xffffffffu, push);
   uint32_t base = 0;
@@ -2590,7 +2592,9 @@ __global__ void __launch_bounds__(kRenderBlock, 4) k_di_small_reservoirs(RenderA
   if (i >= W.paths) return;
   wf_generate(A, W, i);
   wf_trace(A, W, H, i, stack);
-  if (di_primary(A, W, i)) {
+  bool candidate = false;
+  di_primary(A, W, i, candidate);
+  if (candidate) {
     wf_trace(A, W, H, i, stack);
     if (gi_secondary(A, W, i)) H.occ[i] = wf_occluded(A, W.sray, i, stack) ? 1 : 0;
   }
@@ -3693,11 +3697,9 @@ vt_status di_reservoirs(const WfStages &S, const RenderArgs &A, WfArgs W) {
   const uint32_t warps = (uint32_t)ctx->sm_count * 16u, lanes = (P + warps - 1u) / warps;
   if (lanes <= 32u) {
     const uint32_t blocks = (P + lanes * (kRenderBlock / 32) - 1u) / (lanes * (kRenderBlock / 32));
-    if (S.pbr) k_di_primary<true, true><<<blocks, kRenderBlock, 0, s>>>(A, W, lanes);
-    else k_di_primary<false, true><<<blocks, kRenderBlock, 0, s>>>(A, W, lanes);
+    k_di_primary<true><<<blocks, kRenderBlock, 0, s>>>(A, W, lanes);
   } else {
-    if (S.pbr) k_di_primary<true, false><<<pixels, kRenderBlock, 0, s>>>(A, W, 32u);
-    else k_di_primary<false, false><<<pixels, kRenderBlock, 0, s>>>(A, W, 32u);
+    k_di_primary<false><<<pixels, kRenderBlock, 0, s>>>(A, W, 32u);
   }
   if (A.maxDepth > 1u) {
     vt_launch_closest(S.mesh, ray, P, hit, ctx->sm_count, S.word(1, kWfExtendHead), S.B.q[1], ctx->d_status + 1, s, W.outCount, true, true);

@@ -366,7 +366,8 @@ void vt_launch_any(const vt_mesh *mesh, const vt_ray *rays, uint32_t n, uint8_t 
   if (n == 0) return;
   if (!cleared) cudaMemsetAsync(counter, 0, sizeof(uint32_t), s);
   const bool small = n <= kFewLanes * kFewWarps * (uint32_t)sm_count, few = count || small;
-  launch_persistent(slack ? (few ? k_any<true, true> : k_any<true, false>) : few ? k_any<false, true> : k_any<false, false>, mesh, n, small, sm_count, s, status,
+  // (Shadow rays with slack come from queues only, so they need no form for a launch of many rays.)
+  launch_persistent(slack ? k_any<true, true> : few ? k_any<false, true> : k_any<false, false>, mesh, n, small, sm_count, s, status,
                     ray_set<uint8_t>(rays, n, occ, counter, perm, count, sm_count));
 }
 
