@@ -3075,7 +3075,6 @@ void scene_free(vt_scene *scene) {
   cudaFree(scene->d_face_pos);
   cudaFree(scene->d_di);
   cudaFree(scene->d_wf);
-  cudaFree(scene->d_wf_gi);
   cudaFree(scene->d_env_img);
   cudaFree(scene->d_env_rows);
   cudaFree(scene->d_env_cols);
@@ -3470,13 +3469,13 @@ enum : uint32_t { kWfLive = 0, kWfShadows = 1, kWfExtendHead = 2, kWfShadowHead 
 // hits and occlusion.
 struct WfBuffers {
   uint32_t *q[2], *counts;
-  uint8_t *occ;
+  uint8_t *occ, *gocc;
   int4 *hit;
 };
 
 // Which stages a render takes, and so which arrays its paths need.
 struct WfLayout {
-  bool group, split, nrc;
+  bool group, split, nrc, gi;
 };
 WfLayout wf_layout(const RenderArgs &A, bool nrc) {
   // Regrouping pays where hits differ in kind: scenes with OpenPBR slots, and open scenes (imported ones
@@ -3487,11 +3486,11 @@ WfLayout wf_layout(const RenderArgs &A, bool nrc) {
   // tree, OpenPBR slots and spectral transport. In RGB it gains nothing (4.55 against 4.58 ms for 960 x 540),
   // and on Lambert slots the second pass over the path state costs more than it saves (4.30 against 4.48 ms
   // for 1000 x 600). (A cache-terminated path must not draw at the vertex that ends it.)
-  return {A.layered || A.imported, A.layered && A.spectral && A.imported && A.treeNodes && !nrc && A.mode != 3u, nrc};
+  return {A.layered || A.imported, A.layered && A.spectral && A.imported && A.treeNodes && !nrc && A.mode != 3u, nrc, A.mode == 0u};
 }
 
 // Bytes of wavefront state for `cap` paths (each array 256-byte aligned), and its arrays at `base`: 229 a path, 8 more
-// for a cache's render, 20 for regrouping, 32 for light samples of their own.
+// for a cache's render, 20 for regrouping, 32 for light samples of their own, 53 for sampling mode 0's connections.
 size_t wf_carve(unsigned char *base, uint32_t cap, const WfLayout &need, WfArgs &W, WfBuffers &B) {
   size_t off = 0;
   auto take = [&](size_t bytes) {
@@ -3520,27 +3519,15 @@ size_t wf_carve(unsigned char *base, uint32_t cap, const WfLayout &need, WfArgs 
   W.shQ = reinterpret_cast<uint32_t *>(take(4 * n));
   W.grpQ = need.group ? reinterpret_cast<uint32_t *>(take(4 * kWfClasses * n)) : nullptr;
   W.grpStride = cap;
+  W.gray = need.gi ? reinterpret_cast<float4 *>(take(32 * n)) : nullptr;
+  W.gcon = need.gi ? reinterpret_cast<float4 *>(take(16 * n)) : nullptr;
+  B.gocc = need.gi ? reinterpret_cast<uint8_t *>(take(n)) : nullptr;
+  W.giQ = need.gi ? reinterpret_cast<uint32_t *>(take(4 * n)) : nullptr;
   B.counts = reinterpret_cast<uint32_t *>(take(kWfSlots * kWfWords * sizeof(uint32_t)));
   W.hit = B.hit;
   W.occ = B.occ;
+  W.gocc = B.gocc;
   W.p0 = 0u;
-  return off;
-}
-
-// The connection arrays of sampling mode 0.
-size_t wf_carve_gi(unsigned char *base, uint32_t cap, WfArgs &W, uint8_t **occ) {
-  size_t off = 0;
-  auto take = [&](size_t bytes) {
-    unsigned char *p = base ? base + off : nullptr;
-    off += (bytes + 255) & ~size_t(255);
-    return p;
-  };
-  const size_t n = cap;
-  W.gray = reinterpret_cast<float4 *>(take(32 * n));
-  W.gcon = reinterpret_cast<float4 *>(take(16 * n));
-  *occ = reinterpret_cast<uint8_t *>(take(n));
-  W.gocc = *occ;
-  W.giQ = reinterpret_cast<uint32_t *>(take(4 * n));
   return off;
 }
 
@@ -3658,8 +3645,8 @@ vt_status wf_bounces(const WfStages &S, const RenderArgs &A, WfArgs W, uint32_t 
 // stages: Cornell box 264 x 171 354 / 418 at depth 3 and 529 / 755 at 12, 320 x 236 476 / 451 and 759 / 828; 300,000
 // triangles 320 x 236 1335 / 1353 and 1911 / 2314; OPENPBR grid 180 x 100 541 / 585 and 1036 / 1424, 190 x 149 708 / 644 and
 // 1388 / 1610, 264 x 171 839 / 690 and 1565 / 1683.
-bool small_frame(const WfStages &S, const RenderArgs &A, uint32_t npix) {
-  const uint32_t full = (uint32_t)S.ctx->sm_count * kDiSmallWarps * 32u, most = S.pbr ? full / 4u * 3u : 2u * full;
+bool small_frame(const vt_ctx *ctx, const RenderArgs &A, uint32_t npix) {
+  const uint32_t full = (uint32_t)ctx->sm_count * kDiSmallWarps * 32u, most = A.layered ? full / 4u * 3u : 2u * full;
   return npix <= (A.maxDepth > 8u ? most : most / 3u * 2u);
 }
 
@@ -3715,7 +3702,7 @@ vt_status di_reservoirs(const WfStages &S, const RenderArgs &A, WfArgs W) {
 }
 
 // One band of a mode-0 frame from its reservoirs to the accumulation.
-vt_status di_paths(const WfStages &S, const RenderArgs &A, WfArgs W, uint8_t *gocc) {
+vt_status di_paths(const WfStages &S, const RenderArgs &A, WfArgs W) {
   vt_ctx *ctx = S.ctx;
   cudaStream_t s = S.s;
   const uint32_t P = W.paths, pixels = (P + kRenderBlock - 1) / kRenderBlock;
@@ -3732,7 +3719,7 @@ vt_status di_paths(const WfStages &S, const RenderArgs &A, WfArgs W, uint8_t *go
     else k_di_shade<false, false><<<pixels, kRenderBlock, 0, s>>>(A, W);
   }
   if (!S.nrc && A.maxDepth > 1u) {
-    vt_launch_any(S.mesh, reinterpret_cast<const vt_ray *>(W.gray), P, gocc, ctx->sm_count, S.word(0, kWfConnectHead), W.giQ,
+    vt_launch_any(S.mesh, reinterpret_cast<const vt_ray *>(W.gray), P, S.B.gocc, ctx->sm_count, S.word(0, kWfConnectHead), W.giQ,
                   ctx->d_status + 1, s, W.giCount, A.imported != 0u, true);
     k_gi_connect<<<S.grid(P), S.block, 0, s>>>(W);
   }
@@ -3786,10 +3773,18 @@ vt_status render_impl(vt_ctx *ctx, vt_scene *scene, const vt_frame_params *p, ui
   }
   if (p->sampling_mode == 0u) {
     // ReSTIR: frames in order, each through the wavefront stages (k_di_primary's comment lists them).
+    // A small frame's path state lies behind the scene's reservoirs (one allocation less on its first frame: 1.28 -> 1.05 ms
+    // for 180 x 100, as before frames kept path state).
+    WfArgs W{};
+    WfBuffers B;
+    const WfLayout layout = wf_layout(A, nrc != nullptr);
+    const bool small = small_frame(ctx, A, npix);
+    const size_t reservoirs = (20 * (size_t)npix * sizeof(float4) + 255) & ~size_t(255), behind = small ? wf_carve(nullptr, npix, layout, W, B) : 0;
     if (!scene->d_di || scene->di_width != p->width || scene->di_height != p->height) {
       cudaFree(scene->d_di);
       scene->d_di = nullptr;
-      VT_CUDA(ctx, cudaMalloc(&scene->d_di, 20 * (size_t)npix * sizeof(float4)));
+      VT_CUDA(ctx, cudaMalloc(&scene->d_di, reservoirs + behind));
+      scene->di_behind = behind;
       scene->di_width = p->width;
       scene->di_height = p->height;
       scene->di_frames = 0;
@@ -3808,33 +3803,22 @@ vt_status render_impl(vt_ctx *ctx, vt_scene *scene, const vt_frame_params *p, ui
                            A.up.x, A.up.y, A.up.z, A.aspect, A.fovScale};
     // The stages' state for a band of pixels: the whole frame up to 4M pixels, less where memory is short.
     uint32_t band = std::min(npix, kWfMaxPaths);
-    WfArgs W{};
-    WfBuffers B;
-    uint8_t *gocc = nullptr;
-    const WfLayout layout = wf_layout(A, nrc != nullptr);
-    for (;;) {
-      cudaError_t e = cudaSuccess;
-      if (const size_t bytes = wf_carve(nullptr, band, layout, W, B); scene->wf_bytes < bytes) {
-        cudaFree(scene->d_wf);
-        scene->d_wf = nullptr;
-        scene->wf_bytes = 0;
-        e = cudaMalloc(&scene->d_wf, bytes);
-        if (e == cudaSuccess) scene->wf_bytes = bytes;
+    const bool fits = small && behind <= scene->di_behind;
+    for (; !fits; band = (band + 1u) / 2u) {
+      const size_t bytes = wf_carve(nullptr, band, layout, W, B);
+      if (bytes <= scene->wf_bytes) break;
+      cudaFree(scene->d_wf);
+      scene->d_wf = nullptr;
+      scene->wf_bytes = 0;
+      const cudaError_t e = cudaMalloc(&scene->d_wf, bytes);
+      if (e == cudaSuccess) {
+        scene->wf_bytes = bytes;
+        break;
       }
-      if (e == cudaSuccess && scene->wf_gi_cap < band) {
-        cudaFree(scene->d_wf_gi);
-        scene->d_wf_gi = nullptr;
-        scene->wf_gi_cap = 0;
-        e = cudaMalloc(&scene->d_wf_gi, wf_carve_gi(nullptr, band, W, &gocc));
-        if (e == cudaSuccess) scene->wf_gi_cap = band;
-      }
-      if (e == cudaSuccess) break;
       cudaGetLastError();
       if (e != cudaErrorMemoryAllocation || band <= (1u << 16)) return vt_cuda_fail(ctx, e, "allocating the frame's path state");
-      band = (band + 1u) / 2u;
     }
-    wf_carve(scene->d_wf, band, layout, W, B);
-    wf_carve_gi(scene->d_wf_gi, scene->wf_gi_cap, W, &gocc);
+    wf_carve(fits ? reinterpret_cast<unsigned char *>(scene->d_di) + reservoirs : scene->d_wf, band, layout, W, B);
     W.npix = npix;
     W.deadFlags = 0u;
     A.kernelId = nrc ? 5u : 4u;
@@ -3858,23 +3842,23 @@ vt_status render_impl(vt_ctx *ctx, vt_scene *scene, const vt_frame_params *p, ui
       A.paspect = pc[12];
       A.pfovScale = pc[13];
       W.k0 = k;
-      const bool whole = band >= npix, small = whole && small_frame(S, A, npix);
-      if (small) {
+      const bool whole = band >= npix, threads = whole && small;
+      if (threads) {
         W.p0 = 0u;
         W.paths = npix;
         if (const vt_status st = di_small(S, A, W)) return st;
       }
-      for (uint32_t p0 = 0; p0 < npix && !small; p0 += band) {
+      for (uint32_t p0 = 0; p0 < npix && !threads; p0 += band) {
         W.p0 = p0;
         W.paths = std::min(band, npix - p0);
         vt_status st = di_reservoirs(S, A, W);
-        if (st == VT_OK && whole) st = di_paths(S, A, W, gocc);
+        if (st == VT_OK && whole) st = di_paths(S, A, W);
         if (st != VT_OK) return st;
       }
       for (uint32_t p0 = 0; p0 < npix && !whole; p0 += band) {
         W.p0 = p0;
         W.paths = std::min(band, npix - p0);
-        const vt_status st = di_paths(S, A, W, gocc);
+        const vt_status st = di_paths(S, A, W);
         if (st != VT_OK) return st;
       }
       scene->di_parity ^= 1u;

@@ -68,7 +68,7 @@ struct vt_mesh {
   float build_ms = 0.0f;
   float lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
   vt_wide_node *d_nodes = nullptr;   // nnodes, reference layout (128 B, 16-B vector loads)
-  float4 *d_tris = nullptr;          // 3 per BVH position: (a, face id bits), (b, face tag bits), (c, 0)
+  float4 *d_tris = nullptr;          // 3 per BVH position: (a, face id bits), (b, face tag bits), (c, 1 on a leaf's last, else 0)
   int32_t *d_order = nullptr;        // BVH position -> input face
   uint32_t *d_codes = nullptr;       // sorted Morton codes
   int32_t *d_sorted = nullptr;       // sorted position -> input face
@@ -140,13 +140,12 @@ struct vt_scene {
   float4 *d_ebasis = nullptr;
   float4 *d_di = nullptr;
   uint32_t di_width = 0, di_height = 0, di_frames = 0, di_parity = 0;
+  size_t di_behind = 0;  // bytes behind the reservoirs (a small frame's path state)
   // Wavefront integrator (vt_render_wavefront): the paths' state, rays and queues, one allocation
   // of wf_bytes, carved anew for each render.
   unsigned char *d_wf = nullptr;
   size_t wf_bytes = 0;
   bool wf_short = false;  // memory was too short for the state of the largest passes
-  unsigned char *d_wf_gi = nullptr;  // sampling mode 0's connection arrays, for wf_gi_cap paths
-  uint32_t wf_gi_cap = 0;
   float di_cam[14] = {};  // previous frame's camera: position, forward, right, up, aspect, fov scale
 };
 

@@ -7,7 +7,7 @@ The reference's own checks (tests/Fix_integrator.swift:188-240) restated:
   reservoirs merged history (M above the frame's own candidates), and the last frame's energy is
   within 15 % of an MIS render from the final view;
 * a cut (vt_accum_reset) clears the history.
-And against the FP64 oracle, which runs the same two passes per frame over the same sampler streams:
+And against the FP64 oracle, which runs the reference's two passes per frame over the same sampler streams:
 mean radiance within 0.5 % and per-pixel relMSE within the estimator's own.
 """
 import numpy as np
@@ -183,3 +183,20 @@ def test_small_and_staged_frames_of_layered_slots_agree(ctx, depth):
     mesh.close()
     assert abs(threads.mean() / stages.mean() - 1) < 0.02 and abs(threads.mean() / mis.mean() - 1) < 0.06, (
         threads.mean(), stages.mean(), mis.mean())
+
+
+def test_threads_and_stages_share_a_scene(ctx, cornell):
+    """A frame size that goes by stages at depth 3 and by threads at depth 10, on one scene in either order and after a
+    wavefront render: each image is a fresh scene's, bit for bit."""
+    faces, verts, mats, light, cam, mesh = cornell
+    w, h = 260, (small_frame_pixels(3, False) + small_frame_pixels(10, False)) // 2 // 260
+    fresh = {d: render(ctx, mesh, mats, light, cam, w, h, 2, 0, d) for d in (3, 10)}
+    for depths in ((3, 10, 3), (10, 3, 10)):
+        scene = vt.Scene(ctx, mesh, mats, light)
+        for i, d in enumerate(depths):
+            if i == 2:
+                scene.render_wavefront(vt.make_params(cam, w, h, 4, 1, False, 1), 1)
+            scene.reset()
+            scene.render(vt.make_params(cam, w, h, d, 1, False, 0), 2)
+            assert np.array_equal(scene.readback()[0], fresh[d]), (depths, i)
+        scene.close()
