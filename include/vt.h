@@ -319,8 +319,10 @@ vt_status vt_render(vt_ctx *ctx, vt_scene *scene, const vt_frame_params *params,
  * state lives in device memory between stage kernels over queues of live paths (camera rays;
  * per bounce the closest-hit traversal of the queue, shading with NEE and the BSDF continuation,
  * the shadow rays' any-hit traversal; then the accumulation), with the megakernel's sampler draws
- * and arithmetic per path; a path's primary and continuation radiance are summed apart, so the image
- * equals vt_render's to float rounding (1e-6 relative per pixel). The
+ * per path; a path's primary and continuation radiance are summed apart and its BSDFs compiled for the stages,
+ * so the image equals vt_render's to float rounding: 99.5 % of pixels within 1e-6 relative, with layered
+ * OPENPBR slots (film, coat, fuzz, anisotropy) 98 % within 1e-4 (a rounding at a decision's edge sends a path another
+ * way). With glass or mirror slots the call blocks the host past max_depth (live paths are counted). The
  * reference has no wavefront path; its design note proposes the split (docs/KERNEL_SPLIT_DESIGN.md:
  * 72-74). A frame has at most 4M pixels; a pass holds as many whole samples as fit 16M paths (4M where
  * memory is short); the state takes 229 bytes per path, 249 with OPENPBR slots or imported meshes, 281 for spectral
@@ -684,7 +686,7 @@ vt_status vt_nrc_train(vt_ctx *ctx, vt_nrc *nrc, const vt_nrc_input *in, const f
  * first; VT_NRC_RENDER: render spp samples per pixel whose paths end where the cache's query rule
  * (query_vertex, spread) stops them, with the cache's prediction (sampling modes 0 and 1), added to
  * the scene's accumulation; sampling mode 1 renders through the wavefront integrator
- * (vt_render_wavefront's stages), mode 0 through ReSTIR DI's two passes. The frame's transport must
+ * (vt_render_wavefront's stages), mode 0 as vt_render's ReSTIR frames. The frame's transport must
  * match the cache's `spectral` setting. */
 vt_status vt_render_nrc(vt_ctx *ctx, vt_scene *scene, vt_nrc *nrc, const vt_frame_params *p, uint32_t spp,
                         uint32_t flags, void *stream);

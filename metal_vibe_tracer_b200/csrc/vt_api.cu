@@ -498,10 +498,10 @@ extern "C" {
 
 // Host pipeline: chunk c goes on stream c % 2 as copy-in, trace, copy-out; the two streams let
 // chunk c + 1's copy-in and chunk c - 1's copy-out overlap chunk c's traversal. Pageable buffers go
-// through pinned staging, filled and drained by several host threads (host_pipeline). Measured on one
-// B200, rays in ordinary arrays against 200,000 triangles, closest hit: 1,000,003 rays 3.9 -> 2.1 ms, 4M
-// 12.9 -> 7.3, 200,000 0.92 -> 0.64 (chunks of 4M rays with two slots and threads started per copy left
-// nothing to overlap below 8M).
+// through pinned staging, filled and drained by several host threads (host_pipeline) from 12 MB on. Measured
+// on one B200's host, closest hits of rays in ordinary arrays on 200,000 triangles into a new result array:
+// 1,000,003 rays 4.0-4.7 -> 2.2-2.6 ms, 4M 15-17 -> 8-11, and whole below, 200,000 1.1 as before (chunks of 4M rays
+// with two slots and threads started per copy left nothing to overlap below 8M).
 static vt_status trace_host(vt_ctx *ctx, const vt_mesh *mesh, const vt_ray *rays, uint32_t n,
                             void *out, size_t out_stride, bool closest) {
   vt_status st = check_trace_args(ctx, mesh, rays, out, n);

@@ -6,9 +6,9 @@ for them (no scattering event spent, no NEE, emission weight 1 after an ideal bo
 * a Cornell box with a mirror tall box, a glass short box and a rough GLOSSY (OpenPBR metal) wall, in
   RGB, in spectral transport with a thin film on the mirror, and with the Z++ sampler;
 * the wavefront integrator's images equal the megakernel's;
-* ReSTIR DI (sampling mode 0) renders the scene as the oracle does;
-* the radiance cache renders it in sampling mode 1 and refuses it in mode 0, whose cache-terminated
-  kernels are built without glass and mirrors.
+* ReSTIR DI (sampling mode 0) renders the scene as the oracle does, by threads and by stages, and does
+  not block the host;
+* the radiance cache renders it in sampling mode 1 and refuses it in mode 0.
 
 The GPU draws the oracle's numbers, so nearly every pixel agrees to 1e-3. Refraction in float and in
 double can still part at a total-internal-reflection or Fresnel threshold, and a path that then reaches

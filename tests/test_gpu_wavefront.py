@@ -1,14 +1,16 @@
 """The wavefront integrator (vt_render_wavefront) against the megakernel (vt_render) on the B200.
 
-Both draw the same numbers from the same samplers and run the same device functions per vertex; the
-wavefront's traversals are the persistent quantised-node kernels of traverse.cu (the megakernel
-walks the 128-byte nodes), whose closest hit can differ only between triangles hit at exactly the
-same distance. So the images agree pixel for pixel to FP64 summation order except on a handful of
-pixels, and their means to well within the estimator's noise:
+Both draw the same numbers from the same samplers; the wavefront's traversals are the persistent
+quantised-node kernels of traverse.cu (the megakernel walks the 128-byte nodes), whose closest hit can
+differ only between triangles hit at exactly the same distance, and its stages prepare an OPENPBR vertex
+once for all its uses where the megakernel prepares it at each (other contractions of the same
+formulas). So the images agree pixel for pixel to float rounding, 1e-6, except on a handful of pixels (with
+layered OPENPBR slots 1e-4 on 98 %, since narrow lobes amplify a rounding), and their means to well within
+the estimator's noise:
 * Cornell box, spectral and RGB, sampling modes 1-3;
 * the OpenPBR Cornell box (spectral), an imported scene under its light tree and an open scene with
   the procedural sky (shadow rays with the endpoint slack, MIS-weighted escapes);
-* several passes (more samples than one pass's 4M paths hold) and a strided frame.
+* a pass of 8M paths, more samples than one pass's 16M paths hold, and a strided frame.
 """
 import numpy as np
 import pytest
@@ -146,7 +148,7 @@ def test_openpbr_under_a_light_tree_equals_megakernel(ctx, mode, sampler):
 
 def test_passes_and_stride(ctx, cornell):
     mats, light, cam, mesh = cornell
-    # 1024 x 1024 x 8 spp = 8M paths: two passes of 4M.
+    # 1024 x 1024 x 8 spp = 8M paths in one pass (test_largest_passes takes two).
     mega, wave = both(ctx, mesh, mats, light, vt.make_params(cam, 1024, 1024, 4, 1, False, 1), 8, False)
     assert_same(mega, wave)
     mega, wave = both(ctx, mesh, mats, light, vt.make_params(cam, 96, 64, 8, 1, True, 1, pixel_stride=3), 8, True)
